@@ -358,11 +358,9 @@ void enqueue_run(leo2d_batch* b) {
         RtBatchFlake& r = fl[f];
         r.data = m->rt_data.p;
         r.wbeg = m->rt_wbeg.p;
-        r.kst = m->rt_kst.p;
+        r.blk = m->rt_blk.p;
+        r.bbeg = m->rt_bbeg.p;
         r.n = m->n;
-        r.nrb = m->rt_blocks;
-        r.group = m->rt_group;
-        r.chunk = m->rt_chunk;
         r.x0 = b->x0.p + v.row_off * C;
         r.x1 = b->x1.p + v.row_off * C;
         r.partials[0] = b->partials.p + (size_t)b->block_first[f] * 2 * C;

@@ -100,6 +100,8 @@ struct leo2d_csr {
   unsigned rt_grid = 0;
   leo2d::DevBuf<int64_t> rt_kst;      // [blocks] k-steps of each block
   leo2d::DevBuf<int64_t> rt_wbeg;     // [grid * warps + 1] first k-step of each warp
+  leo2d::DevBuf<int2> rt_blk;         // [blocks + 1] (block, k-steps) in processing order
+  leo2d::DevBuf<int32_t> rt_bbeg;     // [grid * warps + 1] first entry of each warp in rt_blk
   leo2d::DevBuf<unsigned char> rt_data;  // 32 + 32 rt_rows bytes per k-step
   // shared-memory windows of the row blocks (rbw_spmm.cu): per tile of 16 blocks
   // the sorted distinct columns of its slots; slots hold window positions

@@ -104,9 +104,9 @@ constexpr int kRtBatchWarps = 16, kRtBatchDepth = 3;  // the launch shape of eve
 struct RtBatchFlake {
   const unsigned char* data = nullptr;  // the flake's k-steps (csr->rt_data)
   const int64_t* wbeg = nullptr;
-  const int64_t* kst = nullptr;
-  int64_t n = 0, nrb = 0;
-  int group = 0, chunk = 0;
+  const int2* blk = nullptr;
+  const int32_t* bbeg = nullptr;
+  int64_t n = 0;
   float* x0 = nullptr;            // T_0 (step parity 0 reads x0, writes x1)
   float* x1 = nullptr;
   double* partials[2] = {nullptr, nullptr};  // by step parity, [CTAs of the flake][64]

@@ -29,9 +29,10 @@
 //                        the B fragment of mma.m16n8k8 (B = V^T, k = slot, n = row)
 //   Blocks are stored in the order the kernel processes them: warp w of CTA c
 //   takes runs of G consecutive blocks (one run per tile of W runs, tiles in
-//   chunked round-robin over the CTAs), so each warp streams one contiguous
-//   range of k-steps, rt_wbeg[c W + w] .. rt_wbeg[c W + w + 1]; rt_kst holds
-//   each block's k-step count (the kernel's block boundaries).
+//   chunked round-robin over the CTAs; the blocks after the last whole round in
+//   even shares), so each warp streams one contiguous range of k-steps,
+//   rt_wbeg[c W + w] .. rt_wbeg[c W + w + 1]; rt_blk lists each warp's blocks
+//   with their k-step counts in that order, from rt_bbeg[c W + w] on.
 // Kernel (one CTA per SM, W warps, no CTA-wide barrier in the main loop)
 //   Each warp runs a software pipeline over its k-steps with cp.async groups:
 //   at iteration u it copies the matrix data of k-step u + D + DM and the 8 T_n
@@ -45,9 +46,19 @@
 //   4 cg + i is logical column g + 8 i of the MMA). At a block's last k-step
 //   the lane owns rows 2t and 2t + 1 of the block, columns 4 cg .. 4 cg + 3: it
 //   writes T_{n+1} and adds its moment dots (FP32 over 16 blocks, then FP64).
+//   The T_n and T_{n-1} rows of that epilogue are copied into shared memory at
+//   the block's start (each lane its own 16-byte chunks, so its own wait orders
+//   them): held in registers through the block they cost 16 registers, and the
+//   loads of T_{n-1}, which comes from HBM, stalled the warp.
+//   Bound: instruction issue (61 %) and the L1 / shared-memory pipe (59 %); HBM
+//   50 %, tensor pipe 31 % (1M orbitals). One step at 2.4M orbitals 0.602 ms
+//   with the rows in registers, 0.573 ms with 16 warps, 0.559 ms with 20 (the
+//   freed registers); 10M orbitals 2.44 -> 2.26 ms; the complex step at 400k
+//   orbitals 0.187 -> 0.153 ms.
 //   cp.async waits are hardware waits on copies already issued: no spin loop.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "kpm.cuh"
@@ -122,10 +133,10 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1
 struct RtArgs {
   CUtensorMap tmap;  // kRtTma: T_n as [n][32] FP32, boxes of one 128-byte row, 128-byte swizzle
   int64_t n;    // rows
-  int64_t nrb;  // row blocks
   const unsigned char* __restrict__ data;  // k-steps in processing order
   const int64_t* __restrict__ wbeg;        // [grid * W + 1] first k-step of each warp
-  const int64_t* __restrict__ kst;         // [blocks] k-steps of each block
+  const int2* __restrict__ blk;            // [blocks + 1] (block, k-steps) in processing order
+  const int32_t* __restrict__ bbeg;        // [grid * W + 1] first entry of each warp in blk
   const float* __restrict__ tn;
   float* __restrict__ tp;
   const float* __restrict__ tprev;  // null: T_{n-1} is read from tp
@@ -134,8 +145,6 @@ struct RtArgs {
   double* __restrict__ partials;
   const double* __restrict__ prev_partials;
   double* __restrict__ prev_dots;
-  int group;        // G: consecutive blocks per run
-  int chunk;        // consecutive tiles per CTA between grid-wide jumps
   // kRtTma: row waits give up after spin_limit polls or two seconds and set *status
   uint64_t spin_limit;
   int* status;
@@ -239,9 +248,10 @@ __device__ __forceinline__ float2 ld_stream_f2(const void* p) {
 //    8t + cg). The matrix stream is read with loads that skip L1: the columns 2D
 //    k-steps ahead (they address the row loads), the values D ahead.
 // Either way the matrix stream is prefetched into L2 in bulk further ahead.
-// Each warp walks its blocks in the build's processing order: runs of G
-// consecutive blocks, run i in tile (bid + (i / chunk) grid) chunk + i % chunk;
-// a block ends after its k-step count (kst), read one block ahead.
+// Each warp walks its blocks in the build's processing order, a list of (block,
+// k-steps) read one block ahead. The cp.async form prefetches the matrix 8
+// k-steps ahead of its copies: 32 ahead held 42 MB of the L2 with 16-row k-steps
+// and pushed T_n rows out (0.68 -> 0.60 ms at 2.4M orbitals).
 // The epilogue's reads of T_n and T_{n-1} rows: through the read-only path, or,
 // in a launch that runs several steps (COH), from L2, since other CTAs of the
 // launch wrote those rows after L1 may have cached older ones.
@@ -262,6 +272,8 @@ __device__ __forceinline__ float4 ld_rows_tprev(const float* p) {
 // rows, the products P_re = X Re(V)^T and P_im = X Im(V)^T give
 //   (H X)_re = P_re[re col] - P_im[im col],  (H X)_im = P_re[im col] + P_im[re col],
 // combined in the lane's own four columns (two pairs) at the block's end.
+__device__ __forceinline__ float4 ld_f4(const unsigned char* p) { return *reinterpret_cast<const float4*>(p); }
+
 template <int W, int D, int STAGE, int R, bool COH = false, bool CPX = false>
 __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const int nblk) {
   constexpr bool REGS = STAGE == kRtRegs;
@@ -270,6 +282,9 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
   constexpr int NTR = RB / kRtRows;      // n-tiles of the block's rows
   static_assert(!CPX || R == 16, "complex blocks: 8 rows in the 16-row k-step layout");
   constexpr int KB = rt_step_bytes(R);   // bytes of one k-step
+  // the epilogue's T_n and T_{n-1} rows: copied into shared memory at the block's
+  // start (cp.async form), else held in registers through the block
+  constexpr bool LATE = STAGE == kRtCpAsync;
   static_assert((R == 8 || R == 16) && (R == 8 || STAGE == kRtCpAsync), "16-row blocks: cp.async form only");
   static_assert(!COH || STAGE == kRtCpAsync, "multi-step launches: the cp.async form (its gathers bypass L1)");
   constexpr int C = 32;
@@ -277,7 +292,7 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
   constexpr int XS = D + 1;      // shared ring of staged T_n rows (k-steps)
   constexpr int MS = 2 * XS;     // shared ring of matrix k-steps
   constexpr int DM = MS - 1 - D; // matrix lookahead beyond the rows'
-  constexpr int kPf = REGS ? 48 : 32;  // matrix k-steps prefetched into L2 ahead
+  constexpr int kPf = STAGE == kRtCpAsync ? 8 : REGS ? 48 : 32;  // matrix k-steps prefetched into L2 ahead
   constexpr int kDotFlush = 16;        // blocks summed in FP32 between FP64 flushes
   static_assert(REGS || ((XS & (XS - 1)) == 0 && DM >= D + 1), "power-of-two rings, matrix ahead of the rows");
   extern __shared__ __align__(1024) unsigned char rt_smem_raw[];
@@ -290,36 +305,24 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
   const int g = lane >> 2, t = lane & 3, q = lane >> 3, p = lane & 7;
   const int cg = (g >> 1) | ((g & 1) << 2);  // the lane's chunk of 4 memory columns
   const int64_t n = a.n;
-  const int first = a.first, group = a.group, chunk = a.chunk;
+  const int first = a.first;
   const float alpha = a.alpha != 0.f ? a.alpha : (first ? 1.f : 2.f);
   const float* tprev = a.tprev ? a.tprev : a.tp;
   float* tp = a.tp;
   const float* tnc = a.tn + 4 * cg;
   const unsigned char* tnb = reinterpret_cast<const unsigned char*>(a.tn + 4 * p);  // + column * 128
-  const int64_t* kst = a.kst;
   const int64_t k0 = a.wbeg[bid * W + warp];
   const int nk = (int)(a.wbeg[bid * W + warp + 1] - k0);
   const unsigned char* gdata = a.data + k0 * KB;
 
-  // block walk, block-end countdown and epilogue operands
-  // run i of the warp lies in tile (bid + (i / chunk) nblk) chunk + i % chunk;
-  // the walk keeps that tile split as (tb, ic) for the run after the current
-  // one, advanced without divisions
-  int jb = 0;
-  int64_t tb = (int64_t)bid * chunk;
-  int ic = 0;
-  auto run_row = [&]() -> int64_t { return ((tb + ic) * W + warp) * group * RB; };
-  auto next_run = [&]() {
-    if (++ic == chunk) {
-      ic = 0;
-      tb += (int64_t)nblk * chunk;
-    }
-  };
-  int64_t rbase = run_row(), row0 = 0;  // first row of the current run
-  next_run();
-  int64_t nbase = run_row();  // first row of the next run
-  int left = 0;                                       // k-steps of the current block still to run
-  int next_left = nk > 0 ? (int)kst[rbase / RB] : 0;  // the next block's k-steps
+  // the warp's blocks in processing order, (block, k-steps) read one block ahead
+  const int2* bp = a.blk + a.bbeg[bid * W + warp];
+  int2 next = nk > 0 ? __ldg(bp) : make_int2(0, 0);
+  int64_t row0 = 0;  // first row of the current block
+  int left = 0;      // k-steps of the current block still to run
+  int bk = 0;        // k-steps of the current block already run (LATE)
+  // LATE: the lane's 16-byte chunks of the block's T_n rows (2 per n-tile), then T_{n-1}
+  unsigned char* ebuf = rt_smem + (size_t)W * (XS * 1024 + MS * KB) + (size_t)warp * (NTR * 2048);
   // T_n and T_{n-1} of the lane's rows 8 nt + 2t and 8 nt + 2t + 1 of the block
   float4 xn0[NTI], xn1[NTI], xp0[NTI], xp1[NTI];
 #pragma unroll
@@ -351,11 +354,24 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
     for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
   };
   auto begin_block = [&]() {
-    row0 = rbase + (int64_t)jb * RB;
-    left = next_left;
-    // the k-steps of the block after this one (its run may start elsewhere)
-    const int64_t nrow = jb + 1 < group ? row0 + RB : nbase;
-    if (nrow / RB < a.nrb) next_left = (int)kst[nrow / RB];
+    row0 = (int64_t)next.x * RB;
+    left = next.y;
+    next = __ldg(++bp);  // (the list has one entry of padding)
+    if constexpr (LATE) {
+      bk = 0;
+      unsigned char* eb = ebuf + 16 * lane;
+#pragma unroll
+      for (int nt = 0; nt < NTR; ++nt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int64_t r = row0 + 8 * nt + 2 * t + h;
+          if (r < n) {
+            cp_async_cg16(eb + (4 * nt + h) * 512, tnc + r * C);
+            if (!first) cp_async_cg16(eb + (4 * nt + 2 + h) * 512, tprev + r * C + 4 * cg);
+          }
+        }
+      return;
+    }
 #pragma unroll
     for (int nt = 0; nt < NTR; ++nt) {
       const int64_t r0 = row0 + 8 * nt + 2 * t;
@@ -388,6 +404,9 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
 #pragma unroll
   for (int nt = 0; nt < NTI; ++nt) acc[nt].zero();
   auto end_block = [&]() {
+    if constexpr (LATE) {
+      if (bk <= D) cp_async_wait<0>();
+    }
     if constexpr (CPX) {
       float4 a0, a1, b0, b1;  // real-part and imaginary-part products, rows 2t and 2t + 1
       acc[0].rows(a0, a1);
@@ -398,8 +417,15 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
       const float4 h0 = make_float4(a0.x - b0.y, a0.y + b0.x, a0.z - b0.w, a0.w + b0.z);
       const float4 h1 = make_float4(a1.x - b1.y, a1.y + b1.x, a1.z - b1.w, a1.w + b1.z);
       const int64_t r0 = row0 + 2 * t;
-      row_out(r0, h0, xp0[0], xn0[0]);
-      row_out(r0 + 1, h1, xp1[0], xn1[0]);
+      if constexpr (LATE) {
+        const unsigned char* eb = ebuf + 16 * lane;
+        const float4 zn0 = ld_f4(eb), zn1 = ld_f4(eb + 512), zp0 = ld_f4(eb + 1024), zp1 = ld_f4(eb + 1536);
+        row_out(r0, h0, zp0, zn0);
+        row_out(r0 + 1, h1, zp1, zn1);
+      } else {
+        row_out(r0, h0, xp0[0], xn0[0]);
+        row_out(r0 + 1, h1, xp1[0], xn1[0]);
+      }
     } else {
 #pragma unroll
       for (int nt = 0; nt < NTI; ++nt) {
@@ -407,15 +433,16 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
         acc[nt].rows(h0, h1);
         acc[nt].zero();
         const int64_t r0 = row0 + 8 * nt + 2 * t;
-        row_out(r0, h0, xp0[nt], xn0[nt]);
-        row_out(r0 + 1, h1, xp1[nt], xn1[nt]);
+        if constexpr (LATE) {
+          const unsigned char* eb = ebuf + 16 * lane + 4 * nt * 512;
+          const float4 zn0 = ld_f4(eb), zn1 = ld_f4(eb + 512), zp0 = ld_f4(eb + 1024), zp1 = ld_f4(eb + 1536);
+          row_out(r0, h0, zp0, zn0);
+          row_out(r0 + 1, h1, zp1, zn1);
+        } else {
+          row_out(r0, h0, xp0[nt], xn0[nt]);
+          row_out(r0 + 1, h1, xp1[nt], xn1[nt]);
+        }
       }
-    }
-    if (++jb == group) {
-      jb = 0;
-      rbase = nbase;
-      next_run();
-      nbase = run_row();
     }
     if (++since_flush == kDotFlush) {
       since_flush = 0;
@@ -432,7 +459,7 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
   if constexpr (STAGE == kRtCpAsync) {
     constexpr int kWarpBytes = XS * 1024 + MS * KB;
     constexpr int kChunks = KB / 16;  // 16-byte chunks of a matrix k-step (18 or 34)
-    static_assert(MS % 8 == 0, "L2 prefetch every 8 matrix k-steps at fixed slots of the unrolled loop");
+    static_assert(MS == 2 * XS, "the matrix ring is two halves of the row ring's length");
     unsigned char* xr = rt_smem + (size_t)warp * kWarpBytes;
     unsigned char* mr = xr + XS * 1024;
     // Lane (g, t) copies, and later reads, chunk cg of the T_n rows of slots t
@@ -442,33 +469,38 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
     // matrix k-steps (copied in 16-byte chunks by all lanes, read by all) are
     // ordered by one __syncwarp per iteration.
     const int ro0 = t * 128 + 16 * (cg ^ t), ro1 = 512 + t * 128 + 16 * (cg ^ (t + 4));
-    // iteration u (matrix slot sm = u mod MS): wait for the copies of iteration
+    // iteration u (row slot j = u mod XS, its matrix slot in the half `mc` of the
+    // matrix ring, the other half at `mo`): wait for the copies of iteration
     // u - D (the rows of k-step u, matrix k-step u + DM), copy matrix k-step
     // u + D + DM and the rows of k-step u + D, run k-step u's MMAs. The matrix
     // source of the iteration is mb + off (mb: k-step u's chunk of this lane).
-    auto iter = [&](int u, int sm, const unsigned char* mb, int off, bool checks, bool pf) {
+    // kind: 0 the first copies (no k-step to run yet), 1 the unrolled loop (every
+    // copy exists), 2 the last k-steps.
+    auto iter = [&](auto kind, int u, int j, unsigned char* mc, unsigned char* mo, const unsigned char* mb, int off) {
+      constexpr int kind_v = decltype(kind)::value;
+      auto slot = [&](int i) { return i < XS ? mc + i * KB : mo + (i - XS) * KB; };  // i mod MS, from the half's start
       cp_async_wait<D - 1>();
       __syncwarp();  // every lane's matrix copies have landed; k-step u - 1 is read
       const int vm = u + D + DM, vx = u + D;
-      if (!checks || vm < nk) {
-        unsigned char* md = mr + ((sm + MS - 1) & (MS - 1)) * KB + 16 * lane;
+      if (kind_v == 1 || vm < nk) {
+        unsigned char* md = slot((j + MS - 1) & (MS - 1)) + 16 * lane;
         const unsigned char* msrc = mb + (off + (D + DM) * KB);
         if (lane < kChunks) cp_async_cg16(md, msrc);
         if (kChunks > 32 && lane < kChunks - 32) cp_async_cg16(md + 512, msrc + 512);
       }
-      if (pf && lane == 0 && vm + kPf < nk)
-        prefetch_l2_bulk(gdata + (size_t)(vm + kPf) * KB, (uint32_t)min(8, nk - vm - kPf) * KB);
-      if (!checks || (vx >= 0 && vx < nk)) {
+      if (((j + D + DM) & (XS - 1)) == 0 && lane == 0 && vm + kPf < nk)
+        prefetch_l2_bulk(gdata + (size_t)(vm + kPf) * KB, (uint32_t)min(XS, nk - vm - kPf) * KB);
+      if (kind_v == 1 || (vx >= 0 && vx < nk)) {
         // the columns of k-step vx (slots t, t + 4) landed DM iterations ago
-        const int2 cc = *reinterpret_cast<const int2*>(mr + ((sm + D) & (MS - 1)) * KB + 8 * t);
-        unsigned char* dst = xr + ((sm + D) & (XS - 1)) * 1024;
+        const int2 cc = *reinterpret_cast<const int2*>(slot((j + D) & (MS - 1)) + 8 * t);
+        unsigned char* dst = xr + ((j + D) & (XS - 1)) * 1024;
         cp_async_cg16(dst + ro0, tnc + (uint64_t)(uint32_t)cc.x * C);
         cp_async_cg16(dst + ro1, tnc + (uint64_t)(uint32_t)cc.y * C);
       }
       cp_async_commit();
-      if (checks && u < 0) return;
-      const unsigned char* xs = xr + (sm & (XS - 1)) * 1024;
-      const unsigned char* ms = mr + sm * KB;
+      if constexpr (kind_v == 0) return;
+      const unsigned char* xs = xr + j * 1024;
+      const unsigned char* ms = mc + j * KB;
       RtA A;
       A.split(*reinterpret_cast<const float4*>(xs + ro0), *reinterpret_cast<const float4*>(xs + ro1));
       if constexpr (NTI == 1) {
@@ -480,6 +512,7 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
         acc[0].mma(A, v.x, v.y);
         acc[1].mma(A, v.z, v.w);
       }
+      if constexpr (LATE) ++bk;
       if (--left == 0) {
         end_block();
         if (u + 1 < nk) begin_block();
@@ -487,16 +520,47 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
     };
     if (nk > 0) begin_block();
     const unsigned char* mlan = gdata + 16 * lane;  // this lane's chunk of matrix k-step 0
+    // The loop is unrolled over one half of the matrix ring for 16-row k-steps and
+    // over both halves for 8-row ones: the block's end is inlined in every
+    // iteration, and 8 copies of the 16-row one overflow the instruction cache
+    // (ncu: 3.5 of 10 cycles per instruction without one; 0.84 -> 0.58 ms on a
+    // 2.4M-orbital flake), while 8 copies of the 8-row one still fit and save the
+    // addresses of the swapped halves (0.594 -> 0.573 ms).
+    constexpr int UN = NTI == 1 ? MS : XS;
+    unsigned char *mc = mr, *mo = mr + XS * KB;
+    auto swap_halves = [&]() {
+      unsigned char* x = mc;
+      mc = mo;
+      mo = x;
+    };
     int u = -(D + DM);
-    for (; u < 0; ++u) iter(u, u & (MS - 1), mlan, u * KB, true, (((u + D + DM) & 7) == 0));
-    const int main_end = nk - (D + DM) > 0 ? ((nk - (D + DM)) & ~(MS - 1)) : 0;
-    for (; u < main_end; u += MS) {
-      const unsigned char* mb = mlan + (size_t)u * KB;
-#pragma unroll
-      for (int j = 0; j < MS; ++j) iter(u + j, j, mb, j * KB, false, ((j + D + DM) & 7) == 0);
+    if (u & XS) swap_halves();
+#pragma unroll 1
+    for (; u < 0; ++u) {
+      iter(std::integral_constant<int, 0>{}, u, u & (XS - 1), mc, mo, mlan, u * KB);
+      if (((u + 1) & (XS - 1)) == 0) swap_halves();
     }
-    for (; u < nk; ++u)
-      iter(u, u & (MS - 1), mlan, u * KB, true, (((u + D + DM) & 7) == 0));
+    const int main_end = nk - (D + DM) > 0 ? ((nk - (D + DM)) & ~(UN - 1)) : 0;
+#pragma unroll 1
+    for (; u < main_end; u += UN) {  // (u = 0: the halves are in order)
+      const unsigned char* mb = mlan + (size_t)u * KB;
+      if constexpr (UN == MS) {
+#pragma unroll
+        for (int j = 0; j < XS; ++j) iter(std::integral_constant<int, 1>{}, u + j, j, mr, mr + XS * KB, mb, j * KB);
+#pragma unroll
+        for (int j = 0; j < XS; ++j)
+          iter(std::integral_constant<int, 1>{}, u + XS + j, j, mr + XS * KB, mr, mb, (XS + j) * KB);
+      } else {
+#pragma unroll
+        for (int j = 0; j < XS; ++j) iter(std::integral_constant<int, 1>{}, u + j, j, mc, mo, mb, j * KB);
+        swap_halves();
+      }
+    }
+#pragma unroll 1
+    for (; u < nk; ++u) {
+      iter(std::integral_constant<int, 2>{}, u, u & (XS - 1), mc, mo, mlan, u * KB);
+      if (((u + 1) & (XS - 1)) == 0) swap_halves();
+    }
     cp_async_wait<0>();
   } else if constexpr (STAGE == kRtTma) {
     // Each warp owns XS entries of 2 KB (1 KB aligned): row entry e holds slots
@@ -737,10 +801,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_cheb_rt_batch(const __grid_consta
   for (int k = 0; k < p.steps; ++k) {
     RtArgs a{};
     a.n = F.n;
-    a.nrb = F.nrb;
     a.data = F.data;
     a.wbeg = F.wbeg;
-    a.kst = F.kst;
+    a.blk = F.blk;
+    a.bbeg = F.bbeg;
     a.tn = k % 2 == 0 ? F.x0 : F.x1;
     a.tp = k % 2 == 0 ? F.x1 : F.x0;
     a.tprev = nullptr;
@@ -749,8 +813,6 @@ __global__ void __launch_bounds__(W * 32, 1) k_cheb_rt_batch(const __grid_consta
     a.partials = F.partials[k % 2];
     a.prev_partials = k == 0 ? nullptr : F.partials[(k + 1) % 2];
     a.prev_dots = k == 0 ? nullptr : F.dots + (size_t)(k - 1) * 2 * C;
-    a.group = F.group;
-    a.chunk = F.chunk;
     a.spin_limit = p.spin_limit;
     a.status = p.status;
     rt_body<W, D, kRtCpAsync, kRtRows, true>(a, bid, nblk);
@@ -1016,10 +1078,19 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
   }
 }
 
-__global__ void k_rt_gather_i64(const int32_t* __restrict__ seq, const int64_t* __restrict__ src, int64_t count,
-                                int64_t* __restrict__ dst) {
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < count; j += (int64_t)gridDim.x * blockDim.x)
-    dst[j] = src[seq[j]];
+// The k-steps of the blocks in processing order, alone and beside their block
+// (one entry of padding: the kernel reads a block ahead).
+__global__ void k_rt_order(const int32_t* __restrict__ seq, const int64_t* __restrict__ kst, int64_t count,
+                           int64_t* __restrict__ kseq, int2* __restrict__ blk) {
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j <= count; j += (int64_t)gridDim.x * blockDim.x) {
+    if (j == count) {
+      blk[j] = make_int2(0, 0);
+      continue;
+    }
+    const int32_t b = seq[j];
+    kseq[j] = kst[b];
+    blk[j] = make_int2(b, (int)kst[b]);
+  }
 }
 
 __global__ void k_rt_scatter_i64(const int32_t* __restrict__ seq, const int64_t* __restrict__ pos, int64_t count,
@@ -1028,7 +1099,7 @@ __global__ void k_rt_scatter_i64(const int32_t* __restrict__ seq, const int64_t*
     dst[seq[j]] = pos[j];
 }
 
-__global__ void k_rt_warp_begin(const int64_t* __restrict__ first_pos, const int64_t* __restrict__ pos, int count,
+__global__ void k_rt_warp_begin(const int32_t* __restrict__ first_pos, const int64_t* __restrict__ pos, int count,
                                 int64_t* __restrict__ wbeg) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
     wbeg[i] = pos[first_pos[i]];
@@ -1041,18 +1112,15 @@ __global__ void k_rt_warp_begin(const int64_t* __restrict__ first_pos, const int
 namespace {
 
 struct RtShape {
-  int64_t nrb, nruns, ntiles;
+  int64_t nrb;
   unsigned grid;
 };
 
-RtShape rt_shape(const leo2d_ctx* ctx, int64_t n, int warps, int group, int chunk, int rows, int max_grid = 0) {
+RtShape rt_shape(const leo2d_ctx* ctx, int64_t n, int warps, int rows, int max_grid = 0) {
   RtShape s;
   s.nrb = (n + rows - 1) / rows;
-  s.nruns = (s.nrb + group - 1) / group;
-  s.ntiles = (s.nruns + warps - 1) / warps;
-  const int64_t chunks = (s.ntiles + chunk - 1) / chunk;
   const int64_t cap = max_grid > 0 ? max_grid : (int64_t)ctx->sm_count;
-  s.grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(cap, chunks));
+  s.grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(cap, (s.nrb + warps - 1) / warps));
   return s;
 }
 
@@ -1060,7 +1128,7 @@ RtShape rt_shape(const leo2d_ctx* ctx, int64_t n, int warps, int group, int chun
 // matrix: 2 (D + 1) k-steps of blocks of `rows` rows): packed for cp.async; for
 // TMA gathers 2 KB per row entry (the matrix in its holes) and its mbarrier.
 constexpr int rt_warp_bytes(int depth, int stage, int rows) {
-  return stage == kRtTma ? (depth + 1) * (2048 + 8) : (depth + 1) * 1024 + 2 * (depth + 1) * rt_step_bytes(rows);
+  return stage == kRtTma ? (depth + 1) * (2048 + 8) : (depth + 1) * 1024 + 2 * (depth + 1) * rt_step_bytes(rows) + rows / 8 * 2048;
 }
 
 // TMA maps of the T_n buffers a thread launched the TMA form on (three
@@ -1099,7 +1167,7 @@ size_t rt_smem_bytes(int warps, int depth, int stage, int rows) {
 }
 
 unsigned rt_grid(leo2d_ctx* ctx, const leo2d_csr* csr, int warps, int rows) {
-  return rt_shape(ctx, csr->n, warps, rt_group_of(ctx), rt_chunk_of(ctx), rows).grid;
+  return rt_shape(ctx, csr->n, warps, rows).grid;
 }
 
 void csr_drop_rt(leo2d_csr* csr) {
@@ -1107,6 +1175,8 @@ void csr_drop_rt(leo2d_csr* csr) {
   csr->rt_built = false;
   csr->rt_kst.release();
   csr->rt_wbeg.release();
+  csr->rt_blk.release();
+  csr->rt_bbeg.release();
   csr->rt_data.release();
   csr->rt_blocks = csr->rt_ksteps = csr->rt_union = 0;
   csr->rt_max_slots = 0;
@@ -1122,7 +1192,7 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
   LEO_REQUIRE(!cpx || (rows == 8 && csr->pval_im32.p), "a complex Hamiltonian takes 8-row blocks");
   const int64_t n = csr->n;
   const int KB = rt_step_bytes(cpx ? 16 : rows);  // complex: real and imaginary panels
-  const RtShape sh = rt_shape(ctx, n, warps, group, chunk, rows, max_grid);
+  const RtShape sh = rt_shape(ctx, n, warps, rows, max_grid);
   if (csr->rt_built && csr->rt_rows == rows && csr->rt_patch == csr->reorder_patch &&
       csr->rt_curve == csr->reorder_curve && csr->rt_warps == warps && csr->rt_group == group &&
       csr->rt_chunk == chunk && csr->rt_grid == sh.grid)
@@ -1162,33 +1232,38 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
     LEO_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), ctx->stream));
   }
   csr->rt_built = false;
-  // processing order: CTA c, warp w, its runs (tile by tile), the blocks of a run
+  // Processing order. Whole rounds first: a round gives every warp `chunk` runs of
+  // `group` consecutive blocks, the tiles (one run per warp of a CTA) of a CTA
+  // next to each other, so the grid's blocks in flight form one band of rows and
+  // their T_n rows stay in L2. The blocks after the last whole round are dealt
+  // evenly in contiguous shares, so two warps differ by one block at most
+  // (whole runs only left up to `chunk` x `group` blocks between CTAs, 17 % of
+  // a step on a 200k-orbital flake).
+  const int64_t nw = (int64_t)sh.grid * warps;
+  const int64_t rounds = sh.nrb / (nw * chunk * group), rest0 = rounds * nw * chunk * group, rest = sh.nrb - rest0;
   std::vector<int32_t> seq;
   seq.reserve((size_t)sh.nrb);
-  std::vector<int64_t> first((size_t)sh.grid * warps + 1);
-  for (unsigned c = 0; c < sh.grid; ++c)
-    for (int w = 0; w < warps; ++w) {
-      first[(size_t)c * warps + w] = (int64_t)seq.size();
-      for (int64_t i = 0;; ++i) {
-        const int64_t tile = ((int64_t)c + (i / chunk) * (int64_t)sh.grid) * chunk + i % chunk;
-        if (tile >= sh.ntiles) break;
-        const int64_t run = tile * warps + w;
-        if (run >= sh.nruns) break;
-        for (int j = 0; j < group; ++j) {
-          const int64_t b = run * group + j;
-          if (b >= sh.nrb) break;
-          seq.push_back((int32_t)b);
-        }
+  std::vector<int32_t> first((size_t)nw + 1);
+  for (int64_t i = 0; i < nw; ++i) {
+    const int64_t c = i / warps, w = i % warps;
+    first[(size_t)i] = (int32_t)seq.size();
+    for (int64_t r = 0; r < rounds; ++r)
+      for (int64_t k = 0; k < chunk; ++k) {
+        const int64_t b0 = (((r * sh.grid + c) * chunk + k) * warps + w) * group;
+        for (int64_t b = b0; b < b0 + group; ++b) seq.push_back((int32_t)b);
       }
-    }
-  first[(size_t)sh.grid * warps] = (int64_t)seq.size();
+    for (int64_t b = rest0 + rest * i / nw; b < rest0 + rest * (i + 1) / nw; ++b) seq.push_back((int32_t)b);
+  }
+  first[(size_t)nw] = (int32_t)seq.size();
   LEO_REQUIRE((int64_t)seq.size() == sh.nrb, "row-block order does not cover the matrix");
   DevBuf<int32_t> dseq(std::max<int64_t>(sh.nrb, 1));
-  DevBuf<int64_t> kseq(std::max<int64_t>(sh.nrb, 1)), pos(sh.nrb + 1), dfirst(first.size());
+  DevBuf<int64_t> kseq(std::max<int64_t>(sh.nrb, 1)), pos(sh.nrb + 1);
   h2d(ctx, dseq.p, seq.data(), seq.size());
-  h2d(ctx, dfirst.p, first.data(), first.size());
+  csr->rt_bbeg.alloc(first.size());
+  csr->rt_blk.alloc((size_t)sh.nrb + 1);
+  h2d(ctx, csr->rt_bbeg.p, first.data(), first.size());
   const unsigned g = grid_for(sh.nrb, 256, (int64_t)ctx->sm_count * 16);
-  launch(ctx, "rt_order", [&] { k_rt_gather_i64<<<g, 256, 0, ctx->stream>>>(dseq.p, csr->rt_kst.p, sh.nrb, kseq.p); });
+  launch(ctx, "rt_order", [&] { k_rt_order<<<g, 256, 0, ctx->stream>>>(dseq.p, csr->rt_kst.p, sh.nrb, kseq.p, csr->rt_blk.p); });
   exclusive_scan_i64(ctx, kseq.p, pos.p, sh.nrb);
   int64_t total = 0;
   d2h(ctx, &total, pos.p + sh.nrb, 1);
@@ -1197,8 +1272,8 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
   launch(ctx, "rt_order", [&] { k_rt_scatter_i64<<<g, 256, 0, ctx->stream>>>(dseq.p, pos.p, sh.nrb, kstart.p); });
   csr->rt_wbeg.alloc(first.size());
   launch(ctx, "rt_order", [&] {
-    k_rt_warp_begin<<<grid_for((int64_t)first.size(), 256), 256, 0, ctx->stream>>>(dfirst.p, pos.p, (int)first.size(),
-                                                                                   csr->rt_wbeg.p);
+    k_rt_warp_begin<<<grid_for((int64_t)first.size(), 256), 256, 0, ctx->stream>>>(csr->rt_bbeg.p, pos.p,
+                                                                                   (int)first.size(), csr->rt_wbeg.p);
   });
   csr->rt_data.release();
   csr->rt_data.alloc((size_t)std::max<int64_t>(total, 1) * KB);
@@ -1225,7 +1300,7 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
 }
 
 unsigned rt_batch_cap(leo2d_ctx* ctx, const leo2d_csr* csr) {
-  return rt_shape(ctx, csr->n, kRtBatchWarps, rt_group_of(ctx), rt_chunk_of(ctx), kRtRows).grid;
+  return rt_shape(ctx, csr->n, kRtBatchWarps, kRtRows).grid;
 }
 
 size_t rt_batch_smem() { return rt_smem_bytes(kRtBatchWarps, kRtBatchDepth, kRtCpAsync, kRtRows); }
@@ -1292,10 +1367,10 @@ void rt_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape
   a.status = ctx->status.p;
   a.never_wait = ctx->test_unsatisfied_wait;
   a.n = csr->n;
-  a.nrb = csr->rt_blocks;
   a.data = csr->rt_data.p;
   a.wbeg = csr->rt_wbeg.p;
-  a.kst = csr->rt_kst.p;
+  a.blk = csr->rt_blk.p;
+  a.bbeg = csr->rt_bbeg.p;
   a.tn = tn;
   a.tp = tp;
   a.tprev = tprev;
@@ -1304,8 +1379,6 @@ void rt_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape
   a.partials = partials;
   a.prev_partials = prev_partials;
   a.prev_dots = prev_dots;
-  a.group = csr->rt_group;
-  a.chunk = csr->rt_chunk;
   auto go = [&](auto kern, int warps) {
     LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // the register form keeps no dynamic shared memory: the carveout goes to L1
