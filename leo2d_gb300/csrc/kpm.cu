@@ -371,7 +371,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
     // 8-row blocks of the locality-ordered copy, stored for this launch shape
     const int w = shape.rt_warps;
     const int panel = m->complex_h ? 16 : shape.rt_rows;  // complex: real and imaginary panels
-    const bool fits = rt_smem_bytes(w, shape.rt_depth, shape.rt_stage, panel) + 8 * 1024 <= ctx->smem_optin;
+    const bool fits = rt_smem_bytes(w, shape.rt_depth, shape.rt_stage, panel) + w * 512 + 1024 <= ctx->smem_optin;
     if (fits && csr_build_rt(ctx, mm, w, rt_group_of(ctx), rt_chunk_of(ctx), shape.rt_rows)) {
       dyn_smem = rt_smem_bytes(w, shape.rt_depth, shape.rt_stage, panel);
       grid = m->rt_grid;

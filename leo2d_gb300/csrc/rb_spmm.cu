@@ -142,12 +142,11 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
   const float alpha = a.alpha != 0.f ? a.alpha : (a.first ? 1.f : 2.f);
   const float* tprev = a.tprev ? a.tprev : a.tp;
   const float* tq = a.tn + 4 * q;
-  // dots: FP32 over kDotFlush row blocks (64 rows), then FP64 (the FP64 pipe
-  // is a small fraction of the FP32 one: converting every block's partials
-  // would bound the kernel). A flush sums the four groups' FP32 partials and
-  // hands column `lane` to lane `lane`, so the FP64 sums take 2 registers.
+  // dots: FP32 over kDotFlush row blocks (64 rows), then pairs of FP32 over the
+  // CTA (PairSum), FP64 beyond. A flush sums the four groups' FP32 partials and
+  // hands column `lane` to lane `lane`.
   constexpr int kDotFlush = 16;
-  double d0 = 0.0, d1 = 0.0;  // column `lane`
+  PairSum d0, d1;             // column `lane`
   float e0[4], e1[4];         // columns 4q..4q+3, this lane's rows
   int since_flush = 0;
 #pragma unroll
@@ -171,8 +170,8 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
         v1 = s1;
       }
     }
-    d0 += (double)v0;
-    d1 += (double)v1;
+    d0.add(v0);
+    d1.add(v1);
 #pragma unroll
     for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
   };
@@ -347,18 +346,19 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
   // (the velocity step computes no moment dots and writes no partials)
   if constexpr (DJ) return;
   flush();
-  // warps add their columns in warp order (deterministic)
-  __shared__ double bsum[2 * C];
-  for (int t = threadIdx.x; t < 2 * C; t += NT) bsum[t] = 0.0;
+  // the warps' sums through the stages' memory (every copy has landed), added in
+  // warp order (deterministic)
   __syncthreads();
-  for (int w = 0; w < WARPS; ++w) {
-    if (warp == w) {
-      bsum[2 * lane] += d0;
-      bsum[2 * lane + 1] += d1;
-    }
-    __syncthreads();
+  PairSum* ws = reinterpret_cast<PairSum*>(smem);  // [WARPS][2C]
+  ws[warp * 2 * C + 2 * lane] = d0;
+  ws[warp * 2 * C + 2 * lane + 1] = d1;
+  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * C; t += NT) {
+    PairSum s;
+#pragma unroll 8
+    for (int w = 0; w < WARPS; ++w) s.add(ws[w * 2 * C + t]);
+    a.partials[(size_t)bid * 2 * C + t] = s.value();
   }
-  for (int t = threadIdx.x; t < 2 * C; t += NT) a.partials[(size_t)bid * 2 * C + t] = bsum[t];
 }
 
 template <int WARPS, bool PACKED, int U, bool CPX = false, bool DJ = false>
@@ -889,7 +889,9 @@ int rb_stages(leo2d_ctx* ctx, leo2d_csr* csr, int warps, bool velocity) {
 }
 
 size_t rb_smem_bytes(leo2d_ctx* ctx, leo2d_csr* csr, int warps, bool velocity) {
-  return (size_t)rb_stages(ctx, csr, warps, velocity) * (size_t)rb_stage_bytes(ctx, csr, warps, velocity);
+  // (at least the warps' sums of a step's end: 64 pairs a warp)
+  return std::max((size_t)rb_stages(ctx, csr, warps, velocity) * (size_t)rb_stage_bytes(ctx, csr, warps, velocity),
+                  (size_t)warps * 64 * 8);
 }
 
 unsigned rb_grid(leo2d_ctx* ctx, const leo2d_csr* csr, int warps) {

@@ -327,8 +327,8 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
   float4 xn0[NTI], xn1[NTI], xp0[NTI], xp1[NTI];
 #pragma unroll
   for (int nt = 0; nt < NTI; ++nt) xn0[nt] = xn1[nt] = xp0[nt] = xp1[nt] = make_float4(0.f, 0.f, 0.f, 0.f);
-  // dots: FP32 over kDotFlush blocks, then FP64; lane (g, t) ends with column 4 cg + t
-  double d0 = 0.0, d1 = 0.0;
+  // dots: FP32 over kDotFlush blocks, then pairs of FP32 (PairSum); lane (g, t) ends with column 4 cg + t
+  PairSum d0, d1;
   float e0[4], e1[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
@@ -348,8 +348,8 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
         v0 = e0[c];
         v1 = e1[c];
       }
-    d0 += (double)v0;
-    d1 += (double)v1;
+    d0.add(v0);
+    d1.add(v1);
 #pragma unroll
     for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
   };
@@ -712,19 +712,18 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
     }
   }
   flush();
-  // warps add their columns in warp order (deterministic)
-  __shared__ double bsum[2 * C];
-  for (int i = threadIdx.x; i < 2 * C; i += NT) bsum[i] = 0.0;
-  __syncthreads();
+  // the warps' sums, added in warp order (deterministic)
+  __shared__ PairSum wsum[W][2 * C];
   const int col = 4 * cg + t;
-  for (int w = 0; w < W; ++w) {
-    if (warp == w) {
-      bsum[2 * col] += d0;
-      bsum[2 * col + 1] += d1;
-    }
-    __syncthreads();
+  wsum[warp][2 * col] = d0;
+  wsum[warp][2 * col + 1] = d1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * C; i += NT) {
+    PairSum s;
+#pragma unroll 8
+    for (int w = 0; w < W; ++w) s.add(wsum[w][i]);
+    a.partials[(size_t)bid * 2 * C + i] = s.value();
   }
-  for (int i = threadIdx.x; i < 2 * C; i += NT) a.partials[(size_t)bid * 2 * C + i] = bsum[i];
 }
 
 template <int W, int D, int STAGE, int R = kRtRows, bool CPX = false>

@@ -80,31 +80,58 @@ struct StepArgs {
   double* __restrict__ prev_dots;            // where the previous step's dots go
 };
 
-// Fixed-order tree reduction of partials[b][t] over b < nb into out[t], for the
-// values t assigned to this block.
+// A running sum of FP32 terms as an unevaluated pair hi + lo: Knuth's exact
+// addition (hi + x = s + e without rounding), e goes into lo. It keeps some 48 bits
+// where FP64 keeps 53, at FP32 cost: GB300's FP64 unit takes a warp's addition
+// every 16 cycles of an SM and answers late, so FP64 sums at the end of a step
+// (a chain over the warps) were microseconds of each step. Sums over CTAs are FP64.
+struct PairSum {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
+    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    h = s;
+  }
+  __device__ __forceinline__ void add(const PairSum& o) {
+    add(o.h);
+    l = __fadd_rn(l, o.l);
+  }
+  __device__ __forceinline__ PairSum shfl_xor(int o) const {
+    PairSum r;
+    r.h = __shfl_xor_sync(0xffffffffu, h, o);
+    r.l = __shfl_xor_sync(0xffffffffu, l, o);
+    return r;
+  }
+  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+};
+
+// Fixed-order reduction of partials[b][t] over b < nb into out[t], for the values
+// t assigned to this block: a thread per value while blocks are few (a small
+// matrix), else a warp per value (lane l adds b = l, l + 32, ..., then a
+// butterfly). No block barrier: the other warps start their rows meanwhile.
+// FP64 additions are what costs here (a warp's takes 16 cycles of an SM): a
+// block-wide tree per value took 200 us a step on a 76-orbital matrix, whose
+// grid is one block with 64 values.
 // `bid` / `nblk`: this block's index and the block count of its group (the grid,
 // or the blocks of one flake in a batched launch).
 template <int C, int NT = kThreads>
 __device__ __forceinline__ void reduce_prev(const double* __restrict__ partials,
                                             double* __restrict__ out, int nb, int bid, int nblk) {
-  constexpr int kPow = NT >= 512 ? 512 : 256;  // tree over the first kPow lanes
-  __shared__ double red[kPow];
-  for (int t = bid; t < 2 * C; t += nblk) {
+  if (nb <= 16) {
+    for (int t = bid + nblk * (int)threadIdx.x; t < 2 * C; t += nblk * NT) {
+      double s = __ldcg(partials + t);
+      for (int b = 1; b < nb; ++b) s += __ldcg(partials + (size_t)b * 2 * C + t);
+      out[t] = s;
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  for (int t = bid + nblk * (int)(threadIdx.x >> 5); t < 2 * C; t += nblk * (NT / 32)) {
     double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += NT) s += __ldcg(partials + (size_t)b * 2 * C + t);
-    for (int base = 0; base < NT; base += kPow) {  // fold lanes >= kPow in, in order
-      if ((int)threadIdx.x >= base && (int)threadIdx.x < base + kPow) {
-        if (base == 0) red[threadIdx.x] = s;
-        else red[threadIdx.x - base] += s;
-      }
-      __syncthreads();
-    }
-    for (int w = kPow / 2; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[t] = red[0];
-    __syncthreads();
+    for (int b = lane; b < nb; b += 32) s += __ldcg(partials + (size_t)b * 2 * C + t);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[t] = s;
   }
 }
 
