@@ -485,6 +485,8 @@ def run_cfg0(args):
         t, d = _timed(stream, lambda: dos(csr.kpm_dos(cfg)), args.steps, 0)
     launches = (ctx.launch_count() - l0) // args.steps
     k_n, k_ms = ctx.kernel_stats("cheb_step")
+    if k_n == 0:  # every step of a run in a few launches: the time of one step
+        k_n, k_ms = args.steps * ((2 * R + cols - 1) // cols) * (Pc // 2), ctx.kernel_stats("cheb_steps")[1]
     ctx.set_profiling(False)
 
     def e2e_once():
@@ -525,7 +527,8 @@ def run_cfg0(args):
            "gpu_launches": int(launches),
            "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                         "frac": round(achieved / peak, 4), "traffic": None,
-                        "kernel": {0: "k_cheb_tile<double>", 1: "k_cheb_step<double>"}.get(kernel_id, str(kernel_id)),
+                        "kernel": {0: "k_cheb_tile<double>", 1: "k_cheb_step<double>",
+                                   6: "k_cheb_sell (FP64 rows, every step in one launch)"}.get(kernel_id, str(kernel_id)),
                         "bytes_per_launch": bytes_step, "launch_ms": round(launch_ms, 4), "peak_kind": peak_kind,
                         "note": "working set in L2: the fraction of HBM is a bandwidth figure, not an HBM bound"},
            # what bounds this workload: the FP64 FMAs (2 flops per entry and column)
@@ -1010,7 +1013,8 @@ def main():
     kernel_name = {0: "k_cheb_tile (tiled CSR gathers)", 1: "k_cheb_step (register gathers)",
                    2: "k_cheb_tc (tensor cores)", 3: "k_cheb_rb (row blocks)",
                    4: "k_cheb_rbw (row blocks, shared-memory windows)",
-                   5: "k_cheb_rt (8-row blocks, tensor cores)"}[kernel_id]
+                   5: "k_cheb_rt (8-row blocks, tensor cores)",
+                   6: "k_cheb_win (rows over shared-memory windows, every step in one launch)"}[kernel_id]
 
     import torch
     torch.cuda.set_device(local)

@@ -479,7 +479,8 @@ class Csr:
 
     def step_kernel(self, cfg):
         """(kernel, block): the step kernel a kpm_dos call with cfg runs (0 tiled, 1 register,
-        2 tensor cores, 3 row blocks) and its vector-block width."""
+        2 tensor cores, 3 row blocks, 5 row blocks on the tensor cores, 6 every step in one launch
+        over the CSR rows) and its vector-block width."""
         k, b = ctypes.c_int32(), ctypes.c_int32()
         self.ctx.check(self.ctx.lib.leo2d_kpm_step_kernel(self.ctx.h, self.h, ctypes.byref(cfg),
                                                           ctypes.byref(k), ctypes.byref(b)))

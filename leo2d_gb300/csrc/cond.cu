@@ -189,6 +189,7 @@ bool cond_trace_rows(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kpm_cfg* 
   leo2d_csr* m = const_cast<leo2d_csr*>(csr);
   StepShape s = choose_shape(ctx, csr, false, 32, 32, 0);
   s.rb = true;
+  s.row = false;
   s.rt = false;  // the velocity step exists in the 4-row form only
   s.tc = false;
   s.rb_window = false;
@@ -211,6 +212,7 @@ bool cond_trace_rows(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kpm_cfg* 
   // 4-row step otherwise); its moment dots go to a scratch row nobody reads
   StepShape sb = choose_shape(ctx, csr, false, 32, 32, 0);
   sb.rb = false;
+  sb.row = false;
   sb.tc = false;
   sb.rt = ctx->kernel_variant == -1 || ctx->kernel_variant == 5;
   Recursion rt;
@@ -345,6 +347,7 @@ leo2d_status leo2d_kpm_cond(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kp
     const int64_t total_cols = local ? num_targets : (int64_t)cfg->num_vectors * group;
     StepShape shape = choose_shape(ctx, csr, false, (int)std::min<int64_t>(total_cols, 8),
                                    cfg->block > 0 ? cfg->block : 8, cfg->rows_per_warp);
+    shape.row = false;  // the Kubo path takes its steps one by one
     Recursion r;
     r.allow_perm = false;
     r.setup(ctx, csr, shape, 1);

@@ -103,6 +103,26 @@ struct leo2d_csr {
   leo2d::DevBuf<int2> rt_blk;         // [blocks + 1] (block, k-steps) in processing order
   leo2d::DevBuf<int32_t> rt_bbeg;     // [grid * warps + 1] first entry of each warp in rt_blk
   leo2d::DevBuf<unsigned char> rt_data;  // 32 + 32 rt_rows bytes per k-step
+  // rows in slices of 16, the j-th entries of a slice's rows next to each other
+  // (row_spmm.cu): positions padded to the slice's longest row
+  bool sell_perm = false;             // built from the locality-ordered copy
+  leo2d::DevBuf<int64_t> sell_off;    // [slices + 1] first position of each slice
+  leo2d::DevBuf<int32_t> sell_col;    // [16 positions] columns and FP64 values
+  leo2d::DevBuf<double> sell_val;
+  // the same slices in chunks of 8 positions, [chunk][16 rows][8], for tiles of
+  // slices whose T_n rows go through shared memory (FP32, row_spmm.cu): columns
+  // as positions in the tile's window, its sorted distinct columns
+  bool win_perm = false;
+  int win_cs = 0, win_group = 0;      // column slice and CTAs the tiles were cut for
+  int win_cls = 0;                    // classes the entries are ordered by (1: kept in order)
+  int64_t win_tiles = 0, win_stride = 0;
+  int win_tile_slices = 0, win_slice_cap = 0;
+  leo2d::DevBuf<int64_t> win_off;     // [slices + 1] first chunk of each slice
+  leo2d::DevBuf<int32_t> win_slen;    // [slices] positions
+  leo2d::DevBuf<int32_t> win_list;    // [tiles][win_stride] window rows
+  leo2d::DevBuf<int32_t> win_cnt;     // [tiles]
+  leo2d::DevBuf<float> win_val;
+  leo2d::DevBuf<uint16_t> win_idx;
   // shared-memory windows of the row blocks (rbw_spmm.cu): per tile of 16 blocks
   // the sorted distinct columns of its slots; slots hold window positions
   bool rbw_built = false;
@@ -155,4 +175,7 @@ void csr_drop_rt(leo2d_csr* csr);
 // nothing) when a tile of 16 blocks has more than 8192 slots or 2048 distinct columns.
 bool csr_build_rbw(leo2d_ctx* ctx, leo2d_csr* csr);
 void csr_drop_rbw(leo2d_csr* csr);
+// Drop the formats of row_spmm.cu.
+void csr_drop_sell(leo2d_csr* csr);
+void csr_drop_win(leo2d_csr* csr);
 }  // namespace leo2d

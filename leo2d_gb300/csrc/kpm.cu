@@ -281,6 +281,7 @@ struct ShapeKey {
 };
 struct Tuned {
   int rows = 0, warps = 0;
+  bool row = false; // the multi-step row kernel won for this block width
   bool tc = false;  // the tensor-core step won for this block width
   bool rb = false;  // the row-block step won for this block width
   int rb_warps = 0, rb_unroll = 0;
@@ -324,8 +325,13 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
   if (shape.rt && (!can_perm || s.fp64 || s.cols != 32 || ctx->reorder == 0)) shape.rt = false;
   if (shape.rt) shape.rb = false;
   if (shape.rb || shape.rt) shape.tc = false;
+  const int used = s.cols_used > 0 ? s.cols_used : s.cols;
+  if (shape.tc || shape.rb || shape.rt || m->nnz == 0 ||
+      (shape.row && !s.row_built && !row_pays(m, s.fp64, steps_)))
+    shape.row = false;
   const bool want_perm = can_perm && (shape.tc || shape.rb || shape.rt || ctx->reorder == 1 ||
-                                      (ctx->reorder == -1 && n >= 100000));
+                                      (ctx->reorder == -1 &&
+                                       (n >= 100000 || (shape.row && row_wants_order(n, s.fp64)))));
   const double patch = reorder_patch_for(ctx, shape.rb || shape.rt);
   if (want_perm && (!m->reordered || (s.fp64 && !m->reorder_fp64) || m->reorder_patch != patch ||
                     m->reorder_curve_req != ctx->reorder_curve))
@@ -381,6 +387,15 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
       shape.rt = false;  // a block too heavy for the 8-row build: the gather kernels run
     }
   }
+  if (shape.row) {
+    LEO_REQUIRE(s.cols == 8 || s.cols == 16 || s.cols == 32 || s.cols == 64 || (s.cols == 128 && !s.fp64),
+                s.fp64 ? "FP64 block width must be 8, 16, 32 or 64 columns"
+                       : "FP32 block width must be 8, 16, 32, 64 or 128 columns");
+    shape.row = row_prepare(ctx, mm, use_perm, s.fp64, s.cols, used, rows);
+    shape.tiled = !shape.row;
+    if (shape.row) bar.alloc(kRowBarWords);
+    if (shape.row && rows.exact) x2.alloc((size_t)n * s.cols * sizeof(float));
+  }
   if (shape.tiled && !shape.tc && !shape.rb && !shape.rt) {
     const int ns = tile_slots(s.cols, s.fp64, s.warps);
     const int ri = s.rows_per_item > 0 ? s.rows_per_item : std::max(1, 32 / ns);
@@ -429,7 +444,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
       grid = (unsigned)g;
     }
   }
-  if (!shape.tiled && !shape.tc && !shape.rb && !shape.rt) {
+  if (!shape.tiled && !shape.tc && !shape.rb && !shape.rt && !shape.row) {
     if (shape.rows_per_item <= 0) shape.rows_per_item = 4;
     const int occ = std::max(1, occupancy(s.cols, s.fp64));
     const int lpr = s.cols <= 32 ? s.cols : 32;  // lanes per row slot
@@ -443,7 +458,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
   const size_t esz = s.fp64 ? sizeof(double) : sizeof(float);
   x0.alloc((size_t)n * s.cols * esz);
   x1.alloc((size_t)n * s.cols * esz);
-  partials.alloc((size_t)2 * grid * 2 * s.cols);
+  partials.alloc(shape.row ? row_partials(rows, steps) : (size_t)2 * grid * 2 * s.cols);
   dots.alloc((size_t)steps * 2 * s.cols);
 }
 
@@ -451,7 +466,7 @@ template <typename T>
 void one_step(Recursion& r, const void* in, void* out, const void* prev, bool first, double alpha, int matrix) {
   leo2d_ctx* ctx = r.ctx;
   const int C = r.shape.cols;
-  LEO_REQUIRE(!r.use_perm && !r.shape.tc && !r.shape.rb && !r.shape.rt,
+  LEO_REQUIRE(!r.use_perm && !r.shape.tc && !r.shape.rb && !r.shape.rt && !r.shape.row,
               "a recursion over dxH needs the unpermuted matrix");
   StepArgs<T> a;
   a.n = r.n;
@@ -494,9 +509,11 @@ void Recursion::step(const void* in, void* out, const void* prev, bool first, do
 }
 
 void Recursion::run() {
-  if (shape.fp64) enqueue_steps<double>(*this);
+  if (shape.row)
+    row_run(ctx, csr, rows, use_perm, shape.fp64, shape.cols, steps, x0.p, x1.p, x2.p, partials.p, bar.p, dots.p);
+  else if (shape.fp64) enqueue_steps<double>(*this);
   else enqueue_steps<float>(*this);
-  if (shape.tiled || shape.tc || shape.rb || shape.rt) ctx_check_status(ctx, "Chebyshev recursion");
+  if (shape.tiled || shape.tc || shape.rb || shape.rt || shape.row) ctx_check_status(ctx, "Chebyshev recursion");
 }
 
 Recursion::~Recursion() {
@@ -548,7 +565,10 @@ StepShape choose_shape(leo2d_ctx* ctx, const leo2d_csr* csr, bool fp64, int cols
   else if (ctx->kernel_variant == -1) s.rt = rt_ok && (cached ? it->second.rt : s.rb);
   if (s.rt) s.rb = false;
   if (s.rb || s.rt) s.tc = false;
+  // else every step in one launch over the CSR rows, unless a step kernel is asked for
+  s.row = ctx->kernel_variant == -1 && !s.tc && !s.rb && !s.rt && (cached ? it->second.row : true);
   if (csr->complex_h) {
+    s.row = false;
     s.rb = !s.rt;  // the 4-row step, or the 8-row step when asked for
     s.tc = false;
     s.tiled = true;
@@ -728,9 +748,11 @@ void run_trace(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kpm_cfg* cfg, c
   const int total_cols = cfg->num_vectors * group;
   StepShape shape = choose_shape(ctx, csr, fp64, total_cols, cfg->block, cfg->rows_per_warp);
   LEO_REQUIRE(shape.cols % group == 0, "block width must hold whole complex vectors");
-  const int vec_per_block = shape.cols / group;
+  shape.cols_used = std::min(shape.cols, total_cols);
   Recursion r;
   r.setup(ctx, csr, shape, steps);
+  shape = r.shape;
+  const int vec_per_block = shape.cols / group;
   std::vector<double> dots((size_t)steps * 2 * shape.cols);
   DirectMoments dm(ctx, csr, r);
   for (int v0 = 0; v0 < cfg->num_vectors; v0 += vec_per_block) {
@@ -782,8 +804,10 @@ leo2d_status leo2d_kpm_ldos(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kp
     const int group = csr->complex_h ? 2 : 1;  // complex H: a (real, imaginary) column pair per target
     StepShape shape = choose_shape(ctx, csr, fp64, (int)std::min<int64_t>(num_targets * group, 128),
                                    cfg->block, cfg->rows_per_warp);
+    shape.cols_used = (int)std::min<int64_t>(shape.cols, num_targets * group);
     Recursion r;
     r.setup(ctx, csr, shape, steps);
+    shape = r.shape;
     std::vector<double> dots((size_t)steps * 2 * shape.cols);
     DirectMoments dm(ctx, csr, r);
     const int per_block = shape.cols / group;
@@ -839,6 +863,7 @@ extern "C" leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr,
           sh.tc = false;
           sh.rb = false;
           sh.rt = false;
+          sh.row = false;
           Recursion r;
           r.setup(ctx, csr, sh, steps);
           fill_phase(ctx, r, 1, 0, cols / 2);
@@ -853,6 +878,28 @@ extern "C" leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr,
             best_c = per;
             best_t.rows = rows;
             best_t.warps = warps;
+          }
+        }
+      }
+      // every step in one launch over the CSR rows
+      if (ctx->kernel_variant == -1) {
+        StepShape sh = choose_shape(ctx, csr, fp64, cols, cols, 0);
+        sh.tc = sh.rb = sh.rt = false;
+        sh.row = sh.row_built = true;
+        const int many = 64;  // (one launch: enough steps to hide its start)
+        Recursion r;
+        r.setup(ctx, csr, sh, many);
+        if (r.shape.row) {
+          fill_phase(ctx, r, 1, 0, cols / 2);
+          r.run();  // warm
+          ctx_sync(ctx);
+          const auto before = ctx->stats["cheb_steps"];
+          r.run();
+          ctx_sync(ctx);
+          const double per = (ctx->stats["cheb_steps"].ms - before.ms) / many;
+          if (per < best_c) {
+            best_c = per;
+            best_t.row = true;
           }
         }
       }
@@ -878,6 +925,7 @@ extern "C" leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr,
           if (per < best_c) {
             best_c = per;
             best_t.tc = true;
+            best_t.row = false;
           }
         }
       }
@@ -912,7 +960,7 @@ extern "C" leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr,
           const double per = (after.ms - before.ms) / std::max<int64_t>(1, after.launches - before.launches);
           if (per < best_c) {
             best_c = per;
-            best_t.tc = false;
+            best_t.tc = best_t.row = false;
             best_t.rb = true;
             best_t.rb_warps = sh.rb_warps;
             best_t.rb_unroll = sh.rb_unroll;
@@ -957,7 +1005,7 @@ extern "C" leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr,
           const double per = (after.ms - before.ms) / std::max<int64_t>(1, after.launches - before.launches);
           if (per < best_c) {
             best_c = per;
-            best_t.tc = false;
+            best_t.tc = best_t.row = false;
             best_t.rb = false;
             best_t.rt = true;
             best_t.rt_warps = sh.rt_warps;
@@ -996,7 +1044,8 @@ extern "C" leo2d_status leo2d_kpm_step_kernel(leo2d_ctx* ctx, const leo2d_csr* c
     if (s.rb && (!can_perm || s.fp64 || s.cols != 32 || ctx->reorder == 0)) s.rb = false;
     if (s.rt && (!can_perm || s.fp64 || s.cols != 32 || ctx->reorder == 0)) s.rt = false;
     if (s.tc && !can_perm) s.tc = false;
-    *kernel = s.rt ? 5 : s.rb ? (s.rb_window ? 4 : 3) : s.tc ? 2 : s.tiled ? 0 : 1;
+    if (s.tc || s.rb || s.rt || csr->nnz == 0 || !row_pays(csr, s.fp64, cfg->poly_order / 2)) s.row = false;
+    *kernel = s.row ? 6 : s.rt ? 5 : s.rb ? (s.rb_window ? 4 : 3) : s.tc ? 2 : s.tiled ? 0 : 1;
     *block = s.cols;
   });
 }

@@ -26,7 +26,35 @@ struct StepShape {
   int rt_stage = 1;        // 8-row step: T_n rows staged in 0 registers, 1 shared memory by cp.async,
                            // 2 shared memory by TMA gathers
   int rt_rows = 8;         // rows per block (8; 16 with rt_stage 1)
+  bool row = false;        // every step in one launch over the CSR rows (row_spmm.cu; a real H)
+  bool row_built = false;  // build its format whatever the steps of the run (the autotuner's trial)
+  int cols_used = 0;       // columns that hold vectors (0: all); the row step leaves the other slices out
 };
+
+// Launch of the multi-step row kernel (row_spmm.cu): the columns in `slices` of
+// cs, `group` CTAs each, `chunk` steps per launch.
+constexpr int kRowSmall = 0, kRowSell = 1, kRowWin = 2;
+struct RowShape {
+  int cs = 32, slices = 1, group = 1, chunk = 1;
+  int form = 0;        // kRowSmall, kRowSell (FP64) or kRowWin (FP32)
+  bool exact = false;  // kRowWin: the tiled step's FP32 sums, a third vector buffer
+  int dot_slots = 1, dot_rows = 1;
+  int ent_cap = 0, row_cap = 0;  // small: room of a CTA
+  int warps = 0;  // compute warps of a CTA
+  size_t smem = 0;
+};
+constexpr int kRowBarWords = 8;  // barrier counters of up to 4 slices; the last word is the abort flag
+// Chooses the form and builds its format (once per matrix); false when none fits.
+bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s);
+// Whether the row form is worth its format (and ordering) for a run of `steps`.
+bool row_pays(const leo2d_csr* csr, bool fp64, int steps);
+// Whether the form for n rows gains from the locality ordering (its windows).
+bool row_wants_order(int64_t n, bool fp64);
+// doubles of the CTAs' partial dots of one launch
+size_t row_partials(const RowShape& s, int steps);
+// Every step [0, steps) on T_0 in x0 (x2: the third buffer of the exact form), dots[step][cols][2].
+void row_run(leo2d_ctx* ctx, const leo2d_csr* csr, const RowShape& s, bool perm, bool fp64, int cols, int steps,
+             void* x0, void* x1, void* x2, double* partials, unsigned* bar, double* dots);
 
 // Vector block resident on the device: two buffers of n x cols (T_k, T_{k-1}).
 struct Recursion {
@@ -36,12 +64,15 @@ struct Recursion {
   int64_t n = 0;
   unsigned grid = 0;
   DevBuf<char> x0, x1;          // T buffers (float or double)
+  DevBuf<char> x2;              // the exact row form's third
   DevBuf<double> partials;      // [grid][cols][2]
   DevBuf<unsigned> counter;     // last-block ticket
   DevBuf<double> dots;          // [steps][cols][2]: <T_k|T_k>, <T_{k+1}|T_k>
   int steps = 0;
   int tile_stages = 2, tile_chunk = 1, tile_rows = 0, tile_cap = 0, tile_rp_bytes = 0, tile_col_bytes = 0, tile_stage_bytes = 0;
   size_t dyn_smem = 0;
+  RowShape rows;                // shape.row
+  DevBuf<unsigned> bar;         // shape.row: the slices' barriers
   cudaGraphExec_t graph = nullptr;
   int graph_steps = -1;
   bool use_perm = false;  // stream the locality-ordered copy of the matrix
