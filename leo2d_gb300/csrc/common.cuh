@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <map>
@@ -133,6 +134,7 @@ struct leo2d_ctx {
   int64_t kubo_chunk = 0;     // Kubo trace: B-side moments held at once (0: as many as memory allows)
   int mlp_fused = 1;          // network forward over many sites: 1 one fused launch, 0 one GEMM per layer
   leo2d::DevBuf<int> status;  // one int, reset before kernels that may set it
+  leo2d::DevBuf<char> scratch;  // small work arrays of the transforms (ctx_scratch)
 };
 
 namespace leo2d {
@@ -207,6 +209,23 @@ template <class T>
 void d2h(leo2d_ctx* ctx, T* dst, const T* src, size_t count) {
   if (count) LEO_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
 }
+
+// Work space of one call on this context, kept up to 64 MiB (a call synchronises
+// before it returns, and a context serves one thread at a time, so the next call
+// may reuse it): the transforms' four allocations took longer than their kernels.
+constexpr size_t kScratchKept = (size_t)64 << 20;
+template <class T>
+T* ctx_scratch(leo2d_ctx* ctx, size_t count) {
+  const size_t bytes = count * sizeof(T);
+  if (ctx->scratch.n < bytes || (ctx->scratch.n > kScratchKept && bytes <= kScratchKept)) {
+    ctx->scratch.release();
+    ctx->scratch.alloc(std::max(bytes, (size_t)1 << 16));
+  }
+  return reinterpret_cast<T*>(ctx->scratch.p);
+}
+
+// tab[m] = cos(pi m / (2P)), 0 <= m < 4P (transform.cu).
+void cos_table(leo2d_ctx* ctx, int P, double* tab);
 
 // Exclusive prefix sum of n int64 values: out[0..n] with out[n] = total.
 // `out` may alias `in` only if it is a distinct buffer of n+1 elements.
