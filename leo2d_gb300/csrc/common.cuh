@@ -210,13 +210,15 @@ void d2h(leo2d_ctx* ctx, T* dst, const T* src, size_t count) {
   if (count) LEO_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
 }
 
-// Work space of one call on this context, kept up to 64 MiB (a call synchronises
+// Work space of one call on this context, one live request at a time, kept up to 64 MiB (a call synchronises
 // before it returns, and a context serves one thread at a time, so the next call
 // may reuse it): the transforms' four allocations took longer than their kernels.
 constexpr size_t kScratchKept = (size_t)64 << 20;
 template <class T>
 T* ctx_scratch(leo2d_ctx* ctx, size_t count) {
   const size_t bytes = count * sizeof(T);
+  if (g_alloc_cap && bytes > g_alloc_cap)  // also when a kept buffer would do
+    fail(LEO2D_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes exceeds the context's alloc_cap_mb");
   if (ctx->scratch.n < bytes || (ctx->scratch.n > kScratchKept && bytes <= kScratchKept)) {
     ctx->scratch.release();
     ctx->scratch.alloc(std::max(bytes, (size_t)1 << 16));

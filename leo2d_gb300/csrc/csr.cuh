@@ -149,6 +149,15 @@ void csr_alloc_entries(leo2d_ctx* ctx, leo2d_csr* csr, int64_t nnz, bool with_dx
 void csr_build_reordered(leo2d_ctx* ctx, leo2d_csr* csr, double patch, bool with_fp64, bool curve = false);
 // Per-orbital disregistry (Hstruct::getShiftConfigs) into device memory out[n][2]; bilayers.
 void csr_shift_configs(leo2d_ctx* ctx, const leo2d_csr* csr, double* out);
+// The same disregistry as fractions of a turn in 64-bit fixed point: component d
+// of grid cell (i, j) on sheet s is (c[d] + i mi[d] + j mj[d]) mod 2^64, in units
+// of 2^-64 (ph[s]). The site findNearest picks on the other sheet only moves the
+// offset by whole lattice vectors, so modulo 1 the offset is affine in (i, j), and
+// integer multiplication wraps by itself. Rounding: |i| 2^-53, as in FP64.
+struct SitePhase {
+  uint64_t mi[2], mj[2], c[2];
+};
+void csr_site_phases(const leo2d_csr* csr, SitePhase* ph);
 void csr_drop_reordered(leo2d_csr* csr);
 // Builds the tensor-core tiles of the locality-ordered copy; returns false (and
 // builds nothing) when a tile has more than 1024 distinct columns, 16384

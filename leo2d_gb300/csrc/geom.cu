@@ -1285,21 +1285,11 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
 
 namespace leo2d {
 
-// Disregistry of every orbital into device memory out[n][2].
-void csr_shift_configs(leo2d_ctx* ctx, const leo2d_csr* csr, double* out) {
-  LEO_REQUIRE(csr->has_geom && csr->grid4.p, "matrix has no geometry (uploaded without it)");
-  const leo2d_geom& g = csr->geom;
-  LEO_REQUIRE(g.num_sheets == 2, "disregistry is defined for bilayers (two sheets)");
-  GeomDev G;
-  std::memset(&G, 0, sizeof(G));
-  G.S = g.num_sheets;
-  G.model = g.model;
-  G.bc = g.boundary_condition;
-  for (int s = 0; s < G.S; ++s) fill_sheet(g, s, G.sh[s]);
+static CellInv cell_inverses(const leo2d_geom& g, const SheetDev* sh) {
   CellInv ci;
   for (int s = 0; s < 2; ++s) {
     const double theta = g.angles[s];
-    const SheetDev& d = G.sh[s];
+    const SheetDev& d = sh[s];
     double u[2][2];
     u[0][0] = std::cos(theta) * d.a[0][0] - std::sin(theta) * d.a[0][1];
     u[0][1] = std::sin(theta) * d.a[0][0] + std::cos(theta) * d.a[0][1];
@@ -1311,11 +1301,60 @@ void csr_shift_configs(leo2d_ctx* ctx, const leo2d_csr* csr, double* out) {
     ci.inv[s][1][0] = -u[0][1] / det;
     ci.inv[s][1][1] = u[0][0] / det;
   }
+  return ci;
+}
+
+static void require_bilayer(const leo2d_csr* csr) {
+  LEO_REQUIRE(csr->has_geom && csr->grid4.p, "matrix has no geometry (uploaded without it)");
+  LEO_REQUIRE(csr->geom.num_sheets == 2, "disregistry is defined for bilayers (two sheets)");
+}
+
+// Disregistry of every orbital into device memory out[n][2].
+void csr_shift_configs(leo2d_ctx* ctx, const leo2d_csr* csr, double* out) {
+  require_bilayer(csr);
+  const leo2d_geom& g = csr->geom;
+  GeomDev G;
+  std::memset(&G, 0, sizeof(G));
+  G.S = g.num_sheets;
+  G.model = g.model;
+  G.bc = g.boundary_condition;
+  for (int s = 0; s < G.S; ++s) fill_sheet(g, s, G.sh[s]);
+  const CellInv ci = cell_inverses(g, G.sh);
   if (csr->n > 0)
     launch(ctx, "shift_configs", [&] {
       k_shift_configs<<<grid_for(csr->n, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
           G, ci, csr->n, csr->grid4.p, out);
     });
+}
+
+void csr_site_phases(const leo2d_csr* csr, SitePhase* out) {
+  require_bilayer(csr);
+  const leo2d_geom& g = csr->geom;
+  SheetDev sh[2];
+  for (int s = 0; s < 2; ++s) fill_sheet(g, s, sh[s]);
+  const CellInv ci = cell_inverses(g, sh);
+  auto fixed = [](double x) {  // x mod 1 in units of 2^-64
+    const double f = x - std::floor(x);
+    return f < 1.0 ? (uint64_t)std::ldexp(f, 64) : (uint64_t)0;
+  };
+  for (int s = 0; s < 2; ++s) {
+    const SheetDev &a = sh[s], &b = sh[1 - s];
+    // global position of (i, j): R_a (i a_0 + j a_1 + atom_0), minus the other
+    // sheet's atom: three columns (of i, of j, constant)
+    const double col[3][2] = {{a.cos_t * a.a[0][0] - a.sin_t * a.a[0][1], a.sin_t * a.a[0][0] + a.cos_t * a.a[0][1]},
+                              {a.cos_t * a.a[1][0] - a.sin_t * a.a[1][1], a.sin_t * a.a[1][0] + a.cos_t * a.a[1][1]},
+                              {a.cos_t * a.atom[0][0] - a.sin_t * a.atom[0][1] -
+                                   (b.cos_t * b.atom[0][0] - b.sin_t * b.atom[0][1]),
+                               a.sin_t * a.atom[0][0] + a.cos_t * a.atom[0][1] -
+                                   (b.sin_t * b.atom[0][0] + b.cos_t * b.atom[0][1])}};
+    for (int d = 0; d < 2; ++d) {
+      const double* inv = ci.inv[1 - s][d];
+      out[s].mi[d] = fixed(inv[0] * col[0][0] + inv[1] * col[0][1]);
+      out[s].mj[d] = fixed(inv[0] * col[1][0] + inv[1] * col[1][1]);
+      out[s].c[d] = fixed(inv[0] * col[2][0] + inv[1] * col[2][1]) + out[s].mi[d] * (uint64_t)(int64_t)a.min0 +
+                    out[s].mj[d] * (uint64_t)(int64_t)a.min1;
+    }
+  }
 }
 
 }  // namespace leo2d

@@ -43,6 +43,117 @@ __device__ __forceinline__ uint32_t mix32(uint64_t a, uint64_t b) {
   return (uint32_t)((z ^ (z >> 31)) >> 32);
 }
 
+// A value as an unevaluated sum of two FP32 numbers (about 2^-45 relative).
+struct Pair {
+  float h, l;
+};
+__device__ __forceinline__ Pair pair_fast_sum(float a, float b) {  // |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return {s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+  const float p = __fmul_rn(a.h, b.h);
+  float e = __fmaf_rn(a.h, b.h, -p);
+  e = __fmaf_rn(a.h, b.l, e);
+  e = __fmaf_rn(a.l, b.h, e);
+  return {p, e};
+}
+// a + b rounded to FP32
+__device__ __forceinline__ float pair_sum(Pair a, Pair b) {
+  const float s = __fadd_rn(a.h, b.h);
+  const float t = __fsub_rn(s, a.h);
+  const float e = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, t)), __fsub_rn(b.h, t));
+  return __fadd_rn(s, __fadd_rn(e, __fadd_rn(a.l, b.l)));
+}
+__device__ __forceinline__ Pair pair_neg(Pair a) { return {-a.h, -a.l}; }
+
+// cos and sin of p 2^-64 turns. The quarter turn comes off exactly in integers;
+// the rest (at most 1/8 turn) goes through the Taylor series of sin and cos, their
+// first terms in pairs and the tail (below 1/60) in FP32: errors up to 5e-9, so
+// the rounded FP32 value is that of the FP64 function but for 3 in 1000 near ties
+// (then its neighbour).
+__device__ __forceinline__ void phase_cos_sin(uint64_t p, Pair& c, Pair& s) {
+  const uint32_t q = (uint32_t)((p + (1ull << 61)) >> 62);
+  const int64_t r = (int64_t)(p - ((uint64_t)q << 62));
+  const int32_t a = (int32_t)(r >> 32);
+  const float h = __int2float_rn(a);
+  const float l = __fmaf_rn(__uint2float_rn((uint32_t)r), 0x1p-32f, __int2float_rn(a - (int32_t)h));
+  // x = 2 pi (h + l) 2^-32
+  constexpr double kTurn = 6.283185307179586476925 / 4294967296.0;
+  constexpr float kTurnH = (float)kTurn, kTurnL = (float)(kTurn - (double)kTurnH);
+  const Pair u = pair_mul({h, l}, {kTurnH, kTurnL});
+  const Pair x = pair_fast_sum(u.h, u.l);
+  const Pair z = pair_mul(x, x);
+  constexpr double kSixth = -1.0 / 6.0;
+  constexpr float kSixthH = (float)kSixth, kSixthL = (float)(kSixth - (double)kSixthH);
+  const Pair t = pair_mul(pair_mul(x, z), {kSixthH, kSixthL});
+  float ts = __fmaf_rn(z.h, -1.0f / 39916800.0f, 1.0f / 362880.0f);
+  ts = __fmaf_rn(z.h, ts, -1.0f / 5040.0f);
+  ts = __fmaf_rn(z.h, ts, 1.0f / 120.0f);
+  ts = __fmul_rn(ts, __fmul_rn(x.h, __fmul_rn(z.h, z.h)));
+  const Pair s0 = pair_fast_sum(x.h, t.h);
+  const Pair sn = pair_fast_sum(s0.h, __fadd_rn(s0.l, __fadd_rn(__fadd_rn(x.l, t.l), ts)));
+  float tc = __fmaf_rn(z.h, -1.0f / 3628800.0f, 1.0f / 40320.0f);
+  tc = __fmaf_rn(z.h, tc, -1.0f / 720.0f);
+  tc = __fmaf_rn(z.h, tc, 1.0f / 24.0f);
+  tc = __fmul_rn(tc, __fmul_rn(z.h, z.h));
+  const Pair c0 = pair_fast_sum(1.0f, -0.5f * z.h);
+  const Pair cs = pair_fast_sum(c0.h, __fadd_rn(c0.l, __fmaf_rn(-0.5f, z.l, tc)));
+  c = (q & 1) ? sn : cs;
+  s = (q & 1) ? cs : sn;
+  if (q == 1 || q == 2) c = pair_neg(c);
+  if (q >= 2) s = pair_neg(s);
+}
+
+// BF16 features [n][16] of the sites first .. first + n - 1: site_features() with
+// the disregistry as fixed-point phases (csr_site_phases) and FP32 pairs. This
+// GPU's FP64 pipe gives a warp instruction per 16 cycles and SM: the disregistry
+// in FP64 (60 instructions a site, 134 us per 1M sites) and twelve FP64 sines and
+// cosines with rows padded to 64 columns in memory (680 us) took twice the time
+// of the network; like this the pass is bound by its 48 bytes a site.
+__global__ void __launch_bounds__(256) k_site_rows(int64_t n, int64_t first, const SitePhase ph0, const SitePhase ph1,
+                                                   const int32_t* __restrict__ grid4, float twist_deg,
+                                                   __nv_bfloat16* __restrict__ X) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+    const int4 g = __ldg(reinterpret_cast<const int4*>(grid4) + first + r);  // i, j, orbital, sheet
+    const SitePhase& ph = g.w == 0 ? ph0 : ph1;
+    Pair c[2], s[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d)
+      phase_cos_sin(ph.c[d] + ph.mi[d] * (uint64_t)(int64_t)g.x + ph.mj[d] * (uint64_t)(int64_t)g.y, c[d], s[d]);
+    const Pair cc = pair_mul(c[0], c[1]), ss = pair_mul(s[0], s[1]);
+    const Pair sc = pair_mul(s[0], c[1]), cs = pair_mul(c[0], s[1]);
+    float f[kFeat];
+    f[0] = c[0].h;
+    f[1] = s[0].h;
+    f[2] = c[1].h;
+    f[3] = s[1].h;
+    f[4] = pair_sum(cc, pair_neg(ss));
+    f[5] = pair_sum(sc, cs);
+    f[6] = pair_sum(cc, ss);
+    f[7] = pair_sum(sc, pair_neg(cs));
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      const Pair p = pair_mul(c[d], s[d]);
+      f[8 + 2 * d] = pair_sum(pair_mul(c[d], c[d]), pair_neg(pair_mul(s[d], s[d])));
+      f[9 + 2 * d] = pair_sum(p, p);
+    }
+    f[12] = twist_deg / 3.0f;
+    f[13] = (float)g.w;
+    f[14] = (float)g.z;
+    f[15] = 1.0f;
+    uint32_t w[kFeat / 2];
+#pragma unroll
+    for (int k = 0; k < kFeat / 2; ++k) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+      w[k] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    uint4* dst = reinterpret_cast<uint4*>(X + r * kFeat);
+    dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
 // Site features from the disregistry (Hstruct::getShiftConfigs), twist,
 // layer and sublattice; 16 used columns of 64.
 __device__ __forceinline__ void site_features(double d0, double d1, float twist_deg, int layer, int sub,
@@ -66,18 +177,12 @@ __device__ __forceinline__ void site_features(double d0, double d1, float twist_
   f[15] = 1.0f;
 }
 
-__global__ void k_features(int64_t n, int64_t first, const double* __restrict__ cfg,
-                           const int32_t* __restrict__ grid4, float twist_deg, __nv_bfloat16* __restrict__ X,
-                           float* __restrict__ Xf) {
+__global__ void k_features(int64_t n, const double* __restrict__ cfg,
+                           const int32_t* __restrict__ grid4, float twist_deg, float* __restrict__ Xf) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = first + r;
     float f[kFeat];
-    site_features(cfg[2 * k], cfg[2 * k + 1], twist_deg, grid4[4 * k + 3], grid4[4 * k + 2], f);
-    for (int c = 0; c < kIn; ++c) {
-      const float v = c < kFeat ? f[c] : 0.0f;
-      if (X) X[r * kIn + c] = __float2bfloat16_rn(v);
-      if (Xf && c < kFeat) Xf[r * kFeat + c] = v;
-    }
+    site_features(cfg[2 * r], cfg[2 * r + 1], twist_deg, grid4[4 * r + 3], grid4[4 * r + 2], f);
+    for (int c = 0; c < kFeat; ++c) Xf[r * kFeat + c] = f[c];
   }
 }
 
@@ -420,29 +525,30 @@ void upload_x(leo2d_mlp* M, const float* x, int64_t n, int F) {
   ctx_sync(ctx);
 }
 
-// Forward of `n` rows whose BF16 features sit in X (row-major [n][64]): either
-// Y [n][256] FP32, or the column sums (FP64). By default one fused launch keeps
+// Forward of `n` rows whose BF16 features sit in X (row-major [n][ldx], ldx = 64
+// or 16: the TMA boxes are 64 columns wide either way and fill the columns beyond
+// the tensor with zeros): either Y [n][256] FP32, or the column sums (FP64) with
+// `part` as work space (mlp_fused_part, or a grid of tc_gemm blocks x 256). Only enqueues the fused form. By default one fused launch keeps
 // every activation on chip (mlp_fused.cu); option mlp_fused = 0 runs one GEMM
 // per layer over chunks of kChunk rows, with the activations in HBM.
-void infer_rows(leo2d_mlp* M, const __nv_bfloat16* X, int64_t n, float* Y, double* sums_dev) {
+void infer_rows(leo2d_mlp* M, const __nv_bfloat16* X, int ldx, int64_t n, float* Y, double* sums_dev, double* part,
+                bool accumulate) {
   leo2d_ctx* ctx = M->ctx;
   if (ctx->mlp_fused) {
     CUtensorMap tx;
-    make_tmap_bf16(&tx, X, n, kIn, kGemmBM);
+    make_tmap_bf16(&tx, X, n, ldx, kGemmBM);
     const float* bias[kLayers];
     for (int l = 0; l < kLayers; ++l) bias[l] = M->p.p + M->b_off[l];
-    mlp_forward_fused(ctx, tx, M->tWt, bias, n, Y, sums_dev);
+    mlp_forward_fused(ctx, tx, M->tWt, bias, n, Y, sums_dev, part, accumulate);
     return;
   }
   const int64_t chunk = std::min<int64_t>(kChunk, n);
   DevBuf<__nv_bfloat16> h0((size_t)chunk * kHid), h1((size_t)chunk * kHid);
-  const int grid = tc_gemm_grid(ctx, (int)chunk, kOut);
-  DevBuf<double> part((size_t)grid * kOut);
-  bool first = true;
+  bool first = !accumulate;
   for (int64_t r0 = 0; r0 < n; r0 += chunk) {
     const int rows = (int)std::min<int64_t>(chunk, n - r0);
     CUtensorMap tx, th0, th1;
-    make_tmap_bf16(&tx, X + r0 * kIn, rows, kIn, kGemmBM);
+    make_tmap_bf16(&tx, X + r0 * ldx, rows, ldx, kGemmBM);
     make_tmap_bf16(&th0, h0.p, rows, kHid, kGemmBM);
     make_tmap_bf16(&th1, h1.p, rows, kHid, kGemmBM);
     const CUtensorMap* in_map[kLayers] = {&tx, &th0, &th1, &th0};
@@ -461,11 +567,11 @@ void infer_rows(leo2d_mlp* M, const __nv_bfloat16* X, int64_t n, float* Y, doubl
         g.out_f32 = Y + r0 * kOut;
         tc_gemm(ctx, kEpiBias, *in_map[l], M->tWt[l], g);
       } else {
-        g.colsum = part.p;
+        g.colsum = part;
         const int gr = tc_gemm_grid(ctx, rows, kOut);
         tc_gemm(ctx, kEpiBias, *in_map[l], M->tWt[l], g);
         launch(ctx, "mlp_sum", [&] {
-          k_sum_partials<<<1, kOut, 0, ctx->stream>>>(part.p, gr, sums_dev, first ? 0 : 1);
+          k_sum_partials<<<1, kOut, 0, ctx->stream>>>(part, gr, sums_dev, first ? 0 : 1);
         });
       }
     }
@@ -667,7 +773,7 @@ leo2d_status leo2d_mlp_predict(leo2d_mlp* M, const float* x, int32_t F, int64_t 
     launch(ctx, "mlp_pack", [&] {
       k_pack_x<<<grid_for(n * kIn, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(n, F, src.p, X.p, nullptr, 0);
     });
-    infer_rows(M, X.p, n, Y.p, nullptr);
+    infer_rows(M, X.p, kIn, n, Y.p, nullptr, nullptr, false);
     d2h(ctx, y, Y.p, (size_t)n * kOut);
     ctx_check_status(ctx, "MLP inference");
   });
@@ -683,8 +789,8 @@ leo2d_status leo2d_mlp_site_features(leo2d_ctx* ctx, const leo2d_csr* csr, doubl
     DevBuf<float> xf((size_t)std::max<int64_t>(n, 1) * kFeat);
     if (n > 0)
       launch(ctx, "mlp_features", [&] {
-        k_features<<<grid_for(n, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(n, 0, cfg.p, csr->grid4.p,
-                                                                                 (float)twist_deg, nullptr, xf.p);
+        k_features<<<grid_for(n, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(n, cfg.p, csr->grid4.p,
+                                                                                 (float)twist_deg, xf.p);
       });
     d2h(ctx, x_out, xf.p, (size_t)n * kFeat);
     ctx_sync(ctx);
@@ -698,15 +804,30 @@ leo2d_status leo2d_mlp_site_sum(leo2d_mlp* M, const leo2d_csr* csr, double twist
     LEO_CUDA(cudaSetDevice(ctx->device));
     const int64_t n = csr->n;
     LEO_REQUIRE(n >= 1, "empty matrix");
-    DevBuf<double> cfg(2 * (size_t)n), sums(kOut);
-    csr_shift_configs(ctx, csr, cfg.p);
-    DevBuf<__nv_bfloat16> X((size_t)n * kIn);
-    launch(ctx, "mlp_features", [&] {
-      k_features<<<grid_for(n, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(n, 0, cfg.p, csr->grid4.p,
-                                                                               (float)twist_deg, X.p, nullptr);
-    });
-    infer_rows(M, X.p, n, nullptr, sums.p);
-    d2h(ctx, sum_out, sums.p, kOut);
+    SitePhase ph[2];
+    csr_site_phases(csr, ph);
+    // Work space from the context: features of one chunk of sites (32 bytes each),
+    // the kernel's partial sums, the sums. A chunk is a whole number of tile pairs
+    // for every SM, at most 2M sites, so that all of it stays within what the
+    // context keeps (64 MiB); the 160 MB that 1M sites took before cost 0.36 ms a
+    // call in four allocations.
+    const int64_t wave = (int64_t)ctx->sm_count * 2 * kGemmBM;
+    const int64_t chunk = std::min<int64_t>(n, std::max<int64_t>(1, (2000000 / wave)) * wave);
+    const size_t part_n = std::max(mlp_fused_part(ctx), (size_t)tc_gemm_grid(ctx, (int)chunk, kOut) * kOut);
+    const size_t xw = ((size_t)chunk * kFeat * sizeof(__nv_bfloat16) + 255) / 256 * 256;
+    char* ws = ctx_scratch<char>(ctx, xw + (part_n + kOut) * sizeof(double));
+    __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(ws);
+    double* part = reinterpret_cast<double*>(ws + xw);
+    double* sums = part + part_n;
+    for (int64_t r0 = 0; r0 < n; r0 += chunk) {
+      const int64_t rows = std::min(chunk, n - r0);
+      launch(ctx, "mlp_features", [&] {
+        k_site_rows<<<grid_for(rows, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
+            rows, r0, ph[0], ph[1], csr->grid4.p, (float)twist_deg, X);
+      });
+      infer_rows(M, X, kFeat, rows, nullptr, sums, part, r0 > 0);
+    }
+    d2h(ctx, sum_out, sums, kOut);
     ctx_check_status(ctx, "MLP site sum");
   });
 }
@@ -762,7 +883,7 @@ leo2d_status leo2d_kpm_dos_cv(leo2d_ctx* ctx, const leo2d_csr* csr, leo2d_mlp* M
         k_features_at<<<grid_for(num_sites, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
             num_sites, drows.p, dcfg.p, csr->grid4.p, (float)twist_deg, X.p);
       });
-      infer_rows(M, X.p, num_sites, Y.p, nullptr);
+      infer_rows(M, X.p, kIn, num_sites, Y.p, nullptr, nullptr, false);
       std::vector<float> f((size_t)num_sites * kOut);
       d2h(ctx, f.data(), Y.p, f.size());
       ctx_check_status(ctx, "control-variate sites");

@@ -345,23 +345,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
   if (warp == kMmaWarp) umma::tmem_dealloc(tmem, 2 * kWidth);
 }
 
-// sums[c] = sum over the partial rows of part[.][c], in a fixed order.
+// sums[c] (+)= sum over the partial rows of part[.][c], in a fixed order. Each
+// block takes 8 columns (a 64-byte segment of every row) and 32 groups of rows:
+// one block with a thread per column walked its 608 rows in one dependent chain
+// (47 us of latency; this split 4 us).
 __global__ void __launch_bounds__(256) k_fused_site_sums(const double* __restrict__ part, int rows,
-                                                         double* __restrict__ sums) {
-  const int c = threadIdx.x;
+                                                         double* __restrict__ sums, int accumulate) {
+  __shared__ double sh[32][8];
+  const int j = threadIdx.x & 7, g = threadIdx.x >> 3, c = blockIdx.x * 8 + j;
   double s = 0.0;
-  for (int i = 0; i < rows; ++i) s += part[(size_t)i * kWidth + c];
-  sums[c] = s;
+#pragma unroll 4
+  for (int i = g; i < rows; i += 32) s += part[(size_t)i * kWidth + c];
+  sh[g][j] = s;
+  __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) {
+    if (g < o) sh[g][j] += sh[g + o][j];
+    __syncthreads();
+  }
+  if (g == 0) sums[c] = accumulate ? sums[c] + sh[0][j] : sh[0][j];
 }
 
 }  // namespace
 
 namespace leo2d {
 
+size_t mlp_fused_part(const leo2d_ctx* ctx) { return (size_t)ctx->sm_count * 4 * kWidth; }
+
 void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap* tw, const float* const* bias,
-                       int64_t n, float* Y, double* sums_dev) {
+                       int64_t n, float* Y, double* sums_dev, double* part, bool accumulate) {
   LEO_REQUIRE(n >= 1 && n < (int64_t(1) << 31), "fused MLP forward: n must be 1 .. 2^31 - 1");
-  LEO_REQUIRE(Y || sums_dev, "fused MLP forward: no output");
+  LEO_REQUIRE(Y || (sums_dev && part), "fused MLP forward: no output");
   LEO_REQUIRE(kSmemBytes <= ctx->smem_optin, "fused MLP forward: shared memory per block too small");
   LEO_CUDA(cudaFuncSetAttribute(k_mlp_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
   FusedArgs a{};
@@ -375,13 +388,11 @@ void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap*
   a.y = Y;
   a.status = ctx->status.p;
   const int grid = (int)std::min<int64_t>(ctx->sm_count, (a.tiles + 1) / 2);
-  DevBuf<double> part(Y ? 0 : (size_t)grid * 4 * kWidth);
-  a.part = part.p;
+  a.part = part;
   launch(ctx, "mlp_fused", [&] { k_mlp_fused<<<grid, kThreads, kSmemBytes, ctx->stream>>>(a); });
   if (!Y)
     launch(ctx, "mlp_fused_sums",
-           [&] { k_fused_site_sums<<<1, kWidth, 0, ctx->stream>>>(part.p, grid * 4, sums_dev); });
-  ctx_sync(ctx);  // the partials are freed on return
+           [&] { k_fused_site_sums<<<kWidth / 8, 256, 0, ctx->stream>>>(part, grid * 4, sums_dev, accumulate); });
 }
 
 }  // namespace leo2d

@@ -176,9 +176,11 @@ __device__ __forceinline__ void mlp_gelu2(float& a, float& b) {
 // activation kept on chip (mlp_fused.cu). tx: TMA map of the BF16 features
 // [n][64] (boxes of 64 columns x 128 rows, 128-byte swizzle); tw[l]: TMA maps of
 // the BF16 weights W_l [256][in_l] (boxes of 64 x 256); bias[l]: FP32 [256].
-// Writes Y (FP32 [n][256]) or, with Y null, sums_dev[256] = the FP64 column
-// sums of the outputs over the n rows (overwritten). n < 2^31.
+// Writes Y (FP32 [n][256]) or, with Y null, sums_dev[256] (+)= the FP64 column
+// sums of the outputs over the n rows (added to with `accumulate`); `part` is then
+// work space of mlp_fused_part(ctx) doubles. n < 2^31. Only enqueues.
+size_t mlp_fused_part(const leo2d_ctx* ctx);
 void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap* tw, const float* const* bias,
-                       int64_t n, float* Y, double* sums_dev);
+                       int64_t n, float* Y, double* sums_dev, double* part, bool accumulate);
 
 }  // namespace leo2d
