@@ -19,18 +19,26 @@
 //                   frees weight stages, hands the accumulator to the epilogue
 //                   and, after the last layer, frees the activation buffer;
 //   warps 0..15     epilogue: warp w reads TMEM lanes 32 (w & 3) .. + 31 (one
-//                   site each), columns 64 (w >> 2) .. + 63, in chunks of 32
-//                   (tcgen05.ld.32x32b.x32). Hidden layers: + bias, GELU, BF16,
+//                   site each), columns 64 (w >> 2) .. + 63, in chunks of 16
+//                   (tcgen05.ld.32x32b.x16: chunks of 32 left the compiler
+//                   too few of the 96 registers to overlap the GELUs). Hidden layers: + bias, GELU, BF16,
 //                   stored into the slot's activation buffer in the K-major
 //                   128-byte-swizzled layout the next MMA reads (the layout TMA
 //                   writes). Last layer: + bias, then either the FP32 outputs
-//                   to HBM or, for the site sum, a warp transpose-reduce of
-//                   each 32 x 32 chunk (lane j ends with column j's sum over
-//                   the warp's sites) added into per-lane partials (FP32 over
-//                   8 tile pairs, then FP64).
+//                   to HBM or, for the site sum, column sums: read in the
+//                   16x256b shape, where a lane holds 4 rows of 16 columns, so
+//                   that they add up in registers (no shuffles; the bias enters
+//                   once, times the sites).
 // Order of work: (slot 0, layer 0), (slot 1, layer 0), (slot 0, layer 1), ...
 // for each pair of tiles; the MMA and the epilogue both walk it, so the MMA
 // of (slot s, layer l) waits only for the epilogue of (s, l - 1).
+// What bounds it: the GELU's packed FP32 work. A pair of activations takes 20 issue
+// slots and 22 cycles of the FMA pipe, 2,816 cycles a tile and layer, against 2,048
+// of the tensor pipe; the rest of a pair's time is the hand-over between the two.
+// Sums over 1M sites: 470 us with a transpose-reduce by 31 shuffles per 32 x 32
+// block in the last layer, 444 us with the 16x256b read, 422 us with chunks of 16
+// (with the next chunk's read in flight 429; column sums through shared memory,
+// which the MMAs' operands need, 499; 104 registers by setmaxnreg 558).
 // Shared memory: 2 x 64 KB activation buffers + 3 x 32 KB weight stages.
 // Every mbarrier wait gives up after two seconds, records a timeout in the
 // status word and lets the block drain its copies and MMAs, free its TMEM and
@@ -69,27 +77,9 @@ struct FusedArgs {
   int64_t n;             // sites
   int64_t tiles;         // ceil(n / 128)
   float* y;              // [n][256] FP32 outputs, or null
-  double* part;          // y null: [grid][4][256] FP64 column sums of the block's sites
+  double* part;          // y null: [grid][4][256] FP64 column sums of the block's sites, without the bias
   int* status;
 };
-
-// 32 consecutive FP32 columns of this thread's TMEM lane (32x32b shape), with
-// the wait in the same statement so no use of the registers can move above it.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);  // lo at the lower address
@@ -110,20 +100,22 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
-// v[0..31] of every lane -> lane j returns sum over the warp's lanes of v[j]
-// (five halving exchange steps, 31 shuffles).
-__device__ __forceinline__ float warp_transpose_sum(float* v, int lane) {
+// Eight 8-column blocks of 16 TMEM lanes (16x256b shape): register 4 b + 2 e + c of
+// lane t is row t / 4 + 8 e, column 8 b + 2 (t % 4) + c.
+__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, float* v) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
 #pragma unroll
-  for (int w = 16; w >= 1; w >>= 1) {
-    const bool up = (lane & w) != 0;
-#pragma unroll
-    for (int i = 0; i < w; ++i) {
-      const float send = up ? v[i] : v[i + w];
-      const float keep = up ? v[i + w] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
-    }
-  }
-  return v[0];
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant__ FusedArgs a) {
@@ -253,14 +245,33 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
     // epilogue: site r = 32 q + lane of the tile, columns kEpiCols h .. + kEpiCols - 1
     const int q = warp & 3, h = warp >> 2, r = q * 32 + lane;
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    // site sums: FP32 over 8 tile pairs, then FP64 (the FP64 pipe is narrow)
-    double csum[kEpiCols / 32];
-    float fsum[kEpiCols / 32];
+    // site sums: acc[2 b + c] is column 8 b + 2 (lane % 4) + c of the warp's 64 over
+    // rows lane / 4 + 8 e, FP32 over four tile pairs (32 rows). A flush adds them up
+    // over the eight lanes of a column by halving exchanges, which leaves lane t the
+    // columns 8 (t / 4) + 2 (t % 4) + c, in FP32 pairs (the FP64 pipe is narrow)
+    constexpr int kAcc = kEpiCols / 4;
+    float acc[kAcc], sum_h[2] = {0.f, 0.f}, sum_l[2] = {0.f, 0.f};
 #pragma unroll
-    for (int ci = 0; ci < kEpiCols / 32; ++ci) {
-      csum[ci] = 0.0;
-      fsum[ci] = 0.f;
-    }
+    for (int k = 0; k < kAcc; ++k) acc[k] = 0.f;
+    auto flush = [&]() {
+#pragma unroll
+      for (int w = kAcc / 2; w >= 2; w >>= 1) {
+        const bool up = (lane & (2 * w)) != 0;
+#pragma unroll
+        for (int k = 0; k < w; ++k) {
+          const float send = up ? acc[k] : acc[k + w], keep = up ? acc[k + w] : acc[k];
+          acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * w);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float t = __fadd_rn(sum_h[k], acc[k]), d = __fsub_rn(t, sum_h[k]);
+        sum_l[k] += __fadd_rn(__fsub_rn(sum_h[k], __fsub_rn(t, d)), __fsub_rn(acc[k], d));
+        sum_h[k] = t;
+      }
+#pragma unroll
+      for (int k = 0; k < kAcc; ++k) acc[k] = 0.f;
+    };
     // byte offset of K column k (multiple of 8) of this site in an activation buffer
     auto a_off = [&](int k) -> uint32_t {
       return (uint32_t)(k >> 6) * kAKBlock + (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u +
@@ -282,38 +293,52 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
           const uint32_t tacc = tmem + (uint32_t)(s * kWidth) + lane_off;
           const float* bl = a.bias[l];
           const uint32_t ab = umma::saddr(abuf + s * kABytes);
+          if (!a.y && l == 3) {
+            // whole rows of every column are wanted, not whole columns of a row: the
+            // TMEM shape that gives a lane few columns of several rows
 #pragma unroll
-          for (int ci = 0; ci < kEpiCols / 32; ++ci) {
-            const int c0 = h * kEpiCols + ci * 32;
-            float v[32];
-            tmem_ld32(tacc + (uint32_t)c0, v);
+            for (int e = 0; e < 2; ++e) {
+              float v[32];
+              tmem_ld_16x64(tacc + ((uint32_t)(16 * e) << 16) + (uint32_t)(h * kEpiCols), v);
+              if ((t + 1) * kRows > a.n) {  // the tile of the last site, and padding tiles
+                const int64_t row = t * kRows + q * 32 + 16 * e + (lane >> 2);
+                const bool ok0 = t < a.tiles && row < a.n, ok1 = t < a.tiles && row + 8 < a.n;
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 b = __ldg(reinterpret_cast<const float4*>(bl + c0 + i));
-              add2(v[i], v[i + 1], b.x, b.y);
-              add2(v[i + 2], v[i + 3], b.z, b.w);
-            }
-            if (l < 3) {
-              uint32_t pk[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                mlp_gelu2(v[2 * i], v[2 * i + 1]);
-                pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+                for (int i = 0; i < 32; ++i) v[i] = ((i & 2) ? ok1 : ok0) ? v[i] : 0.f;
               }
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                st_shared_v4(ab + a_off(c0 + 8 * i), pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
-            } else if (a.y) {
-              if (valid) {
+              for (int b = 0; b < kAcc / 2; ++b) {
+                add2(acc[2 * b], acc[2 * b + 1], v[4 * b], v[4 * b + 1]);
+                add2(acc[2 * b], acc[2 * b + 1], v[4 * b + 2], v[4 * b + 3]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int ci = 0; ci < kEpiCols / 16; ++ci) {
+              const int c0 = h * kEpiCols + ci * 16;
+              float v[16];
+              umma::tmem_ld16(tacc + (uint32_t)c0, v);
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                const float4 b = __ldg(reinterpret_cast<const float4*>(bl + c0 + i));
+                add2(v[i], v[i + 1], b.x, b.y);
+                add2(v[i + 2], v[i + 3], b.z, b.w);
+              }
+              if (l < 3) {
+                uint32_t pk[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  mlp_gelu2(v[2 * i], v[2 * i + 1]);
+                  pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                  st_shared_v4(ab + a_off(c0 + 8 * i), pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+              } else if (valid) {
                 float4* dst = reinterpret_cast<float4*>(a.y + site * kWidth + c0);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
               }
-            } else {
-              if (!valid)
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = 0.f;
-              fsum[ci] += warp_transpose_sum(v, lane);
             }
           }
           umma::fence_before_sync();
@@ -325,18 +350,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
         give_up();
         break;
       }
-      if ((it & 7) == 7) {
-#pragma unroll
-        for (int ci = 0; ci < kEpiCols / 32; ++ci) {
-          csum[ci] += (double)fsum[ci];
-          fsum[ci] = 0.f;
-        }
-      }
+      if (!a.y && (it & 3) == 3) flush();
     }
     if (!a.y) {
+      flush();
 #pragma unroll
-      for (int ci = 0; ci < kEpiCols / 32; ++ci)
-        a.part[((size_t)bid * 4 + q) * kWidth + h * kEpiCols + ci * 32 + lane] = csum[ci] + (double)fsum[ci];
+      for (int k = 0; k < 2; ++k)
+        a.part[((size_t)bid * 4 + q) * kWidth + h * kEpiCols + 8 * (lane >> 2) + 2 * (lane & 3) + k] =
+            (double)sum_h[k] + (double)sum_l[k];
     }
   }
   umma::fence_before_sync();
@@ -345,11 +366,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
   if (warp == kMmaWarp) umma::tmem_dealloc(tmem, 2 * kWidth);
 }
 
-// sums[c] (+)= sum over the partial rows of part[.][c], in a fixed order. Each
+// sums[c] (+)= n bias[c] + the sum over the partial rows of part[.][c], in a fixed order. Each
 // block takes 8 columns (a 64-byte segment of every row) and 32 groups of rows:
 // one block with a thread per column walked its 608 rows in one dependent chain
 // (47 us of latency; this split 4 us).
 __global__ void __launch_bounds__(256) k_fused_site_sums(const double* __restrict__ part, int rows,
+                                                         const float* __restrict__ bias, double n,
                                                          double* __restrict__ sums, int accumulate) {
   __shared__ double sh[32][8];
   const int j = threadIdx.x & 7, g = threadIdx.x >> 3, c = blockIdx.x * 8 + j;
@@ -362,7 +384,10 @@ __global__ void __launch_bounds__(256) k_fused_site_sums(const double* __restric
     if (g < o) sh[g][j] += sh[g + o][j];
     __syncthreads();
   }
-  if (g == 0) sums[c] = accumulate ? sums[c] + sh[0][j] : sh[0][j];
+  if (g == 0) {
+    const double t = sh[0][j] + n * (double)bias[c];
+    sums[c] = accumulate ? sums[c] + t : t;
+  }
 }
 
 }  // namespace
@@ -392,7 +417,8 @@ void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap*
   launch(ctx, "mlp_fused", [&] { k_mlp_fused<<<grid, kThreads, kSmemBytes, ctx->stream>>>(a); });
   if (!Y)
     launch(ctx, "mlp_fused_sums",
-           [&] { k_fused_site_sums<<<kWidth / 8, 256, 0, ctx->stream>>>(part, grid * 4, sums_dev, accumulate); });
+           [&] { k_fused_site_sums<<<kWidth / 8, 256, 0, ctx->stream>>>(part, grid * 4, bias[3], (double)n, sums_dev,
+                                                                     accumulate); });
 }
 
 }  // namespace leo2d
