@@ -231,45 +231,82 @@ __global__ void k_gather(int64_t n_train, int B, const __nv_bfloat16* __restrict
 }
 
 // dY = (2/n) w (Y - T) -> BF16 [n][256], its transpose, FP32; per-block loss sums.
-__global__ void __launch_bounds__(256) k_loss(int n, const float* __restrict__ Y, const float* __restrict__ T,
+// A block takes 32 rows; a thread 4 columns of 8 rows. The transpose goes through
+// shared memory: 2-byte stores a row length apart and six FP64 instructions an
+// element for the loss took 28 us at 8192 rows (10 now). w d^2 is summed as an
+// exact product in FP32 pairs (2^-45 relative), a thread's 32 terms, then in FP64.
+constexpr int kLossRows = 32;
+__global__ void __launch_bounds__(512) k_loss(int n, const float* __restrict__ Y, const float* __restrict__ T,
                                               const float* __restrict__ w, __nv_bfloat16* __restrict__ dZ,
                                               __nv_bfloat16* __restrict__ dZt, int64_t ldt, float* __restrict__ dZ32,
                                               double* __restrict__ part) {
-  __shared__ double red[256];
-  double acc = 0.0;
-  const int64_t total = (int64_t)n * kOut;
+  __shared__ __nv_bfloat16 tile[kOut][kLossRows + 2];
+  __shared__ double red[16];
+  const int j = 4 * (threadIdx.x & 63), g8 = threadIdx.x >> 6;
+  const int r0 = blockIdx.x * kLossRows;
   const float scale = 2.0f / (float)n;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(e / kOut), j = (int)(e % kOut);
-    const float d = Y[e] - T[e];
-    const float g = scale * w[j] * d;
-    acc += (double)w[j] * (double)d * (double)d;
-    dZ32[e] = g;
-    const __nv_bfloat16 b = __float2bfloat16_rn(g);
-    dZ[e] = b;
-    dZt[(int64_t)j * ldt + r] = b;
+  const float4 w4 = *reinterpret_cast<const float4*>(w + j);
+  const float wj[4] = {w4.x, w4.y, w4.z, w4.w};
+  float sh = 0.f, sl = 0.f;
+#pragma unroll
+  for (int i = 0; i < kLossRows / 8; ++i) {
+    const int rr = g8 + 8 * i;
+    if (r0 + rr >= n) break;
+    const size_t e = (size_t)(r0 + rr) * kOut + j;
+    const float4 y4 = *reinterpret_cast<const float4*>(Y + e), t4 = *reinterpret_cast<const float4*>(T + e);
+    const float d[4] = {y4.x - t4.x, y4.y - t4.y, y4.z - t4.z, y4.w - t4.w};
+    float gr[4];
+    __nv_bfloat16 b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      gr[k] = scale * wj[k] * d[k];
+      b[k] = __float2bfloat16_rn(gr[k]);
+      tile[j + k][rr] = b[k];
+      const Pair q = pair_mul({wj[k], 0.f}, pair_mul({d[k], 0.f}, {d[k], 0.f}));
+      const float s = __fadd_rn(sh, q.h), v = __fsub_rn(s, sh);  // two-sum
+      sl = __fadd_rn(sl, __fadd_rn(q.l, __fadd_rn(__fsub_rn(sh, __fsub_rn(s, v)), __fsub_rn(q.h, v))));
+      sh = s;
+    }
+    *reinterpret_cast<float4*>(dZ32 + e) = make_float4(gr[0], gr[1], gr[2], gr[3]);
+    *reinterpret_cast<uint2*>(dZ + e) = *reinterpret_cast<const uint2*>(b);
   }
-  red[threadIdx.x] = acc;
+  double acc = (double)sh + (double)sl;
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  for (int e = threadIdx.x; e < kOut * kLossRows; e += blockDim.x) {
+    const int c = e / kLossRows, r = e % kLossRows;
+    if (r0 + r < n) dZt[(size_t)c * ldt + r0 + r] = tile[c][r];
+  }
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int k = 0; k < 16; ++k) s += red[k];
+    part[blockIdx.x] = s;
+  }
+}
+
+// The mean of the block sums, 256 strided chains and a tree (one thread's chain of
+// 1024 loads took 51 us).
+__global__ void __launch_bounds__(256) k_loss_final(const double* __restrict__ part, int nb, int n,
+                                                    const int64_t* __restrict__ step, double* __restrict__ hist,
+                                                    int64_t hist_cap, double* __restrict__ last) {
+  __shared__ double red[256];
+  double s = 0.0;
+  for (int b = threadIdx.x; b < nb; b += 256) s += part[b];
+  red[threadIdx.x] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-__global__ void k_loss_final(const double* __restrict__ part, int nb, int n, const int64_t* __restrict__ step,
-                             double* __restrict__ hist, int64_t hist_cap, double* __restrict__ last) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int b = 0; b < nb; ++b) s += part[b];
-  s /= (double)n;
+  if (threadIdx.x != 0) return;
+  s = red[0] / (double)n;
   *last = s;
   const int64_t t = step ? *step : 0;
   if (hist && t < hist_cap) hist[t] = s;
 }
 
-// Column sums of x [n][256] (FP32) in two fixed-order passes.
+// Column sums of x [n][256] (FP32) over blocks of rows, in a fixed order.
 __global__ void __launch_bounds__(256) k_colsum_part(int n, int rows_per_block, const float* __restrict__ x,
                                                      float* __restrict__ part) {
   const int j = threadIdx.x;
@@ -278,11 +315,31 @@ __global__ void __launch_bounds__(256) k_colsum_part(int n, int rows_per_block, 
   for (int r = r0; r < r1; ++r) s += x[(int64_t)r * kOut + j];
   part[(int64_t)blockIdx.x * kOut + j] = s;
 }
-__global__ void __launch_bounds__(256) k_colsum_final(const float* __restrict__ part, int nb, float* __restrict__ out) {
-  const int j = threadIdx.x;
-  float s = 0.0f;
-  for (int b = 0; b < nb; ++b) s += part[(int64_t)b * kOut + j];
-  out[j] = s;
+
+// The last additions of every layer in one launch: dW_l = sum of its K-range splits,
+// db_l = sum of its column-sum blocks (fixed orders; as two launches a layer these
+// took 30 us of a gradient at 8192 rows, together 13).
+struct GradParts {
+  const float* dw[kLayers];  // [splits][256 in]
+  const float* cs[kLayers];  // [blocks][256]
+  int64_t w_off[kLayers], b_off[kLayers];
+  int splits, blocks;
+};
+__global__ void __launch_bounds__(256) k_grad_final(const GradParts a, float* __restrict__ g) {
+  const int l = blockIdx.y;
+  const int64_t nw = (int64_t)kHid * (l == 0 ? kIn : kHid);
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (blockIdx.x == gridDim.x - 1) {
+    float s = 0.0f;
+#pragma unroll 8
+    for (int b = 0; b < a.blocks; ++b) s += a.cs[l][(int64_t)b * kOut + threadIdx.x];
+    g[a.b_off[l] + threadIdx.x] = s;
+  } else if (e < nw) {
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < a.splits; ++k) s += a.dw[l][(size_t)k * nw + e];
+    g[a.w_off[l] + e] = s;
+  }
 }
 
 __global__ void k_adam(int64_t np, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -342,9 +399,10 @@ struct leo2d_mlp {
   // training workspace (batch B)
   int B = 0;
   DevBuf<__nv_bfloat16> Xb, Xbt, A[kLayers], At[kLayers], dZ[2], dZt[2];
-  DevBuf<float> Tb, Z[kLayers], Y, dZ32[2], cs_part, dw_split;
+  DevBuf<float> Tb, Z[kLayers], Y, dZ32[2], cs_part[kLayers], dw_split[kLayers];
   DevBuf<double> loss_part, loss_last, loss_hist;
   int64_t hist_cap = 0;
+  CUtensorMap tWf[kLayers];  // boxes of 256 rows, for the fused forward
   CUtensorMap tX, tA[kLayers], tWt[kLayers], tWn[kLayers], tXt, tAt[kLayers], tdZ[2], tdZt[2];
   // training set
   int64_t n_train = 0;
@@ -371,6 +429,9 @@ void refresh_bf16(leo2d_mlp* M) {
   }
 }
 
+// K-range splits of the weight-gradient products of n rows
+int dw_splits(int n) { return std::max(1, std::min(kDwSplits, n / 256)); }
+
 void ensure_batch(leo2d_mlp* M, int B) {
   if (M->B == B) return;
   LEO_REQUIRE(B >= 64 && B % 64 == 0 && B <= (1 << 20), "batch must be a multiple of 64 in [64, 2^20]");
@@ -395,16 +456,17 @@ void ensure_batch(leo2d_mlp* M, int B) {
     M->dZt[i].alloc((size_t)kHid * B);
     M->dZ32[i].alloc((size_t)B * kHid);
   }
-  M->dw_split.alloc((size_t)kDwSplits * kHid * kHid);
-  const int cs_blocks = (B + 63) / 64;
-  M->cs_part.alloc((size_t)cs_blocks * kOut);
-  M->loss_part.alloc(1024);
+  for (int l = 0; l < kLayers; ++l) {
+    M->dw_split[l].alloc((size_t)dw_splits(B) * kHid * kInDim[l]);
+    M->cs_part[l].alloc((size_t)((B + 63) / 64) * kOut);
+  }
+  M->loss_part.alloc((size_t)(B + kLossRows - 1) / kLossRows);
   M->loss_last.alloc(1);
   make_tmap_bf16(&M->tX, M->Xb.p, B, kIn, kGemmBM);
-  make_tmap_bf16(&M->tXt, M->Xbt.p, kIn, B, 256);
+  make_tmap_bf16(&M->tXt, M->Xbt.p, kIn, B, kGemmBoxB);
   for (int l = 1; l < kLayers; ++l) {
     make_tmap_bf16(&M->tA[l], M->A[l].p, B, kHid, kGemmBM);
-    make_tmap_bf16(&M->tAt[l], M->At[l].p, kHid, B, 256);
+    make_tmap_bf16(&M->tAt[l], M->At[l].p, kHid, B, kGemmBoxB);
   }
   for (int i = 0; i < 2; ++i) {
     make_tmap_bf16(&M->tdZ[i], M->dZ[i].p, B, kHid, kGemmBM);
@@ -440,24 +502,28 @@ void forward_train(leo2d_mlp* M, int n) {
 void backward_train(leo2d_mlp* M, int n) {
   leo2d_ctx* ctx = M->ctx;
   const int B = M->B;
-  const int lb = (int)std::min<int64_t>(1024, grid_for((int64_t)n * kOut, 256));
+  const int lb = (n + kLossRows - 1) / kLossRows;
   launch(ctx, "mlp_loss", [&] {
-    k_loss<<<lb, 256, 0, ctx->stream>>>(n, M->Y.p, M->Tb.p, M->lw.p, M->dZ[1].p, M->dZt[1].p, B, M->dZ32[1].p,
+    k_loss<<<lb, 512, 0, ctx->stream>>>(n, M->Y.p, M->Tb.p, M->lw.p, M->dZ[1].p, M->dZt[1].p, B, M->dZ32[1].p,
                                         M->loss_part.p);
   });
   launch(ctx, "mlp_loss", [&] {
-    k_loss_final<<<1, 32, 0, ctx->stream>>>(M->loss_part.p, lb, n, M->step.p, M->loss_hist.p, M->hist_cap,
-                                            M->loss_last.p);
+    k_loss_final<<<1, 256, 0, ctx->stream>>>(M->loss_part.p, lb, n, M->step.p, M->loss_hist.p, M->hist_cap,
+                                             M->loss_last.p);
   });
+  const int rpb = 64;
+  GradParts gp{};
+  gp.splits = dw_splits(n);
+  gp.blocks = (n + rpb - 1) / rpb;
   int cur = 1;  // dZ of layer l lives in buffer `cur`
   for (int l = kLayers - 1; l >= 0; --l) {
+    gp.dw[l] = M->dw_split[l].p;
+    gp.cs[l] = M->cs_part[l].p;
+    gp.w_off[l] = M->w_off[l];
+    gp.b_off[l] = M->b_off[l];
     // bias gradient
-    const int rpb = 64, nb = (n + rpb - 1) / rpb;
     launch(ctx, "mlp_colsum", [&] {
-      k_colsum_part<<<nb, 256, 0, ctx->stream>>>(n, rpb, M->dZ32[cur].p, M->cs_part.p);
-    });
-    launch(ctx, "mlp_colsum", [&] {
-      k_colsum_final<<<1, 256, 0, ctx->stream>>>(M->cs_part.p, nb, M->g.p + M->b_off[l]);
+      k_colsum_part<<<gp.blocks, 256, 0, ctx->stream>>>(n, rpb, M->dZ32[cur].p, M->cs_part[l].p);
     });
     // weight gradient dW_l [out][in] = dZ_l^T A_l
     {
@@ -465,11 +531,11 @@ void backward_train(leo2d_mlp* M, int n) {
       g.M = kHid;
       g.N = kInDim[l];
       g.K = n;
-      g.out_f32 = M->g.p + M->w_off[l];
+      g.out_f32 = M->dw_split[l].p;  // a single split writes its product here
       g.status = ctx->status.p;
       // K = n rows: split over up to 32 work items per output tile
-      g.k_splits = std::max(1, std::min(kDwSplits, n / 256));
-      g.split_buf = M->dw_split.p;
+      g.k_splits = gp.splits;
+      g.split_buf = M->dw_split[l].p;
       tc_gemm(ctx, kEpiF32, M->tdZt[cur], l == 0 ? M->tXt : M->tAt[l], g);
     }
     if (l == 0) break;
@@ -490,6 +556,9 @@ void backward_train(leo2d_mlp* M, int n) {
       cur = nxt;
     }
   }
+  launch(ctx, "mlp_grad_final", [&] {
+    k_grad_final<<<dim3(kHid * kHid / 256 + 1, kLayers), 256, 0, ctx->stream>>>(gp, M->g.p);
+  });
 }
 
 void adam_update(leo2d_mlp* M, float lr) {
@@ -516,13 +585,12 @@ void train_step_enqueue(leo2d_mlp* M, uint64_t seed, float lr) {
 
 void upload_x(leo2d_mlp* M, const float* x, int64_t n, int F) {
   leo2d_ctx* ctx = M->ctx;
-  DevBuf<float> src((size_t)n * F);
-  h2d(ctx, src.p, x, (size_t)n * F);
+  float* src = ctx_scratch<float>(ctx, (size_t)n * F);  // in stream order, free again after the call's next sync
+  h2d(ctx, src, x, (size_t)n * F);
   launch(ctx, "mlp_pack", [&] {
-    k_pack_x<<<grid_for(n * kIn, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(n, F, src.p, M->Xb.p, M->Xbt.p,
+    k_pack_x<<<grid_for(n * kIn, 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(n, F, src, M->Xb.p, M->Xbt.p,
                                                                                  M->B);
   });
-  ctx_sync(ctx);
 }
 
 // Forward of `n` rows whose BF16 features sit in X (row-major [n][ldx], ldx = 64
@@ -539,7 +607,7 @@ void infer_rows(leo2d_mlp* M, const __nv_bfloat16* X, int ldx, int64_t n, float*
     make_tmap_bf16(&tx, X, n, ldx, kGemmBM);
     const float* bias[kLayers];
     for (int l = 0; l < kLayers; ++l) bias[l] = M->p.p + M->b_off[l];
-    mlp_forward_fused(ctx, tx, M->tWt, bias, n, Y, sums_dev, part, accumulate);
+    mlp_forward_fused(ctx, tx, M->tWf, bias, n, Y, sums_dev, part, accumulate);
     return;
   }
   const int64_t chunk = std::min<int64_t>(kChunk, n);
@@ -633,10 +701,11 @@ leo2d_status leo2d_mlp_create(leo2d_ctx* ctx, uint64_t seed, leo2d_mlp** out) {
     LEO_CUDA(cudaMemsetAsync(M->step.p, 0, sizeof(int64_t), ctx->stream));
     for (int l = 0; l < kLayers; ++l) {
       M->wt[l].alloc((size_t)kHid * kInDim[l]);
-      make_tmap_bf16(&M->tWt[l], M->wt[l].p, kHid, kInDim[l], 256);
+      make_tmap_bf16(&M->tWf[l], M->wt[l].p, kHid, kInDim[l], 256);
+      make_tmap_bf16(&M->tWt[l], M->wt[l].p, kHid, kInDim[l], kGemmBoxB);
       if (l > 0) {
         M->wn[l].alloc((size_t)kInDim[l] * kHid);
-        make_tmap_bf16(&M->tWn[l], M->wn[l].p, kInDim[l], kHid, 256);
+        make_tmap_bf16(&M->tWn[l], M->wn[l].p, kInDim[l], kHid, kGemmBoxB);
       }
     }
     refresh_bf16(M.get());

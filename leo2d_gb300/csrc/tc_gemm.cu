@@ -10,23 +10,25 @@ using namespace leo2d;
 
 namespace {
 
-constexpr int BM = kGemmBM, BK = kGemmBK, ST = kGemmStages, BN = 256;
-constexpr uint32_t kABytes = BM * BK * 2, kBBytes = BN * BK * 2, kStage = kABytes + kBBytes;
-constexpr uint32_t kIdesc = umma::idesc_bf16(BM, BN);
+constexpr int BM = kGemmBM, BK = kGemmBK, ST = kGemmStages;
+constexpr uint32_t kABytes = BM * BK * 2, kBBox = kGemmBoxB * BK * 2;
 
 __device__ __forceinline__ float gelu(float z) { return mlp_gelu(z); }
 __device__ __forceinline__ float gelu_grad(float z) { return mlp_gelu_grad(z); }
 
-template <int EPI>
-__global__ void __launch_bounds__(256, 1)
+// BN: 64 or 256 columns of an output tile (tc_gemm() chooses)
+template <int EPI, int BN>
+__global__ void __launch_bounds__(256, BN == 64 ? 2 : 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const GemmArgs g) {
+  constexpr uint32_t kStage = kABytes + BN / kGemmBoxB * kBBox;
+  constexpr uint32_t kIdesc = umma::idesc_bf16(BM, BN);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[ST], empty[ST], done;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
-  __shared__ double wsum[4][EPI == kEpiBias ? BN : 1];
+  __shared__ double wsum[4][EPI == kEpiBias && BN == 256 ? BN : 1];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -38,7 +40,7 @@ __global__ void __launch_bounds__(256, 1)
     umma::bar_fence_init();
     abort_flag = 0;
   }
-  if (EPI == kEpiBias)
+  if (EPI == kEpiBias && BN == 256)
     for (int i = threadIdx.x; i < 4 * BN; i += blockDim.x) (&wsum[0][0])[i] = 0.0;
   if (warp == 0) umma::tmem_alloc(&tmem_base, BN);
   umma::fence_before_sync();
@@ -68,7 +70,9 @@ __global__ void __launch_bounds__(256, 1)
         unsigned char* st = smem + (size_t)s * kStage;
         umma::bar_expect_tx(&full[s], kStage);
         umma::tma_load_2d(st, &ta, (kb_first + kb) * BK, mt * BM, &full[s]);
-        umma::tma_load_2d(st + kABytes, &tb, (kb_first + kb) * BK, nt * BN, &full[s]);
+#pragma unroll
+        for (int b = 0; b < BN / kGemmBoxB; ++b)
+          umma::tma_load_2d(st + kABytes + b * kBBox, &tb, (kb_first + kb) * BK, nt * BN + b * kGemmBoxB, &full[s]);
       }
     } else if (warp == 1 && lane == 0) {
       // MMA issuer
@@ -114,7 +118,7 @@ __global__ void __launch_bounds__(256, 1)
         for (int j = 0; j < 16; ++j) v[j] = 0.0f;  // an empty K range contributes nothing
       }
       const int cnt = min(16, g.N - n0);
-      if (EPI == kEpiBias && g.colsum) {
+      if (EPI == kEpiBias && BN == 256 && g.colsum) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           double x = (row_ok && j < cnt) ? (double)(v[j] + g.bias[n0 + j]) : 0.0;
@@ -137,7 +141,9 @@ __global__ void __launch_bounds__(256, 1)
           for (int j = 0; j < 16; j += 4)
             *reinterpret_cast<float4*>(out32 + base + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
         } else {
-          for (int j = 0; j < cnt; ++j) out32[base + j] = o[j];
+          #pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < cnt) out32[base + j] = o[j];
         }
       } else if (EPI == kEpiBiasGelu) {
         float z[16];
@@ -158,13 +164,16 @@ __global__ void __launch_bounds__(256, 1)
             reinterpret_cast<uint4*>(g.out_bf16 + base)[1] = hv[1];
           }
         } else {
-          for (int j = 0; j < cnt; ++j) {
-            if (g.zout) g.zout[base + j] = z[j];
-            if (g.out_bf16) g.out_bf16[base + j] = h[j];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (j < cnt && g.zout) g.zout[base + j] = z[j];
+            if (j < cnt && g.out_bf16) g.out_bf16[base + j] = h[j];
           }
         }
         if (g.out_bf16_t)
-          for (int j = 0; j < cnt; ++j) g.out_bf16_t[(size_t)(n0 + j) * g.ld_t + r] = h[j];
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < cnt) g.out_bf16_t[(size_t)(n0 + j) * g.ld_t + r] = h[j];
       } else {  // kEpiGeluBwd
         float zi[16], gz[16];
         __nv_bfloat16 h[16];
@@ -175,6 +184,7 @@ __global__ void __launch_bounds__(256, 1)
             zi[j] = q.x; zi[j + 1] = q.y; zi[j + 2] = q.z; zi[j + 3] = q.w;
           }
         } else {
+#pragma unroll
           for (int j = 0; j < 16; ++j) zi[j] = j < cnt ? g.zin[base + j] : 0.0f;
         }
 #pragma unroll
@@ -193,13 +203,16 @@ __global__ void __launch_bounds__(256, 1)
             reinterpret_cast<uint4*>(g.out_bf16 + base)[1] = hv[1];
           }
         } else {
-          for (int j = 0; j < cnt; ++j) {
-            if (g.out_f32) g.out_f32[base + j] = gz[j];
-            if (g.out_bf16) g.out_bf16[base + j] = h[j];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (j < cnt && g.out_f32) g.out_f32[base + j] = gz[j];
+            if (j < cnt && g.out_bf16) g.out_bf16[base + j] = h[j];
           }
         }
         if (g.out_bf16_t)
-          for (int j = 0; j < cnt; ++j) g.out_bf16_t[(size_t)(n0 + j) * g.ld_t + r] = h[j];
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < cnt) g.out_bf16_t[(size_t)(n0 + j) * g.ld_t + r] = h[j];
       }
     }
     umma::fence_before_sync();
@@ -208,19 +221,10 @@ __global__ void __launch_bounds__(256, 1)
   umma::fence_before_sync();
   __syncthreads();
   if (abort_flag && threadIdx.x == 0) atomicExch(g.status, kStatusTimeout);
-  if (EPI == kEpiBias && g.colsum)
+  if (EPI == kEpiBias && BN == 256 && g.colsum)
     for (int n = threadIdx.x; n < g.N && n < BN; n += blockDim.x)
       g.colsum[(size_t)blockIdx.x * g.N + n] = ((wsum[0][n] + wsum[1][n]) + wsum[2][n]) + wsum[3][n];
   if (warp == 0) umma::tmem_dealloc(tmem, BN);
-}
-
-// out[e] = sum over the K-range splits of part[s][e] (fixed order).
-__global__ void k_split_sum(const float* __restrict__ part, int splits, int64_t total, float* __restrict__ out) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int k = 0; k < splits; ++k) s += part[(size_t)k * total + e];
-    out[e] = s;
-  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -260,49 +264,60 @@ void make_tmap_bf16_ld(CUtensorMap* map, const void* base, int64_t rows, int64_t
   LEO_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled rejected the tensor");
 }
 
-void tc_gemm_prepare(leo2d_ctx* ctx) {
-  if (ctx->tc_gemm_ready) return;
+template <int BN>
+static void prepare_bn() {
   const int smem = (int)gemm_smem_bytes(BN);
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiBias>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiBiasGelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiGeluBwd>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ctx->tc_gemm_ready = true;
+  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiF32, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiBias, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiBiasGelu, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiGeluBwd, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
 }
 
-void tc_gemm(leo2d_ctx* ctx, GemmEpi epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g,
-             int grid_cap) {
-  LEO_REQUIRE(g.M > 0 && g.N > 0 && g.K > 0, "empty GEMM");
-  const size_t smem = gemm_smem_bytes(BN);
-  const int splits = (epi == kEpiF32 && g.k_splits > 1 && g.split_buf) ? g.k_splits : 1;
-  LEO_REQUIRE(splits == 1 || epi == kEpiF32, "only the plain product splits its K range");
-  const int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) * splits;
-  int grid = std::min(tiles, ctx->sm_count);
-  if (grid_cap > 0) grid = std::min(grid, grid_cap);
-  tc_gemm_prepare(ctx);
-  GemmArgs ga = g;
-  ga.k_splits = splits;
+template <int BN>
+static void launch_bn(leo2d_ctx* ctx, GemmEpi epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g,
+               int grid) {
   auto go = [&](auto kern) {
-    launch(ctx, "tc_gemm", [&] { kern<<<grid, 256, smem, ctx->stream>>>(ta, tb, ga); });
+    launch(ctx, "tc_gemm", [&] { kern<<<grid, 256, gemm_smem_bytes(BN), ctx->stream>>>(ta, tb, g); });
   };
   switch (epi) {
-    case kEpiF32:
-      go(k_tc_gemm<kEpiF32>);
-      if (splits > 1)
-        launch(ctx, "tc_gemm_sum", [&] {
-          k_split_sum<<<grid_for((int64_t)g.M * g.N, 256, (int64_t)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
-              g.split_buf, splits, (int64_t)g.M * g.N, g.out_f32);
-        });
-      return;
-    case kEpiBias: return go(k_tc_gemm<kEpiBias>);
-    case kEpiBiasGelu: return go(k_tc_gemm<kEpiBiasGelu>);
-    case kEpiGeluBwd: return go(k_tc_gemm<kEpiGeluBwd>);
+    case kEpiF32: return go(k_tc_gemm<kEpiF32, BN>);
+    case kEpiBias: return go(k_tc_gemm<kEpiBias, BN>);
+    case kEpiBiasGelu: return go(k_tc_gemm<kEpiBiasGelu, BN>);
+    case kEpiGeluBwd: return go(k_tc_gemm<kEpiGeluBwd, BN>);
   }
   fail(LEO2D_ERR_BAD_ARG, "unknown GEMM epilogue");
 }
 
+void tc_gemm_prepare(leo2d_ctx* ctx) {
+  if (ctx->tc_gemm_ready) return;
+  prepare_bn<256>();
+  prepare_bn<64>();
+  ctx->tc_gemm_ready = true;
+}
+
+// Tiles are 128 x 256 where those alone fill the SMs, else 128 x 64, two blocks an
+// SM: a training batch of 8192 rows has 64 tiles of the wide kind, whose epilogues
+// (a third of a megabyte of FP32 and BF16 each) then ran on 64 of 152 SMs. The
+// products of one gradient at 8192 rows: forward 3 x 24 us + 14, input gradients
+// 3 x 28, weight gradients 4 x 10 with wide tiles; 3 x 12 + 9, 3 x 15, 4 x 7.4 with
+// narrow ones and the epilogues' arrays in registers. The K order of an output element is the same in both. Column sums need the wide tiles.
+void tc_gemm(leo2d_ctx* ctx, GemmEpi epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g) {
+  LEO_REQUIRE(g.M > 0 && g.N > 0 && g.K > 0, "empty GEMM");
+  const int splits = (epi == kEpiF32 && g.k_splits > 1 && g.split_buf) ? g.k_splits : 1;
+  LEO_REQUIRE(splits == 1 || epi == kEpiF32, "only the plain product splits its K range");
+  const int m_tiles = (g.M + BM - 1) / BM;
+  const int wide = m_tiles * ((g.N + 255) / 256) * splits, narrow = m_tiles * ((g.N + 63) / 64) * splits;
+  tc_gemm_prepare(ctx);
+  GemmArgs ga = g;
+  ga.k_splits = splits;
+  if (wide >= ctx->sm_count || g.colsum)
+    launch_bn<256>(ctx, epi, ta, tb, ga, std::min(wide, ctx->sm_count));
+  else
+    launch_bn<64>(ctx, epi, ta, tb, ga, std::min(narrow, 2 * ctx->sm_count));
+}
+
 int tc_gemm_grid(leo2d_ctx* ctx, int M, int N) {
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int tiles = ((M + BM - 1) / BM) * ((N + 255) / 256);
   return std::min(tiles, ctx->sm_count);
 }
 
@@ -324,7 +339,7 @@ extern "C" leo2d_status leo2d_tc_gemm(leo2d_ctx* ctx, const uint16_t* a, const u
     h2d(ctx, reinterpret_cast<uint16_t*>(db.p), b, (size_t)N * K);
     CUtensorMap ta, tb;
     make_tmap_bf16(&ta, da.p, M, K, BM);
-    make_tmap_bf16(&tb, db.p, N, K, BN);
+    make_tmap_bf16(&tb, db.p, N, K, kGemmBoxB);
     GemmArgs g{};
     g.M = (int)M;
     g.N = (int)N;

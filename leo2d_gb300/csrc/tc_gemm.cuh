@@ -7,13 +7,13 @@
 //   weight grad  A = dZ^T [out][rows],        B = activations^T [in][rows]
 // (the epilogues write the transposed copies the next product needs).
 //
-// Kernel: persistent, one 128 x BN output tile at a time per block of 128
-// threads. Lane 0 of warp 0 streams 128x64 and BNx64 BF16 tiles with TMA
+// Kernel: persistent, one 128 x BN output tile (BN = 256 or 64) at a time per block
+// of 256 threads. Lane 0 of warp 0 streams 128x64 and BNx64 BF16 tiles with TMA
 // (128-byte swizzle) into a 4-stage ring; lane 0 of warp 1 issues
 // tcgen05.mma (M = 128, N = BN, K = 16) into a BN-column TMEM accumulator and
-// frees each stage with tcgen05.commit; all four warps then read the
-// accumulator with tcgen05.ld (warp w owns rows 32w..32w+31) and apply the
-// epilogue. Every wait gives up after two seconds, records a status and lets
+// frees each stage with tcgen05.commit; all eight warps then read the
+// accumulator with tcgen05.ld (warps w and w + 4 share rows 32w..32w+31 and split
+// the columns) and apply the epilogue. Every wait gives up after two seconds, records a status and lets
 // the block free its TMEM and exit.
 #pragma once
 
@@ -43,12 +43,13 @@ struct GemmArgs {
   double* colsum;              // [gridDim.x][N] (kEpiBias only, optional)
   int* status;
   // kEpiF32 only: the K range is split over k_splits work items per output tile;
-  // item s writes split_buf + s*M*N and a second pass adds them into out_f32
+  // item s writes split_buf + s*M*N (the caller adds them up; out_f32 is not written)
   int k_splits;
   float* split_buf;
 };
 
-constexpr int kGemmBM = 128, kGemmBK = 64, kGemmStages = 4;
+// kGemmBoxB: rows of B's TMA box; a tile of BN columns takes BN / kGemmBoxB boxes
+constexpr int kGemmBM = 128, kGemmBK = 64, kGemmStages = 4, kGemmBoxB = 64;
 
 inline size_t gemm_smem_bytes(int BN) {
   return (size_t)kGemmStages * (kGemmBM + BN) * kGemmBK * 2 + 1024;
@@ -78,9 +79,9 @@ void tc_gemm_f32x3_acc(leo2d_ctx* ctx, const float* A, const float* B, int M, in
 // call before capturing GEMM launches into a graph).
 void tc_gemm_prepare(leo2d_ctx* ctx);
 
-// Launches D = A B^T with the epilogue; A is [M][K] behind ta, B is [N][K] behind tb.
-void tc_gemm(leo2d_ctx* ctx, GemmEpi epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g,
-             int grid_cap = 0);
+// Launches D = A B^T with the epilogue; A is [M][K] behind ta (boxes of kGemmBM
+// rows), B is [N][K] behind tb (boxes of kGemmBoxB rows).
+void tc_gemm(leo2d_ctx* ctx, GemmEpi epi, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g);
 
 // The activation of the control variate's network: GELU(z) = z Phi(z) =
 // z (1 + erf(z / sqrt 2)) / 2, with erf taken in the form of Abramowitz &
