@@ -114,11 +114,13 @@ __device__ __forceinline__ int find_nearest_sheet(const SheetDev& s, const doubl
   return min(max(int(floor(j_new)), s.min1), s.max1) - s.min1;
 }
 
-// Hstruct::findNearest (global frame, rotated by -angle, zero shifts)
+// Hstruct::findNearest (global frame, rotated by -angle, zero shifts). The
+// reference adds 0 x lattice vector to both coordinates; that can only turn -0
+// into +0, which the cell index below does not see, so the eight FP64
+// instructions a search are left out.
 __device__ __forceinline__ int find_nearest_h(const SheetDev& s, const double p[3], int dim) {
-  const double z0 = 0.0;
-  double x_new = p[0] * s.cos_mt - p[1] * s.sin_mt + z0 * s.a[0][0] + z0 * s.a[1][0];
-  double y_new = p[0] * s.sin_mt + p[1] * s.cos_mt + z0 * s.a[0][1] + z0 * s.a[1][1];
+  const double x_new = p[0] * s.cos_mt - p[1] * s.sin_mt;
+  const double y_new = p[0] * s.sin_mt + p[1] * s.cos_mt;
   if (dim == 0) {
     double i_new = s.a_inv[0][0] * x_new + s.a_inv[0][1] * y_new;
     return min(max(int(floor(i_new)), s.min0), s.max0) - s.min0;
@@ -208,6 +210,44 @@ __device__ __forceinline__ double interlayer_t(int model, int orow, int ocol, do
   }
   const double v = c_to_c(orow, ocol, v0, v1, v2, th_row, th_col);
   return v != 0.0 ? v / rescale : 0.0;
+}
+
+// interlayer_t of the simple model in k_flake_rows, where FP64 instructions are the
+// bound (one per 16 cycles and SM): 24 of them for a pair instead of about 40.
+//  - sqrt: the FP32 reciprocal root (22 bits) and one cubic step (Halley),
+//    r (1 + e/2 + 3 e^2/8) with e = 1 - d2 y^2, which leaves e^3 < 2^-60;
+//  - exp: 2^(u/64), u = 64 log2(e) (3.35 - r) / 0.45 = n + f: table of 2^(k/64) for
+//    k = n mod 64, the Taylor series of 2^(f/64) to f^5 (the next term is below
+//    2^-54), the power of two n / 64 into the exponent field.
+// Both are within 2 ulp; the argument rounds as the library form's does. Distances
+// at the 8 A cutoff, very short and non-finite ones take the library form, so the
+// pairs that count are the same.
+__device__ __forceinline__ double simple_t(double v0, double v1, double v2, double amp,
+                                           const double* __restrict__ pow2_64) {
+  const double d2 = __fma_rn(v2, v2, __fma_rn(v1, v1, __dmul_rn(v0, v0)));
+  const float d2f = (float)d2;
+  if (d2f > 64.001f && d2f < 1e30f) return 0.0;
+  if (!(d2f > 1.0f && d2f < 63.999f))
+    return interlayer_t(LEO2D_MODEL_SIMPLE, 0, 0, v0, v1, v2, 0.0, 0.0, 1.0, amp);
+  const double y = (double)rsqrtf(d2f);
+  const double r0 = __dmul_rn(d2, y);
+  const double e = __fma_rn(-r0, y, 1.0);
+  const double r = __fma_rn(__dmul_rn(r0, e), __fma_rn(0.375, e, 0.5), r0);
+  constexpr double kC = 64.0 * 1.4426950408889634 / 0.45;  // 64 log2(e) / 0.45
+  constexpr double kMagic = 6755399441055744.0;            // 1.5 x 2^52: rounds to an integer
+  constexpr double kL = 0.6931471805599453 / 64.0;         // ln 2 / 64
+  const double u = __fma_rn(-kC, r, 3.35 * kC);
+  const double m = __dadd_rn(u, kMagic);
+  const int n = __double2loint(m);
+  const double f = __dadd_rn(u, -__dadd_rn(m, -kMagic));
+  double p = __fma_rn(kL * kL * kL * kL * kL / 120.0, f, kL * kL * kL * kL / 24.0);
+  p = __fma_rn(p, f, kL * kL * kL / 6.0);
+  p = __fma_rn(p, f, kL * kL / 2.0);
+  p = __fma_rn(p, f, kL);
+  p = __fma_rn(p, f, 1.0);
+  const double t = __dmul_rn(__dmul_rn(pow2_64[n & 63], p), amp);
+  // amp may be anything finite: scale by 2^(n >> 6) as a factor (1 <= r: n < 2^10)
+  return __dmul_rn(t, __hiloint2double((1023 + (n >> 6)) << 20, 0));
 }
 
 __device__ __forceinline__ int sheet_of(const GeomDev& G, int64_t k) {
@@ -353,12 +393,31 @@ __global__ void k_pos32(const double* __restrict__ pos, int64_t n, float4* __res
 // test decides, so the kept pairs and their values are those of FP64 alone.
 constexpr float kPrefilterMargin = 0.05f;
 
+// The cells nearest to orbital `row`: [0] in its own sheet, [1] in the one below, [2]
+// in the one above.
+__device__ __forceinline__ void nearest_cells(const GeomDev& G, int64_t row, const int32_t* __restrict__ grid4,
+                                              const double* __restrict__ pos, int* near_i, int* near_j) {
+  const int4 g = reinterpret_cast<const int4*>(grid4)[row];
+  double lp[3];
+  pos_grid(G.sh[g.w], g.x, g.y, g.z, lp);
+  near_i[0] = find_nearest_sheet(G.sh[g.w], lp, 0);
+  near_j[0] = find_nearest_sheet(G.sh[g.w], lp, 1);
+  const double ph[3] = {pos[3 * row], pos[3 * row + 1], 0.0};
+#pragma unroll
+  for (int k = 1; k < 3; ++k) {
+    const int s0 = k == 1 ? g.w - 1 : g.w + 1;
+    if (s0 < 0 || s0 >= G.S) continue;
+    near_i[k] = find_nearest_h(G.sh[s0], ph, 0);
+    near_j[k] = find_nearest_h(G.sh[s0], ph, 1);
+  }
+}
+
 // kMode 0: count entries per row; 1: fill at the scanned row pointers; 2: fill
 // and count in one pass, row r at r * pad_cap of padded arrays (entries past
 // pad_cap are counted, not stored, and raise `overflow`).
 template <int kMode>
 __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_constant__ GeomDev G, int64_t n,
-                                                    const int32_t* __restrict__ grid4,
+                                                    int run, const int32_t* __restrict__ grid4,
                                                     const double* __restrict__ pos,
                                                     const float4* __restrict__ pos32,
                                                     const double* __restrict__ spos,
@@ -368,28 +427,36 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
   __shared__ int32_t s_code[kRowWarps][kInterSeg];
   __shared__ int16_t s_queue[kRowWarps][kInterSeg];
   __shared__ double s_hop[kRowWarps][kInterSeg];
+  __shared__ double s_pow[64];
+  if (kFill && threadIdx.x < 64) s_pow[threadIdx.x] = exp2((double)threadIdx.x / 64.0);
+  __syncthreads();
   const unsigned lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < n; row += warps) {
+  // A warp takes `run` rows at a time: the cells nearest to their positions (in their
+  // own sheet, the one below, the one above) come from one lane a row. Every lane of
+  // the warp used to compute the row's own, 50 of its 165 FP64 instructions.
+  int near_i[3] = {0, 0, 0}, near_j[3] = {0, 0, 0};
+  int rr = 0;
+  for (int64_t row = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * run; row < n;
+       row += ++rr == run ? warps * run - run + 1 : 1) {
+    if (rr == run) rr = 0;
+    if (rr == 0 && (int)lane < run && row + lane < n) nearest_cells(G, row + lane, grid4, pos, near_i, near_j);
     const int ih = grid4[4 * row], jh = grid4[4 * row + 1], l0 = grid4[4 * row + 2],
               s = grid4[4 * row + 3];
     const SheetDev& sh = G.sh[s];
     // pos: the unshifted positions, which choose the pairs (the reference's pair
     // lists come from the unshifted geometry); spos: the job's shifted i2pos,
     // which give the values (setConfigPositions, locality.cpp:3618-3642)
-    const double x1 = pos[3 * row] + 0.0, y1 = pos[3 * row + 1] + 0.0, z1 = pos[3 * row + 2];
-    const double sx1 = spos[3 * row] + 0.0, sy1 = spos[3 * row + 1] + 0.0, sz1 = spos[3 * row + 2];
+    const double x1 = pos[3 * row], y1 = pos[3 * row + 1];
+    const double sx1 = spos[3 * row], sy1 = spos[3 * row + 1], sz1 = spos[3 * row + 2];
     int64_t o = kPad ? row * (int64_t)out.pad_cap : (kFill ? out.rowptr[row] : 0);
     const int64_t o_end = kPad ? o + out.pad_cap : 0;
     int64_t n_ent = 0, n_intra = 0, n_inter = 0;
 
     // intralayer: window [i0-4, i0+4) x [j0-4, j0+4) x orbitals, every candidate kept
     {
-      double lp[3];
-      pos_grid(sh, ih, jh, l0, lp);
-      double ph[3] = {lp[0] + 0.0, lp[1] + 0.0, lp[2]};
-      const int i0 = find_nearest_sheet(sh, ph, 0), j0 = find_nearest_sheet(sh, ph, 1);
+      const int i0 = __shfl_sync(0xffffffffu, near_i[0], rr), j0 = __shfl_sync(0xffffffffu, near_j[0], rr);
       const int side = 2 * kIntraSearch;
       const int nc = side * side * sh.n_orb;
       for (int c0 = 0; c0 < nc; c0 += 32) {
@@ -442,9 +509,9 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
     // hoppings of the queue, on every lane; (3) the entries in candidate
     // order, as a single pass would write them.
     {
-      const double ph[3] = {x1, y1, z1};
-      const float x1f = (float)x1, y1f = (float)y1;
-      const float sx1f = (float)sx1, sy1f = (float)sy1, sz1f = (float)sz1;
+      const float4 p1f = pos32[row], sp1f = spos32[row];
+      const float x1f = p1f.x, y1f = p1f.y;
+      const float sx1f = sp1f.x, sy1f = sp1f.y, sz1f = sp1f.z;
       constexpr float kWinLo = (float)(kInterCutoff - kPrefilterMargin), kWinHi = (float)(kInterCutoff + kPrefilterMargin);
       // every hopping is zero from 8 A on (in-plane for the reference model, 3-D for the simple one)
       constexpr float kHopHi = 8.0f + kPrefilterMargin, kHopLo = 8.0f - kPrefilterMargin;
@@ -455,7 +522,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
         const int s0 = side_k == 0 ? s - 1 : s + 1;
         if (s0 < 0 || s0 >= G.S) continue;
         const SheetDev& o0 = G.sh[s0];
-        const int i0 = find_nearest_h(o0, ph, 0), j0 = find_nearest_h(o0, ph, 1);
+        const int i0 = __shfl_sync(0xffffffffu, near_i[1 + side_k], rr);
+        const int j0 = __shfl_sync(0xffffffffu, near_j[1 + side_k], rr);
         const int ilo = max(0, i0 - kInterSearch), ihi = min(o0.H, i0 + kInterSearch);
         const int jlo = max(0, j0 - kInterSearch), jhi = min(o0.W, j0 + kInterSearch);
         if (ihi <= ilo || jhi <= jlo) continue;
@@ -488,7 +556,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
                   in_window = false;
                 } else {
                   const double x2 = pos[3 * kk], y2 = pos[3 * kk + 1];
-                  in_window = (x2 - ph[0]) * (x2 - ph[0]) + (y2 - ph[1]) * (y2 - ph[1]) < kInterCutoff * kInterCutoff;
+                  in_window = (x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1) < kInterCutoff * kInterCutoff;
                 }
                 if (in_window) {
                   // the hopping cutoffs test the shifted positions
@@ -526,6 +594,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
                   nz = sqrt(v0 * v0 + v1 * v1 + v2 * v2) < 8.0;
                 }
                 t = nz ? 1.0 : 0.0;
+              } else if (kFill && G.model == LEO2D_MODEL_SIMPLE) {
+                t = simple_t(spos[3 * kk] - sx1, spos[3 * kk + 1] - sy1, spos[3 * kk + 2] - sz1, G.simple_amp, s_pow);
               } else {
                 const int l = (seg0 + slot) % o0.n_orb;
                 const double x2 = spos[3 * kk], y2 = spos[3 * kk + 1], z2 = spos[3 * kk + 2];
@@ -1148,7 +1218,10 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
       LEO_CUDA(cudaFuncSetAttribute(k_periodic_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       LEO_CUDA(cudaFuncSetAttribute(k_periodic_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     }
-    const unsigned rows_grid = grid_for(n, kRowWarps, (int64_t)ctx->sm_count * 64);
+    // rows a warp takes at a time (k_flake_rows): as many as leave every one of the
+    // 24 resident warps of an SM two runs, at most a warp's lanes
+    const int run = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / ((int64_t)ctx->sm_count * 48)));
+    const unsigned rows_grid = grid_for(n, kRowWarps * run, (int64_t)ctx->sm_count * 64);
     DevBuf<float4> pos32(G.bc == 0 ? std::max<int64_t>(n, 1) : 1);
     DevBuf<float4> spos32(G.bc == 0 && G.shifted ? std::max<int64_t>(n, 1) : 0);
     if (G.bc == 0 && n > 0)
@@ -1188,7 +1261,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
         rp.pad_cap = kPadCap;
         rp.overflow = overflow.p;
         launch(ctx, "flake_rows_fill", [&] {
-          k_flake_rows<2><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, pos32.p, spos,
+          k_flake_rows<2><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, rp);
         });
         int over = 0;
@@ -1229,7 +1302,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
     if (n > 0) {
       if (G.bc == 0)
         launch(ctx, "flake_rows_count", [&] {
-          k_flake_rows<0><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, pos32.p, spos,
+          k_flake_rows<0><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, ro);
         });
       else
@@ -1261,7 +1334,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
     if (n > 0) {
       if (G.bc == 0)
         launch(ctx, "flake_rows_fill", [&] {
-          k_flake_rows<1><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, pos32.p, spos,
+          k_flake_rows<1><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, ro);
         });
       else
