@@ -8,7 +8,10 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <new>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -47,6 +50,57 @@ struct Error : std::exception {
 // API call (guard() sets it for the calling thread).
 inline thread_local size_t g_alloc_cap = 0;
 
+// Released device memory, kept for the next allocations. Mapping and unmapping the
+// arrays of a job took 14 of its 122 ms (2.4M orbitals) and 8 of the 46 ms of a Kubo
+// trace; of a 76-orbital k point's 2.8 ms, 0.2.
+//
+// Order: a context runs everything on its one stream, so a block that a call releases
+// while kernels still use it may serve the same context's next allocation (its
+// pending blocks). When no call runs on the context and its stream is idle, they pass
+// to the blocks that every context of the device may take. A buffer goes back through
+// the context that made it, inside a call on that context or outside any call (calls
+// synchronise before they return, also when they fail); one released inside a call on
+// another context is freed with cudaFree, which waits.
+// Bounds: everything kept in the process is at most 16 GiB or a sixteenth of the
+// device's memory, whichever is less, oldest first out; an allocation that fails
+// gives it back to the device and tries again, and so does closing the last context.
+// Thread-safe.
+class MemPool {
+ public:
+  MemPool(int device, cudaStream_t stream, size_t device_bytes);
+  ~MemPool();
+  void enter();  // a call on the context begins / ends (calls nest)
+  void leave();
+  void* take(size_t bytes, size_t* got);  // null: nothing fits
+  bool give(void* p, size_t bytes);       // false: not kept, the caller frees it
+  void close();                           // the context goes: keeps nothing more
+  static size_t kept();                   // bytes kept in the process
+  static void flush();                    // gives them back
+ private:
+  int device_, depth_ = 0;
+  cudaStream_t stream_;
+  size_t cap_;
+  bool closed_ = false;
+};
+
+// The size an allocation is rounded up to, so that jobs of nearly equal sizes find
+// each other's blocks: whole driver pages from 1 MB on, steps of a sixteenth above
+// 32 MB and of 64 MB from 1 GB on.
+inline size_t pool_size(size_t bytes) {
+  size_t unit = 512;
+  if (bytes >= ((size_t)1 << 20))
+    for (unit = (size_t)2 << 20; unit < ((size_t)64 << 20) && unit * 32 <= bytes;) unit *= 2;
+  return (bytes + unit - 1) / unit * unit;
+}
+
+// The pool of the context whose call runs on this thread (guard() sets it).
+inline thread_local const std::shared_ptr<MemPool>* g_pool = nullptr;
+
+// cudaMalloc, after giving back what the pools keep if it does not fit at first.
+cudaError_t device_malloc(void** p, size_t bytes);
+// Free device memory, counting what the pools keep.
+void device_mem_info(size_t* free_bytes, size_t* total_bytes);
+
 // Owning device allocation (move-only).
 template <class T>
 struct DevBuf {
@@ -56,9 +110,12 @@ struct DevBuf {
   explicit DevBuf(size_t count) { alloc(count); }
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+  DevBuf(DevBuf&& o) noexcept { take_from(o); }
   DevBuf& operator=(DevBuf&& o) noexcept {
-    if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+    if (this != &o) {
+      release();
+      take_from(o);
+    }
     return *this;
   }
   ~DevBuf() { release(); }
@@ -68,15 +125,33 @@ struct DevBuf {
     if (g_alloc_cap && count * sizeof(T) > g_alloc_cap)
       fail(LEO2D_ERR_OOM, "device allocation of " + std::to_string(count * sizeof(T)) +
                               " bytes exceeds the context's alloc_cap_mb");
-    LEO_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    size_t got = pool_size(count * sizeof(T));
+    void* q = g_pool ? (*g_pool)->take(got, &got) : nullptr;
+    if (!q) LEO_CUDA(device_malloc(&q, got));
+    if (g_pool) home_ = *g_pool;
+    p = static_cast<T*>(q);
+    held_ = got;
     n = count;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && !(home_ && (!g_pool || *g_pool == home_) && home_->give(p, held_))) cudaFree(p);
+    home_.reset();
     p = nullptr;
-    n = 0;
+    n = held_ = 0;
   }
   size_t bytes() const { return n * sizeof(T); }
+
+ private:
+  void take_from(DevBuf& o) noexcept {
+    p = o.p;
+    n = o.n;
+    held_ = o.held_;
+    home_ = std::move(o.home_);
+    o.p = nullptr;
+    o.n = o.held_ = 0;
+  }
+  size_t held_ = 0;                // bytes behind p
+  std::shared_ptr<MemPool> home_;  // the pool it returns to
 };
 
 struct KStat {
@@ -133,6 +208,8 @@ struct leo2d_ctx {
   int kubo_velocity = -1;     // Kubo trace: -1 D built in the row-block step where possible, 0 stored dxH
   int64_t kubo_chunk = 0;     // Kubo trace: B-side moments held at once (0: as many as memory allows)
   int mlp_fused = 1;          // network forward over many sites: 1 one fused launch, 0 one GEMM per layer
+  std::shared_ptr<leo2d::MemPool> pool;   // released device memory kept for the next allocations
+  std::set<const void*> smem_ready;       // kernels allowed the device's largest dynamic shared memory
   leo2d::DevBuf<int> status;  // one int, reset before kernels that may set it
   leo2d::DevBuf<char> scratch;  // small work arrays of the transforms (ctx_scratch)
 };
@@ -147,8 +224,28 @@ leo2d_status guard(leo2d_ctx* ctx, F&& f) {
     explicit CapScope(size_t cap) : saved(g_alloc_cap) { g_alloc_cap = cap; }
     ~CapScope() { g_alloc_cap = saved; }
   } cap_scope(ctx ? ctx->alloc_cap : g_alloc_cap);
+  struct PoolScope {
+    const std::shared_ptr<MemPool>* saved;
+    explicit PoolScope(const std::shared_ptr<MemPool>* p) : saved(g_pool) {
+      g_pool = p;
+      if (p) (*p)->enter();
+    }
+    ~PoolScope() {
+      if (g_pool) (*g_pool)->leave();
+      g_pool = saved;
+    }
+  } pool_scope(ctx && ctx->pool ? &ctx->pool : g_pool);
+  // a call that fails leaves nothing running on memory that its buffers gave back
+  struct Drain {
+    leo2d_ctx* ctx;
+    bool armed = true;
+    ~Drain() {
+      if (armed && ctx && ctx->stream) cudaStreamSynchronize(ctx->stream);
+    }
+  } drain{ctx};
   try {
     f();
+    drain.armed = false;
     if (ctx) ctx->last_error.clear();
     return LEO2D_OK;
   } catch (const Error& e) {
@@ -164,6 +261,18 @@ leo2d_status guard(leo2d_ctx* ctx, F&& f) {
     if (ctx) ctx->last_error = "unknown error";
     return LEO2D_ERR_CUDA;
   }
+}
+
+// Lets `kern` be launched with any dynamic shared memory the device has, once per
+// context: the attribute call cost a Chebyshev step of a small cell 1.2 us of its 7,
+// and a call with one step's size could undercut another thread's launch.
+inline void allow_smem(leo2d_ctx* ctx, const void* kern) {
+  if (ctx->smem_ready.count(kern)) return;
+  cudaFuncAttributes at{};
+  LEO_CUDA(cudaFuncGetAttributes(&at, kern));
+  LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(ctx->smem_optin - at.sharedSizeBytes)));
+  ctx->smem_ready.insert(kern);
 }
 
 cudaEvent_t ctx_event(leo2d_ctx* ctx);

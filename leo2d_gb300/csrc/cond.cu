@@ -300,7 +300,7 @@ bool cond_trace_rows(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kpm_cfg* 
     mc = std::min<int64_t>(P, ctx->kubo_chunk);
   } else {
     size_t fr = 0, tot = 0;
-    LEO_CUDA(cudaMemGetInfo(&fr, &tot));
+    device_mem_info(&fr, &tot);
     const size_t reserve = (size_t)3 << 30;  // GEMM partials, ordering and launch scratch
     const int64_t fit = fr > reserve ? (int64_t)((fr - reserve) / (vec * sizeof(float))) - 2 : 0;
     if (fit < P) mc = fit >= 256 ? fit / 256 * 256 : fit / 4 * 4;

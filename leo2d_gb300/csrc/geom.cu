@@ -1245,7 +1245,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
     if (G.bc == 0 && n > 0 && G.model == LEO2D_MODEL_SIMPLE && !G.keep_zeros) {
       const size_t per = sizeof(int32_t) + sizeof(double) * (1 + (G.with_dx ? 2 : 0) + (G.cpx ? 1 : 0));
       size_t fr = 0, tot = 0;
-      LEO_CUDA(cudaMemGetInfo(&fr, &tot));
+      device_mem_info(&fr, &tot);
       if ((size_t)n * kPadCap * per <= fr / 4) {
         const size_t pn = (size_t)n * kPadCap;
         DevBuf<int32_t> pcol(pn);

@@ -935,7 +935,7 @@ void rb_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape
   a.xs = vel ? csr->rb_xs.p : nullptr;
   a.out2 = out2;
   auto go = [&](auto kern, int warps) {
-    LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ctx, (const void*)kern);
     launch(ctx, vel ? "cheb_step_vel" : "cheb_step", [&] { kern<<<grid, warps * 32, smem, ctx->stream>>>(a); });
   };
   if (vel) {
@@ -1026,7 +1026,7 @@ void rb_batch_launch(leo2d_ctx* ctx, const RbBatchFlake* fl, const int* block_fi
     a.never_wait = ctx->test_unsatisfied_wait;
   }
   auto kern = k_cheb_rb_batch<24, true, 8>;
-  LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)kern);
   launch(ctx, "cheb_batch_step",
          [&] { kern<<<(unsigned)block_first[nflakes], warps * 32, smem, ctx->stream>>>(p); });
 }

@@ -1379,7 +1379,7 @@ void rt_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape
   a.prev_partials = prev_partials;
   a.prev_dots = prev_dots;
   auto go = [&](auto kern, int warps) {
-    LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ctx, (const void*)kern);
     // the register form keeps no dynamic shared memory: the carveout goes to L1
     if (smem == 0) LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 0));
     launch(ctx, "cheb_step", [&] { kern<<<grid, warps * 32, smem, ctx->stream>>>(a); });
