@@ -114,7 +114,8 @@ struct leo2d_csr {
   // as positions in the tile's window, its sorted distinct columns
   bool win_perm = false;
   int win_cs = 0, win_group = 0;      // column slice and CTAs the tiles were cut for
-  int win_cls = 0;                    // classes the entries are ordered by (1: kept in order)
+  bool win_twice = false;             // a row stores a column twice: no panels
+  bool win_exact = false;             // rows in order, for the exact sums; else panels of 4 rows
   int64_t win_tiles = 0, win_stride = 0;
   int win_tile_slices = 0, win_slice_cap = 0;
   leo2d::DevBuf<int64_t> win_off;     // [slices + 1] first chunk of each slice
@@ -123,6 +124,7 @@ struct leo2d_csr {
   leo2d::DevBuf<int32_t> win_cnt;     // [tiles]
   leo2d::DevBuf<float> win_val;
   leo2d::DevBuf<uint16_t> win_idx;
+  leo2d::DevBuf<int32_t> win_blk;     // panels: [slices][blocks of a slice] 4-row blocks by size within a tile
   // shared-memory windows of the row blocks (rbw_spmm.cu): per tile of 16 blocks
   // the sorted distinct columns of its slots; slots hold window positions
   bool rbw_built = false;

@@ -41,6 +41,7 @@ struct RowShape {
   int dot_slots = 1, dot_rows = 1;
   int ent_cap = 0, row_cap = 0;  // small: room of a CTA
   int warps = 0;  // compute warps of a CTA
+  int slice_warps = 0;  // kRowWin panels: those that take slices
   size_t smem = 0;
 };
 constexpr int kRowBarWords = 8;  // barrier counters of up to 4 slices; the last word is the abort flag

@@ -19,21 +19,22 @@
 //   they wait; the CTAs' sums are stored per step and added in CTA order by one
 //   reduction per launch. Between steps the matrix does not change: a warp asks
 //   for its first entries of the next step before the barrier.
-// FP32 (k_cheb_win): the T_n rows a CTA needs (its window) are copied into shared
-//   memory at the step's start, and LPE lanes own a row whose entries stream
-//   through a ring: the loop sees shared-memory latency only. Bound by the
-//   shared-memory pipe (32 columns: 46 wavefronts per 8 entries of 4 rows), and
-//   for few rows by three trips to L2 and back (window, rows out, barrier), 6 us.
+// FP32: the T_n rows a CTA needs (its window) are copied into shared memory at the
+//   step's start, and the entries stream through a ring: the loop sees shared-memory
+//   latency only. Up to 8000 rows k_cheb_win, LPE lanes a row, sums in the tiled
+//   step's order; bound by three trips to L2 and back (window, rows out, barrier),
+//   6 us. More rows k_cheb_pan, LPE lanes a block of 4 rows; bound by issue and the
+//   shared-memory pipe, two thirds busy each between the same trips.
 // FP64 small (k_cheb_small): the CTA's entries stay in shared memory for the whole
 //   launch, a warp takes one row at a time, GR = 32 / LPE entries at once with up to U
 //   groups in flight; a reduce-scatter over the groups ends a row.
 // FP64 (k_cheb_sell): rows in slices of 16, the j-th entries of 16 rows next to
 //   each other, LPE lanes own a row. Bound by the FP64 pipe (89 % active).
 // Measured per step, tiled step before -> now: the 11,908-orbital cell with 128
-//   columns 99 -> 26 us, a 2188-orbital cell with 12 targets 49 -> 8.2 us, 8 columns of
-//   a 200k-orbital flake 62 -> 27 us, FP64 with 32 columns of 52k orbitals 251 -> 223
-//   us. Gathers through L1 instead of the window took 34 and 42 us for the first
-//   and third: some misses in every group of gathers, about 1000 cycles each.
+//   columns 99 -> 16 us, a 2188-orbital cell with 12 targets 49 -> 8.2 us, 8 columns of
+//   a 200k-orbital flake 62 -> 22 us, FP64 with 32 columns of 52k orbitals 251 -> 223
+//   us. The first and third, LPE lanes a row: 26 and 27 us over the window, 34 and 42
+//   with gathers through L1 (some misses in every group, about 1000 cycles each).
 //
 // Waits: the service warp polls the slice's counter, at most spin_limit polls or
 //   two seconds; then the CTA records a timeout, raises the abort flag that every
@@ -73,6 +74,8 @@ struct RowArgs {
   const int32_t* __restrict__ wcnt;    // [tiles]
   int64_t tiles, win_stride;
   int tile_slices, win_cap, slice_cap;
+  const int32_t* __restrict__ blk;     // panels: [slices][blocks] the 4-row block at each place
+  int warps;                           // panels: warps of a CTA that take slices
   int dot_slots, dot_rows;             // exact sums: the tiled step's row slots of a tile and rows per slot
   int ent_cap;                         // small: entries of a CTA that fit its shared memory
   int row_cap;                         // small: rows of a CTA that fit
@@ -480,10 +483,7 @@ __global__ void __launch_bounds__(kSellWarps * 32 + 32, 1) k_cheb_sell(const __g
 
 // FP32: the rows of T_n that a tile of rows needs (its window) are copied into
 // shared memory once a step, all copies in flight at once; the entries stream
-// through a ring per warp, 6 chunks ahead. What is left in the loop has
-// shared-memory latency: gathers through L1 (a few misses in every group of
-// eight, each about 1000 cycles) took 34 us a step on the 11,908-orbital cell
-// with 128 columns and 42 us with 8 columns of a 200k-orbital flake.
+// through a ring per warp, 6 chunks ahead.
 constexpr int kWinWarps = 23;                                 // + the service warp: 24 warps of 80 registers
 constexpr int kWinChunk = 8;                                  // positions of a chunk
 // chunks of a warp's ring (6 chunks ahead; 3 for 16 rows, whose chunks are as large)
@@ -505,15 +505,14 @@ __device__ __forceinline__ void row_cp8(uint32_t dst, const void* src) {
 // of the moments by the order and more, so a local density of a small cell would
 // otherwise move by 1e-3 of its norm. The dots of step k - 1 are taken by the service
 // warp during step k from T_{k-1} and T_k, which a third vector buffer keeps.
-template <int CS, bool EXACT>
+template <int CS>
 __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __grid_constant__ RowArgs<float> a) {
   using T = float;
   constexpr int W = kWinWarps;
   constexpr int VL = 4, LPE = CS / VL, RW = 32 / LPE, IPS = kSellRows / RW;
-  constexpr int kFlush = 16, kWinRing = win_ring(RW), kWinAhead = RW == 16 ? 3 : 6;
+  constexpr int kWinRing = win_ring(RW), kWinAhead = RW == 16 ? 3 : 6;
   constexpr int kVal = kWinChunk * RW * 4, kIdx = kWinChunk * RW * 2;  // bytes of a ring chunk's parts
   extern __shared__ __align__(128) unsigned char row_smem[];
-  __shared__ RowSum<T> wsum[2][W][2 * CS];
   __shared__ int go;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rl = lane / LPE, sub = lane % LPE;
@@ -596,7 +595,7 @@ __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __gri
   if (warp < W) restart();
 
   auto buf = [&](int i) { return i == 0 ? a.x0 : i == 1 ? a.x1 : a.x2; };
-  // EXACT: the dots of step k from T_k and T_{k+1}, the CTA's share of the groups
+  // the dots of step k from T_k and T_{k+1}, the CTA's share of the groups
   auto exact_dots = [&](int k) {
     const float* t0 = buf(k % 3) + slice * CS;
     const float* t1 = buf((k + 1) % 3) + slice * CS;
@@ -645,17 +644,11 @@ __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __gri
   };
 
   for (int k = a.k0; k < a.k1; ++k) {
-    RowSum<T>(*ws)[2 * CS] = wsum[k & 1];
-    // (EXACT: T_{k-1} from one buffer, T_{k+1} into the third)
-    const T* tn = buf(EXACT ? k % 3 : k & 1);
-    T* tp = buf(EXACT ? (k + 1) % 3 : (k + 1) & 1);
-    const T* tm = EXACT ? buf((k + 2) % 3) : tp;
+    // (T_{k-1} from one buffer, T_{k+1} into the third)
+    const T* tn = buf(k % 3);
+    T* tp = buf((k + 1) % 3);
+    const T* tm = buf((k + 2) % 3);
     const T alpha = k == 0 ? T(1) : T(2);
-    T f[2 * VL];  // FP32 over kFlush items; [2 v + d]: column VL sub + v, dot d
-    RowSum<T> s[2 * VL];
-#pragma unroll
-    for (int v = 0; v < 2 * VL; ++v) f[v] = T(0);
-    int since = 0;
     for (int t = 0; t < ntile; ++t) {
       // the tile's window
       const int64_t l0 = (t_first + t) * a.win_stride;
@@ -681,11 +674,8 @@ __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __gri
           const int len = slen[sl];
           const bool in = row < a.n;
           const int64_t at = row * C + slice * CS + VL * sub;
-          float4 xn = make_float4(0.f, 0.f, 0.f, 0.f), xp = xn;
-          if (in) {
-            if (!EXACT) xn = __ldcg(reinterpret_cast<const float4*>(tn + at));
-            if (k != 0) xp = __ldcg(reinterpret_cast<const float4*>(tm + at));
-          }
+          float4 xp = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (in && k != 0) xp = __ldcg(reinterpret_cast<const float4*>(tm + at));
           T acc[VL];
 #pragma unroll
           for (int v = 0; v < VL; ++v) acc[v] = T(0);
@@ -722,18 +712,243 @@ __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __gri
           }
           if (in) {
             RowVec<T> y;
-            const T xs[4] = {xn.x, xn.y, xn.z, xn.w}, ps[4] = {xp.x, xp.y, xp.z, xp.w};
+            const T ps[4] = {xp.x, xp.y, xp.z, xp.w};
 #pragma unroll
-            for (int v = 0; v < VL; ++v) {
-              y.v[v] = k == 0 ? alpha * acc[v] : alpha * acc[v] - ps[v];
-              if (!EXACT) {
-                f[2 * v] += xs[v] * xs[v];
-                f[2 * v + 1] += y.v[v] * xs[v];
-              }
-            }
+            for (int v = 0; v < VL; ++v) y.v[v] = k == 0 ? alpha * acc[v] : alpha * acc[v] - ps[v];
             y.store(tp + at);
           }
-          if (!EXACT && ++since == kFlush) {
+        }
+      }
+      if (t + 1 < ntile) __syncthreads();  // the window is read
+    }
+    const bool last = k + 1 == a.k1;
+    if (warp < W) {
+      if (!last) restart();
+    } else if (k > a.k0) {
+      exact_dots(k - 1);
+    }
+    if (a.group == 1) __threadfence();  // (the next step reads the rows past L1)
+    __syncthreads();
+    if (a.group > 1) {  // (also after the last step: its dots need every CTA's rows)
+      if (threadIdx.x == W * 32) {
+        row_announce(a, slice);
+        go = row_await(a, k, slice);
+      }
+      __syncthreads();
+      if (go == 0) break;
+    }
+    if (last && warp == W) exact_dots(k);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// ---------------------------------------------------------------- panels
+
+// FP32, more rows: blocks of 4 consecutive rows (under the locality ordering, of a
+// compact cluster) share the union of their columns. LPE lanes own a block: a
+// gathered T_n row and its 4 values make 16 FMAs a lane, so 16 rows of 32 columns
+// cost 5 wavefronts of shared memory for each of their 98 or so common positions where
+// row by row they cost 5.75 for each of 4 x 67 entries. The values stored for the zeros
+// of the union are paid back by a single index per position (427 bytes a row for 402).
+// Per step, the 11,908-orbital cell with 128 columns / 8 columns of a 200k flake:
+// 26 / 27 us row by row; panels in row order 23 / 35 (slices padded to their longest
+// block); blocks by size within a tile 19 / 24; chunks of 8 to 16 positions and warps
+// in fours 17.5 / 23; packed FMAs (half the issue slots of the products) 16 / 22.
+// The window and the entry ring are those of k_cheb_win.
+constexpr int kPanRows = 4;
+constexpr int kPanWarps = 15;  // + the service warp: 16 warps of 128 registers
+// blocks of a warp's item (= a slice of the format), positions of a chunk
+__host__ __device__ constexpr int pan_blocks(int cs) { return 128 / cs; }
+__host__ __device__ constexpr int pan_chunk(int cs) { return cs == 32 ? 16 : 8; }
+constexpr int kPanRing = 3;  // chunks of a warp's ring, all but one of them ahead
+__host__ __device__ constexpr int pan_ring_bytes(int cs) { return kPanRing * pan_chunk(cs) * pan_blocks(cs) * 18; }
+
+// (a, b) += w (x, y), both lanes of one fma.rn.f32x2
+__device__ __forceinline__ void pan_fma2(float& a, float& b, float w, float x, float y) {
+  unsigned long long r;
+  asm("{\n\t.reg .b64 s, t, u;\n\tmov.b64 s, {%3, %3};\n\tmov.b64 t, {%4, %5};\n\tmov.b64 u, {%1, %2};\n\t"
+      "fma.rn.f32x2 %0, s, t, u;\n\t}"
+      : "=l"(r)
+      : "f"(a), "f"(b), "f"(w), "f"(x), "f"(y));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+
+template <int CS>
+__global__ void __launch_bounds__(kPanWarps * 32 + 32, 1) k_cheb_pan(const __grid_constant__ RowArgs<float> a) {
+  using T = float;
+  constexpr int W = kPanWarps;
+  constexpr int VL = 4, LPE = CS / VL, RW = pan_blocks(CS), PC = pan_chunk(CS), RB = kPanRows;
+  constexpr int kSliceRows = RW * RB, kFlush = 4;  // items (16 rows a lane) of an FP32 sum
+  constexpr int kVal = PC * RW * 16, kIdx = PC * RW * 2, kSlot = kVal + kIdx;
+  extern __shared__ __align__(128) unsigned char row_smem[];
+  __shared__ RowSum<T> wsum[2][W][2 * CS];
+  __shared__ int go;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rl = lane / LPE, sub = lane % LPE;
+  const int slice = (int)blockIdx.x / a.group, bid = (int)blockIdx.x % a.group;
+  const int C = a.C;
+  // this CTA's tiles, of tile_slices slices each
+  const int64_t nsl = (a.n + kSliceRows - 1) / kSliceRows;
+  const int64_t t_first = a.tiles * bid / a.group, t_end = a.tiles * (bid + 1) / a.group;
+  const int64_t s_first = min(nsl, t_first * a.tile_slices), s_end = min(nsl, t_end * a.tile_slices);
+  const int nslice = (int)(s_end - s_first);
+  // shared memory: window | rings | chunk offsets of the slices | lengths | window list
+  float* win = reinterpret_cast<float*>(row_smem);
+  unsigned char* ring = row_smem + (size_t)a.win_cap * CS * 4 + (size_t)warp * pan_ring_bytes(CS);
+  int* spos = reinterpret_cast<int*>(row_smem + (size_t)a.win_cap * CS * 4 + (size_t)W * pan_ring_bytes(CS));
+  int* slen = spos + a.slice_cap + 1;
+  int* list = slen + a.slice_cap + 1;
+  const int64_t c_first = a.off[s_first];
+  for (int i = threadIdx.x; i <= nslice; i += blockDim.x) {
+    spos[i] = (int)(a.off[s_first + i] - c_first);
+    if (i < nslice) slen[i] = a.slen[s_first + i];
+  }
+  __syncthreads();
+
+  // The copy side of the warp's entry stream: slices warp, warp + step, ... of each
+  // tile in turn, chunk by chunk (warps from `step` on have none).
+  const int first = warp < a.warps ? warp : 1 << 28, step = a.warps;
+  const int ntile = (int)(t_end - t_first);
+  auto tile_items = [&](int t) { return min(a.tile_slices, nslice - t * a.tile_slices); };
+  const uint32_t ring_u = (uint32_t)__cvta_generic_to_shared(ring);
+  const float* pv = nullptr;
+  const uint16_t* pi = nullptr;
+  int ft = 0, fi = 0, fleft = 0;  // tile, item of the tile, chunks of it still to copy
+  uint32_t fslot = 0, cslot = 0;  // byte offsets of the ring chunks to fill and to use next
+  auto fetch_item = [&]() {       // item (ft, fi), or the first one after it that exists
+    while (ft < ntile && fi >= tile_items(ft)) {
+      ++ft;
+      fi = first;
+    }
+    if (ft < ntile) {
+      const int sl = ft * a.tile_slices + fi;
+      fleft = spos[sl + 1] - spos[sl];
+      pv = a.wval + (c_first + spos[sl]) * (kVal / 4) + 4 * lane;
+      pi = a.widx + (c_first + spos[sl]) * (kIdx / 2) + 8 * lane;
+    }
+  };
+  auto fetch = [&]() {  // one chunk (or an empty group past the last one)
+    while (fleft == 0 && ft < ntile) {
+      fi += step;
+      fetch_item();
+    }
+    if (fleft > 0) {
+      const uint32_t d = ring_u + fslot + 16 * lane;
+#pragma unroll
+      for (int i = 0; i < kVal / 512; ++i) row_cp16(d + 512 * i, pv + 128 * i);
+      if (lane < kIdx / 16) row_cp16(d + kVal, pi);
+      pv += kVal / 4;
+      pi += kIdx / 2;
+      --fleft;
+    }
+    fslot = fslot == (kPanRing - 1) * kSlot ? 0u : fslot + kSlot;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto restart = [&]() {  // the first chunks of a step (the matrix does not change: also before the barrier)
+    __syncwarp();
+    fslot = cslot = 0;
+    ft = 0;
+    fi = first;
+    fleft = 0;
+    fetch_item();
+#pragma unroll 1
+    for (int i = 0; i < kPanRing - 1; ++i) fetch();
+  };
+  if (warp < W) restart();
+
+  for (int k = a.k0; k < a.k1; ++k) {
+    RowSum<T>(*ws)[2 * CS] = wsum[k & 1];
+    const T* tn = (k & 1) ? a.x1 : a.x0;
+    T* tp = (k & 1) ? a.x0 : a.x1;
+    const T alpha = k == 0 ? T(1) : T(2);
+    T f[2 * VL];  // FP32 over kFlush items; [2 v + d]: column VL sub + v, dot d
+    RowSum<T> s[2 * VL];
+#pragma unroll
+    for (int v = 0; v < 2 * VL; ++v) f[v] = T(0);
+    int since = 0;
+    for (int t = 0; t < ntile; ++t) {
+      // the tile's window
+      const int64_t l0 = (t_first + t) * a.win_stride;
+      const int nwin = a.wcnt[t_first + t];
+      if (ntile > 1 || k == a.k0) {
+        for (int i = threadIdx.x; i < nwin; i += blockDim.x) list[i] = __ldg(a.wlist + l0 + i);
+        __syncthreads();
+      }
+      {
+        const uint32_t w_u = (uint32_t)__cvta_generic_to_shared(win);
+        const T* src = tn + slice * CS;
+        for (int i = threadIdx.x; i < nwin * LPE; i += blockDim.x)
+          row_cp16(w_u + 16 * i, src + (int64_t)list[i / LPE] * C + 4 * (i % LPE));
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncthreads();
+      if (warp < W) {
+        const int items = tile_items(t);
+        for (int item = first; item < items; item += step) {
+          const int sl = t * a.tile_slices + item;
+          const int64_t row0 = (int64_t)__ldg(a.blk + (s_first + sl) * RW + rl) * RB;
+          const int len = slen[sl];
+          float acc[RB][VL];
+#pragma unroll
+          for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int v = 0; v < VL; ++v) acc[r][v] = 0.f;
+#pragma unroll 1
+          for (int j = 0; j < len; j += PC) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kPanRing - 2) : "memory");
+            __syncwarp();
+            fetch();
+            const unsigned char* rc = ring + cslot;
+            cslot = cslot == (kPanRing - 1) * kSlot ? 0u : cslot + kSlot;
+            const uint2* pix = reinterpret_cast<const uint2*>(rc + kVal + rl * (PC * 2));
+            auto four = [&](int h) {  // positions 4 h .. 4 h + 3 of the chunk
+              const uint2 ix = pix[h];
+              const uint32_t c[4] = {ix.x & 0xffffu, ix.x >> 16, ix.y & 0xffffu, ix.y >> 16};
+              float4 x[4], w[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                x[u] = *reinterpret_cast<const float4*>(win + c[u] * CS + VL * sub);
+                w[u] = *reinterpret_cast<const float4*>(rc + ((4 * h + u) * RW + rl) * 16);
+              }
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const float ww[4] = {w[u].x, w[u].y, w[u].z, w[u].w};
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                  pan_fma2(acc[r][0], acc[r][1], ww[r], x[u].x, x[u].y);
+                  pan_fma2(acc[r][2], acc[r][3], ww[r], x[u].z, x[u].w);
+                }
+              }
+            };
+            four(0);
+#pragma unroll
+            for (int h = 1; h < PC / 4; ++h)
+              if (j + 4 * h < len) four(h);
+          }
+          const int64_t at = row0 * C + slice * CS + VL * sub;
+          float4 xn[RB], xp[RB];
+#pragma unroll
+          for (int r = 0; r < RB; ++r) {
+            xn[r] = xp[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row0 + r < a.n) {
+              xn[r] = __ldcg(reinterpret_cast<const float4*>(tn + at + (int64_t)r * C));
+              if (k != 0) xp[r] = __ldcg(reinterpret_cast<const float4*>(tp + at + (int64_t)r * C));
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < RB; ++r) {
+            const float xs[4] = {xn[r].x, xn[r].y, xn[r].z, xn[r].w}, ps[4] = {xp[r].x, xp[r].y, xp[r].z, xp[r].w};
+            RowVec<T> y;
+#pragma unroll
+            for (int v = 0; v < VL; ++v) {
+              y.v[v] = k == 0 ? alpha * acc[r][v] : alpha * acc[r][v] - ps[v];
+              f[2 * v] += xs[v] * xs[v];
+              f[2 * v + 1] += y.v[v] * xs[v];
+            }
+            if (row0 + r < a.n) y.store(tp + at + (int64_t)r * C);
+          }
+          if (++since == kFlush) {
             since = 0;
 #pragma unroll
             for (int v = 0; v < 2 * VL; ++v) {
@@ -745,33 +960,13 @@ __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __gri
       }
       if (t + 1 < ntile) __syncthreads();  // the window is read
     }
-    if constexpr (EXACT) {
-      const bool last = k + 1 == a.k1;
-      if (warp < W) {
-        if (!last) restart();
-      } else if (k > a.k0) {
-        exact_dots(k - 1);
-      }
-      if (a.group == 1) __threadfence();  // (the next step reads the rows past L1)
-      __syncthreads();
-      if (a.group > 1) {  // (also after the last step: its dots need every CTA's rows)
-        if (threadIdx.x == W * 32) {
-          row_announce(a, slice);
-          go = row_await(a, k, slice);
-        }
-        __syncthreads();
-        if (go == 0) break;
-      }
-      if (last && warp == W) exact_dots(k);
-    } else {
-      if (warp < W) {
-        if (k + 1 < a.k1) restart();
+    if (warp < W) {
+      if (k + 1 < a.k1) restart();
 #pragma unroll
-        for (int v = 0; v < 2 * VL; ++v) s[v].add(f[v]);
-        row_warp_sums<T, CS>(s, ws[warp], rl, sub);
-      }
-      if (!row_step_end<T, CS, W>(a, ws, k, slice, bid, &go)) break;
+      for (int v = 0; v < 2 * VL; ++v) s[v].add(f[v]);
+      row_warp_sums<T, CS>(s, ws[warp], rl, sub);
     }
+    if (!row_step_end<T, CS, W>(a, ws, k, slice, bid, &go)) break;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
@@ -894,14 +1089,7 @@ __global__ void __launch_bounds__(kWinThreads) k_win_list(int64_t n, int tile_ro
 // One CTA per tile, a warp per row: the chunks of its slices, [chunk][16 rows][8],
 // the columns as window positions. Rows shorter than the slice end in zero values
 // at their first column (their own index when they are empty).
-// The order of a row's entries is free, and decides the bank conflicts of the
-// gathers: a quarter warp reads `cls` rows of the window at once (4 for slices of 8
-// columns, 2 of 16, 1 of 32), without a conflict when their positions differ modulo cls.
-// So row r's m-th entry of class c (position modulo cls) goes to place
-// cls m + (c - r) mod cls, as long as every class has an m-th entry; the others follow.
-// cls = 1 keeps the entries in order (slices of 32 columns, and the EXACT form)
-// (in row order 8 columns of a 200k-orbital flake had 2.1 wavefronts per read, 37 us a step).
-__global__ void __launch_bounds__(kWinThreads) k_win_fill(int64_t n, int64_t nsl, int tile_slices, int cls,
+__global__ void __launch_bounds__(kWinThreads) k_win_fill(int64_t n, int64_t nsl, int tile_slices,
                                                           const int64_t* __restrict__ rowptr,
                                                           const int64_t* __restrict__ off,
                                                           const int32_t* __restrict__ col, const float* __restrict__ val,
@@ -929,39 +1117,155 @@ __global__ void __launch_bounds__(kWinThreads) k_win_fill(int64_t n, int64_t nsl
     const int64_t beg = row < n ? rowptr[row] : 0;
     const int len = row < n ? (int)(rowptr[row + 1] - beg) : 0;
     auto place = [&](int j) { return ((p0 + j / kWinChunk) * kSellRows + r) * kWinChunk + j % kWinChunk; };
-    int count[4] = {0, 0, 0, 0};
-    for (int j0 = 0; j0 < len; j0 += 32) {
-      const int c = j0 + lane < len ? find((uint32_t)col[beg + j0 + lane]) % cls : -1;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) count[q] += __popc(__ballot_sync(0xffffffffu, c == q));
-    }
-    int least = count[0];
-    for (int q = 1; q < cls; ++q) least = min(least, count[q]);
-    int seen[4] = {0, 0, 0, 0};
-    for (int j0 = 0; j0 < len; j0 += 32) {
-      const int64_t e = beg + j0 + lane;
-      const bool in = j0 + lane < len;
-      const int w = in ? find((uint32_t)col[e]) : 0, c = in ? w % cls : -1;
-      int k = 0, before = 0;  // entries of this class before it; leftovers of the classes before it
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const unsigned b = __ballot_sync(0xffffffffu, c == q);
-        if (c == q) k = seen[q] + __popc(b & ((1u << lane) - 1u));
-        if (c > q) before += count[q] - least;
-        seen[q] += __popc(b);
-      }
-      if (in) {
-        const int j = k < least ? cls * k + ((c - r) & (cls - 1)) : cls * least + before + (k - least);
-        const int64_t at = place(j);
-        widx[at] = (uint16_t)w;
-        wval[at] = val[e];
-      }
+    for (int j = lane; j < len; j += 32) {
+      const int64_t at = place(j);
+      widx[at] = (uint16_t)find((uint32_t)col[beg + j]);
+      wval[at] = val[beg + j];
     }
     const uint16_t pad = row >= n ? 0 : (uint16_t)find(len > 0 ? (uint32_t)col[beg] : (uint32_t)row);
     for (int j = len + lane; j < room; j += 32) {
       const int64_t at = place(j);
       widx[at] = pad;
       wval[at] = 0.f;
+    }
+  }
+}
+
+// Panels, one CTA per tile, a warp per block of 4 rows. A bit per window position and
+// row gives the block's union; `fill` = 0: size[block] = its positions, and *over is
+// raised when a row stores a column twice; 1: the chunks of the tile's slices, values
+// [chunk][PC][RW][4], positions [chunk][RW][PC] (both zero before, so that places past
+// the union read window row 0 with weight 0).
+// The order of a block's positions is free, and decides the bank conflicts of the
+// gathers: a quarter warp reads `cls` rows of the window at once (4 for slices of 8
+// columns, 2 of 16, 1 of 32), without a conflict when their positions differ modulo cls.
+// So block b's m-th position of class c (position modulo cls) goes to place
+// cls m + (c - b) mod cls, as long as every class has an m-th one; the others follow.
+constexpr int kPanWords = kWinMax / 32;
+constexpr size_t kPanFillSmem =
+    (size_t)kWinMax * 4 + (size_t)(kWinThreads / 32) * kPanWords * (kPanRows * 4 + 8);
+__global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl, int tile_slices, int RW, int PC, int cls,
+                                                          int fill, const int64_t* __restrict__ rowptr,
+                                                          const int32_t* __restrict__ col,
+                                                          const float* __restrict__ val, int64_t stride,
+                                                          const int32_t* __restrict__ list,
+                                                          const int32_t* __restrict__ cnt, int32_t* __restrict__ size,
+                                                          const int32_t* __restrict__ order,
+                                                          const int64_t* __restrict__ off, float* __restrict__ wval,
+                                                          uint16_t* __restrict__ widx, int* __restrict__ over) {
+  extern __shared__ __align__(16) uint32_t win_keys[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // per word of 32 positions: how many earlier ones of each class the union holds
+  unsigned long long* pre = reinterpret_cast<unsigned long long*>(win_keys + kWinMax) + (size_t)warp * kPanWords;
+  uint32_t* bits = win_keys + kWinMax + (size_t)(kWinThreads / 32) * kPanWords * 2 + (size_t)warp * kPanRows * kPanWords;
+  const int m = cnt[blockIdx.x], words = (m + 31) / 32;
+  for (int i = threadIdx.x; i < m; i += kWinThreads) win_keys[i] = (uint32_t)list[blockIdx.x * stride + i];
+  __syncthreads();
+  auto find = [&](uint32_t c) {  // (present)
+    int lo = 0, hi = m - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (win_keys[mid] < c) lo = mid + 1;
+      else hi = mid;
+    }
+    return lo;
+  };
+  auto mask = [&](int c) { return (cls == 4 ? 0x11111111u : cls == 2 ? 0x55555555u : ~0u) << c; };
+  auto united = [&](int i) {
+    uint32_t u = 0;
+#pragma unroll
+    for (int r = 0; r < kPanRows; ++r) u |= bits[r * kPanWords + i];
+    return u;
+  };
+  const int64_t s0 = (int64_t)blockIdx.x * tile_slices, s1 = min(nsl, s0 + tile_slices);
+  for (int64_t at = s0 * RW + warp; at < s1 * RW; at += kWinThreads / 32) {
+    const int64_t s = at / RW, b = fill ? order[at] : at, row0 = b * kPanRows;
+    const int rl = (int)(at % RW);
+    for (int i = lane; i < words; i += 32)
+#pragma unroll
+      for (int r = 0; r < kPanRows; ++r) bits[r * kPanWords + i] = 0u;
+    __syncwarp();
+    bool twice = false;
+    for (int r = 0; r < kPanRows && row0 + r < n; ++r)
+      for (int64_t e = rowptr[row0 + r] + lane; e < rowptr[row0 + r + 1]; e += 32) {
+        const int w = find((uint32_t)col[e]);
+        const uint32_t bit = 1u << (w & 31);
+        if (atomicOr(&bits[r * kPanWords + (w >> 5)], bit) & bit) twice = true;
+      }
+    __syncwarp();
+    // the lane's words, 8 at most
+    const int per = (words + 31) / 32, i0 = min(words, lane * per), i1 = min(words, i0 + per);
+    int own[4] = {0, 0, 0, 0};
+    for (int i = i0; i < i1; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (c < cls) own[c] += __popc(united(i) & mask(c));
+    int first[4], total[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      int x = own[c];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      first[c] = x - own[c];
+      total[c] = __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (fill == 0) {
+      if (__any_sync(0xffffffffu, twice) && lane == 0) atomicExch(over, 1);
+      if (lane == 0) size[b] = total[0] + total[1] + total[2] + total[3];
+      __syncwarp();
+      continue;
+    }
+    int least = total[0];
+    for (int c = 1; c < cls; ++c) least = min(least, total[c]);
+    for (int i = i0; i < i1; ++i) {
+      unsigned long long p = 0;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        p |= (unsigned long long)first[c] << (16 * c);
+        if (c < cls) first[c] += __popc(united(i) & mask(c));
+      }
+      pre[i] = p;
+    }
+    __syncwarp();
+    for (int r = 0; r < kPanRows && row0 + r < n; ++r)
+      for (int64_t e = rowptr[row0 + r] + lane; e < rowptr[row0 + r + 1]; e += 32) {
+        const int w = find((uint32_t)col[e]), i = w >> 5, c = w & (cls - 1);
+        const int k = (int)((pre[i] >> (16 * c)) & 0xffffu) +
+                      __popc(united(i) & mask(c) & ((1u << (w & 31)) - 1u));
+        int before = 0;  // positions of the classes before it that have no partner
+        for (int q = 0; q < c; ++q) before += total[q] - least;
+        const int j = k < least ? cls * k + ((c - rl) & (cls - 1)) : cls * least + before + (k - least);
+        const int64_t chunk = off[s] + j / PC;
+        widx[(chunk * RW + rl) * PC + j % PC] = (uint16_t)w;
+        wval[((chunk * PC + j % PC) * RW + rl) * 4 + r] = val[e];
+      }
+    __syncwarp();
+  }
+}
+
+// One CTA per tile: its blocks by falling size (slices of blocks of equal length: in
+// row order a slice of 16 was padded to its longest by half), the length of each
+// slice and its chunks of PC positions.
+__global__ void __launch_bounds__(kWinThreads) k_pan_order(int64_t nsl, int tile_slices, int RW, int PC,
+                                                           const int32_t* __restrict__ size,
+                                                           int32_t* __restrict__ order, int32_t* __restrict__ slen,
+                                                           int64_t* __restrict__ count) {
+  const int64_t s0 = (int64_t)blockIdx.x * tile_slices, s1 = min(nsl, s0 + tile_slices), b0 = s0 * RW;
+  const int nb = (int)((s1 - s0) * RW);
+  for (int i = threadIdx.x; i < nb; i += kWinThreads) {
+    const int mine = size[b0 + i];
+    int rank = 0;
+    for (int j = 0; j < nb; ++j) {
+      const int other = __ldg(size + b0 + j);
+      rank += other > mine || (other == mine && j < i) ? 1 : 0;
+    }
+    order[b0 + rank] = (int32_t)(b0 + i);
+    if (rank % RW == 0) {
+      slen[s0 + rank / RW] = mine;
+      count[s0 + rank / RW] = (mine + PC - 1) / PC;
     }
   }
 }
@@ -980,11 +1284,11 @@ void row_coop_launch(leo2d_ctx* ctx, const void* kern, unsigned grid, int thread
 const void* small_kernel(int cs) {
   return cs == 8 ? (const void*)k_cheb_small<8> : cs == 16 ? (const void*)k_cheb_small<16> : (const void*)k_cheb_small<32>;
 }
-template <bool EXACT>
 const void* win_kernel(int cs) {
-  return cs == 8    ? (const void*)k_cheb_win<8, EXACT>
-         : cs == 16 ? (const void*)k_cheb_win<16, EXACT>
-                    : (const void*)k_cheb_win<32, EXACT>;
+  return cs == 8 ? (const void*)k_cheb_win<8> : cs == 16 ? (const void*)k_cheb_win<16> : (const void*)k_cheb_win<32>;
+}
+const void* pan_kernel(int cs) {
+  return cs == 8 ? (const void*)k_cheb_pan<8> : cs == 16 ? (const void*)k_cheb_pan<16> : (const void*)k_cheb_pan<32>;
 }
 const void* sell_kernel(int cs) {
   return cs == 8 ? (const void*)k_cheb_sell<8> : cs == 16 ? (const void*)k_cheb_sell<16> : (const void*)k_cheb_sell<32>;
@@ -1001,32 +1305,29 @@ size_t small_smem(int row_cap, int ent_cap) {
 // static shared memory of the kernels: the warps' sums of two steps and a little more
 size_t row_static_smem(int warps, int cs) { return (size_t)2 * warps * 2 * cs * 8 + 256; }
 
-size_t win_smem(int win_cap, int slice_cap, int cs) {
-  return (size_t)win_cap * (cs * 4 + 4) + (size_t)kWinWarps * win_ring_bytes(128 / cs) + 2 * ((size_t)slice_cap + 1) * 4;
+size_t win_smem(const RowShape& s, int win_cap, int slice_cap) {
+  const size_t rings = s.exact ? (size_t)kWinWarps * win_ring_bytes(128 / s.cs) : (size_t)kPanWarps * pan_ring_bytes(s.cs);
+  return (size_t)win_cap * (s.cs * 4 + 4) + rings + 2 * ((size_t)slice_cap + 1) * 4;
 }
+int win_slice_rows(const RowShape& s) { return s.exact ? kSellRows : kPanRows * pan_blocks(s.cs); }
 
-// The window format for `group` CTAs a slice; false when a 16-row slice alone
-// has too wide a window.
+// The window format (rows for the EXACT form, else panels) for `group` CTAs a slice;
+// false when a slice alone has too wide a window or a row stores a column twice
+// (panels).
 bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
-  const int64_t n = csr->n, nsl = (n + kSellRows - 1) / kSellRows;
+  if (!s.exact && csr->win_twice) return false;
+  const int SR = win_slice_rows(s), PC = s.exact ? kWinChunk : pan_chunk(s.cs);
+  const int64_t n = csr->n, nsl = (n + SR - 1) / SR;
   const int64_t* rp = perm ? csr->prow.p : csr->rowptr.p;
   const int32_t* col = perm ? csr->pcol.p : csr->col.p;
-  const size_t room = ctx->smem_optin - row_static_smem(kWinWarps, s.cs);
-  const int cls = s.exact ? 1 : 32 / s.cs;
+  const float* val = perm ? csr->pval32.p : csr->val32.p;
+  const size_t room = ctx->smem_optin - row_static_smem(s.warps, s.cs);
   const bool current = csr->win_off.p && csr->win_perm == perm && csr->win_cs == s.cs && csr->win_group == s.group &&
-                       csr->win_cls == cls;
+                       csr->win_exact == s.exact;
   if (!current) {
     csr_drop_win(csr);
     csr->win_off.alloc(nsl + 1);
     csr->win_slen.alloc(nsl);
-    {
-      DevBuf<int64_t> count(nsl);
-      launch(ctx, "win_build", [&] {
-        k_slice_len<<<grid_for(nsl, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(n, nsl, rp, kWinChunk, count.p,
-                                                                                         csr->win_slen.p);
-      });
-      exclusive_scan_i64(ctx, count.p, csr->win_off.p, nsl);
-    }
     const size_t list_smem = (size_t)(kWinSet + kWinMax) * sizeof(uint32_t);
     LEO_CUDA(cudaFuncSetAttribute(k_win_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem));
     DevBuf<int> over(1);
@@ -1036,16 +1337,19 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
       const int64_t tiles = (nsl + ts - 1) / ts;
       const int64_t per_cta = (tiles + s.group - 1) / s.group;
       const int64_t slice_cap = ts * per_cta;
-      const size_t fixed = win_smem(0, (int)slice_cap, s.cs);
-      if (fixed >= room) return false;
+      const size_t fixed = win_smem(s, 0, (int)slice_cap);
+      if (fixed >= room) {
+        csr_drop_win(csr);
+        return false;
+      }
       const int64_t cap = std::min<int64_t>((int64_t)((room - fixed) / (s.cs * 4 + 4)) / 4 * 4, kWinMax);
       // (a window holds the tile's own rows and, on a bilayer, as many of the other sheet)
-      if (ts > 1 && ts * kSellRows > cap) continue;
+      if (ts > 1 && ts * SR > cap) continue;
       csr->win_list.alloc((size_t)(tiles * cap));
       csr->win_cnt.alloc((size_t)tiles);
       LEO_CUDA(cudaMemsetAsync(over.p, 0, sizeof(int), ctx->stream));
       launch(ctx, "win_build", [&] {
-        k_win_list<<<(unsigned)tiles, kWinThreads, list_smem, ctx->stream>>>(n, (int)(ts * kSellRows), rp, col, cap,
+        k_win_list<<<(unsigned)tiles, kWinThreads, list_smem, ctx->stream>>>(n, (int)(ts * SR), rp, col, cap,
                                                                          csr->win_list.p, csr->win_cnt.p, over.p);
       });
       int h = 0;
@@ -1064,24 +1368,69 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
       csr->win_slice_cap = (int)slice_cap;
       break;
     }
+    DevBuf<int32_t> size(s.exact ? 0 : (size_t)nsl * pan_blocks(s.cs));
+    auto panels = [&](int fill) {
+      launch(ctx, "win_build", [&] {
+        k_pan_fill<<<(unsigned)csr->win_tiles, kWinThreads, kPanFillSmem, ctx->stream>>>(
+            n, nsl, csr->win_tile_slices, pan_blocks(s.cs), PC, 32 / s.cs, fill, rp, col, val, csr->win_stride,
+            csr->win_list.p, csr->win_cnt.p, size.p, csr->win_blk.p, csr->win_off.p, csr->win_val.p, csr->win_idx.p,
+            over.p);
+      });
+    };
+    {
+      DevBuf<int64_t> count(nsl);
+      if (s.exact) {
+        launch(ctx, "win_build", [&] {
+          k_slice_len<<<grid_for(nsl, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(n, nsl, rp, kWinChunk, count.p, csr->win_slen.p);
+        });
+      } else {
+        LEO_CUDA(cudaFuncSetAttribute(k_pan_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanFillSmem));
+        csr->win_blk.alloc((size_t)nsl * pan_blocks(s.cs));
+        panels(0);
+        launch(ctx, "win_build", [&] {
+          k_pan_order<<<(unsigned)csr->win_tiles, kWinThreads, 0, ctx->stream>>>(
+              nsl, csr->win_tile_slices, pan_blocks(s.cs), PC, size.p, csr->win_blk.p, csr->win_slen.p, count.p);
+        });
+      }
+      exclusive_scan_i64(ctx, count.p, csr->win_off.p, nsl);
+    }
     int64_t chunks = 0;
+    int twice = 0;
     d2h(ctx, &chunks, csr->win_off.p + nsl, 1);
+    d2h(ctx, &twice, over.p, 1);
     ctx_sync(ctx);
-    const size_t count = (size_t)std::max<int64_t>(chunks, 1) * kSellRows * kWinChunk;
+    if (twice != 0) {
+      csr_drop_win(csr);
+      csr->win_twice = true;
+      return false;
+    }
+    const size_t count = (size_t)std::max<int64_t>(chunks, 1) * SR * PC;  // values
+    const size_t positions = s.exact ? count : count / kPanRows;
     csr->win_val.alloc(count);
-    csr->win_idx.alloc(count);
-    launch(ctx, "win_build", [&] {
-      k_win_fill<<<(unsigned)csr->win_tiles, kWinThreads, (size_t)kWinMax * sizeof(uint32_t), ctx->stream>>>(
-          n, nsl, csr->win_tile_slices, cls, rp, csr->win_off.p, col, perm ? csr->pval32.p : csr->val32.p, csr->win_stride,
-          csr->win_list.p, csr->win_cnt.p, csr->win_val.p, csr->win_idx.p);
-    });
+    csr->win_idx.alloc(positions);
+    if (s.exact) {
+      launch(ctx, "win_build", [&] {
+        k_win_fill<<<(unsigned)csr->win_tiles, kWinThreads, (size_t)kWinMax * sizeof(uint32_t), ctx->stream>>>(
+            n, nsl, csr->win_tile_slices, rp, csr->win_off.p, col, val, csr->win_stride, csr->win_list.p, csr->win_cnt.p,
+            csr->win_val.p, csr->win_idx.p);
+      });
+    } else {
+      LEO_CUDA(cudaMemsetAsync(csr->win_val.p, 0, count * sizeof(float), ctx->stream));
+      LEO_CUDA(cudaMemsetAsync(csr->win_idx.p, 0, positions * sizeof(uint16_t), ctx->stream));
+      panels(1);
+    }
     csr->win_perm = perm;
     csr->win_cs = s.cs;
     csr->win_group = s.group;
-    csr->win_cls = cls;
+    csr->win_exact = s.exact;
   }
   s.group = (int)std::min<int64_t>(s.group, csr->win_tiles);
-  s.smem = win_smem((int)csr->win_stride, csr->win_slice_cap, s.cs);
+  s.smem = win_smem(s, (int)csr->win_stride, csr->win_slice_cap);
+  // Warps that take slices: as few as need the same number of rounds over a tile, in
+  // fours, one to each scheduler (20 slices: 12 warps and 8, not 15 and 5, whose
+  // latency nothing would cover).
+  const int rounds = (csr->win_tile_slices + kPanWarps - 1) / kPanWarps;
+  s.slice_warps = std::min(kPanWarps, ((csr->win_tile_slices + rounds - 1) / rounds + 3) / 4 * 4);
   return true;
 }
 
@@ -1127,7 +1476,8 @@ void csr_drop_win(leo2d_csr* csr) {
   csr->win_cnt.release();
   csr->win_val.release();
   csr->win_idx.release();
-  csr->win_cs = csr->win_group = csr->win_cls = 0;
+  csr->win_blk.release();
+  csr->win_cs = csr->win_group = 0;
 }
 
 static int row_slices(int cols, int cols_used) {
@@ -1148,14 +1498,14 @@ bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols,
   s = RowShape{};
   s.cs = std::min(cols, 32);
   s.slices = row_slices(cols, cols_used);
-  const int64_t n = csr->n, nsl = (n + kSellRows - 1) / kSellRows, most = std::max(1, ctx->sm_count / s.slices);
+  const int64_t n = csr->n, most = std::max(1, ctx->sm_count / s.slices);
   if (!fp64) {
     s.form = kRowWin;
-    s.warps = kWinWarps;
     s.exact = n <= kSmallRows && !perm;
-    // a slice of 16 rows per CTA and up: the rows' latency and the shared-memory
-    // bandwidth are spread over every SM
-    s.group = (int)std::min<int64_t>(most, nsl);
+    s.warps = s.exact ? kWinWarps : kPanWarps;
+    // a slice (16 rows; panels: 64 of 8 columns, 16 of 32) per CTA and up: the rows'
+    // latency and the shared-memory bandwidth are spread over every SM
+    s.group = (int)std::min<int64_t>(most, (n + win_slice_rows(s) - 1) / win_slice_rows(s));
     // the tiled step's row slots per tile and rows per slot (kpm.cu)
     const int lpr = cols / (cols == 8 ? 2 : 4);
     s.dot_slots = (cols == 32 || cols == 64 ? 24 : 8) * (32 / lpr);
@@ -1221,6 +1571,8 @@ void row_run(leo2d_ctx* ctx, const leo2d_csr* csr, const RowShape& s, bool perm,
       a.tile_slices = csr->win_tile_slices;
       a.win_cap = (int)csr->win_stride;
       a.slice_cap = csr->win_slice_cap;
+      a.blk = csr->win_blk.p;
+      a.warps = s.slice_warps;
       a.dot_slots = s.dot_slots;
       a.dot_rows = s.dot_rows;
     }
@@ -1247,7 +1599,7 @@ void row_run(leo2d_ctx* ctx, const leo2d_csr* csr, const RowShape& s, bool perm,
     }
   };
   if (fp64) go((double*)nullptr, s.form == kRowSmall ? small_kernel(s.cs) : sell_kernel(s.cs));
-  else go((float*)nullptr, s.exact ? win_kernel<true>(s.cs) : win_kernel<false>(s.cs));
+  else go((float*)nullptr, s.exact ? win_kernel(s.cs) : pan_kernel(s.cs));
 }
 
 }  // namespace leo2d
