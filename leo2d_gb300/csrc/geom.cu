@@ -731,26 +731,60 @@ __device__ void block_bitonic_sort(uint64_t* keys, int n2) {
   }
 }
 
-template <bool kFill>
+// A CTA per row. kMode as in k_flake_rows.
+// Bound by the FP64 pipe (an instruction per 16 cycles and SM), so FP64 is left to the
+// pairs that have a hopping, each evaluated once and on full warps: the cells nearest
+// to the row's images come from one lane an image, FP32 distances sort out the
+// candidates (as in k_flake_rows), and the hoppings are taken after the sort, which
+// puts the interlayer pairs next to each other. With every thread finding its
+// image's cells and evaluating its own candidate, in a counting and a filling pass, the
+// rows of a 2188-orbital cell of the reference model took 1.55 ms (0.23 now).
+template <int kMode>
 __global__ void __launch_bounds__(256) k_periodic_rows(const __grid_constant__ GeomDev G, int64_t n,
                                                        const int32_t* __restrict__ grid4,
                                                        const double* __restrict__ pos,
-                                                       const double* __restrict__ spos, int cap,
+                                                       const float4* __restrict__ pos32,
+                                                       const double* __restrict__ spos,
+                                                       const float4* __restrict__ spos32, int cap, int hop_cap,
                                                        RowOut out, int* status) {
-  extern __shared__ uint64_t keys[];
-  __shared__ int cnt, n_intra_s, n_inter_s, n_run;
+  constexpr bool kFill = kMode != 0, kPad = kMode == 2;
+  extern __shared__ uint64_t keys[];  // [cap] | hoppings [hop_cap] | nearest cells, FP32 shift [images][6 + 2]
+  double* const hop = reinterpret_cast<double*>(keys + cap);
+  int* const near = reinterpret_cast<int*>(hop + hop_cap);
+  __shared__ int cnt, n_intra_s, n_inter_s;
   __shared__ int warp_sums[8];
   const int ss = G.sc_search;
   const int n_img = (2 * ss + 1) * (2 * ss + 1);
+  constexpr float kWinLo = (float)(kInterCutoff - kPrefilterMargin), kWinHi = (float)(kInterCutoff + kPrefilterMargin);
+  constexpr float kHopHi = 8.0f + kPrefilterMargin;  // (every hopping is zero from 8 A on)
   for (int64_t row = blockIdx.x; row < n; row += gridDim.x) {
     if (threadIdx.x == 0) { cnt = 0; n_intra_s = 0; n_inter_s = 0; }
-    __syncthreads();
     const int ih = grid4[4 * row], jh = grid4[4 * row + 1], l0 = grid4[4 * row + 2],
               s = grid4[4 * row + 3];
     const SheetDev& sh = G.sh[s];
-    double lp[3];
-    pos_grid(sh, ih, jh, l0, lp);
-    const double khx = pos[3 * row], khy = pos[3 * row + 1], khz = pos[3 * row + 2];
+    const double khx = pos[3 * row], khy = pos[3 * row + 1];
+    for (int img = threadIdx.x; img < n_img; img += blockDim.x) {
+      int dxs, dys;
+      image_of(img, ss, dxs, dys);
+      double lp[3];
+      pos_grid(sh, ih, jh, l0, lp);
+      const double own[3] = {lp[0] + (dxs * sh.sc[0][0] + dys * sh.sc[1][0]),
+                             lp[1] + (dxs * sh.sc[0][1] + dys * sh.sc[1][1]), lp[2]};
+      near[8 * img] = find_nearest_sheet(sh, own, 0);
+      near[8 * img + 1] = find_nearest_sheet(sh, own, 1);
+      const double scx = dxs * G.supercell[0][0] + dys * G.supercell[1][0];
+      const double scy = dxs * G.supercell[0][1] + dys * G.supercell[1][1];
+      const double ph[3] = {khx + scx, khy + scy, 0.0};
+      near[8 * img + 6] = __float_as_int((float)scx);
+      near[8 * img + 7] = __float_as_int((float)scy);
+      for (int side_k = 0; side_k < 2; ++side_k) {
+        const int s0 = side_k == 0 ? s - 1 : s + 1;
+        if (s0 < 0 || s0 >= G.S) continue;
+        near[8 * img + 2 + 2 * side_k] = find_nearest_h(G.sh[s0], ph, 0);
+        near[8 * img + 3 + 2 * side_k] = find_nearest_h(G.sh[s0], ph, 1);
+      }
+    }
+    __syncthreads();
 
     // intralayer candidates of every image (Sheet::getIntraPairs)
     const int side = 2 * kIntraSearch;
@@ -759,67 +793,65 @@ __global__ void __launch_bounds__(256) k_periodic_rows(const __grid_constant__ G
       const int img = c / per_img, cc = c % per_img;
       int dxs, dys;
       image_of(img, ss, dxs, dys);
-      const double scx = dxs * sh.sc[0][0] + dys * sh.sc[1][0];
-      const double scy = dxs * sh.sc[0][1] + dys * sh.sc[1][1];
-      double ph[3] = {lp[0] + scx, lp[1] + scy, lp[2]};
-      const int i0 = find_nearest_sheet(sh, ph, 0), j0 = find_nearest_sheet(sh, ph, 1);
       const int l = cc % sh.n_orb;
-      const int j = j0 - kIntraSearch + (cc / sh.n_orb) % side;
-      const int i = i0 - kIntraSearch + cc / (sh.n_orb * side);
+      const int j = near[8 * img + 1] - kIntraSearch + (cc / sh.n_orb) % side;
+      const int i = near[8 * img] - kIntraSearch + cc / (sh.n_orb * side);
       const int k2 = grid_to_index(sh, i, j, l);
       if (k2 == -1) continue;
       int gd0 = i - ih, gd1 = j - jh;
       gd0 = gd0 - dxs * sh.stride[0][0] - dys * sh.stride[1][0];
       gd1 = gd1 - dxs * sh.stride[0][1] - dys * sh.stride[1][1];
-      const double raw = intralayer(G.model, l0, l, gd0, gd1);
-      const bool keep = raw != 0 || (dxs == 0 && dys == 0);
-      if (!keep) continue;
+      const bool nonzero = t_nonzero(intralayer(G.model, l0, l, gd0, gd1));
+      if (!nonzero && (dxs != 0 || dys != 0)) continue;
       atomicAdd(&n_intra_s, 1);
       const int64_t k2g = k2 + sh.base;
-      if (!G.keep_zeros) {
-        const double t = k2g == row ? (raw + G.shift) / G.rescale : raw / G.rescale;
-        if (t == 0 && k2g != row) continue;
-      }
+      if (!G.keep_zeros && !nonzero && k2g != row) continue;
       const int slot = atomicAdd(&cnt, 1);
       if (slot < cap) keys[slot] = ((uint64_t)k2g << 16) | (uint64_t)img;
     }
-    // interlayer candidates of every image (Hstruct::getInterPairs)
-    for (int img = 0; img < n_img; ++img) {
-      int dxs, dys;
-      image_of(img, ss, dxs, dys);
-      const double scx = dxs * G.supercell[0][0] + dys * G.supercell[1][0];
-      const double scy = dxs * G.supercell[0][1] + dys * G.supercell[1][1];
-      const double ph[3] = {khx + scx, khy + scy, khz};
-      for (int side_k = 0; side_k < 2; ++side_k) {
-        const int s0 = side_k == 0 ? s - 1 : s + 1;
-        if (s0 < 0 || s0 >= G.S) continue;
-        const SheetDev& o0 = G.sh[s0];
-        const int i0 = find_nearest_h(o0, ph, 0), j0 = find_nearest_h(o0, ph, 1);
-        const int ilo = max(0, i0 - kInterSearch), ihi = min(o0.H, i0 + kInterSearch);
-        const int jlo = max(0, j0 - kInterSearch), jhi = min(o0.W, j0 + kInterSearch);
-        if (ihi <= ilo || jhi <= jlo) continue;
-        const int wj = jhi - jlo;
-        const int nc = (ihi - ilo) * wj * o0.n_orb;
-        for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-          const int l = c % o0.n_orb;
-          const int j = jlo + (c / o0.n_orb) % wj;
-          const int i = ilo + c / (o0.n_orb * wj);
-          const int k2 = grid_to_index(o0, i, j, l);
-          if (k2 == -1) continue;
-          const int64_t kk = k2 + o0.base;
+    // interlayer candidates of every image (Hstruct::getInterPairs), the sheet below
+    // and the sheet above; without KEEP_ZEROS those that may have a hopping
+    const int wide = 2 * kInterSearch;
+    for (int side_k = 0; side_k < 2; ++side_k) {
+      const int s0 = side_k == 0 ? s - 1 : s + 1;
+      if (s0 < 0 || s0 >= G.S) continue;
+      const SheetDev& o0 = G.sh[s0];
+      const int per = wide * wide * o0.n_orb;
+      for (int c = threadIdx.x; c < n_img * per; c += blockDim.x) {
+        const int img = c / per, cc = c % per;
+        const int l = cc % o0.n_orb;
+        const int j = near[8 * img + 3 + 2 * side_k] - kInterSearch + (cc / o0.n_orb) % wide;
+        const int i = near[8 * img + 2 + 2 * side_k] - kInterSearch + cc / (o0.n_orb * wide);
+        const int k2 = grid_to_index(o0, i, j, l);
+        if (k2 == -1) continue;
+        const int64_t kk = k2 + o0.base;
+        const float4 q = pos32[kk], h = pos32[row];
+        const float scx = __int_as_float(near[8 * img + 6]), scy = __int_as_float(near[8 * img + 7]);
+        const float dxf = q.x - (h.x + scx), dyf = q.y - (h.y + scy);
+        const float d2f = dxf * dxf + dyf * dyf;
+        if (d2f > kWinHi * kWinHi) continue;
+        if (d2f >= kWinLo * kWinLo) {
+          int dxs, dys;
+          image_of(img, ss, dxs, dys);
+          const double px = khx + (dxs * G.supercell[0][0] + dys * G.supercell[1][0]);
+          const double py = khy + (dxs * G.supercell[0][1] + dys * G.supercell[1][1]);
           const double x2 = pos[3 * kk], y2 = pos[3 * kk + 1];
-          if (!((x2 - ph[0]) * (x2 - ph[0]) + (y2 - ph[1]) * (y2 - ph[1]) <
-                kInterCutoff * kInterCutoff))
-            continue;
-          atomicAdd(&n_inter_s, 1);
-          if (!G.keep_zeros) {
-            double xx, yy;
-            const double t = periodic_value(G, row, grid4, spos, true, kk, img, xx, yy);
-            if (t == 0) continue;
-          }
-          const int slot = atomicAdd(&cnt, 1);
-          if (slot < cap) keys[slot] = kKeyInter | ((uint64_t)kk << 16) | (uint64_t)img;
+          if (!((x2 - px) * (x2 - px) + (y2 - py) * (y2 - py) < kInterCutoff * kInterCutoff)) continue;
         }
+        atomicAdd(&n_inter_s, 1);
+        if (!G.keep_zeros) {
+          float hd2 = d2f;
+          float hz = q.z - h.z;
+          if (G.shifted) {
+            const float4 sq = spos32[kk], sr = spos32[row];
+            const float ax = sq.x - (sr.x + scx), ay = sq.y - (sr.y + scy);
+            hd2 = ax * ax + ay * ay;
+            hz = sq.z - sr.z;
+          }
+          if ((G.model == LEO2D_MODEL_SIMPLE ? hd2 + hz * hz : hd2) > kHopHi * kHopHi) continue;
+        }
+        const int slot = atomicAdd(&cnt, 1);
+        if (slot < cap) keys[slot] = kKeyInter | ((uint64_t)kk << 16) | (uint64_t)img;
       }
     }
     __syncthreads();
@@ -834,29 +866,36 @@ __global__ void __launch_bounds__(256) k_periodic_rows(const __grid_constant__ G
     for (int i = m + threadIdx.x; i < n2; i += blockDim.x) keys[i] = kKeyPad;
     __syncthreads();
     block_bitonic_sort(keys, n2);
-
-    // one output entry per run of equal (intra/inter, column)
-    if (!kFill) {
-      int local = 0;
-      for (int p = threadIdx.x; p < m; p += blockDim.x)
-        if (p == m - 1 || (keys[p] >> 16) != (keys[p + 1] >> 16)) ++local;
-      if (threadIdx.x == 0) n_run = 0;
+    auto value = [&](int p) {
+      const uint64_t key = keys[p];
+      double x1, y1;
+      return periodic_value(G, row, grid4, spos, (key & kKeyInter) != 0, (int64_t)((key >> 16) & 0xffffffffull),
+                            (int)(key & 0xffffull), x1, y1);
+    };
+    const bool held = m <= hop_cap;  // (a search so wide that the hoppings have no room takes them again)
+    if (held) {
+      for (int p = threadIdx.x; p < m; p += blockDim.x) hop[p] = value(p);
       __syncthreads();
-      atomicAdd(&n_run, local);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        out.cnt_ent[row] = n_run;
-        out.cnt_intra[row] = n_intra_s;
-        out.cnt_inter[row] = n_inter_s;
-      }
-      __syncthreads();
-      continue;
     }
-    // fill: ordered slots by a block-wide scan of run-end flags, chunk by chunk
-    int64_t base_out = out.rowptr[row];
+
+    // one output entry per run of equal (intra/inter, column), unless it is an
+    // interlayer run without a hopping; ordered slots by a block-wide scan of the
+    // flags at the runs' ends, chunk by chunk
+    int64_t base_out = kPad ? row * (int64_t)out.pad_cap : (kFill ? out.rowptr[row] : 0);
+    const int64_t pad_end = base_out + out.pad_cap;
+    int entries = 0;
     for (int p0 = 0; p0 < m; p0 += blockDim.x) {
       const int p = p0 + threadIdx.x;
-      const bool end = p < m && (p == m - 1 || (keys[p] >> 16) != (keys[p + 1] >> 16));
+      bool end = p < m && (p == m - 1 || (keys[p] >> 16) != (keys[p + 1] >> 16));
+      int q = p;
+      if (end) {
+        while (q > 0 && (keys[q - 1] >> 16) == (keys[p] >> 16)) --q;
+        if ((keys[p] & kKeyInter) != 0 && !G.keep_zeros) {
+          bool any = false;
+          for (int e = q; e <= p; ++e) any |= t_nonzero(held ? hop[e] : value(e));
+          end = any;
+        }
+      }
       const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
       const unsigned bal = __ballot_sync(0xffffffffu, end);
       if (lane == 0) warp_sums[warp] = __popc(bal);
@@ -867,17 +906,18 @@ __global__ void __launch_bounds__(256) k_periodic_rows(const __grid_constant__ G
         total += warp_sums[w];
       }
       before += __popc(bal & ((1u << lane) - 1u));
-      if (end) {
-        int q = p;
-        while (q > 0 && (keys[q - 1] >> 16) == (keys[p] >> 16)) --q;
-        const bool inter = (keys[p] & kKeyInter) != 0;
+      const int64_t e_out = base_out + before;
+      if (kFill && end && (!kPad || e_out < pad_end)) {
         const int64_t k2 = (int64_t)((keys[p] >> 16) & 0xffffffffull);
         double v = 0.0, vdx = 0.0, vdy = 0.0, vim = 0.0;
         for (int e = q; e <= p; ++e) {
-          const int img = (int)(keys[e] & 0xffffull);
-          double x1, y1;
-          const double t = periodic_value(G, row, grid4, spos, inter, k2, img, x1, y1);
-          if (t != 0) {
+          const double t = held ? hop[e] : value(e);
+          if (!t_nonzero(t)) continue;
+          if (G.cpx || G.with_dx) {
+            int dxs, dys;
+            image_of((int)(keys[e] & 0xffffull), ss, dxs, dys);
+            const double x1 = spos[3 * row] + (dxs * G.supercell[0][0] + dys * G.supercell[1][0]);
+            const double y1 = spos[3 * row + 1] + (dxs * G.supercell[0][1] + dys * G.supercell[1][1]);
             if (G.cpx) {
               // std::polar(t, phase) summed over the images, the phase the Peierls
               // phase plus k.(r2 - r1) with r1 the row's orbital shifted by the
@@ -889,25 +929,33 @@ __global__ void __launch_bounds__(256) k_periodic_rows(const __grid_constant__ G
               sincos(ph, &sn, &cs);
               v += t * cs;
               vim += t * sn;
-            } else {
-              v += t;
             }
-            vdx += (x1 - spos[3 * k2]) * t;
-            vdy += (y1 - spos[3 * k2 + 1]) * t;
+            if (G.with_dx) {
+              vdx += (x1 - spos[3 * k2]) * t;
+              vdy += (y1 - spos[3 * k2 + 1]) * t;
+            }
           }
+          if (!G.cpx) v += t;
         }
-        const int64_t e = base_out + before;
-        out.col[e] = (int32_t)k2;
-        out.val[e] = v;
-        if (G.cpx) out.val_im[e] = vim;
+        out.col[e_out] = (int32_t)k2;
+        out.val[e_out] = v;
+        if (G.cpx) out.val_im[e_out] = vim;
         if (G.with_dx) {
-          out.dx[e] = vdx;
-          out.dy[e] = vdy;
+          out.dx[e_out] = vdx;
+          out.dy[e_out] = vdy;
         }
       }
       base_out += total;
+      entries += total;
       __syncthreads();
     }
+    if ((!kFill || kPad) && threadIdx.x == 0) {
+      out.cnt_ent[row] = entries;
+      out.cnt_intra[row] = n_intra_s;
+      out.cnt_inter[row] = n_inter_s;
+      if (kPad && entries > out.pad_cap) atomicOr(out.overflow, 1);
+    }
+    __syncthreads();  // the counters and the keys are read
   }
 }
 
@@ -1204,7 +1252,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
         cnt_inter(std::max<int64_t>(n, 1));
     csr_alloc_rowptr(ctx, csr, n);
     RowOut ro{cnt_ent.p, cnt_intra.p, cnt_inter.p, csr->rowptr.p, nullptr, nullptr, nullptr, nullptr, nullptr};
-    int cap = 0;
+    int cap = 0, hop_cap = 0;
     size_t smem = 0;
     if (G.bc == 1) {
       const int n_img = (2 * G.sc_search + 1) * (2 * G.sc_search + 1);
@@ -1213,18 +1261,21 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
                           neigh * (2 * kInterSearch) * (2 * kInterSearch) * 2);
       cap = 1;
       while (cap < need) cap <<= 1;
-      smem = (size_t)cap * sizeof(uint64_t);
-      LEO_REQUIRE(smem <= ctx->smem_optin, "periodic search too large for shared memory");
-      LEO_CUDA(cudaFuncSetAttribute(k_periodic_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      LEO_CUDA(cudaFuncSetAttribute(k_periodic_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const size_t fixed = (size_t)cap * sizeof(uint64_t) + (size_t)n_img * 8 * sizeof(int), room = ctx->smem_optin - 1024;
+      LEO_REQUIRE(fixed <= room, "periodic search too large for shared memory");
+      hop_cap = (int)std::min<size_t>((size_t)need, (room - fixed) / sizeof(double));
+      smem = fixed + (size_t)hop_cap * sizeof(double);
+      allow_smem(ctx, (const void*)k_periodic_rows<0>);
+      allow_smem(ctx, (const void*)k_periodic_rows<1>);
+      allow_smem(ctx, (const void*)k_periodic_rows<2>);
     }
     // rows a warp takes at a time (k_flake_rows): as many as leave every one of the
     // 24 resident warps of an SM two runs, at most a warp's lanes
     const int run = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / ((int64_t)ctx->sm_count * 48)));
     const unsigned rows_grid = grid_for(n, kRowWarps * run, (int64_t)ctx->sm_count * 64);
-    DevBuf<float4> pos32(G.bc == 0 ? std::max<int64_t>(n, 1) : 1);
-    DevBuf<float4> spos32(G.bc == 0 && G.shifted ? std::max<int64_t>(n, 1) : 0);
-    if (G.bc == 0 && n > 0)
+    DevBuf<float4> pos32(std::max<int64_t>(n, 1));
+    DevBuf<float4> spos32(G.shifted ? std::max<int64_t>(n, 1) : 0);
+    if (n > 0)
       launch(ctx, "pos32", [&] {
         k_pos32<<<grid_for(n, 256, (int64_t)ctx->sm_count * 32), 256, 0, ctx->stream>>>(csr->pos.p, n, pos32.p);
         if (G.shifted)
@@ -1236,18 +1287,18 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
       if (G.shifted) csr->pos = std::move(spos_buf);
     };
     const unsigned cta_grid = grid_for(n, 1, (int64_t)ctx->sm_count * 8);
-    // A flake of the simple model without stored zeros (about 67 entries per
-    // row) takes one pass: rows are filled into padded arrays of kPadCap
-    // entries while they are counted, then compacted. A row with more entries,
+    // Without stored zeros, a flake of the simple model (about 67 entries per
+    // row) and a supercell take one pass: rows are filled into padded arrays of
+    // `pad` entries while they are counted, then compacted. A row with more entries,
     // or padded arrays too large for a quarter of free memory, takes the
     // count and fill passes.
-    constexpr int kPadCap = 96;
-    if (G.bc == 0 && n > 0 && G.model == LEO2D_MODEL_SIMPLE && !G.keep_zeros) {
+    const int pad = G.bc == 0 ? 96 : 256;
+    if (n > 0 && !G.keep_zeros && (G.bc != 0 || G.model == LEO2D_MODEL_SIMPLE)) {
       const size_t per = sizeof(int32_t) + sizeof(double) * (1 + (G.with_dx ? 2 : 0) + (G.cpx ? 1 : 0));
       size_t fr = 0, tot = 0;
       device_mem_info(&fr, &tot);
-      if ((size_t)n * kPadCap * per <= fr / 4) {
-        const size_t pn = (size_t)n * kPadCap;
+      if ((size_t)n * pad * per <= fr / 4) {
+        const size_t pn = (size_t)n * pad;
         DevBuf<int32_t> pcol(pn);
         DevBuf<double> pval(pn), pdx(G.with_dx ? pn : 0), pdy(G.with_dx ? pn : 0), pim(G.cpx ? pn : 0);
         DevBuf<int> overflow(1);
@@ -1258,10 +1309,16 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
         rp.dx = pdx.p;
         rp.dy = pdy.p;
         rp.val_im = pim.p;
-        rp.pad_cap = kPadCap;
+        rp.pad_cap = pad;
         rp.overflow = overflow.p;
-        launch(ctx, "flake_rows_fill", [&] {
-          k_flake_rows<2><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
+        if (G.bc != 0)
+          launch(ctx, "periodic_rows_fill", [&] {
+            k_periodic_rows<2><<<cta_grid, 256, smem, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, pos32.p, spos,
+                                                                     spos32p, cap, hop_cap, rp, ctx->status.p);
+          });
+        else
+          launch(ctx, "flake_rows_fill", [&] {
+            k_flake_rows<2><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, rp);
         });
         int over = 0;
@@ -1277,6 +1334,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
           csr->n_inter = reduce_sum_i64(ctx, cnt_inter.p, n);
           csr_alloc_entries(ctx, csr, nnz, G.with_dx != 0);
           csr->complex_h = G.cpx != 0;
+          csr->nonhermitian = csr->complex_h && G.bc == 1 && G.b_field != 0.0;
           if (csr->complex_h) {
             csr->val_im64.alloc(nnz + kCsrPad);
             LEO_CUDA(cudaMemsetAsync(csr->val_im64.p, 0, (nnz + kCsrPad) * sizeof(double), ctx->stream));
@@ -1289,7 +1347,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
           fo.val_im = csr->val_im64.p;
           launch(ctx, "unpad_rows", [&] {
             k_unpad_rows<<<grid_for(n * 32, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-                n, kPadCap, csr->rowptr.p, pcol.p, pval.p, pdx.p, pdy.p, pim.p, fo);
+                n, pad, csr->rowptr.p, pcol.p, pval.p, pdx.p, pdy.p, pim.p, fo);
           });
           ctx_check_status(ctx, "leo2d_build_csr (single pass)");
           keep_shifted_positions();
@@ -1307,8 +1365,8 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
         });
       else
         launch(ctx, "periodic_rows_count", [&] {
-          k_periodic_rows<false><<<cta_grid, 256, smem, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, spos,
-                                                                       cap, ro, ctx->status.p);
+          k_periodic_rows<0><<<cta_grid, 256, smem, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, pos32.p, spos,
+                                                                   spos32p, cap, hop_cap, ro, ctx->status.p);
         });
     }
     ctx_check_status(ctx, "leo2d_build_csr (count)");
@@ -1339,8 +1397,8 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
         });
       else
         launch(ctx, "periodic_rows_fill", [&] {
-          k_periodic_rows<true><<<cta_grid, 256, smem, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, spos,
-                                                                      cap, ro, ctx->status.p);
+          k_periodic_rows<1><<<cta_grid, 256, smem, ctx->stream>>>(G, n, csr->grid4.p, csr->pos.p, pos32.p, spos,
+                                                                   spos32p, cap, hop_cap, ro, ctx->status.p);
         });
     }
     ctx_check_status(ctx, "leo2d_build_csr (fill)");
