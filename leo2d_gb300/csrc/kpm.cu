@@ -199,6 +199,13 @@ template <typename T>
 void enqueue_steps(Recursion& r) {
   leo2d_ctx* ctx = r.ctx;
   const int C = r.shape.cols;
+  if constexpr (std::is_same<T, float>::value) {
+    if (!r.direct && rb_one_fits(ctx, r.csr, r.shape, r.grid)) {
+      rb_run_one(ctx, r.csr, r.steps, reinterpret_cast<float*>(r.buf(0)), reinterpret_cast<float*>(r.buf(1)),
+                 r.dots.p);
+      return;
+    }
+  }
   for (int k = 0; k < r.steps; ++k) {
     if constexpr (std::is_same<T, float>::value) {
       if (r.direct) {

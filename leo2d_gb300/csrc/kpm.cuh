@@ -112,6 +112,11 @@ unsigned rb_grid(leo2d_ctx* ctx, const leo2d_csr* csr, int warps);
 // With out2 (the velocity step; csr_build_rb_xs first, smem and grid for
 // velocity stages) the launch also writes out2 = D T_n, D_ij = (x_i - x_j) H~_ij
 // (a flake's dxH), from the same gathers, and computes no moment dots.
+// Whether every step of the run fits one launch of one CTA (a small complex matrix:
+// matrix and vectors in shared memory, up to about 40 row blocks), and that launch:
+// T_0 in x0, dots[steps][64].
+bool rb_one_fits(const leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape, unsigned grid);
+void rb_run_one(leo2d_ctx* ctx, const leo2d_csr* csr, int steps, float* x0, float* x1, double* dots);
 void rb_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape, unsigned grid, size_t smem,
                     const float* tn, float* tp, const float* tprev, int first, float alpha, double* partials,
                     const double* prev_partials, double* prev_dots, float* out2 = nullptr);

@@ -83,6 +83,76 @@ struct RbArgs {
   int never_wait;  // test hook: wait on a barrier that nobody completes
 };
 
+// A warp's moment dots: FP32 over kFlush row blocks (64 rows), then pairs of FP32 over
+// the CTA (PairSum), FP64 beyond. A flush sums the four groups' FP32 partials and
+// hands column `lane` to lane `lane`.
+struct RbDots {
+  static constexpr int kFlush = 16;
+  PairSum d0, d1;                                          // column `lane`
+  float e0[4] = {0.f, 0.f, 0.f, 0.f}, e1[4] = {0.f, 0.f, 0.f, 0.f};  // columns 4q..4q+3, this lane's rows
+  int since = 0;
+  __device__ __forceinline__ void add(const float4& xn, const float4& y) {
+    e0[0] += xn.x * xn.x;
+    e0[1] += xn.y * xn.y;
+    e0[2] += xn.z * xn.z;
+    e0[3] += xn.w * xn.w;
+    e1[0] += y.x * xn.x;
+    e1[1] += y.y * xn.y;
+    e1[2] += y.z * xn.z;
+    e1[3] += y.w * xn.w;
+  }
+  __device__ __forceinline__ void next(int lane) {  // a row block is done (warp-uniform)
+    if (++since == kFlush) {
+      since = 0;
+      flush(lane);
+    }
+  }
+  __device__ __forceinline__ void flush(int lane) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      e0[c] += __shfl_xor_sync(0xffffffffu, e0[c], 8);
+      e1[c] += __shfl_xor_sync(0xffffffffu, e1[c], 8);
+      e0[c] += __shfl_xor_sync(0xffffffffu, e0[c], 16);
+      e1[c] += __shfl_xor_sync(0xffffffffu, e1[c], 16);
+    }
+    // column `lane` = 4 * (lane >> 2) + (lane & 3) lives in lane (lane >> 2)
+    float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float s0 = __shfl_sync(0xffffffffu, e0[c], lane >> 2);
+      const float s1 = __shfl_sync(0xffffffffu, e1[c], lane >> 2);
+      if ((lane & 3) == c) {
+        v0 = s0;
+        v1 = s1;
+      }
+    }
+    d0.add(v0);
+    d1.add(v1);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
+  }
+};
+
+// Reduce-scatter over the four groups of 8 lanes: group g keeps row g.
+__device__ __forceinline__ void rb_scatter(const float (&p)[4][4], float (&h)[4], int g) {
+  const bool upper = g >= 2, odd = (g & 1) != 0;
+  float hh[2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float send = upper ? p[i][c] : p[2 + i][c];
+      const float keep = upper ? p[2 + i][c] : p[i][c];
+      hh[i][c] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const float send = odd ? hh[0][c] : hh[1][c];
+    const float keep = odd ? hh[1][c] : hh[0][c];
+    h[c] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+}
+
 // One CTA's share of a step: CTA `bid` of `nblk` working on the matrix of `a`
 // (the whole grid for one matrix, a block group of a batched launch).
 template <int WARPS, bool PACKED, int U, bool CPX = false, bool DJ = false>
@@ -142,39 +212,7 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
   const float alpha = a.alpha != 0.f ? a.alpha : (a.first ? 1.f : 2.f);
   const float* tprev = a.tprev ? a.tprev : a.tp;
   const float* tq = a.tn + 4 * q;
-  // dots: FP32 over kDotFlush row blocks (64 rows), then pairs of FP32 over the
-  // CTA (PairSum), FP64 beyond. A flush sums the four groups' FP32 partials and
-  // hands column `lane` to lane `lane`.
-  constexpr int kDotFlush = 16;
-  PairSum d0, d1;             // column `lane`
-  float e0[4], e1[4];         // columns 4q..4q+3, this lane's rows
-  int since_flush = 0;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
-  auto flush = [&]() {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      e0[c] += __shfl_xor_sync(0xffffffffu, e0[c], 8);
-      e1[c] += __shfl_xor_sync(0xffffffffu, e1[c], 8);
-      e0[c] += __shfl_xor_sync(0xffffffffu, e0[c], 16);
-      e1[c] += __shfl_xor_sync(0xffffffffu, e1[c], 16);
-    }
-    // column `lane` = 4 * (lane >> 2) + (lane & 3) lives in lane (lane >> 2)
-    float v0 = 0.f, v1 = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float s0 = __shfl_sync(0xffffffffu, e0[c], lane >> 2);
-      const float s1 = __shfl_sync(0xffffffffu, e1[c], lane >> 2);
-      if ((lane & 3) == c) {
-        v0 = s0;
-        v1 = s1;
-      }
-    }
-    d0.add(v0);
-    d1.add(v1);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) e0[c] = e1[c] = 0.f;
-  };
+  RbDots dots;
 
   bool gave_up = false;
   if (a.never_wait && !bounded_wait(&never, 0u, a.spin_limit)) {
@@ -266,35 +304,16 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
           if (u < rem) add(x[u], 4 * (b + u));
         (void)vb;
       }
-      // reduce-scatter over the four groups: group g keeps row g
-      const bool upper = g >= 2, odd = (g & 1) != 0;
-      auto scatter = [&](const float (&p)[4][4], float (&h)[4]) {
-        float hh[2][4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float send = upper ? p[i][c] : p[2 + i][c];
-            const float keep = upper ? p[2 + i][c] : p[i][c];
-            hh[i][c] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-          }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float send = odd ? hh[0][c] : hh[1][c];
-          const float keep = odd ? hh[1][c] : hh[0][c];
-          h[c] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-        }
-      };
       float h[4];
       {
         float p[4][4];
         acc.get(p);
-        scatter(p, h);
+        rb_scatter(p, h, g);
       }
       if constexpr (DJ) {
         float p[4][4], hj[4];
         accj.get(p);
-        scatter(p, hj);
+        rb_scatter(p, hj, g);
         if (ok) st_na4(a.out2 + row * C + 4 * q, make_float4(hj[0], hj[1], hj[2], hj[3]));
       }
       if (ok) {
@@ -307,23 +326,10 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
         }
         st_na4(a.tp + row * C + 4 * q, y);
         if constexpr (!DJ) {
-          const float4 xn = ldg4(tq + row * C);
-          e0[0] += xn.x * xn.x;
-          e0[1] += xn.y * xn.y;
-          e0[2] += xn.z * xn.z;
-          e0[3] += xn.w * xn.w;
-          e1[0] += y.x * xn.x;
-          e1[1] += y.y * xn.y;
-          e1[2] += y.z * xn.z;
-          e1[3] += y.w * xn.w;
+          dots.add(ldg4(tq + row * C), y);
         }
       }
-      if constexpr (!DJ) {
-        if (++since_flush == kDotFlush) {  // warp-uniform
-          since_flush = 0;
-          flush();
-        }
-      }
+      if constexpr (!DJ) dots.next(lane);
     }
     // release the stage; the last warp refills it
     __syncwarp();
@@ -345,13 +351,13 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
 
   // (the velocity step computes no moment dots and writes no partials)
   if constexpr (DJ) return;
-  flush();
+  dots.flush(lane);
   // the warps' sums through the stages' memory (every copy has landed), added in
   // warp order (deterministic)
   __syncthreads();
   PairSum* ws = reinterpret_cast<PairSum*>(smem);  // [WARPS][2C]
-  ws[warp * 2 * C + 2 * lane] = d0;
-  ws[warp * 2 * C + 2 * lane + 1] = d1;
+  ws[warp * 2 * C + 2 * lane] = dots.d0;
+  ws[warp * 2 * C + 2 * lane + 1] = dots.d1;
   __syncthreads();
   for (int t = threadIdx.x; t < 2 * C; t += NT) {
     PairSum s;
@@ -364,6 +370,112 @@ __device__ __forceinline__ void rb_body(const RbArgs& a, const int bid, const in
 template <int WARPS, bool PACKED, int U, bool CPX = false, bool DJ = false>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_cheb_rb(const __grid_constant__ RbArgs a) {
   rb_body<WARPS, PACKED, U, CPX, DJ>(a, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// Every step of a small complex matrix (a k point of a small cell) in one launch of
+// one CTA: the matrix and both vector buffers stay in shared memory. The arithmetic
+// is that of rb_body on one CTA: the same batches, sums and orders, which the density of
+// a small cell needs (its reconstruction amplifies the moments' rounding by the
+// order and more). A step of its own launch took 7 us on a 76-orbital cell, nearly all
+// of it the launch, the copy of the matrix and L2 latency; here 3.5 us, half of it the
+// issue slots of the products on one SM.
+struct RbOneArgs {
+  int64_t n;
+  int nrb, steps;
+  int64_t slots;
+  const int64_t* __restrict__ off;
+  const unsigned char* __restrict__ data;
+  const float* __restrict__ im;
+  float* x0;  // T_k for even k, in and out
+  float* x1;
+  double* __restrict__ dots;  // [steps][2C]
+};
+constexpr int kRbOneWarps = 24;
+
+size_t rb_one_smem(int64_t n, int64_t nrb, int64_t slots) {
+  return 2 * (size_t)n * 32 * sizeof(float) + (size_t)slots * (kRbSlotBytes + kRbRows * sizeof(float)) +
+         2 * (size_t)kRbOneWarps * 64 * sizeof(PairSum) + ((size_t)nrb + 1) * sizeof(int);
+}
+
+__global__ void __launch_bounds__(kRbOneWarps * 32, 1) k_cheb_rb_one(const __grid_constant__ RbOneArgs a) {
+  constexpr int C = 32, WARPS = kRbOneWarps, NT = WARPS * 32, U = 4;
+  extern __shared__ __align__(128) unsigned char smem[];
+  float* t0 = reinterpret_cast<float*>(smem);
+  float* t1 = t0 + a.n * C;
+  unsigned char* data = reinterpret_cast<unsigned char*>(t1 + a.n * C);
+  float4* im = reinterpret_cast<float4*>(data + a.slots * kRbSlotBytes);
+  PairSum* ws = reinterpret_cast<PairSum*>(im + a.slots);  // [2][WARPS][2C]
+  int* off = reinterpret_cast<int*>(ws + 2 * WARPS * 2 * C);
+  for (int i = threadIdx.x; i < a.n * (C / 4); i += NT)
+    reinterpret_cast<float4*>(t0)[i] = reinterpret_cast<const float4*>(a.x0)[i];
+  for (int i = threadIdx.x; i < a.slots * kRbSlotBytes / 16; i += NT)
+    reinterpret_cast<uint4*>(data)[i] = reinterpret_cast<const uint4*>(a.data)[i];
+  for (int i = threadIdx.x; i < a.slots; i += NT) im[i] = reinterpret_cast<const float4*>(a.im)[i];
+  for (int i = threadIdx.x; i <= a.nrb; i += NT) off[i] = (int)a.off[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 3, q = lane & 7;
+  for (int k = 0; k < a.steps; ++k) {
+    const float* tn = k & 1 ? t1 : t0;
+    float* tp = k & 1 ? t0 : t1;
+    const float alpha = k == 0 ? 1.f : 2.f;
+    const float* tq = tn + 4 * q;
+    RbDots dots;
+    for (int rb = warp; rb < a.nrb; rb += WARPS) {
+      const int sb = off[rb], K = off[rb + 1] - sb;
+      const unsigned char* base = data + (size_t)sb * kRbSlotBytes;
+      const int32_t* csg = reinterpret_cast<const int32_t*>(base) + g;
+      const float4* vsg = reinterpret_cast<const float4*>(base + (size_t)K * 4) + g;
+      const float4* wsg = im + sb + g;
+      const int64_t row = (int64_t)rb * kRbRows + g;
+      const bool ok = row < a.n;
+      PanelAccCpx acc;
+      acc.zero();
+      const int nb = K >> 2;
+      for (int b = 0; b < nb; b += U) {
+        float4 x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (b + u < nb) x[u] = *reinterpret_cast<const float4*>(tq + (size_t)csg[4 * (b + u)] * C);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (b + u < nb) acc.add(x[u], vsg[4 * (b + u)], wsg[4 * (b + u)]);
+      }
+      float h[4], p[4][4];
+      acc.get(p);
+      rb_scatter(p, h, g);
+      if (ok) {
+        float4* out = reinterpret_cast<float4*>(tp + row * C + 4 * q);
+        float4 y;
+        if (k == 0) {
+          y = make_float4(alpha * h[0], alpha * h[1], alpha * h[2], alpha * h[3]);
+        } else {
+          const float4 xp = *out;
+          y = make_float4(alpha * h[0] - xp.x, alpha * h[1] - xp.y, alpha * h[2] - xp.z, alpha * h[3] - xp.w);
+        }
+        *out = y;
+        dots.add(*reinterpret_cast<const float4*>(tq + row * C), y);
+      }
+      dots.next(lane);
+    }
+    dots.flush(lane);
+    PairSum* w = ws + (k & 1) * WARPS * 2 * C;
+    w[warp * 2 * C + 2 * lane] = dots.d0;
+    w[warp * 2 * C + 2 * lane + 1] = dots.d1;
+    __syncthreads();  // T_{k+1} and the sums are written
+    // the last two warps (the ones without a second row block) add them, in warp order
+    const int t = (int)threadIdx.x - (NT - 2 * C);
+    if (t >= 0) {
+      PairSum s;
+#pragma unroll 8
+      for (int v = 0; v < WARPS; ++v) s.add(w[v * 2 * C + t]);
+      a.dots[(size_t)k * 2 * C + t] = s.value();
+    }
+  }
+  for (int i = threadIdx.x; i < a.n * (C / 4); i += NT) {
+    reinterpret_cast<float4*>(a.x0)[i] = reinterpret_cast<const float4*>(t0)[i];
+    reinterpret_cast<float4*>(a.x1)[i] = reinterpret_cast<const float4*>(t1)[i];
+  }
 }
 
 // Several matrices in one launch: matrix f runs on the CTAs [block_first[f],
@@ -898,6 +1010,30 @@ unsigned rb_grid(leo2d_ctx* ctx, const leo2d_csr* csr, int warps) {
   const int64_t tiles = (csr->rb_blocks + warps - 1) / warps;
   const int64_t chunks = (tiles + ctx->tile_chunk - 1) / std::max(1, ctx->tile_chunk);
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->sm_count, chunks));
+}
+
+bool rb_one_fits(const leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape, unsigned grid) {
+  return csr->complex_h && shape.rb && !shape.rb_window && shape.rb_warps == kRbOneWarps && grid == 1 &&
+         ctx->kernel_variant == -1 && !ctx->test_unsatisfied_wait &&
+         rb_one_smem(csr->n, csr->rb_blocks, csr->rb_slots) <= ctx->smem_optin;
+}
+
+void rb_run_one(leo2d_ctx* ctx, const leo2d_csr* csr, int steps, float* x0, float* x1, double* dots) {
+  RbOneArgs a{};
+  a.n = csr->n;
+  a.nrb = (int)csr->rb_blocks;
+  a.steps = steps;
+  a.slots = csr->rb_slots;
+  a.off = csr->rb_off.p;
+  a.data = csr->rb_data.p;
+  a.im = csr->rb_im.p;
+  a.x0 = x0;
+  a.x1 = x1;
+  a.dots = dots;
+  allow_smem(ctx, (const void*)k_cheb_rb_one);
+  launch(ctx, "cheb_steps", [&] {
+    k_cheb_rb_one<<<1, kRbOneWarps * 32, rb_one_smem(csr->n, csr->rb_blocks, csr->rb_slots), ctx->stream>>>(a);
+  });
 }
 
 void rb_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shape, unsigned grid, size_t smem,
