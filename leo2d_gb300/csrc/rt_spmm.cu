@@ -57,6 +57,7 @@
 //   orbitals 0.187 -> 0.153 ms.
 //   cp.async waits are hardware waits on copies already issued: no spin loop.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -78,9 +79,10 @@ constexpr int kRtStepBytes = 288;    // one k-step of an 8-row block: 8 columns 
 __host__ __device__ constexpr int rt_step_bytes(int R) { return 32 + 32 * R; }
 constexpr int kRtMaxEnt = 2048;      // stored entries of one block (build limit)
 constexpr int kRtHashCols = 1024;    // distinct columns a block may have for the hashed fill
-// shared memory of one build warp: the keys (or the hash table) and the column list
-constexpr size_t kRtBuildSlice = (size_t)kRtMaxEnt * 8 + (size_t)kRtHashCols * 4;
 constexpr int kRtBuildWarps = 4;
+// shared memory of one build warp: the keys (or the hash table) of blocks of up to
+// `cap` entries and the column list
+size_t rt_build_slice(int cap) { return (size_t)cap * 8 + (size_t)std::min(cap, kRtHashCols) * 4; }
 // staging of the gathered T_n rows (the kernel's STAGE parameter)
 constexpr int kRtRegs = 0;     // registers, fragments exchanged by shuffles
 constexpr int kRtCpAsync = 1;  // shared-memory ring filled by cp.async (16 bytes a lane)
@@ -822,9 +824,21 @@ __global__ void __launch_bounds__(W * 32, 1) k_cheb_rt_batch(const __grid_consta
 
 // ---------------------------------------------------------------- format build
 
+// Entries of the largest block of RB rows.
+__global__ void k_rt_max_ent(int64_t n, int64_t nrb, int RB, const int64_t* __restrict__ prow, int* __restrict__ most) {
+  int m = 0;
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nrb; b += (int64_t)gridDim.x * blockDim.x)
+    m = max(m, (int)min((int64_t)INT_MAX, prow[min(n, (b + 1) * RB)] - prow[b * RB]));
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(most, m);
+}
+
 // One warp per block of R rows, at most kRtMaxEnt stored entries; the distinct
 // columns are the slots. Pass 0 counts them in a hash set in the warp's slice of
-// shared memory and writes the k-steps of each block; pass 1 sorts the keys
+// shared memory and writes the k-steps of each block (slices hold `cap` >= the entries
+// of any block, a power of two: with the build's limit of 2048 instead, two thirds of
+// a pass went into clearing and scanning empty table words, on 8 warps an SM; both
+// passes over 2.4M orbitals 12.3 -> 6.1 ms); pass 1 sorts the keys
 // (column << 16 | entry index) in that slice and writes the block's k-steps at
 // kstart[b] (data zero-filled before): the
 // columns in the interleaved order, the values in fragment order (lane 4g + t
@@ -835,11 +849,11 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
     k_rt_build(int64_t n, int64_t nrb, const int64_t* __restrict__ prow, const int32_t* __restrict__ pcol,
                const float* __restrict__ pval, const float* __restrict__ pim, int pass, int64_t* __restrict__ kst,
                const int64_t* __restrict__ kstart, unsigned char* __restrict__ data, int* __restrict__ err,
-               unsigned long long* __restrict__ ssum) {
+               unsigned long long* __restrict__ ssum, int cap, int slice) {
   extern __shared__ __align__(16) unsigned char rt_build_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(rt_build_smem + (size_t)w * kRtBuildSlice);
-  uint32_t* list = reinterpret_cast<uint32_t*>(rt_build_smem + (size_t)w * kRtBuildSlice + (size_t)kRtMaxEnt * 8);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(rt_build_smem + (size_t)w * slice);
+  uint32_t* list = reinterpret_cast<uint32_t*>(rt_build_smem + (size_t)w * slice + (size_t)cap * 8);
   const int64_t warps = (int64_t)gridDim.x * kRtBuildWarps;
   // rows of a block: R, or 8 for a complex H (its values and imaginary parts in
   // n-tiles 0 and 1 of the 16-row k-step layout)
@@ -867,7 +881,7 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
     };
     const int64_t q0 = srp[0];
     const int E = (int)(srp_at(rows) - q0);
-    if (E > kRtMaxEnt) {
+    if (E > cap) {  // (cap = kRtMaxEnt then)
       if (lane == 0) {
         atomicOr(err, 1);
         if (pass == 0) kst[b] = 1;
@@ -877,10 +891,11 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
     __syncwarp();  // the previous block's keys are read
     if (pass == 0) {
       // counting needs the distinct columns only: a hash set in the warp's slice
-      // (2 kRtMaxEnt 32-bit slots, load <= 1/2), no sort (was half the build)
+      // (2 cap 32-bit slots, load <= 1/2), no sort (was half the build)
       uint32_t* set = reinterpret_cast<uint32_t*>(keys);
-      constexpr int kSet = 2 * kRtMaxEnt;
-      for (int i = lane; i < kSet; i += 32) set[i] = 0xFFFFFFFFu;
+      const int kSet = 2 * cap;
+      for (int i = lane; i < kSet / 4; i += 32)
+        reinterpret_cast<uint4*>(set)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
       __syncwarp();
       int fresh = 0;
       for (int i = lane; i < E; i += 32) {
@@ -922,9 +937,10 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
       // of an 8-row block), and each entry finds its slot in the table. A
       // (row, column) pair stored twice falls through to the sort below, which
       // sums the pair in entry order.
-      constexpr int kSet = kRtMaxEnt;  // 64-bit words; load <= 1/2
+      const int kSet = cap;  // 64-bit words; at least as many as entries
       constexpr unsigned long long kEmpty = ~0ull;
-      for (int i = lane; i < kSet; i += 32) keys[i] = kEmpty;
+      for (int i = lane; i < kSet / 2; i += 32)
+        reinterpret_cast<uint4*>(keys)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
       __syncwarp();
       auto find = [&](uint32_t c) {  // the table slot holding column c (present)
         uint32_t h = (c * 2654435761u) & (kSet - 1);
@@ -952,9 +968,9 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
       if (!__any_sync(0xffffffffu, dup)) {
         __syncwarp();
         // the distinct columns, compacted in table order, then sorted
-        constexpr int kPer = kSet / 32;
+        // (a lane's words 32 apart: no bank conflicts)
         int cnt = 0;
-        for (int j = 0; j < kPer; ++j) cnt += keys[lane * kPer + j] != kEmpty ? 1 : 0;
+        for (int j = lane; j < kSet; j += 32) cnt += keys[j] != kEmpty ? 1 : 0;
         int incl = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -963,8 +979,8 @@ __global__ void __launch_bounds__(kRtBuildWarps * 32)
         }
         const int K = __shfl_sync(0xffffffffu, incl, 31);
         int at = incl - cnt;
-        for (int j = 0; j < kPer; ++j) {
-          const unsigned long long v = keys[lane * kPer + j];
+        for (int j = lane; j < kSet; j += 32) {
+          const unsigned long long v = keys[j];
           if (v != kEmpty) list[at++] = (uint32_t)(v >> 32);
         }
         int P2 = 32;
@@ -1196,11 +1212,23 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
       csr->rt_curve == csr->reorder_curve && csr->rt_warps == warps && csr->rt_group == group &&
       csr->rt_chunk == chunk && csr->rt_grid == sh.grid)
     return true;
-  const size_t smem = (size_t)kRtBuildWarps * kRtBuildSlice;
+  DevBuf<int> err(2);
+  LEO_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), ctx->stream));
+  int cap = 256;
+  {
+    int most = 0;
+    launch(ctx, "rt_build", [&] {
+      k_rt_max_ent<<<grid_for(sh.nrb, 256, (int64_t)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
+          n, sh.nrb, cpx ? 8 : rows, csr->prow.p, err.p);
+    });
+    d2h(ctx, &most, err.p, 1);
+    ctx_sync(ctx);
+    while (cap < most && cap < kRtMaxEnt) cap *= 2;
+  }
+  const size_t slice = rt_build_slice(cap), smem = kRtBuildWarps * slice;
   auto build_kernel = cpx ? k_rt_build<16, true> : rows == 16 ? k_rt_build<16> : k_rt_build<8>;
   LEO_CUDA(cudaFuncSetAttribute(build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const unsigned bgrid = grid_for(sh.nrb * 32, kRtBuildWarps * 32, (int64_t)ctx->sm_count * 8);
-  DevBuf<int> err(2);
   DevBuf<unsigned long long> ssum(1);
   LEO_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), ctx->stream));
   LEO_CUDA(cudaMemsetAsync(ssum.p, 0, sizeof(unsigned long long), ctx->stream));
@@ -1211,7 +1239,7 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
     launch(ctx, "rt_build", [&] {
       build_kernel<<<bgrid, kRtBuildWarps * 32, smem, ctx->stream>>>(n, sh.nrb, csr->prow.p, csr->pcol.p,
                                                                        csr->pval32.p, nullptr, 0, csr->rt_kst.p,
-                                                                       nullptr, nullptr, err.p, ssum.p);
+                                                                       nullptr, nullptr, err.p, ssum.p, cap, (int)slice);
     });
     int h[2] = {0, 0};
     unsigned long long hs = 0;
@@ -1282,7 +1310,7 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
     build_kernel<<<bgrid, kRtBuildWarps * 32, smem, ctx->stream>>>(n, sh.nrb, csr->prow.p, csr->pcol.p,
                                                                      csr->pval32.p, cpx ? csr->pval_im32.p : nullptr,
                                                                      1, csr->rt_kst.p, kstart.p, csr->rt_data.p,
-                                                                     err.p, ssum.p);
+                                                                     err.p, ssum.p, cap, (int)slice);
   });
   int h0 = 0;
   d2h(ctx, &h0, err.p, 1);
