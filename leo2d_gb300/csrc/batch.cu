@@ -63,14 +63,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 1)
 // captured graph can be replayed with new vectors.
 __global__ void k_batch_fill_phase(int64_t n, int C, float* __restrict__ x, const uint64_t* __restrict__ sf,
                                    uint64_t pass_first, int n_complex, const int32_t* __restrict__ new2old) {
-  const uint64_t seed = sf[0], first = sf[1] + pass_first;
-  const int64_t total = n * C;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = new2old ? (int64_t)new2old[e / C] : e / C;
-    const int c = (int)(e % C);
-    x[e] = (c >> 1) < n_complex ? (float)phase_entry(row, c, seed, first) : 0.0f;
-  }
+  __shared__ PhaseTable tab;
+  tab.fill();
+  fill_phase_rows<float>(n, C, x, sf[0], sf[1] + pass_first, n_complex, new2old, tab);
 }
 
 template <int C>
@@ -344,7 +339,7 @@ void enqueue_run(leo2d_batch* b) {
       const FlakeView& v = b->fl[f];
       float* x = b->x0.p + v.row_off * C;
       launch(ctx, "batch_fill", [&] {
-        k_batch_fill_phase<<<grid_for(v.n * C, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
+        k_batch_fill_phase<<<grid_for(v.n * (C / 2), 256, (int64_t)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
             v.n, C, x, b->seed_first.p, (uint64_t)pass * per_pass, nv, v.new2old);
       });
     }
@@ -455,7 +450,7 @@ float time_steps(leo2d_batch* b, int reps) {
   for (int f = 0; f < F; ++f) {
     const FlakeView& v = b->fl[f];
     launch(ctx, "batch_fill", [&] {
-      k_batch_fill_phase<<<grid_for(v.n * C, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
+      k_batch_fill_phase<<<grid_for(v.n * (C / 2), 256, (int64_t)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
           v.n, C, b->x0.p + v.row_off * C, b->seed_first.p, 0, C / 2, v.new2old);
     });
   }

@@ -602,8 +602,8 @@ StepShape choose_shape(leo2d_ctx* ctx, const leo2d_csr* csr, bool fp64, int cols
 }
 
 void fill_phase(leo2d_ctx* ctx, Recursion& r, uint64_t seed, uint64_t first, int n_complex) {
-  const int64_t total = r.n * r.shape.cols;
-  const unsigned g = grid_for(total, 256, (int64_t)ctx->sm_count * 32);
+  const int64_t total = r.n * (r.shape.cols / 2);
+  const unsigned g = grid_for(total, 256, (int64_t)ctx->sm_count * 8);
   if (r.shape.fp64)
     launch(ctx, "fill_phase", [&] {
       k_fill_phase<double><<<g, 256, 0, ctx->stream>>>(r.n, r.shape.cols, (double*)r.x0.p, seed, first, n_complex, r.perm());

