@@ -65,3 +65,18 @@ def test_a_column_stored_twice_takes_another_step():
         assert ctx.kernel_stats("cheb_steps")[0] == 0
         np.testing.assert_array_equal(got, two.kpm_dos(cfg))
     assert np.max(np.abs(got - ref)) <= 2e-5 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("P,row", [(60, False), (64, True)])
+def test_short_runs(P, row):
+    """From 32 steps on a run builds the windows; below it takes the tiled step."""
+    with L.Context(0) as ctx:
+        csr = ctx.upload_csr(*_band(9001, 30, 60, 4))
+        cfg = L.kpm_cfg(P, R=4, seed=3)
+        assert (csr.step_kernel(cfg)[0] == ROW) == row
+        ctx.reset_stats()
+        got = csr.kpm_dos(cfg)
+        assert (ctx.kernel_stats("cheb_steps")[0] > 0) == row
+        ctx.set_option("step_kernel", 0)
+        ref = csr.kpm_dos(cfg)
+    assert np.max(np.abs(got - ref)) <= 2e-5 * np.max(np.abs(ref))
