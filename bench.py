@@ -772,7 +772,7 @@ def run_mlp(args):
         ms = 0.0
         for nm in names:
             k_n, k_ms = ctx.kernel_stats(nm)
-            ms += k_ms / max(args.steps, 1)
+            ms += k_ms / (args.steps + 1)  # (the warm-up call is counted too)
         ctx.set_profiling(False)
         fwd[fused] = (t_call, ms / 1000.0)
     t_inf, t_fwd = fwd[1]
