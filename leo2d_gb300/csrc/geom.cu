@@ -1288,17 +1288,19 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
       if (G.shifted) csr->pos = std::move(spos_buf);
     };
     const unsigned cta_grid = grid_for(n, 1, (int64_t)ctx->sm_count * 8);
-    // Without stored zeros, a flake of the simple model (about 67 entries per
-    // row) and a supercell take one pass: rows are filled into padded arrays of
-    // `pad` entries while they are counted, then compacted. A row with more entries,
-    // or padded arrays too large for a quarter of free memory, takes the
-    // count and fill passes.
-    const int pad = G.bc == 0 ? 96 : 256;
-    if (n > 0 && !G.keep_zeros && (G.bc != 0 || G.model == LEO2D_MODEL_SIMPLE)) {
+    // Without stored zeros rows take one pass: they are filled into padded arrays of
+    // `pad` entries while they are counted, then compacted. A bilayer's row has about
+    // 67 entries in the simple model and up to 120 in the reference's (whose hoppings,
+    // some 600 FP64 instructions a pair, the count and fill passes evaluate twice: 28.2 and
+    // 28.4 ms at 401,000 rows, this pass 28.7 ms), a supercell's a few more. A row with
+    // more entries, or padded arrays past a quarter of free memory or the context's limit
+    // on one allocation, takes the count and fill passes.
+    const int pad = G.bc != 0 ? 256 : G.model == LEO2D_MODEL_SIMPLE ? 96 : G.S > 2 ? 224 : 144;
+    if (n > 0 && !G.keep_zeros) {
       const size_t per = sizeof(int32_t) + sizeof(double) * (1 + (G.with_dx ? 2 : 0) + (G.cpx ? 1 : 0));
       size_t fr = 0, tot = 0;
       device_mem_info(&fr, &tot);
-      if ((size_t)n * pad * per <= fr / 4) {
+      if ((size_t)n * pad * per <= fr / 4 && (!g_alloc_cap || (size_t)n * pad * sizeof(double) <= g_alloc_cap)) {
         const size_t pn = (size_t)n * pad;
         DevBuf<int32_t> pcol(pn);
         DevBuf<double> pval(pn), pdx(G.with_dx ? pn : 0), pdy(G.with_dx ? pn : 0), pim(G.cpx ? pn : 0);
