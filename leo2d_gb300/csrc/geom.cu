@@ -42,7 +42,7 @@ constexpr int kIntraSearch = 4;    // (int) Graphene::intra_search_radius (graph
 constexpr int kInterSearch = 6;    // (int) Graphene::inter_search_radius (graphene.h:95)
 constexpr double kInterCutoff = 12.5;  // hstruct.cpp:310
 constexpr int kIntraShellMax = 16;     // no intralayer hopping beyond this neighbour shell
-constexpr int kRowWarps = 8;           // k_flake_rows: warps (rows in flight) per 256-thread block
+constexpr int kRowWarps = 8;           // k_flake_rows, k_flake_rows_one: warps per 256-thread block
 constexpr int kInterSeg = 288;         // k_flake_rows: interlayer candidates per segment (a 12 x 12 x 2 window)
 
 struct SheetDev {
@@ -157,11 +157,33 @@ __device__ __forceinline__ double intralayer(int model, int orow, int ocol, int 
   return intra_shell_t(model, intra_shell(orow, ocol, d0, d1));
 }
 
+// The height-dependent coefficients of c_to_c, the reference's fit and order of operations.
+struct StackZ {
+  double lambda_0, xi_0, kappa_0, lambda_3, xi_3, x_3, lambda_6, xi_6, x_6, kappa_6;
+};
+__device__ __forceinline__ StackZ stack_z(double v2) {
+  const double z_eq = 3.35;
+  const double z_eps = (fabs(v2) - z_eq) / z_eq;
+  StackZ z;
+  z.lambda_0 = 0.310 - 1.882 * z_eps + 7.741 * z_eps * z_eps;
+  z.xi_0 = 1.750 - 1.618 * z_eps + 1.848 * z_eps * z_eps;
+  z.kappa_0 = 1.990 + 1.007 * z_eps + 2.427 * z_eps * z_eps;
+  z.lambda_3 = -0.068 + 0.399 * z_eps - 1.739 * z_eps * z_eps;
+  z.xi_3 = 3.286 - 0.914 * z_eps + 12.011 * z_eps * z_eps;
+  z.x_3 = 0.500 + 0.322 * z_eps + 0.908 * z_eps * z_eps;
+  z.lambda_6 = -0.008 + 0.046 * z_eps - 0.183 * z_eps * z_eps;
+  z.xi_6 = 2.272 - 0.721 * z_eps - 4.414 * z_eps * z_eps;
+  z.x_6 = 1.217 + 0.027 * z_eps - 0.658 * z_eps * z_eps;
+  z.kappa_6 = 1.562 - 0.371 * z_eps - 0.134 * z_eps * z_eps;
+  return z;
+}
+
 // Coupling::Interlayer::C_to_C (graphene.cpp:91-222). abs() at graphene.cpp:117
 // binds to the int overload in the reference, hence the truncation. The
 // fitted coefficients and the order of operations are the reference's.
+// z: stack_z(v2).
 __device__ double c_to_c(int orow, int ocol, double v0, double v1, double v2, double theta_row,
-                         double theta_col) {
+                         double theta_col, const StackZ& z) {
   const double kPi = 3.14159265358979323846, kPi_6 = 0.523598775598298873077;
   if (abs((int)v2) > 5) return 0;
   double r = sqrt(v0 * v0 + v1 * v1);
@@ -172,21 +194,9 @@ __device__ double c_to_c(int orow, int ocol, double v0, double v1, double v2, do
     double theta12 = ac - theta_col + kPi;
     if (ocol == 1) theta12 += kPi_6; else theta12 -= kPi_6;
     double rs = r / 2.4768;
-    double z_eq = 3.35;
-    double z_eps = (fabs(v2) - z_eq) / z_eq;
-    double lambda_0 = 0.310 - 1.882 * z_eps + 7.741 * z_eps * z_eps;
-    double xi_0 = 1.750 - 1.618 * z_eps + 1.848 * z_eps * z_eps;
-    double kappa_0 = 1.990 + 1.007 * z_eps + 2.427 * z_eps * z_eps;
-    double lambda_3 = -0.068 + 0.399 * z_eps - 1.739 * z_eps * z_eps;
-    double xi_3 = 3.286 - 0.914 * z_eps + 12.011 * z_eps * z_eps;
-    double x_3 = 0.500 + 0.322 * z_eps + 0.908 * z_eps * z_eps;
-    double lambda_6 = -0.008 + 0.046 * z_eps - 0.183 * z_eps * z_eps;
-    double xi_6 = 2.272 - 0.721 * z_eps - 4.414 * z_eps * z_eps;
-    double x_6 = 1.217 + 0.027 * z_eps - 0.658 * z_eps * z_eps;
-    double kappa_6 = 1.562 - 0.371 * z_eps - 0.134 * z_eps * z_eps;
-    double V0 = lambda_0 * exp(-xi_0 * (rs) * (rs)) * cos(kappa_0 * rs);
-    double V3 = lambda_3 * rs * rs * exp(-xi_3 * (rs - x_3) * (rs - x_3));
-    double V6 = lambda_6 * exp(-xi_6 * (rs - x_6) * (rs - x_6)) * sin(kappa_6 * rs);
+    double V0 = z.lambda_0 * exp(-z.xi_0 * (rs) * (rs)) * cos(z.kappa_0 * rs);
+    double V3 = z.lambda_3 * rs * rs * exp(-z.xi_3 * (rs - z.x_3) * (rs - z.x_3));
+    double V6 = z.lambda_6 * exp(-z.xi_6 * (rs - z.x_6) * (rs - z.x_6)) * sin(z.kappa_6 * rs);
     double t = V0 + V3 * (cos(3 * theta12) + cos(3 * theta21)) + V6 * (cos(6 * theta12) + cos(6 * theta21));
     double d = 8.0 - r;
     if (d < 1. && d > 0.) t *= exp(1. - 1. / (d * d));
@@ -208,11 +218,11 @@ __device__ __forceinline__ double interlayer_t(int model, int orow, int ocol, do
     const double r = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
     return r < 8.0 ? simple_amp * exp(-(r - 3.35) * kInvDecay) : 0.0;
   }
-  const double v = c_to_c(orow, ocol, v0, v1, v2, th_row, th_col);
+  const double v = c_to_c(orow, ocol, v0, v1, v2, th_row, th_col, stack_z(v2));
   return v != 0.0 ? v / rescale : 0.0;
 }
 
-// interlayer_t of the simple model in k_flake_rows, where FP64 instructions are the
+// interlayer_t of the simple model in k_flake_rows(_one), where FP64 instructions are the
 // bound (one per 16 cycles and SM): 24 of them for a pair instead of about 40.
 //  - sqrt: the FP32 reciprocal root (22 bits) and one cubic step (Halley),
 //    r (1 + e/2 + 3 e^2/8) with e = 1 - d2 y^2, which leaves e^3 < 2^-60;
@@ -382,7 +392,7 @@ __device__ __forceinline__ double diag_value(const GeomDev& G, double raw, doubl
   return G.e_field != 0.0 ? (raw + G.shift + z * G.e_field) / G.rescale : (raw + G.shift) / G.rescale;
 }
 
-// FP32 copy of the positions for the candidate prefilter of k_flake_rows.
+// FP32 copy of the positions for the candidate prefilter (inter_candidate).
 __global__ void k_pos32(const double* __restrict__ pos, int64_t n, float4* __restrict__ p32) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
     p32[k] = make_float4((float)pos[3 * k], (float)pos[3 * k + 1], (float)pos[3 * k + 2], 0.f);
@@ -413,17 +423,97 @@ __device__ __forceinline__ void nearest_cells(const GeomDev& G, int64_t row, con
   }
 }
 
-// kMode 0: count entries per row; 1: fill at the scanned row pointers; 2: fill
-// and count in one pass, row r at r * pad_cap of padded arrays (entries past
-// pad_cap are counted, not stored, and raise `overflow`).
-template <int kMode>
+// Candidate c of row (ih, jh, l0) in the intralayer window [i0-4, i0+4) x [j0-4, j0+4)
+// x orbitals: its column (-1: outside the sheet) and value.
+__device__ __forceinline__ int64_t intra_candidate(const GeomDev& G, const SheetDev& sh, int c, int i0, int j0, int ih,
+                                                   int jh, int l0, int64_t row, double sz1, double* t) {
+  const int side = 2 * kIntraSearch;
+  const int l = c % sh.n_orb;
+  const int j = j0 - kIntraSearch + (c / sh.n_orb) % side;
+  const int i = i0 - kIntraSearch + c / (sh.n_orb * side);
+  const int k2 = grid_to_index(sh, i, j, l);
+  if (k2 == -1) return -1;
+  const int64_t k2g = k2 + sh.base;
+  // the quotients by the rescale from the host's table; a field E
+  // makes the diagonal depend on the orbital's height
+  const int r = intra_shell(l0, l, i - ih, j - jh);
+  if (k2g == row)
+    *t = G.diag_const ? G.diag_q : diag_value(G, intra_shell_t(G.model, r), sz1);
+  else
+    *t = r <= kIntraShellMax ? G.intra_q[r] : 0.0;
+  return k2g;
+}
+
+// The interlayer window of a row in sheet o0: +-6 cells around the nearest one, clipped.
+struct InterWindow {
+  int ilo, jlo, wj, nc;
+};
+__device__ __forceinline__ InterWindow inter_window(const SheetDev& o0, int i0, int j0) {
+  InterWindow w;
+  w.ilo = max(0, i0 - kInterSearch);
+  w.jlo = max(0, j0 - kInterSearch);
+  w.wj = max(0, min(o0.W, j0 + kInterSearch) - w.jlo);
+  w.nc = max(0, min(o0.H, i0 + kInterSearch) - w.ilo) * w.wj * o0.n_orb;
+  return w;
+}
+
+// Candidate c of that window: its column when it is a pair (d_xy < 12.5 A), else -1;
+// *hops: it may have a hopping (within 8 A and a margin, by FP32).
+__device__ __forceinline__ int64_t inter_candidate(const GeomDev& G, const SheetDev& o0, const InterWindow& w, int c,
+                                                   const double* __restrict__ pos, const float4* __restrict__ pos32,
+                                                   const float4* __restrict__ spos32, double x1, double y1,
+                                                   const float4& p1f, const float4& sp1f, bool* hops) {
+  constexpr float kWinLo = (float)(kInterCutoff - kPrefilterMargin), kWinHi = (float)(kInterCutoff + kPrefilterMargin);
+  // every hopping is zero from 8 A on (in-plane for the reference model, 3-D for the simple one)
+  constexpr float kHopHi = 8.0f + kPrefilterMargin;
+  const int l = c % o0.n_orb;
+  const int j = w.jlo + (c / o0.n_orb) % w.wj;
+  const int i = w.ilo + c / (o0.n_orb * w.wj);
+  const int k2 = grid_to_index(o0, i, j, l);
+  if (k2 == -1) return -1;
+  const int64_t kk = k2 + o0.base;
+  const float4 q = pos32[kk];
+  const float dxf = q.x - p1f.x, dyf = q.y - p1f.y;
+  const float d2f = dxf * dxf + dyf * dyf;
+  bool in_window;
+  if (d2f < kWinLo * kWinLo) {
+    in_window = true;
+  } else if (d2f > kWinHi * kWinHi) {
+    in_window = false;
+  } else {
+    const double x2 = pos[3 * kk], y2 = pos[3 * kk + 1];
+    in_window = (x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1) < kInterCutoff * kInterCutoff;
+  }
+  if (!in_window) return -1;
+  // the hopping cutoffs test the shifted positions
+  const float4 sq = G.shifted ? spos32[kk] : q;
+  const float hdx = sq.x - sp1f.x, hdy = sq.y - sp1f.y, hdz = sq.z - sp1f.z;
+  const float hd2 = hdx * hdx + hdy * hdy;
+  const float h2f = G.model == LEO2D_MODEL_SIMPLE ? hd2 + hdz * hdz : hd2;
+  *hops = h2f < kHopHi * kHopHi;
+  return kk;
+}
+
+// Entry e of a row at (sx1, sy1): column k2g, value t, and its products with the distance.
+__device__ __forceinline__ void store_entry(const GeomDev& G, const RowOut& out, const double* __restrict__ spos,
+                                            int64_t e, int64_t k2g, double t, double sx1, double sy1) {
+  out.col[e] = (int32_t)k2g;
+  const double x2 = spos[3 * k2g], y2 = spos[3 * k2g + 1];
+  store_value(G, out, e, t, sx1, sy1, x2, y2);
+  if (G.with_dx) {
+    out.dx[e] = t != 0 ? 0.0 + (sx1 - x2) * t : 0.0;
+    out.dy[e] = t != 0 ? 0.0 + (sy1 - y2) * t : 0.0;
+  }
+}
+
+// kFill false: count entries per row; true: fill at the scanned row pointers.
+template <bool kFill>
 __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_constant__ GeomDev G, int64_t n,
                                                     int run, const int32_t* __restrict__ grid4,
                                                     const double* __restrict__ pos,
                                                     const float4* __restrict__ pos32,
                                                     const double* __restrict__ spos,
                                                     const float4* __restrict__ spos32, RowOut out) {
-  constexpr bool kFill = kMode != 0, kPad = kMode == 2;
   // per warp: the interlayer segment's candidate codes, queue and hoppings
   __shared__ int32_t s_code[kRowWarps][kInterSeg];
   __shared__ int16_t s_queue[kRowWarps][kInterSeg];
@@ -451,8 +541,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
     // which give the values (setConfigPositions, locality.cpp:3618-3642)
     const double x1 = pos[3 * row], y1 = pos[3 * row + 1];
     const double sx1 = spos[3 * row], sy1 = spos[3 * row + 1], sz1 = spos[3 * row + 2];
-    int64_t o = kPad ? row * (int64_t)out.pad_cap : (kFill ? out.rowptr[row] : 0);
-    const int64_t o_end = kPad ? o + out.pad_cap : 0;
+    int64_t o = kFill ? out.rowptr[row] : 0;
     int64_t n_ent = 0, n_intra = 0, n_inter = 0;
 
     // intralayer: window [i0-4, i0+4) x [j0-4, j0+4) x orbitals, every candidate kept
@@ -464,43 +553,19 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
         const int c = c0 + (int)lane;
         int64_t k2g = -1;
         double t = 0.0;
-        if (c < nc) {
-          const int l = c % sh.n_orb;
-          const int j = j0 - kIntraSearch + (c / sh.n_orb) % side;
-          const int i = i0 - kIntraSearch + c / (sh.n_orb * side);
-          const int k2 = grid_to_index(sh, i, j, l);
-          if (k2 != -1) {
-            k2g = k2 + sh.base;
-            // the quotients by the rescale from the host's table; a field E
-            // makes the diagonal depend on the orbital's height
-            const int r = intra_shell(l0, l, i - ih, j - jh);
-            if (k2g == row)
-              t = G.diag_const ? G.diag_q : diag_value(G, intra_shell_t(G.model, r), sz1);
-            else
-              t = r <= kIntraShellMax ? G.intra_q[r] : 0.0;
-          }
-        }
+        if (c < nc) k2g = intra_candidate(G, sh, c, i0, j0, ih, jh, l0, row, sz1, &t);
         const bool keep = k2g >= 0;
         // without KEEP_ZEROS the diagonal stays so a later rescale can shift it
         const bool store = keep && (G.keep_zeros || t_nonzero(t) || k2g == row);
         const unsigned m = __ballot_sync(0xffffffffu, store);
         n_intra += __popc(__ballot_sync(0xffffffffu, keep));
-        if (kFill && store && (!kPad || o + __popc(m & lt_mask) < o_end)) {
-          const int64_t e = o + __popc(m & lt_mask);
-          out.col[e] = (int32_t)k2g;
-          const double x2 = spos[3 * k2g], y2 = spos[3 * k2g + 1];
-          store_value(G, out, e, t, sx1, sy1, x2, y2);
-          if (G.with_dx) {
-            out.dx[e] = t != 0 ? 0.0 + (sx1 - x2) * t : 0.0;
-            out.dy[e] = t != 0 ? 0.0 + (sy1 - y2) * t : 0.0;
-          }
-        }
+        if (kFill && store) store_entry(G, out, spos, o + __popc(m & lt_mask), k2g, t, sx1, sy1);
         o += __popc(m);
         n_ent += __popc(m);
       }
     }
 
-    // interlayer: sheet below, then sheet above; window +-6 clipped; d_xy < 12.5 A.
+    // interlayer: sheet below, then sheet above.
     // Most candidates of the window have no hopping (beyond 8 A), so the FP64
     // hoppings are not taken where the candidates fall, which would leave most
     // lanes of GB300's small FP64 unit idle. Per segment of up to kInterSeg
@@ -511,11 +576,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
     // order, as a single pass would write them.
     {
       const float4 p1f = pos32[row], sp1f = spos32[row];
-      const float x1f = p1f.x, y1f = p1f.y;
       const float sx1f = sp1f.x, sy1f = sp1f.y, sz1f = sp1f.z;
-      constexpr float kWinLo = (float)(kInterCutoff - kPrefilterMargin), kWinHi = (float)(kInterCutoff + kPrefilterMargin);
-      // every hopping is zero from 8 A on (in-plane for the reference model, 3-D for the simple one)
-      constexpr float kHopHi = 8.0f + kPrefilterMargin, kHopLo = 8.0f - kPrefilterMargin;
+      constexpr float kHopLo = 8.0f - kPrefilterMargin;
       int32_t* const seg_code = s_code[threadIdx.x >> 5];
       int16_t* const seg_queue = s_queue[threadIdx.x >> 5];
       double* const seg_t = s_hop[threadIdx.x >> 5];
@@ -525,11 +587,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
         const SheetDev& o0 = G.sh[s0];
         const int i0 = __shfl_sync(0xffffffffu, near_i[1 + side_k], rr);
         const int j0 = __shfl_sync(0xffffffffu, near_j[1 + side_k], rr);
-        const int ilo = max(0, i0 - kInterSearch), ihi = min(o0.H, i0 + kInterSearch);
-        const int jlo = max(0, j0 - kInterSearch), jhi = min(o0.W, j0 + kInterSearch);
-        if (ihi <= ilo || jhi <= jlo) continue;
-        const int wj = jhi - jlo;
-        const int nc = (ihi - ilo) * wj * o0.n_orb;
+        const InterWindow win = inter_window(o0, i0, j0);
+        const int nc = win.nc;
         for (int seg0 = 0; seg0 < nc; seg0 += kInterSeg) {
           const int seg_n = min(kInterSeg, nc - seg0);
           // (1) code: -1 outside the window, else the column with bit 31 set
@@ -539,36 +598,10 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
             const int slot = c0 + (int)lane;
             bool queue = false;
             if (slot < seg_n) {
-              const int c = seg0 + slot;
-              int32_t code = -1;
-              const int l = c % o0.n_orb;
-              const int j = jlo + (c / o0.n_orb) % wj;
-              const int i = ilo + c / (o0.n_orb * wj);
-              const int k2 = grid_to_index(o0, i, j, l);
-              if (k2 != -1) {
-                const int64_t kk = k2 + o0.base;
-                const float4 q = pos32[kk];
-                const float dxf = q.x - x1f, dyf = q.y - y1f;
-                const float d2f = dxf * dxf + dyf * dyf;
-                bool in_window;
-                if (d2f < kWinLo * kWinLo) {
-                  in_window = true;
-                } else if (d2f > kWinHi * kWinHi) {
-                  in_window = false;
-                } else {
-                  const double x2 = pos[3 * kk], y2 = pos[3 * kk + 1];
-                  in_window = (x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1) < kInterCutoff * kInterCutoff;
-                }
-                if (in_window) {
-                  // the hopping cutoffs test the shifted positions
-                  const float4 sq = G.shifted ? spos32[kk] : q;
-                  const float hdx = sq.x - sx1f, hdy = sq.y - sy1f, hdz = sq.z - sz1f;
-                  const float hd2 = hdx * hdx + hdy * hdy;
-                  const float h2f = G.model == LEO2D_MODEL_SIMPLE ? hd2 + hdz * hdz : hd2;
-                  queue = (kFill || !G.keep_zeros) && h2f < kHopHi * kHopHi;
-                  code = (int32_t)((uint32_t)kk | (queue ? 0x80000000u : 0u));
-                }
-              }
+              const int64_t kk =
+                  inter_candidate(G, o0, win, seg0 + slot, pos, pos32, spos32, x1, y1, p1f, sp1f, &queue);
+              queue = queue && (kFill || !G.keep_zeros);
+              const int32_t code = kk < 0 ? -1 : (int32_t)((uint32_t)kk | (queue ? 0x80000000u : 0u));
               seg_code[slot] = code;
             }
             const unsigned qm = __ballot_sync(0xffffffffu, queue);
@@ -627,16 +660,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
             const bool store = keep && (G.keep_zeros || t_nonzero(t));
             const unsigned m = __ballot_sync(0xffffffffu, store);
             n_inter += __popc(__ballot_sync(0xffffffffu, keep));
-            if (kFill && store && (!kPad || o + __popc(m & lt_mask) < o_end)) {
-              const int64_t e = o + __popc(m & lt_mask);
-              out.col[e] = (int32_t)k2g;
-              const double x2 = spos[3 * k2g], y2 = spos[3 * k2g + 1];
-              store_value(G, out, e, t, sx1, sy1, x2, y2);
-              if (G.with_dx) {
-                out.dx[e] = t != 0 ? 0.0 + (sx1 - x2) * t : 0.0;
-                out.dy[e] = t != 0 ? 0.0 + (sy1 - y2) * t : 0.0;
-              }
-            }
+            if (kFill && store) store_entry(G, out, spos, o + __popc(m & lt_mask), k2g, t, sx1, sy1);
             o += __popc(m);
             n_ent += __popc(m);
           }
@@ -644,12 +668,171 @@ __global__ void __launch_bounds__(kRowWarps * 32, 3) k_flake_rows(const __grid_c
         }
       }
     }
-    if ((!kFill || kPad) && lane == 0) {
+    if (!kFill && lane == 0) {
       out.cnt_ent[row] = n_ent;
       out.cnt_intra[row] = n_intra;
       out.cnt_inter[row] = n_inter;
-      if (kPad && n_ent > out.pad_cap) atomicOr(out.overflow, 1);
     }
+  }
+}
+
+// Counting and filling rows in one pass, without stored zeros: row r at r * pad_cap of
+// padded arrays (entries past pad_cap are counted, not stored, and raise `overflow`).
+// The FP64 pipe bounds it, where a warp instruction costs the same whatever lanes are
+// active: the pairs that may have a hopping (64 to 80 of the 288 candidates) go in
+// candidate order into a ring in shared memory that runs on over the warp's rows, and 32
+// at a time are evaluated and stored, every lane with a pair. The height coefficients of
+// c_to_c (a division and 50 instructions) are kept for the last height met on each side.
+// With a queue per row, its last round part full, and the coefficients per pair, 401,000
+// rows took 28.7 ms in the reference model and 2.83 ms in the simple one; now 18.1 and
+// 2.13 (8 rows a run as fast, 32 18.8; 2 blocks an SM, without spills, 19.3 and 2.70).
+__global__ void __launch_bounds__(kRowWarps * 32, 4) k_flake_rows_one(const __grid_constant__ GeomDev G, int64_t n,
+                                                    int run, const int32_t* __restrict__ grid4,
+                                                    const double* __restrict__ pos,
+                                                    const float4* __restrict__ pos32,
+                                                    const double* __restrict__ spos,
+                                                    const float4* __restrict__ spos32, RowOut out) {
+  constexpr int kRing = 64;  // fewer than 32 wait when up to 32 are added
+  __shared__ int32_t s_col[kRowWarps][kRing];
+  __shared__ int32_t s_meta[kRowWarps][kRing];  // orbital << 6 | sheet above << 5 | row of the run
+  __shared__ int32_t s_cnt[kRowWarps][32];      // entries so far of each row of the run
+  // the last heights met below and above, with their coefficients
+  __shared__ double s_key[kRowWarps][2];
+  __shared__ StackZ s_z[kRowWarps][2];
+  __shared__ double s_pow[64];
+  if (threadIdx.x < 64) s_pow[threadIdx.x] = exp2((double)threadIdx.x / 64.0);
+  if (threadIdx.x < 2 * kRowWarps) (&s_key[0][0])[threadIdx.x] = __longlong_as_double(0x7ff8000000000000ll);  // no height
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int64_t warps = (int64_t)gridDim.x * kRowWarps;
+  for (int64_t row0 = ((int64_t)blockIdx.x * kRowWarps + w) * run; row0 < n; row0 += warps * run) {
+    const int rows = (int)min((int64_t)run, n - row0);
+    // nearest cells, counts: lane r holds those of row row0 + r
+    int near_i[3] = {0, 0, 0}, near_j[3] = {0, 0, 0};
+    if (lane < rows) nearest_cells(G, row0 + lane, grid4, pos, near_i, near_j);
+    int n_intra = 0, n_inter = 0;
+    int head = 0, waiting = 0;
+
+    // the first `count` (at most 32) pairs of the ring
+    auto flush = [&](int count) {
+      __syncwarp();
+      const int slot = (head + lane) & (kRing - 1);
+      const int meta = s_meta[w][slot];
+      const int rr = meta & 31;
+      double t = 0.0, sx1 = 0.0, sy1 = 0.0;
+      int64_t kk = 0;
+      const bool on = lane < count;
+      double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+      if (on) {
+        kk = s_col[w][slot];
+        const double* p = spos + 3 * (row0 + rr);
+        sx1 = p[0];
+        sy1 = p[1];
+        v0 = spos[3 * kk] - sx1;
+        v1 = spos[3 * kk + 1] - sy1;
+        v2 = spos[3 * kk + 2] - p[2];
+      }
+      if (G.model == LEO2D_MODEL_SIMPLE) {
+        if (on) t = simple_t(v0, v1, v2, G.simple_amp, s_pow);
+      } else {
+        const int above = (meta >> 5) & 1;
+        const unsigned miss = __ballot_sync(0xffffffffu, on && v2 != s_key[w][above]);
+        StackZ z;
+        if (miss) {
+          z = stack_z(v2);
+          const unsigned up = __ballot_sync(0xffffffffu, above);
+          const unsigned mine = miss & (above ? up : ~up);
+          if (mine && lane == __ffs(mine) - 1) {  // one lane a side
+            s_key[w][above] = v2;
+            s_z[w][above] = z;
+          }
+        } else {
+          z = s_z[w][above];
+        }
+        if (on) {
+          const int4 g = reinterpret_cast<const int4*>(grid4)[row0 + rr];
+          const double v = c_to_c(g.z, meta >> 6, v0, v1, v2, G.sh[g.w].angle, G.sh[above ? g.w + 1 : g.w - 1].angle, z);
+          t = v != 0.0 ? v / G.rescale : 0.0;
+        }
+      }
+      const bool store = on && t_nonzero(t);
+      const unsigned m = __match_any_sync(0xffffffffu, rr) & __ballot_sync(0xffffffffu, store);
+      if (store) {
+        const int e = s_cnt[w][rr] + __popc(m & lt_mask);
+        if (e < out.pad_cap) store_entry(G, out, spos, (row0 + rr) * out.pad_cap + e, kk, t, sx1, sy1);
+      }
+      __syncwarp();
+      if (store && (m & lt_mask) == 0) s_cnt[w][rr] += __popc(m);
+      __syncwarp();
+      head += count;
+      waiting -= count;
+    };
+
+    for (int rr = 0; rr < rows; ++rr) {
+      const int64_t row = row0 + rr;
+      const int4 g = reinterpret_cast<const int4*>(grid4)[row];  // cell, orbital, sheet
+      const SheetDev& sh = G.sh[g.w];
+      // pos chooses the pairs, spos gives the values, as in k_flake_rows
+      const double x1 = pos[3 * row], y1 = pos[3 * row + 1];
+      int ent = 0, intra = 0, inter = 0;
+      {
+        const double sx1 = spos[3 * row], sy1 = spos[3 * row + 1], sz1 = spos[3 * row + 2];
+        const int i0 = __shfl_sync(0xffffffffu, near_i[0], rr), j0 = __shfl_sync(0xffffffffu, near_j[0], rr);
+        const int nc = 4 * kIntraSearch * kIntraSearch * sh.n_orb;
+        for (int c0 = 0; c0 < nc; c0 += 32) {
+          const int c = c0 + lane;
+          int64_t k2g = -1;
+          double t = 0.0;
+          if (c < nc) k2g = intra_candidate(G, sh, c, i0, j0, g.x, g.y, g.z, row, sz1, &t);
+          // the diagonal stays so a later rescale can shift it
+          const bool store = k2g >= 0 && (t_nonzero(t) || k2g == row);
+          const unsigned m = __ballot_sync(0xffffffffu, store);
+          intra += __popc(__ballot_sync(0xffffffffu, k2g >= 0));
+          const int e = ent + __popc(m & lt_mask);
+          if (store && e < out.pad_cap) store_entry(G, out, spos, row * out.pad_cap + e, k2g, t, sx1, sy1);
+          ent += __popc(m);
+        }
+      }
+      if (lane == 0) s_cnt[w][rr] = ent;
+      const float4 p1f = pos32[row], sp1f = spos32[row];
+      for (int above = 0; above < 2; ++above) {
+        const int s0 = above ? g.w + 1 : g.w - 1;
+        if (s0 < 0 || s0 >= G.S) continue;
+        const SheetDev& o0 = G.sh[s0];
+        const InterWindow win = inter_window(o0, __shfl_sync(0xffffffffu, near_i[1 + above], rr),
+                                             __shfl_sync(0xffffffffu, near_j[1 + above], rr));
+        for (int c0 = 0; c0 < win.nc; c0 += 32) {
+          const int c = c0 + lane;
+          bool hops = false;
+          int64_t kk = -1;
+          if (c < win.nc) kk = inter_candidate(G, o0, win, c, pos, pos32, spos32, x1, y1, p1f, sp1f, &hops);
+          inter += __popc(__ballot_sync(0xffffffffu, kk >= 0));
+          const unsigned qm = __ballot_sync(0xffffffffu, hops);
+          if (hops) {
+            const int slot = (head + waiting + __popc(qm & lt_mask)) & (kRing - 1);
+            s_col[w][slot] = (int32_t)kk;
+            s_meta[w][slot] = (c % o0.n_orb) << 6 | above << 5 | rr;
+          }
+          waiting += __popc(qm);
+          if (waiting >= 32) flush(32);
+        }
+      }
+      if (lane == rr) {
+        n_intra = intra;
+        n_inter = inter;
+      }
+    }
+    if (waiting > 0) flush(waiting);
+    __syncwarp();
+    if (lane < rows) {
+      const int ent = s_cnt[w][lane];
+      out.cnt_ent[row0 + lane] = ent;
+      out.cnt_intra[row0 + lane] = n_intra;
+      out.cnt_inter[row0 + lane] = n_inter;
+      if (ent > out.pad_cap) atomicOr(out.overflow, 1);
+    }
+    __syncwarp();
   }
 }
 
@@ -732,7 +915,8 @@ __device__ void block_bitonic_sort(uint64_t* keys, int n2) {
   }
 }
 
-// A CTA per row. kMode as in k_flake_rows.
+// A CTA per row. kMode 0: count; 1: fill at the scanned row pointers; 2: one padded pass, as
+// k_flake_rows_one.
 // Bound by the FP64 pipe (an instruction per 16 cycles and SM), so FP64 is left to the
 // pairs that have a hopping, each evaluated once and on full warps: the cells nearest
 // to the row's images come from one lane an image, FP32 distances sort out the
@@ -1270,9 +1454,10 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
       allow_smem(ctx, (const void*)k_periodic_rows<1>);
       allow_smem(ctx, (const void*)k_periodic_rows<2>);
     }
-    // rows a warp takes at a time (k_flake_rows): as many as leave every one of the
-    // 24 resident warps of an SM two runs, at most a warp's lanes
-    const int run = (int)std::min<int64_t>(32, std::max<int64_t>(1, n / ((int64_t)ctx->sm_count * 48)));
+    // rows a warp takes at a time (k_flake_rows, k_flake_rows_one): as many as leave every
+    // one of the 32 resident warps of an SM three runs, at most 16 (32 leave the SMs uneven:
+    // 18.8 ms against 18.1 at 401,000 orbitals of the reference model)
+    const int run = (int)std::min<int64_t>(16, std::max<int64_t>(1, n / ((int64_t)ctx->sm_count * 96)));
     const unsigned rows_grid = grid_for(n, kRowWarps * run, (int64_t)ctx->sm_count * 64);
     DevBuf<float4> pos32(std::max<int64_t>(n, 1));
     DevBuf<float4> spos32(G.shifted ? std::max<int64_t>(n, 1) : 0);
@@ -1292,7 +1477,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
     // `pad` entries while they are counted, then compacted. A bilayer's row has about
     // 67 entries in the simple model and up to 120 in the reference's (whose hoppings,
     // some 600 FP64 instructions a pair, the count and fill passes evaluate twice: 28.2 and
-    // 28.4 ms at 401,000 rows, this pass 28.7 ms), a supercell's a few more. A row with
+    // 28.4 ms at 401,000 rows, this pass 18.1 ms), a supercell's a few more. A row with
     // more entries, or padded arrays past a quarter of free memory or the context's limit
     // on one allocation, takes the count and fill passes.
     const int pad = G.bc != 0 ? 256 : G.model == LEO2D_MODEL_SIMPLE ? 96 : G.S > 2 ? 224 : 144;
@@ -1321,7 +1506,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
           });
         else
           launch(ctx, "flake_rows_fill", [&] {
-            k_flake_rows<2><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
+            k_flake_rows_one<<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, rp);
         });
         int over = 0;
@@ -1363,7 +1548,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
     if (n > 0) {
       if (G.bc == 0)
         launch(ctx, "flake_rows_count", [&] {
-          k_flake_rows<0><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
+          k_flake_rows<false><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, ro);
         });
       else
@@ -1395,7 +1580,7 @@ extern "C" leo2d_status leo2d_build_csr(leo2d_ctx* ctx, const leo2d_geom* g, uin
     if (n > 0) {
       if (G.bc == 0)
         launch(ctx, "flake_rows_fill", [&] {
-          k_flake_rows<1><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
+          k_flake_rows<true><<<rows_grid, kRowWarps * 32, 0, ctx->stream>>>(G, n, run, csr->grid4.p, csr->pos.p, pos32.p, spos,
                                                               spos32p, ro);
         });
       else

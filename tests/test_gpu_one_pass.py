@@ -25,7 +25,9 @@ def _build(ctx, gp, dx):
     return csr, arrays, counts
 
 
-# sizes: 2.2k to 6k orbitals; pad: entries a row has room for in the single pass
+# pad: entries a row has room for in the single pass. Sizes: 2k to 6k orbitals, a row a
+# warp; then runs of a few rows and of the most, whose pairs share rounds (three sheets:
+# pairs of both sides in one)
 @pytest.mark.parametrize("pad,dx,kw", [
     (144, False, dict(model=REF, size=40, angles_deg=(0.0, 1.05))),
     (144, True, dict(model=REF, size=37, angles_deg=(0.7, -2.2), heights=(0.0, 0.4))),
@@ -33,6 +35,10 @@ def _build(ctx, gp, dx):
     (144, True, dict(model=REF, size=40, angles_deg=(0.0, 2.0), shifts={1: (1 / 3, 1 / 3)}, e_field=0.1)),
     (224, True, dict(model=REF, num_sheets=3, size=33, heights=(0, 3.35, 6.7), angles_deg=(0, 3.0, -1.5))),
     (224, False, dict(model=REF, num_sheets=4, size=30, heights=(0, 3.35, 6.7, 10.05), angles_deg=(0, 3, -1.5, 1))),
+    (144, True, dict(model=REF, size=160, angles_deg=(0.0, 2.6))),
+    (144, False, dict(model=REF, size=330, angles_deg=(0.0, 2.6))),
+    (224, True, dict(model=REF, num_sheets=3, size=110, heights=(0, 3.35, 6.6), angles_deg=(0, 3.0, -1.5))),
+    (96, True, dict(model=SIMPLE, size=190, angles_deg=(0.0, 2.0), shifts={0: (0.2, 0.1)})),
     (96, True, dict(model=SIMPLE, size=50, angles_deg=(0.0, 2.0))),
     (256, False, dict(model=REF, boundary_condition=1, supercell_mn=(13, 12), size=47)),
     (256, False, dict(model=REF, boundary_condition=1, supercell_mn=(13, 12), size=47, k_vec=(0.01, 0.02))),
