@@ -1141,9 +1141,14 @@ __global__ void __launch_bounds__(kWinThreads) k_win_fill(int64_t n, int64_t nsl
 // columns, 2 of 16, 1 of 32), without a conflict when their positions differ modulo cls.
 // So block b's m-th position of class c (position modulo cls) goes to place
 // cls m + (c - b) mod cls, as long as every class has an m-th one; the others follow.
+// Within a class the positions whose weights are all at most a quarter of the block's
+// largest come first: a row's many small products are then rounded at the size of their
+// own sum, not of the few large ones'. LDOS of a 200k flake, 1000 moments, relative error
+// against 64 bits over six sets of targets: 1.2e-6 to 1.8e-6 (1.7e-6 to 3.1e-6 in
+// position order, 2.1e-6 to 3.8e-6 in the tiled step), at the same time a step.
 constexpr int kPanWords = kWinMax / 32;
 constexpr size_t kPanFillSmem =
-    (size_t)kWinMax * 4 + (size_t)(kWinThreads / 32) * kPanWords * (kPanRows * 4 + 8);
+    (size_t)kWinMax * 4 + (size_t)(kWinThreads / 32) * kPanWords * ((kPanRows + 1) * 4 + 16);
 __global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl, int tile_slices, int RW, int PC, int cls,
                                                           int fill, const int64_t* __restrict__ rowptr,
                                                           const int32_t* __restrict__ col,
@@ -1155,9 +1160,11 @@ __global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl
                                                           uint16_t* __restrict__ widx, int* __restrict__ over) {
   extern __shared__ __align__(16) uint32_t win_keys[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // per word of 32 positions: how many earlier ones of each class the union holds
-  unsigned long long* pre = reinterpret_cast<unsigned long long*>(win_keys + kWinMax) + (size_t)warp * kPanWords;
-  uint32_t* bits = win_keys + kWinMax + (size_t)(kWinThreads / 32) * kPanWords * 2 + (size_t)warp * kPanRows * kPanWords;
+  // per word of 32 positions: the places before it of each class, for small and for large weights
+  unsigned long long* pre = reinterpret_cast<unsigned long long*>(win_keys + kWinMax) + (size_t)warp * kPanWords * 2;
+  // the union by row, then the positions with a large weight
+  uint32_t* bits = win_keys + kWinMax + (size_t)(kWinThreads / 32) * kPanWords * 4 + (size_t)warp * (kPanRows + 1) * kPanWords;
+  uint32_t* large = bits + kPanRows * kPanWords;
   const int m = cnt[blockIdx.x], words = (m + 31) / 32;
   for (int i = threadIdx.x; i < m; i += kWinThreads) win_keys[i] = (uint32_t)list[blockIdx.x * stride + i];
   __syncthreads();
@@ -1183,7 +1190,13 @@ __global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl
     const int rl = (int)(at % RW);
     for (int i = lane; i < words; i += 32)
 #pragma unroll
-      for (int r = 0; r < kPanRows; ++r) bits[r * kPanWords + i] = 0u;
+      for (int r = 0; r <= kPanRows; ++r) bits[r * kPanWords + i] = 0u;
+    float top = 0.f;
+    if (fill)
+      for (int64_t e = rowptr[min(n, row0)] + lane; e < rowptr[min(n, row0 + kPanRows)]; e += 32)
+        top = fmaxf(top, fabsf(val[e]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     __syncwarp();
     bool twice = false;
     for (int r = 0; r < kPanRows && row0 + r < n; ++r)
@@ -1191,18 +1204,19 @@ __global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl
         const int w = find((uint32_t)col[e]);
         const uint32_t bit = 1u << (w & 31);
         if (atomicOr(&bits[r * kPanWords + (w >> 5)], bit) & bit) twice = true;
+        if (fill && fabsf(val[e]) > 0.25f * top) atomicOr(&large[w >> 5], bit);
       }
     __syncwarp();
     // the lane's words, 8 at most
     const int per = (words + 31) / 32, i0 = min(words, lane * per), i1 = min(words, i0 + per);
-    int own[4] = {0, 0, 0, 0};
+    int own[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // small ones of each class, large ones
     for (int i = i0; i < i1; ++i)
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (c < cls) own[c] += __popc(united(i) & mask(c));
-    int first[4], total[4];
+      for (int c = 0; c < 8; ++c)
+        if ((c & 3) < cls) own[c] += __popc(united(i) & (c < 4 ? ~large[i] : large[i]) & mask(c & 3));
+    int first[8], total[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 8; ++c) {
       int x = own[c];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1210,7 +1224,13 @@ __global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl
         if (lane >= o) x += y;
       }
       first[c] = x - own[c];
-      total[c] = __shfl_sync(0xffffffffu, x, 31);
+      const int all = __shfl_sync(0xffffffffu, x, 31);
+      if (c < 4) {
+        total[c] = all;
+      } else {
+        first[c] += total[c - 4];
+        total[c - 4] += all;
+      }
     }
     if (fill == 0) {
       if (__any_sync(0xffffffffu, twice) && lane == 0) atomicExch(over, 1);
@@ -1221,20 +1241,26 @@ __global__ void __launch_bounds__(kWinThreads) k_pan_fill(int64_t n, int64_t nsl
     int least = total[0];
     for (int c = 1; c < cls; ++c) least = min(least, total[c]);
     for (int i = i0; i < i1; ++i) {
-      unsigned long long p = 0;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        p |= (unsigned long long)first[c] << (16 * c);
-        if (c < cls) first[c] += __popc(united(i) & mask(c));
+      for (int g = 0; g < 2; ++g) {
+        const uint32_t u = united(i) & (g ? large[i] : ~large[i]);
+        unsigned long long p = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          p |= (unsigned long long)first[4 * g + c] << (16 * c);
+          if (c < cls) first[4 * g + c] += __popc(u & mask(c));
+        }
+        pre[2 * i + g] = p;
       }
-      pre[i] = p;
     }
     __syncwarp();
     for (int r = 0; r < kPanRows && row0 + r < n; ++r)
       for (int64_t e = rowptr[row0 + r] + lane; e < rowptr[row0 + r + 1]; e += 32) {
         const int w = find((uint32_t)col[e]), i = w >> 5, c = w & (cls - 1);
-        const int k = (int)((pre[i] >> (16 * c)) & 0xffffu) +
-                      __popc(united(i) & mask(c) & ((1u << (w & 31)) - 1u));
+        const uint32_t below = mask(c) & ((1u << (w & 31)) - 1u);
+        const int g = (large[i] >> (w & 31)) & 1;
+        const int k = (int)((pre[2 * i + g] >> (16 * c)) & 0xffffu) +
+                      __popc(united(i) & (g ? large[i] : ~large[i]) & below);
         int before = 0;  // positions of the classes before it that have no partner
         for (int q = 0; q < c; ++q) before += total[q] - least;
         const int j = k < least ? cls * k + ((c - rl) & (cls - 1)) : cls * least + before + (k - least);
