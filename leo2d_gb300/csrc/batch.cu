@@ -20,6 +20,10 @@
 // Vector blocks of all flakes are slices of two concatenated n_total x C
 // buffers; each flake streams its locality-reordered copy when it has one
 // (the same policy as the single-matrix recursion).
+// The graph holds addresses inside the matrices (ordering, blocks, values), which
+// other calls on a matrix may build again: a single run in another ordering, a
+// rescale. A run compares each matrix's generation with the one captured, and on
+// a difference orders the matrix as the batch wants it and captures again.
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -127,6 +131,8 @@ struct FlakeView {
   const int64_t* rowptr = nullptr;
   const uint2* ent = nullptr;
   const int32_t* new2old = nullptr;
+  bool perm = false;
+  uint64_t generation = 0;  // of the matrix when the graph was captured
   int64_t row_off = 0;  // first row of the flake in the concatenated vector buffers
 };
 
@@ -159,6 +165,10 @@ struct leo2d_batch {
   std::vector<FlakeView> fl;
   int P = 0, steps = 0, R = 0, passes = 0;
   BatchShape shape;
+  double patch = 0.0;   // the flakes' locality ordering
+  int curve = 0;
+  bool rb4 = false;     // the 4-row step's blocks
+  int stages = 2, chunk = 4;  // of the tiles, as the context had them at creation
   int tile_rows = 0, tile_cap = 0, rp_bytes = 0, col_bytes = 0, stage_bytes = 0;
   size_t dyn_smem = 0;
   unsigned grid = 0;
@@ -170,8 +180,6 @@ struct leo2d_batch {
   DevBuf<uint64_t> seed_first;
   DevBuf<unsigned> bar;  // 8-row form: per-flake step barriers
   DevBuf<int> abort;
-  // 8-row form: what the captured graph points at, per flake (checked before a run)
-  std::vector<const unsigned char*> rt_data;
   BatchParams<float> params[2];  // step parity 0 / 1 differ in buffer roles
   cudaGraphExec_t graph = nullptr;
   int64_t launches_per_run = 0;
@@ -211,7 +219,7 @@ bool layout(leo2d_batch* b, const BatchShape& s) {
     b->rp_bytes = (int)up((int64_t)(b->tile_rows + 4) * 8, 128);
     b->col_bytes = (int)up((int64_t)b->tile_cap * 8, 128);
     b->stage_bytes = (int)up(b->rp_bytes + b->col_bytes, 128);
-    b->dyn_smem = (size_t)ctx->tile_stages * b->stage_bytes;
+    b->dyn_smem = (size_t)b->stages * b->stage_bytes;
     if (b->dyn_smem + 24 * 1024 > ctx->smem_optin) return false;
     int occ = 0;
     batch_dispatch(ctx, s.cols, 0, 0, nullptr, &occ, b->dyn_smem, s.warps);
@@ -230,7 +238,7 @@ bool layout(leo2d_batch* b, const BatchShape& s) {
   for (int f = 0; f < F; ++f) {
     w[f] = (double)b->fl[f].nnz * 8 + (double)b->fl[f].n * (8 + 12.0 * s.cols);
     cap[f] = s.rt ? std::max<int64_t>(1, tiles_of[f])
-                  : std::max<int64_t>(1, (tiles_of[f] + ctx->tile_chunk - 1) / ctx->tile_chunk);
+                  : std::max<int64_t>(1, (tiles_of[f] + b->chunk - 1) / b->chunk);
   }
   std::vector<int> nb(F, 1);
   {
@@ -283,7 +291,7 @@ void fill_params(leo2d_batch* b) {
       a.alpha = 0.0f;
       a.tprev = nullptr;
       a.rows_per_item = b->shape.rows_per_item;
-      ta.lay = TileLayout{ctx->tile_stages, ctx->tile_chunk, b->tile_rows, b->tile_cap, b->rp_bytes, b->col_bytes,
+      ta.lay = TileLayout{b->stages, b->chunk, b->tile_rows, b->tile_cap, b->rp_bytes, b->col_bytes,
                           b->stage_bytes};
       ta.spin_limit = ctx->spin_limit;
       ta.status = ctx->status.p;
@@ -377,30 +385,43 @@ void enqueue_run(leo2d_batch* b) {
   }
 }
 
+// Orders the flakes' matrices as the batch streams them, and points the views there.
+void bind_flakes(leo2d_batch* b) {
+  leo2d_ctx* ctx = b->ctx;
+  for (FlakeView& v : b->fl) {
+    const leo2d_csr* m = v.csr;
+    leo2d_csr* mm = const_cast<leo2d_csr*>(m);
+    if (v.perm && (!m->reordered || m->reorder_patch != b->patch || m->reorder_curve_req != b->curve))
+      csr_build_reordered(ctx, mm, b->patch, m->reorder_fp64, b->curve != 0);
+    if (b->rb4 && (!m->rb_built || m->rb_patch != m->reorder_patch))
+      LEO_REQUIRE(csr_build_rb(ctx, mm), "a batched flake's row blocks exceed the build limits");
+    v.n = m->n;
+    v.nnz = m->nnz;
+    v.rowptr = v.perm ? m->prow.p : m->rowptr.p;
+    v.ent = v.perm ? m->pent.p : m->ent.p;
+    v.new2old = v.perm ? m->new2old.p : nullptr;
+  }
+}
+
 // The 8-row form: each flake's blocks built for the CTAs it gets (a single run on
-// the same matrix rebuilds them for one CTA per SM, so a run checks them first).
+// the same matrix rebuilds them for one CTA per SM).
 void build_rt_formats(leo2d_batch* b) {
   leo2d_ctx* ctx = b->ctx;
   rt_batch_prepare(ctx, b->grid);
-  b->rt_data.assign(b->fl.size(), nullptr);
   for (size_t f = 0; f < b->fl.size(); ++f) {
     leo2d_csr* m = const_cast<leo2d_csr*>(b->fl[f].csr);
     const int nb = b->block_first[f + 1] - b->block_first[f];
     LEO_REQUIRE(csr_build_rt(ctx, m, kRtBatchWarps, rt_group_of(ctx), rt_chunk_of(ctx), 8, nb) &&
                     m->rt_grid == (unsigned)nb,
                 "a batched flake's 8-row blocks exceed the build limits");
-    b->rt_data[f] = m->rt_data.p;
   }
 }
 
-bool rt_formats_current(const leo2d_batch* b) {
-  for (size_t f = 0; f < b->fl.size(); ++f) {
-    const leo2d_csr* m = b->fl[f].csr;
-    const int nb = b->block_first[f + 1] - b->block_first[f];
-    if (!m->rt_built || m->rt_data.p != b->rt_data[f] || m->rt_grid != (unsigned)nb || m->rt_rows != 8 ||
-        m->rt_warps != kRtBatchWarps)
-      return false;
-  }
+// Whether the captured graph still points at the matrices' arrays.
+bool current(const leo2d_batch* b) {
+  if (!b->graph) return false;
+  for (const FlakeView& v : b->fl)
+    if (v.generation != v.csr->generation) return false;
   return true;
 }
 
@@ -440,6 +461,7 @@ void capture(leo2d_batch* b) {
   cudaGraphDestroy(g);
   if (e != cudaSuccess) fail(LEO2D_ERR_CUDA, std::string("graph instantiation: ") + cudaGetErrorString(e));
   b->launches_per_run = ctx->launches - l0;
+  for (FlakeView& v : b->fl) v.generation = v.csr->generation;
 }
 
 // Times `reps` step launches of the current shape (CUDA events, untimed warm-up).
@@ -491,6 +513,8 @@ leo2d_status leo2d_batch_create(leo2d_ctx* ctx, const leo2d_csr* const* csrs, in
     LEO_CUDA(cudaSetDevice(ctx->device));
     auto b = std::make_unique<leo2d_batch>();
     b->ctx = ctx;
+    b->stages = ctx->tile_stages;
+    b->chunk = ctx->tile_chunk;
     b->P = cfg->poly_order;
     b->steps = cfg->poly_order / 2;
     b->R = cfg->num_vectors;
@@ -503,27 +527,20 @@ leo2d_status leo2d_batch_create(leo2d_ctx* ctx, const leo2d_csr* const* csrs, in
       const leo2d_csr* m = csrs[f];
       LEO_REQUIRE(m != nullptr && m->n > 0, "batch matrix is null or empty");
       for (int g = 0; g < f; ++g) LEO_REQUIRE(csrs[g] != m, "a matrix appears twice in the batch");
-      leo2d_csr* mm = const_cast<leo2d_csr*>(m);
       LEO_REQUIRE(m->ent.p != nullptr || m->nnz == 0, "matrix has no FP32 values");
       // the row-block step (every flake ordered, 32 columns) unless the tiled step is asked for
-      const bool perm = rb_mode || (m->pos.p != nullptr && m->nnz > 0 &&
-                                    (ctx->reorder == 1 || (ctx->reorder == -1 && m->n >= 100000)));
-      const double patch = reorder_patch_for(ctx, rb_mode);
-      if (perm && (!m->reordered || m->reorder_patch != patch || m->reorder_curve_req != ctx->reorder_curve))
-        csr_build_reordered(ctx, mm, patch, m->reorder_fp64, ctx->reorder_curve != 0);
-      if (rb_mode && ctx->kernel_variant == 3 && (!m->rb_built || m->rb_patch != m->reorder_patch))
-        LEO_REQUIRE(csr_build_rb(ctx, mm), "a batched flake's row blocks exceed the build limits");
       FlakeView v;
       v.csr = m;
-      v.n = m->n;
-      v.nnz = m->nnz;
-      v.rowptr = perm ? m->prow.p : m->rowptr.p;
-      v.ent = perm ? m->pent.p : m->ent.p;
-      v.new2old = perm ? m->new2old.p : nullptr;
+      v.perm = rb_mode || (m->pos.p != nullptr && m->nnz > 0 &&
+                           (ctx->reorder == 1 || (ctx->reorder == -1 && m->n >= 100000)));
       v.row_off = off;
       off += (m->n + 3) / 4 * 4;  // 16-byte aligned slices for any C
       b->fl.push_back(v);
     }
+    b->patch = reorder_patch_for(ctx, rb_mode);
+    b->curve = ctx->reorder_curve;
+    b->rb4 = rb_mode && ctx->kernel_variant == 3;
+    bind_flakes(b.get());
     b->n_total = off;
     b->seed_first.alloc(2);
     uint64_t sf[2] = {cfg->seed, cfg->first_vector};
@@ -581,10 +598,16 @@ leo2d_status leo2d_batch_run(leo2d_batch* b, uint64_t seed, uint64_t first_vecto
   leo2d_ctx* ctx = b->ctx;
   return guard(ctx, [&] {
     LEO_CUDA(cudaSetDevice(ctx->device));
-    if (b->shape.rt && !rt_formats_current(b)) {
-      // a single run on one of the flakes rebuilt its blocks for another grid:
-      // rebuild them for the batch and capture the run again
-      build_rt_formats(b);
+    if (!current(b)) {
+      // another call built or released what the graph points at (a single run on one
+      // of the flakes, a rescale): build it for the batch and capture the run again
+      bind_flakes(b);
+      // (the same shape and groups as before; measures the blocks' tiles again, which
+      // a capture cannot)
+      const unsigned grid = b->grid;
+      LEO_REQUIRE(layout(b, BatchShape(b->shape)) && b->grid == grid, "batch tiles do not fit in shared memory");
+      fill_params(b);
+      if (b->shape.rt) build_rt_formats(b);
       capture(b);
     }
     uint64_t sf[2] = {seed, first_vector};

@@ -39,6 +39,9 @@ struct leo2d_csr {
   // largest stored-entry count of any tile of `tile_rows` consecutive rows (cached)
   int tile_rows_cached = 0;
   int64_t tile_max_nnz = 0;
+  // counts every build or release of the arrays below and of the FP32 values: what
+  // holds their addresses between calls (a batch's captured graph) checks it
+  uint64_t generation = 0;
   // locality-ordered copy streamed by the recursion (reorder.cu)
   bool reordered = false;
   bool reorder_fp64 = false;

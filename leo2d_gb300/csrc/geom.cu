@@ -1308,7 +1308,7 @@ void csr_alloc_entries(leo2d_ctx* ctx, leo2d_csr* csr, int64_t nnz, bool with_dx
 
 void csr_refresh_fp32(leo2d_ctx* ctx, leo2d_csr* csr) {
   csr->tile_rows_cached = 0;
-  csr_drop_reordered(csr);
+  csr_drop_reordered(csr);  // (and counts the generation on)
   if (csr->nnz == 0) return;
   csr->val32.alloc(csr->nnz + kCsrPad);
   LEO_CUDA(cudaMemsetAsync(csr->val32.p + csr->nnz, 0, kCsrPad * sizeof(float), ctx->stream));

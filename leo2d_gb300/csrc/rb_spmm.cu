@@ -895,6 +895,7 @@ int64_t rb_tile_max_bytes(leo2d_ctx* ctx, const leo2d_csr* csr, int tile) {
 }
 
 void csr_drop_rb(leo2d_csr* csr) {
+  ++csr->generation;
   csr_drop_rbw(csr);
   csr->rb_xs_built = false;
   csr->rb_xrel.release();

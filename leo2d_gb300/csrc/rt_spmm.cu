@@ -1186,6 +1186,7 @@ unsigned rt_grid(leo2d_ctx* ctx, const leo2d_csr* csr, int warps, int rows) {
 }
 
 void csr_drop_rt(leo2d_csr* csr) {
+  ++csr->generation;
   csr->rt_counted = false;
   csr->rt_built = false;
   csr->rt_kst.release();
@@ -1225,6 +1226,7 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
     ctx_sync(ctx);
     while (cap < most && cap < kRtMaxEnt) cap *= 2;
   }
+  ++csr->generation;
   const size_t slice = rt_build_slice(cap), smem = kRtBuildWarps * slice;
   auto build_kernel = cpx ? k_rt_build<16, true> : rows == 16 ? k_rt_build<16> : k_rt_build<8>;
   LEO_CUDA(cudaFuncSetAttribute(build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
