@@ -82,8 +82,7 @@ template <int V, int LPR, int WARPS>
 void batch_kernel_w(leo2d_ctx* ctx, unsigned grid, size_t smem, const BatchParams<float>* p, int* occ,
                     size_t set_smem) {
   if (occ) {
-    LEO_CUDA(cudaFuncSetAttribute(k_cheb_batch<float, V, LPR, WARPS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)set_smem));
+    allow_smem(ctx, (const void*)k_cheb_batch<float, V, LPR, WARPS>);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_cheb_batch<float, V, LPR, WARPS>, WARPS * 32, set_smem);
     return;
   }

@@ -264,8 +264,10 @@ leo2d_status guard(leo2d_ctx* ctx, F&& f) {
 }
 
 // Lets `kern` be launched with any dynamic shared memory the device has, once per
-// context: the attribute call cost a Chebyshev step of a small cell 1.2 us of its 7,
-// and a call with one step's size could undercut another thread's launch.
+// context. The limit belongs to the function on the device, not to a context: a call
+// that sets it to one launch's size can undercut another thread between its own call
+// and its launch, so it is set nowhere else. (Setting it before every launch also
+// cost a Chebyshev step of a small cell 1.2 us of its 7.)
 inline void allow_smem(leo2d_ctx* ctx, const void* kern) {
   if (ctx->smem_ready.count(kern)) return;
   cudaFuncAttributes at{};

@@ -59,8 +59,7 @@ template <typename T, int V, int LPR, int WARPS>
 void tile_kernel_w(leo2d_ctx* ctx, unsigned grid, size_t smem, const TileArgs<T>* a, int* occ,
                    size_t set_smem) {
   if (occ) {
-    LEO_CUDA(cudaFuncSetAttribute(k_cheb_tile<T, V, LPR, WARPS>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)set_smem));
+    allow_smem(ctx, (const void*)k_cheb_tile<T, V, LPR, WARPS>);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k_cheb_tile<T, V, LPR, WARPS>, WARPS * 32, set_smem);
     return;
   }

@@ -401,7 +401,7 @@ void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap*
   LEO_REQUIRE(n >= 1 && n < (int64_t(1) << 31), "fused MLP forward: n must be 1 .. 2^31 - 1");
   LEO_REQUIRE(Y || (sums_dev && part), "fused MLP forward: no output");
   LEO_REQUIRE(kSmemBytes <= ctx->smem_optin, "fused MLP forward: shared memory per block too small");
-  LEO_CUDA(cudaFuncSetAttribute(k_mlp_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+  allow_smem(ctx, (const void*)k_mlp_fused);
   FusedArgs a{};
   a.tx = tx;
   for (int l = 0; l < 4; ++l) {

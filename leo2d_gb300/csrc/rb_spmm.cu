@@ -925,7 +925,7 @@ bool csr_build_rb(leo2d_ctx* ctx, leo2d_csr* csr) {
   LEO_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), ctx->stream));
   LEO_CUDA(cudaMemsetAsync(ssum.p, 0, sizeof(unsigned long long), ctx->stream));
   const size_t smem = (size_t)kRbMaxEnt * sizeof(unsigned long long);
-  LEO_CUDA(cudaFuncSetAttribute(k_rb_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)k_rb_build);
   // a warp per row block; the blocks with more entries than it sorts go to the
   // block-wide kernel (listed in pass 0, the same list in pass 1)
   DevBuf<int64_t> big((size_t)nrb);

@@ -526,7 +526,7 @@ bool csr_build_rbw(leo2d_ctx* ctx, leo2d_csr* csr) {
   LEO_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), ctx->stream));
   LEO_CUDA(cudaMemsetAsync(wsum.p, 0, sizeof(unsigned long long), ctx->stream));
   const size_t smem = (size_t)(kRbwMaxSlots + 2 * kRbwMaxWin + kRbwMaxRuns) * sizeof(uint32_t);
-  LEO_CUDA(cudaFuncSetAttribute(k_rbw_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)k_rbw_build);
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)ctx->sm_count * 4);
   launch(ctx, "rbw_build", [&] {
     k_rbw_build<<<grid, kRbwBuildThreads, smem, ctx->stream>>>(nrb, kRbwTile, csr->rb_off.p, csr->rb_data.p, 0, cnt.p,
@@ -619,7 +619,7 @@ void rbw_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, const StepShape& shap
   a.status = ctx->status.p;
   a.never_wait = ctx->test_unsatisfied_wait;
   auto go = [&](auto kern) {
-    LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ctx, (const void*)kern);
     launch(ctx, "cheb_step", [&] { kern<<<grid, (kRbwTile + 1) * 32, smem, ctx->stream>>>(a); });
   };
   const bool u8 = shape.rb_unroll == 8;

@@ -1298,7 +1298,7 @@ __global__ void __launch_bounds__(kWinThreads) k_pan_order(int64_t nsl, int tile
 
 void row_coop_launch(leo2d_ctx* ctx, const void* kern, unsigned grid, int threads, size_t smem, void* args) {
   int occ = 0;
-  LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, kern);
   LEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
   LEO_REQUIRE(occ >= 1 && grid <= (unsigned)ctx->sm_count, "multi-step launch: the CTAs cannot all be resident");
   void* argv[1] = {args};
@@ -1355,7 +1355,7 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
     csr->win_off.alloc(nsl + 1);
     csr->win_slen.alloc(nsl);
     const size_t list_smem = (size_t)(kWinSet + kWinMax) * sizeof(uint32_t);
-    LEO_CUDA(cudaFuncSetAttribute(k_win_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)list_smem));
+    allow_smem(ctx, (const void*)k_win_list);
     DevBuf<int> over(1);
     // tiles per CTA: the fewest whose windows fit
     for (int64_t m = 1;; m += std::max<int64_t>(1, m / 2)) {
@@ -1410,7 +1410,7 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
           k_slice_len<<<grid_for(nsl, 256, (int64_t)ctx->sm_count * 16), 256, 0, ctx->stream>>>(n, nsl, rp, kWinChunk, count.p, csr->win_slen.p);
         });
       } else {
-        LEO_CUDA(cudaFuncSetAttribute(k_pan_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanFillSmem));
+        allow_smem(ctx, (const void*)k_pan_fill);
         csr->win_blk.alloc((size_t)nsl * pan_blocks(s.cs));
         panels(0);
         launch(ctx, "win_build", [&] {

@@ -1229,7 +1229,7 @@ bool csr_build_rt(leo2d_ctx* ctx, leo2d_csr* csr, int warps, int group, int chun
   ++csr->generation;
   const size_t slice = rt_build_slice(cap), smem = kRtBuildWarps * slice;
   auto build_kernel = cpx ? k_rt_build<16, true> : rows == 16 ? k_rt_build<16> : k_rt_build<8>;
-  LEO_CUDA(cudaFuncSetAttribute(build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)build_kernel);
   const unsigned bgrid = grid_for(sh.nrb * 32, kRtBuildWarps * 32, (int64_t)ctx->sm_count * 8);
   DevBuf<unsigned long long> ssum(1);
   LEO_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), ctx->stream));
@@ -1337,7 +1337,7 @@ size_t rt_batch_smem() { return rt_smem_bytes(kRtBatchWarps, kRtBatchDepth, kRtC
 void rt_batch_prepare(leo2d_ctx* ctx, unsigned grid) {
   auto kern = k_cheb_rt_batch<kRtBatchWarps, kRtBatchDepth>;
   const size_t smem = rt_batch_smem();
-  LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)kern);
   int occ = 0, coop = 0;
   LEO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kRtBatchWarps * 32, smem));
   LEO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));

@@ -265,12 +265,11 @@ void make_tmap_bf16_ld(CUtensorMap* map, const void* base, int64_t rows, int64_t
 }
 
 template <int BN>
-static void prepare_bn() {
-  const int smem = (int)gemm_smem_bytes(BN);
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiF32, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiBias, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiBiasGelu, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm<kEpiGeluBwd, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+static void prepare_bn(leo2d_ctx* ctx) {
+  allow_smem(ctx, (const void*)k_tc_gemm<kEpiF32, BN>);
+  allow_smem(ctx, (const void*)k_tc_gemm<kEpiBias, BN>);
+  allow_smem(ctx, (const void*)k_tc_gemm<kEpiBiasGelu, BN>);
+  allow_smem(ctx, (const void*)k_tc_gemm<kEpiGeluBwd, BN>);
 }
 
 template <int BN>
@@ -290,8 +289,8 @@ static void launch_bn(leo2d_ctx* ctx, GemmEpi epi, const CUtensorMap& ta, const 
 
 void tc_gemm_prepare(leo2d_ctx* ctx) {
   if (ctx->tc_gemm_ready) return;
-  prepare_bn<256>();
-  prepare_bn<64>();
+  prepare_bn<256>(ctx);
+  prepare_bn<64>(ctx);
   ctx->tc_gemm_ready = true;
 }
 
@@ -583,7 +582,7 @@ void tc_gemm_f32x3_acc(leo2d_ctx* ctx, const float* A, const float* B, int M, in
   g.partial = partial.p;
   g.status = ctx->status.p;
   const size_t smem = (size_t)F3_ST * kF3Stage + 1024;
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_gemm_f32x3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)k_tc_gemm_f32x3);
   const unsigned grid = (unsigned)std::min<int64_t>(items, ctx->sm_count);
   launch(ctx, "cond_gemm", [&] { k_tc_gemm_f32x3<<<grid, 192, smem, ctx->stream>>>(ta, tb, g); });
   launch(ctx, "cond_gemm_sum", [&] {

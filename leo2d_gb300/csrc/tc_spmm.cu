@@ -113,7 +113,7 @@ extern "C" leo2d_status leo2d_tc_gemm_tf32x3(leo2d_ctx* ctx, const float* a, con
     h2d(ctx, da.p, a, (size_t)128 * K);
     h2d(ctx, db.p, b, (size_t)N * K);
     const size_t smem = (size_t)2 * N * K * 4 + 1024;
-    LEO_CUDA(cudaFuncSetAttribute(k_tf32x3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ctx, (const void*)k_tf32x3);
     launch(ctx, "tc_tf32x3", [&] {
       k_tf32x3<<<1, 128, smem, ctx->stream>>>(da.p, db.p, (int)N, (int)K, dd.p, ctx->status.p);
     });
@@ -631,7 +631,7 @@ bool csr_build_tc(leo2d_ctx* ctx, leo2d_csr* csr) {
   LEO_CUDA(cudaMemsetAsync(err.p, 0, 3 * sizeof(int), ctx->stream));
   LEO_CUDA(cudaMemsetAsync(wsum.p, 0, sizeof(unsigned long long), ctx->stream));
   const size_t smem = (size_t)(2 * kTcMaxEnt + kTcMaxWin) * 4;
-  LEO_CUDA(cudaFuncSetAttribute(k_tc_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(ctx, (const void*)k_tc_build);
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)ctx->sm_count);
   launch(ctx, "tc_build", [&] {
     k_tc_build<<<grid, kTcThreads, smem, ctx->stream>>>(n, tiles, csr->prow.p, csr->pcol.p, csr->pval32.p,
@@ -683,7 +683,7 @@ void tc_launch_step(leo2d_ctx* ctx, const leo2d_csr* csr, int cols, unsigned gri
   a.prev_dots = prev_dots;
   a.status = ctx->status.p;
   auto go = [&](auto kern) {
-    LEO_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ctx, (const void*)kern);
     launch(ctx, "cheb_step", [&] { kern<<<grid, kTcThreads, smem, ctx->stream>>>(a); });
   };
   if (cols == 32) return go(k_cheb_tc<32>);
