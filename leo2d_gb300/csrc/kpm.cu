@@ -587,15 +587,18 @@ StepShape choose_shape(leo2d_ctx* ctx, const leo2d_csr* csr, bool fp64, int cols
     s.rb_window = false;
     s.rb_warps = 24;
   }
-  // 20 warps hide more of the epilogue where every warp has many blocks (10M
-  // orbitals: 2.26 ms against 2.34 with 16; 2.4M: 0.559 against 0.573), and cost
-  // more at the start and end of a short step (400k: 0.117 against 0.114; 150k:
-  // 0.060 against 0.055)
-  s.rt_warps = ctx->rt_warps > 0 ? ctx->rt_warps
-                                 : (cached && it->second.rt_warps > 0 ? it->second.rt_warps : (csr->n >= 1000000 ? 20 : 16));
   s.rt_stage = ctx->rt_stage >= 0 ? ctx->rt_stage : (cached && it->second.rt ? it->second.rt_stage : 1);
   s.rt_depth = ctx->rt_depth > 0 ? ctx->rt_depth : (cached && it->second.rt_depth > 0 ? it->second.rt_depth : 3);
   s.rt_rows = ctx->rt_rows > 0 ? ctx->rt_rows : (cached && it->second.rt ? it->second.rt_rows : 8);
+  // 20 warps hide more of the epilogue where every warp has many blocks (10M
+  // orbitals: 2.26 ms against 2.34 with 16; 2.4M: 0.559 against 0.573), and cost
+  // more at the start and end of a short step (400k: 0.117 against 0.114; 150k:
+  // 0.060 against 0.055); the line between 400k and 2.4M was not searched for. Only
+  // the 8-row cp.async form of depth 3 is built for 20.
+  const bool form20 = s.rt_stage == 1 && s.rt_rows == 8 && s.rt_depth == 3;
+  s.rt_warps = ctx->rt_warps > 0 ? ctx->rt_warps
+                                 : (cached && it->second.rt_warps > 0 ? it->second.rt_warps
+                                                                      : (form20 && csr->n >= 1000000 ? 20 : 16));
   LEO_REQUIRE(s.rows_per_item >= 0 && s.rows_per_item <= 64, "rows_per_warp must be 0..64");
   return s;
 }
