@@ -333,7 +333,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
   if (shape.rb || shape.rt) shape.tc = false;
   const int used = s.cols_used > 0 ? s.cols_used : s.cols;
   if (shape.tc || shape.rb || shape.rt || m->nnz == 0 ||
-      (shape.row && !s.row_built && !row_pays(m, s.fp64, steps_)))
+      (shape.row && !s.row_built && !row_pays(n, s.fp64, steps_)))
     shape.row = false;
   const bool want_perm = can_perm && (shape.tc || shape.rb || shape.rt || ctx->reorder == 1 ||
                                       (ctx->reorder == -1 &&
@@ -1053,7 +1053,7 @@ extern "C" leo2d_status leo2d_kpm_step_kernel(leo2d_ctx* ctx, const leo2d_csr* c
     if (s.rb && (!can_perm || s.fp64 || s.cols != 32 || ctx->reorder == 0)) s.rb = false;
     if (s.rt && (!can_perm || s.fp64 || s.cols != 32 || ctx->reorder == 0)) s.rt = false;
     if (s.tc && !can_perm) s.tc = false;
-    if (s.tc || s.rb || s.rt || csr->nnz == 0 || !row_pays(csr, s.fp64, cfg->poly_order / 2)) s.row = false;
+    if (s.tc || s.rb || s.rt || csr->nnz == 0 || !row_pays(csr->n, s.fp64, cfg->poly_order / 2)) s.row = false;
     *kernel = s.row ? 6 : s.rt ? 5 : s.rb ? (s.rb_window ? 4 : 3) : s.tc ? 2 : s.tiled ? 0 : 1;
     *block = s.cols;
   });

@@ -48,7 +48,7 @@ constexpr int kRowBarWords = 8;  // barrier counters of up to 4 slices; the last
 // Chooses the form and builds its format (once per matrix); false when none fits.
 bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s);
 // Whether the row form is worth its format (and ordering) for a run of `steps`.
-bool row_pays(const leo2d_csr* csr, bool fp64, int steps);
+bool row_pays(int64_t n, bool fp64, int steps);
 // Whether the form for n rows gains from the locality ordering (its windows).
 bool row_wants_order(int64_t n, bool fp64);
 // doubles of the CTAs' partial dots of one launch

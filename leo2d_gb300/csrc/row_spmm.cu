@@ -1513,14 +1513,15 @@ static int row_slices(int cols, int cols_used) {
 
 bool row_wants_order(int64_t n, bool fp64) { return !fp64 && n > kSmallRows; }
 
-bool row_pays(const leo2d_csr* csr, bool fp64, int steps) {
+bool row_pays(int64_t n, bool fp64, int steps) {
   // Below 8000 rows and in FP64 the format takes a few small launches; the window
   // format of more rows, with the locality ordering, takes 0.4 ms (9k rows) to 1.5 ms
   // (200k) and gains 20 to 90 us a step. From 32 steps on it pays in the first run
   // already: 8 local targets at P = 64, tiled steps / first run with the format built /
   // later runs: 9k orbitals 0.86 / 0.74 / 0.33 ms, 200k 3.3 / 2.4 / 0.84 ms; 16
-  // vectors of 60k 3.2 / 1.4 / 0.64 ms.
-  return fp64 || csr->win_off.p || csr->n <= kSmallRows || steps >= 32;
+  // vectors of 60k 3.2 / 1.4 / 0.64 ms. A shorter run takes the tiled step also where
+  // the format is there: the same call gives the same bits whatever ran before it.
+  return fp64 || n <= kSmallRows || steps >= 32;
 }
 
 bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s) {
