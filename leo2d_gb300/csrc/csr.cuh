@@ -109,6 +109,7 @@ struct leo2d_csr {
   // rows in slices of 16, the j-th entries of a slice's rows next to each other
   // (row_spmm.cu): positions padded to the slice's longest row
   bool sell_perm = false;             // built from the locality-ordered copy
+  bool sell_uneven[2] = {false, false};  // [perm]: rows too uneven in length for it
   leo2d::DevBuf<int64_t> sell_off;    // [slices + 1] first position of each slice
   leo2d::DevBuf<int32_t> sell_col;    // [16 positions] columns and FP64 values
   leo2d::DevBuf<double> sell_val;
@@ -118,6 +119,7 @@ struct leo2d_csr {
   bool win_perm = false;
   int win_cs = 0, win_group = 0;      // column slice and CTAs the tiles were cut for
   bool win_twice = false;             // a row stores a column twice: no panels
+  std::vector<uint64_t> win_refused;  // shapes whose windows do not fit (row_spmm.cu)
   bool win_exact = false;             // rows in order, for the exact sums; else panels of 4 rows
   int64_t win_tiles = 0, win_stride = 0;
   int win_tile_slices = 0, win_slice_cap = 0;
@@ -192,4 +194,6 @@ void csr_drop_rbw(leo2d_csr* csr);
 // Drop the formats of row_spmm.cu.
 void csr_drop_sell(leo2d_csr* csr);
 void csr_drop_win(leo2d_csr* csr);
+// Both, and what is known of the shapes that have none (the ordering or the values change).
+void csr_drop_rows(leo2d_csr* csr);
 }  // namespace leo2d

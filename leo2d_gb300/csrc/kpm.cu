@@ -335,14 +335,35 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
   if (shape.tc || shape.rb || shape.rt || m->nnz == 0 ||
       (shape.row && !s.row_built && !row_pays(n, s.fp64, steps_)))
     shape.row = false;
-  const bool want_perm = can_perm && (shape.tc || shape.rb || shape.rt || ctx->reorder == 1 ||
-                                      (ctx->reorder == -1 &&
-                                       (n >= 100000 || (shape.row && row_wants_order(n, s.fp64)))));
+  auto wants_perm = [&]() {
+    return can_perm && (shape.tc || shape.rb || shape.rt || ctx->reorder == 1 ||
+                        (ctx->reorder == -1 && (n >= 100000 || (shape.row && row_wants_order(n, s.fp64)))));
+  };
+  if (shape.row) {
+    LEO_REQUIRE(s.cols == 8 || s.cols == 16 || s.cols == 32 || s.cols == 64 || (s.cols == 128 && !s.fp64),
+                s.fp64 ? "FP64 block width must be 8, 16, 32 or 64 columns"
+                       : "FP32 block width must be 8, 16, 32, 64 or 128 columns");
+    if (row_refused(ctx, m, wants_perm(), s.fp64, s.cols, used)) shape.row = false;
+  }
+  use_perm = wants_perm();
   const double patch = reorder_patch_for(ctx, shape.rb || shape.rt);
-  if (want_perm && (!m->reordered || (s.fp64 && !m->reorder_fp64) || m->reorder_patch != patch ||
-                    m->reorder_curve_req != ctx->reorder_curve))
-    csr_build_reordered(ctx, mm, patch, s.fp64 || m->reorder_fp64, ctx->reorder_curve != 0);
-  use_perm = want_perm;
+  auto order = [&]() {
+    if (use_perm && (!m->reordered || (s.fp64 && !m->reorder_fp64) || m->reorder_patch != patch ||
+                     m->reorder_curve_req != ctx->reorder_curve))
+      csr_build_reordered(ctx, mm, patch, s.fp64 || m->reorder_fp64, ctx->reorder_curve != 0);
+  };
+  order();
+  if (shape.row) {
+    shape.row = row_prepare(ctx, mm, use_perm, s.fp64, s.cols, used, rows);
+    if (shape.row) {
+      bar.alloc(kRowBarWords);
+      if (rows.exact) x2.alloc((size_t)n * s.cols * sizeof(float));
+      shape.tiled = false;
+    } else {
+      use_perm = wants_perm();
+      order();
+    }
+  }
   if (shape.tc) {
     // tensor-core tiles of the locality-ordered copy (built once per matrix)
     if (!m->tc_built || m->tc_patch != m->reorder_patch) csr_build_tc(ctx, mm);
@@ -392,15 +413,6 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
       LEO_REQUIRE(!m->complex_h, "the complex 8-row blocks do not build here: step_kernel 3 runs the 4-row step");
       shape.rt = false;  // a block too heavy for the 8-row build: the gather kernels run
     }
-  }
-  if (shape.row) {
-    LEO_REQUIRE(s.cols == 8 || s.cols == 16 || s.cols == 32 || s.cols == 64 || (s.cols == 128 && !s.fp64),
-                s.fp64 ? "FP64 block width must be 8, 16, 32 or 64 columns"
-                       : "FP32 block width must be 8, 16, 32, 64 or 128 columns");
-    shape.row = row_prepare(ctx, mm, use_perm, s.fp64, s.cols, used, rows);
-    shape.tiled = !shape.row;
-    if (shape.row) bar.alloc(kRowBarWords);
-    if (shape.row && rows.exact) x2.alloc((size_t)n * s.cols * sizeof(float));
   }
   if (shape.tiled && !shape.tc && !shape.rb && !shape.rt) {
     const int ns = tile_slots(s.cols, s.fp64, s.warps);
@@ -1054,6 +1066,10 @@ extern "C" leo2d_status leo2d_kpm_step_kernel(leo2d_ctx* ctx, const leo2d_csr* c
     if (s.rt && (!can_perm || s.fp64 || s.cols != 32 || ctx->reorder == 0)) s.rt = false;
     if (s.tc && !can_perm) s.tc = false;
     if (s.tc || s.rb || s.rt || csr->nnz == 0 || !row_pays(csr->n, s.fp64, cfg->poly_order / 2)) s.row = false;
+    const bool perm = can_perm && (ctx->reorder == 1 || (ctx->reorder == -1 && (csr->n >= 100000 ||
+                                                                                row_wants_order(csr->n, s.fp64))));
+    // (a shape already found to have no row format; whether an untried one has is not known before its build)
+    if (s.row && row_refused(ctx, csr, perm, s.fp64, s.cols, std::max(1, cfg->num_vectors) * group)) s.row = false;
     *kernel = s.row ? 6 : s.rt ? 5 : s.rb ? (s.rb_window ? 4 : 3) : s.tc ? 2 : s.tiled ? 0 : 1;
     *block = s.cols;
   });

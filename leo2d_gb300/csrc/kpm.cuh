@@ -47,6 +47,9 @@ struct RowShape {
 constexpr int kRowBarWords = 8;  // barrier counters of up to 4 slices; the last word is the abort flag
 // Chooses the form and builds its format (once per matrix); false when none fits.
 bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s);
+// Whether row_prepare found before that this shape has no format (too wide windows, a
+// column stored twice, rows of very uneven length).
+bool row_refused(const leo2d_ctx* ctx, const leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used);
 // Whether the row form is worth its format (and ordering) for a run of `steps`.
 bool row_pays(int64_t n, bool fp64, int steps);
 // Whether the form for n rows gains from the locality ordering (its windows).

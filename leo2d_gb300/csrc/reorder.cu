@@ -207,8 +207,7 @@ void csr_build_reordered(leo2d_ctx* ctx, leo2d_csr* csr, double patch, bool with
   csr_drop_tc(csr);
   csr_drop_rb(csr);
   csr_drop_rt(csr);
-  csr_drop_sell(csr);
-  csr_drop_win(csr);
+  csr_drop_rows(csr);
   const int64_t n = csr->n;
   LEO_REQUIRE(csr->pos.p, "locality ordering needs orbital positions");
   LEO_REQUIRE(patch > 0.5, "patch size must exceed 0.5 A");
@@ -308,8 +307,7 @@ void csr_drop_reordered(leo2d_csr* csr) {
   csr_drop_tc(csr);
   csr_drop_rb(csr);
   csr_drop_rt(csr);
-  csr_drop_sell(csr);
-  csr_drop_win(csr);
+  csr_drop_rows(csr);
   csr->reordered = false;
   csr->reorder_fp64 = false;
   csr->new2old.release();

@@ -1335,13 +1335,16 @@ size_t win_smem(const RowShape& s, int win_cap, int slice_cap) {
   const size_t rings = s.exact ? (size_t)kWinWarps * win_ring_bytes(128 / s.cs) : (size_t)kPanWarps * pan_ring_bytes(s.cs);
   return (size_t)win_cap * (s.cs * 4 + 4) + rings + 2 * ((size_t)slice_cap + 1) * 4;
 }
+// One shape of the window format, for the list of those that do not fit.
+uint64_t win_key(const RowShape& s, bool perm) {
+  return (uint64_t)s.group << 32 | (uint64_t)s.cs << 2 | (s.exact ? 2u : 0u) | (perm ? 1u : 0u);
+}
 int win_slice_rows(const RowShape& s) { return s.exact ? kSellRows : kPanRows * pan_blocks(s.cs); }
 
 // The window format (rows for the EXACT form, else panels) for `group` CTAs a slice;
 // false when a slice alone has too wide a window or a row stores a column twice
 // (panels).
 bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
-  if (!s.exact && csr->win_twice) return false;
   const int SR = win_slice_rows(s), PC = s.exact ? kWinChunk : pan_chunk(s.cs);
   const int64_t n = csr->n, nsl = (n + SR - 1) / SR;
   const int64_t* rp = perm ? csr->prow.p : csr->rowptr.p;
@@ -1357,6 +1360,11 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
     const size_t list_smem = (size_t)(kWinSet + kWinMax) * sizeof(uint32_t);
     allow_smem(ctx, (const void*)k_win_list);
     DevBuf<int> over(1);
+    auto refuse = [&]() {  // (the search is not repeated on the next call)
+      csr_drop_win(csr);
+      csr->win_refused.push_back(win_key(s, perm));
+      return false;
+    };
     // tiles per CTA: the fewest whose windows fit
     for (int64_t m = 1;; m += std::max<int64_t>(1, m / 2)) {
       const int64_t ts = std::max<int64_t>(1, (nsl + s.group * m - 1) / (s.group * m));
@@ -1364,10 +1372,7 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
       const int64_t per_cta = (tiles + s.group - 1) / s.group;
       const int64_t slice_cap = ts * per_cta;
       const size_t fixed = win_smem(s, 0, (int)slice_cap);
-      if (fixed >= room) {
-        csr_drop_win(csr);
-        return false;
-      }
+      if (fixed >= room) return refuse();
       const int64_t cap = std::min<int64_t>((int64_t)((room - fixed) / (s.cs * 4 + 4)) / 4 * 4, kWinMax);
       // (a window holds the tile's own rows and, on a bilayer, as many of the other sheet)
       if (ts > 1 && ts * SR > cap) continue;
@@ -1382,10 +1387,7 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
       d2h(ctx, &h, over.p, 1);
       ctx_sync(ctx);
       if (h != 0) {
-        if (ts == 1) {
-          csr_drop_win(csr);
-          return false;
-        }
+        if (ts == 1) return refuse();
         continue;
       }
       csr->win_tiles = tiles;
@@ -1460,8 +1462,10 @@ bool build_win(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, RowShape& s) {
   return true;
 }
 
-void build_sell(leo2d_ctx* ctx, leo2d_csr* csr, bool perm) {
-  if (csr->sell_off.p && csr->sell_perm == perm) return;
+// False when the padding to each slice's longest row would take as much again as the
+// entries: the matrix's memory is then the caller's to plan with, not this format's.
+bool build_sell(leo2d_ctx* ctx, leo2d_csr* csr, bool perm) {
+  if (csr->sell_off.p && csr->sell_perm == perm) return true;
   csr_drop_sell(csr);
   const int64_t n = csr->n, nsl = (n + kSellRows - 1) / kSellRows;
   const int64_t* rp = perm ? csr->prow.p : csr->rowptr.p;
@@ -1475,6 +1479,11 @@ void build_sell(leo2d_ctx* ctx, leo2d_csr* csr, bool perm) {
   d2h(ctx, &total, csr->sell_off.p + nsl, 1);
   ctx_sync(ctx);
   const size_t count = (size_t)std::max<int64_t>(total, 1) * kSellRows;
+  if (count > 2 * (size_t)csr->nnz + 16 * kSellRows) {  // (a few slices of a small matrix: any padding)
+    csr_drop_sell(csr);
+    csr->sell_uneven[perm] = true;
+    return false;
+  }
   csr->sell_col.alloc(count);
   csr->sell_val.alloc(count);
   launch(ctx, "sell_build", [&] {
@@ -1483,6 +1492,7 @@ void build_sell(leo2d_ctx* ctx, leo2d_csr* csr, bool perm) {
         csr->sell_col.p, csr->sell_val.p);
   });
   csr->sell_perm = perm;
+  return true;
 }
 
 }  // namespace
@@ -1506,6 +1516,13 @@ void csr_drop_win(leo2d_csr* csr) {
   csr->win_cs = csr->win_group = 0;
 }
 
+void csr_drop_rows(leo2d_csr* csr) {
+  csr_drop_sell(csr);
+  csr_drop_win(csr);
+  csr->sell_uneven[0] = csr->sell_uneven[1] = false;
+  csr->win_refused.clear();
+}
+
 static int row_slices(int cols, int cols_used) {
   const int cs = std::min(cols, 32);
   return std::max(1, (std::min(cols_used, cols) + cs - 1) / cs);
@@ -1524,8 +1541,9 @@ bool row_pays(int64_t n, bool fp64, int steps) {
   return fp64 || n <= kSmallRows || steps >= 32;
 }
 
-bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s) {
-  s = RowShape{};
+// The form and its launch, nothing built.
+static RowShape row_shape(const leo2d_ctx* ctx, const leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used) {
+  RowShape s{};
   s.cs = std::min(cols, 32);
   s.slices = row_slices(cols, cols_used);
   const int64_t n = csr->n, most = std::max(1, ctx->sm_count / s.slices);
@@ -1540,7 +1558,6 @@ bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols,
     const int lpr = cols / (cols == 8 ? 2 : 4);
     s.dot_slots = (cols == 32 || cols == 64 ? 24 : 8) * (32 / lpr);
     s.dot_rows = std::max(1, 32 / s.dot_slots);
-    if (!build_win(ctx, csr, perm, s)) return false;
   } else {
     // The small form: one CTA up to 4 rows a warp (a barrier costs more than
     // three more rows), else about two thirds of a row per warp, so that no warp
@@ -1560,9 +1577,24 @@ bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols,
       const int rw = 32 / (s.cs / 2);
       s.group = (int)std::max<int64_t>(1, std::min<int64_t>(most, ((n + rw - 1) / rw + s.warps - 1) / s.warps));
       s.smem = 0;
-      build_sell(ctx, csr, perm);
     }
   }
+  return s;
+}
+
+bool row_refused(const leo2d_ctx* ctx, const leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used) {
+  const RowShape s = row_shape(ctx, csr, perm, fp64, cols, cols_used);
+  if (s.form == kRowSell) return csr->sell_uneven[perm];
+  if (s.form != kRowWin) return false;
+  if (!s.exact && csr->win_twice) return true;
+  return std::find(csr->win_refused.begin(), csr->win_refused.end(), win_key(s, perm)) != csr->win_refused.end();
+}
+
+bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s) {
+  if (row_refused(ctx, csr, perm, fp64, cols, cols_used)) return false;
+  s = row_shape(ctx, csr, perm, fp64, cols, cols_used);
+  if (s.form == kRowWin && !build_win(ctx, csr, perm, s)) return false;
+  if (s.form == kRowSell && !build_sell(ctx, csr, perm)) return false;
   const size_t per_step = (size_t)s.slices * s.group * 2 * s.cs * sizeof(double);
   s.chunk = (int)std::max<size_t>(1, kRowPartialBytes / per_step);
   return true;

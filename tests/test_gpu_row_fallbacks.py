@@ -1,5 +1,7 @@
-"""The multi-step row kernel: what runs does not depend on what ran before on the same
-matrix.
+"""The multi-step row kernel where its format cannot be: windows that do not fit, rows of
+very uneven length. The tiled step runs then, with the bits it gives when asked for, and
+a search that failed is not repeated. What runs does not depend on what ran before on
+the same matrix.
 """
 import numpy as np
 import pytest
@@ -7,6 +9,7 @@ import pytest
 import leo2d_gb300 as L
 
 pytestmark = pytest.mark.gpu
+ROW = 6
 
 
 @pytest.fixture()
@@ -30,6 +33,46 @@ def _matrix(n, per_row, reach, seed):
     rng = np.random.default_rng(seed)
     i = rng.integers(0, n, n * per_row // 2)
     return _symmetric(i, np.clip(i + rng.integers(-reach, reach + 1, len(i)), 0, n - 1), n, rng)
+
+
+def _uneven(n, seed):
+    """Four entries a row, 200 in every 16th."""
+    rng = np.random.default_rng(seed)
+    i = np.concatenate([rng.integers(0, n, 2 * n), np.repeat(np.arange(0, n, 16), 200)])
+    return _symmetric(i, rng.integers(0, n, len(i)), n, rng)
+
+
+def _tiled(ctx, run):
+    ctx.set_option("step_kernel", 0)
+    try:
+        return run()
+    finally:
+        ctx.set_option("step_kernel", -1)
+
+
+@pytest.mark.parametrize("n,R", [(30000, 4), (9000, 64)])
+def test_wide_windows_are_searched_for_once(ctx, n, R):
+    csr = ctx.upload_csr(*_matrix(n, 120, n, 3))  # (every slice of rows needs most of the vectors)
+    cfg = L.kpm_cfg(64, R=R, seed=2)
+    first = csr.kpm_dos(cfg)
+    assert csr.step_kernel(cfg)[0] != ROW
+    ctx.reset_stats()
+    np.testing.assert_array_equal(csr.kpm_dos(cfg), first)
+    assert ctx.kernel_stats("win_build")[0] == 0 and ctx.kernel_stats("cheb_steps")[0] == 0
+    np.testing.assert_array_equal(_tiled(ctx, lambda: csr.kpm_dos(cfg)), first)
+    csr.rescale(1.5, 0.0)
+    assert np.max(np.abs(csr.kpm_dos(cfg) - first)) > 1e-3
+
+
+def test_uneven_rows_in_fp64(ctx):
+    csr = ctx.upload_csr(*_uneven(20000, 5))
+    cfg = L.kpm_cfg(64, R=4, seed=2, precision=L.FP64)
+    first = csr.kpm_dos(cfg)
+    assert csr.step_kernel(cfg)[0] != ROW
+    ctx.reset_stats()
+    np.testing.assert_array_equal(csr.kpm_dos(cfg), first)
+    assert ctx.kernel_stats("sell_build")[0] == 0 and ctx.kernel_stats("cheb_steps")[0] == 0
+    np.testing.assert_array_equal(_tiled(ctx, lambda: csr.kpm_dos(cfg)), first)
 
 
 def test_a_short_run_does_not_depend_on_a_longer_one_before(ctx):
