@@ -352,18 +352,36 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
                      m->reorder_curve_req != ctx->reorder_curve))
       csr_build_reordered(ctx, mm, patch, s.fp64 || m->reorder_fp64, ctx->reorder_curve != 0);
   };
-  order();
+  auto vectors = [&]() {
+    const size_t esz = s.fp64 ? sizeof(double) : sizeof(float);
+    x0.alloc((size_t)n * s.cols * esz);
+    x1.alloc((size_t)n * s.cols * esz);
+    dots.alloc((size_t)steps * 2 * s.cols);
+  };
   if (shape.row) {
-    shape.row = row_prepare(ctx, mm, use_perm, s.fp64, s.cols, used, rows);
-    if (shape.row) {
-      bar.alloc(kRowBarWords);
-      if (rows.exact) x2.alloc((size_t)n * s.cols * sizeof(float));
-      shape.tiled = false;
-    } else {
-      use_perm = wants_perm();
+    try {
       order();
+      shape.row = row_prepare(ctx, mm, use_perm, s.fp64, s.cols, used, rows);
+      if (shape.row) {
+        bar.alloc(kRowBarWords);
+        if (rows.exact) x2.alloc((size_t)n * s.cols * sizeof(float));
+        partials.alloc(row_partials(rows, steps));
+        vectors();
+        shape.tiled = false;
+      }
+    } catch (const Error& e) {
+      // no room for the format beside the matrix: the tiled step needs none
+      if (e.status != LEO2D_ERR_OOM) throw;
+      cudaGetLastError();
+      row_release(mm, s.fp64);
+      bar.release();
+      x2.release();
+      partials.release();
+      shape.row = false;
     }
+    if (!shape.row) use_perm = wants_perm();
   }
+  if (!shape.row) order();
   if (shape.tc) {
     // tensor-core tiles of the locality-ordered copy (built once per matrix)
     if (!m->tc_built || m->tc_patch != m->reorder_patch) csr_build_tc(ctx, mm);
@@ -473,11 +491,10 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
     if (g > need) g = std::max<int64_t>(need, 1);
     grid = (unsigned)g;
   }
-  const size_t esz = s.fp64 ? sizeof(double) : sizeof(float);
-  x0.alloc((size_t)n * s.cols * esz);
-  x1.alloc((size_t)n * s.cols * esz);
-  partials.alloc(shape.row ? row_partials(rows, steps) : (size_t)2 * grid * 2 * s.cols);
-  dots.alloc((size_t)steps * 2 * s.cols);
+  if (!shape.row) {
+    vectors();
+    partials.alloc((size_t)2 * grid * 2 * s.cols);
+  }
 }
 
 template <typename T>

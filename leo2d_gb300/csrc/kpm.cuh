@@ -46,7 +46,11 @@ struct RowShape {
 };
 constexpr int kRowBarWords = 8;  // barrier counters of up to 4 slices; the last word is the abort flag
 // Chooses the form and builds its format (once per matrix); false when none fits.
+// Throws LEO2D_ERR_OOM when the device has no room for it (row_release, then another
+// step kernel runs).
 bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used, RowShape& s);
+// Gives back what row_prepare built or began to build.
+void row_release(leo2d_csr* csr, bool fp64);
 // Whether row_prepare found before that this shape has no format (too wide windows, a
 // column stored twice, rows of very uneven length).
 bool row_refused(const leo2d_ctx* ctx, const leo2d_csr* csr, bool perm, bool fp64, int cols, int cols_used);

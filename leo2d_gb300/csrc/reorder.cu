@@ -204,6 +204,7 @@ namespace leo2d {
 void csr_build_reordered(leo2d_ctx* ctx, leo2d_csr* csr, double patch, bool with_fp64, bool curve) {
   const int curve_req = curve ? 1 : 0;
   ++csr->generation;
+  csr->reordered = false;  // (until every array is there)
   csr_drop_tc(csr);
   csr_drop_rb(csr);
   csr_drop_rt(csr);

@@ -1523,6 +1523,11 @@ void csr_drop_rows(leo2d_csr* csr) {
   csr->win_refused.clear();
 }
 
+void row_release(leo2d_csr* csr, bool fp64) {
+  if (fp64) csr_drop_sell(csr);
+  else csr_drop_win(csr);
+}
+
 static int row_slices(int cols, int cols_used) {
   const int cs = std::min(cols, 32);
   return std::max(1, (std::min(cols_used, cols) + cs - 1) / cs);
@@ -1596,7 +1601,8 @@ bool row_prepare(leo2d_ctx* ctx, leo2d_csr* csr, bool perm, bool fp64, int cols,
   if (s.form == kRowWin && !build_win(ctx, csr, perm, s)) return false;
   if (s.form == kRowSell && !build_sell(ctx, csr, perm)) return false;
   const size_t per_step = (size_t)s.slices * s.group * 2 * s.cs * sizeof(double);
-  s.chunk = (int)std::max<size_t>(1, kRowPartialBytes / per_step);
+  const size_t held = g_alloc_cap ? std::min(kRowPartialBytes, g_alloc_cap) : kRowPartialBytes;
+  s.chunk = (int)std::max<size_t>(1, held / per_step);
   return true;
 }
 

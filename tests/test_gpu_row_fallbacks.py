@@ -1,7 +1,7 @@
 """The multi-step row kernel where its format cannot be: windows that do not fit, rows of
-very uneven length. The tiled step runs then, with the bits it gives when asked for, and
-a search that failed is not repeated. What runs does not depend on what ran before on
-the same matrix.
+very uneven length, no memory beside the matrix. The tiled step runs then, with the
+bits it gives when asked for, and a search that failed is not repeated. What runs
+does not depend on what ran before on the same matrix.
 """
 import numpy as np
 import pytest
@@ -73,6 +73,38 @@ def test_uneven_rows_in_fp64(ctx):
     np.testing.assert_array_equal(csr.kpm_dos(cfg), first)
     assert ctx.kernel_stats("sell_build")[0] == 0 and ctx.kernel_stats("cheb_steps")[0] == 0
     np.testing.assert_array_equal(_tiled(ctx, lambda: csr.kpm_dos(cfg)), first)
+
+
+@pytest.mark.parametrize("precision", [L.FP32, L.FP64])
+def test_no_room_for_the_format(ctx, precision):
+    """8 MiB an allocation: every array of the CSR matrix fits, the format's values do not."""
+    rp, col, val = _matrix(30011, 30, 1250, 7)
+    assert len(val) * 8 < 8 << 20
+    csr = ctx.upload_csr(rp, col, val)
+    cfg = L.kpm_cfg(64, R=4, seed=2, precision=precision)
+    ctx.set_option("alloc_cap_mb", 8)
+    ctx.reset_stats()
+    got = csr.kpm_dos(cfg)
+    assert ctx.kernel_stats("cheb_steps")[0] == 0
+    np.testing.assert_array_equal(got, csr.kpm_dos(cfg))
+    np.testing.assert_array_equal(got, _tiled(ctx, lambda: csr.kpm_dos(cfg)))
+    ctx.set_option("alloc_cap_mb", 0)  # room again: the row kernel runs
+    ctx.reset_stats()
+    more = csr.kpm_dos(cfg)
+    assert ctx.kernel_stats("cheb_steps")[0] > 0
+    assert np.max(np.abs(more - got)) <= (2e-5 if precision == L.FP32 else 1e-12) * np.max(np.abs(got))
+
+
+@pytest.mark.parametrize("n,precision", [(2000, L.FP32), (9000, L.FP32), (2000, L.FP64), (9000, L.FP64)])
+def test_sums_of_a_run_in_small_pieces(ctx, n, precision):
+    """1 MiB an allocation: the CTAs' sums of 500 steps are reduced in several pieces."""
+    csr = ctx.upload_csr(*_matrix(n, 10, 40, n))
+    cfg = L.kpm_cfg(1000, R=4, seed=2, precision=precision)
+    ref = csr.kpm_dos(cfg)
+    ctx.set_option("alloc_cap_mb", 1)
+    ctx.reset_stats()
+    np.testing.assert_array_equal(csr.kpm_dos(cfg), ref)
+    assert ctx.kernel_stats("cheb_steps")[0] > 1
 
 
 def test_a_short_run_does_not_depend_on_a_longer_one_before(ctx):
