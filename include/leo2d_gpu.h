@@ -142,7 +142,9 @@ int64_t leo2d_ctx_launch_count(const leo2d_ctx* ctx);
 /* Tuning switches of a context. Keys: "step_kernel" (-1 = autotuned or the
  * default for the matrix; 0 = shared-memory tiles filled by bulk copies;
  * 1 = register streaming of the matrix; 2 = tensor-core tiles; 3 = row blocks of
- * 4 rows; 5 = row blocks of 8 or 16 rows on the tensor cores),
+ * 4 rows; 5 = row blocks of 8 or 16 rows on the tensor cores; where -1 would take
+ * every step in one launch, a tile_* option off its default or a cfg's
+ * rows_per_warp asks for 0),
  * "tile_stages" (2..4 shared-memory stages of the tiled kernel, default 2),
  * "tile_chunk" (1..65536 consecutive row tiles per block between grid-wide
  * jumps, default 4), "rt_warps" / "rt_depth" / "rt_group" / "rt_chunk" (the

@@ -167,7 +167,7 @@ struct leo2d_batch {
   double patch = 0.0;   // the flakes' locality ordering
   int curve = 0;
   bool rb4 = false;     // the 4-row step's blocks
-  int stages = 2, chunk = 4;  // of the tiles, as the context had them at creation
+  int stages = kTileStages, chunk = kTileChunk;  // of the tiles, as the context had them at creation
   int tile_rows = 0, tile_cap = 0, rp_bytes = 0, col_bytes = 0, stage_bytes = 0;
   size_t dyn_smem = 0;
   unsigned grid = 0;

@@ -164,6 +164,8 @@ struct PendingTimer {
   cudaEvent_t start, stop;
 };
 
+constexpr int kTileStages = 2, kTileChunk = 4;  // the tiled step's defaults
+
 // Device-side status word written by bounded waits (see kStatus*).
 enum : int { kStatusOk = 0, kStatusTimeout = 1, kStatusNonfinite = 2, kStatusBadIndex = 3 };
 
@@ -197,10 +199,10 @@ struct leo2d_ctx {
   int rt_group = 0;           // 8-row tensor-core step: consecutive blocks per warp run: 0 default (2), 1..16
   int rt_chunk = 0;           // 8-row tensor-core step: tiles per CTA between grid-wide jumps: 0 default (2)
   int reorder_curve = 1;      // locality ordering inside a patch: 1 sheet then a fine Hilbert curve, 0 reference index
-  int tile_stages = 2;        // shared-memory stages of the tiled kernel
+  int tile_stages = leo2d::kTileStages;  // shared-memory stages of the tiled kernel
   int test_unsatisfied_wait = 0;  // test hook: tiled steps first wait on a barrier nobody completes
   bool tc_gemm_ready = false;     // shared-memory attributes of the tensor-core GEMM set on this device
-  int tile_chunk = 4;         // consecutive tiles per block between grid-wide jumps
+  int tile_chunk = leo2d::kTileChunk;    // consecutive tiles per block between grid-wide jumps
   int tile_warps = 0;         // warps per block of the tiled kernel (0 = per shape, 8 or 24)
   int reorder = -1;           // locality ordering: -1 auto, 0 off, 1 on
   double reorder_patch = 0.0;   // patch edge (A); 0: the step kernel's own (16 A; 32 A for row blocks)

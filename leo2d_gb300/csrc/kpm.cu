@@ -600,8 +600,11 @@ StepShape choose_shape(leo2d_ctx* ctx, const leo2d_csr* csr, bool fp64, int cols
   else if (ctx->kernel_variant == -1) s.rt = rt_ok && (cached ? it->second.rt : s.rb);
   if (s.rt) s.rb = false;
   if (s.rb || s.rt) s.tc = false;
-  // else every step in one launch over the CSR rows, unless a step kernel is asked for
-  s.row = ctx->kernel_variant == -1 && !s.tc && !s.rb && !s.rt && (cached ? it->second.row : true);
+  // else every step in one launch over the CSR rows, unless a step kernel is asked for,
+  // by its name or by a shape that only the tiled step has
+  const bool tiles_asked = requested_rows > 0 || ctx->tile_warps > 0 || ctx->tile_stages != kTileStages ||
+                           ctx->tile_chunk != kTileChunk;
+  s.row = ctx->kernel_variant == -1 && !tiles_asked && !s.tc && !s.rb && !s.rt && (cached ? it->second.row : true);
   if (csr->complex_h) {
     s.row = false;
     s.rb = !s.rt;  // the 4-row step, or the 8-row step when asked for
