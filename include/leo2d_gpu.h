@@ -19,8 +19,8 @@
  *  - Host buffers are owned by the caller and are complete when the call
  *    returns (calls synchronise the context's stream before returning).
  *  - Device memory that a call or a handle releases is kept for later allocations
- *    of the process (at most 16 GiB or a sixteenth of the device's memory), and
- *    given back when an allocation does not fit or the last context closes.
+ *    of the process on that device (at most 16 GiB or a sixteenth of its memory), and
+ *    given back when an allocation does not fit or the device's last context closes.
  *  - One context = one CUDA device + one stream. A context may be used by one
  *    host thread at a time; use one context per thread.
  *  - Sizes and indices that can exceed 2^31 are 64-bit.

@@ -17,6 +17,8 @@
 #include <utility>
 #include <vector>
 
+#include "mem_pool.h"
+
 #include "../../include/leo2d_gpu.h"
 
 namespace leo2d {
@@ -50,39 +52,6 @@ struct Error : std::exception {
 // API call (guard() sets it for the calling thread).
 inline thread_local size_t g_alloc_cap = 0;
 
-// Released device memory, kept for the next allocations. Mapping and unmapping the
-// arrays of a job took 14 of its 122 ms (2.4M orbitals) and 8 of the 46 ms of a Kubo
-// trace; of a 76-orbital k point's 2.8 ms, 0.2.
-//
-// Order: a context runs everything on its one stream, so a block that a call releases
-// while kernels still use it may serve the same context's next allocation (its
-// pending blocks). When no call runs on the context and its stream is idle, they pass
-// to the blocks that every context of the device may take. A buffer goes back through
-// the context that made it, inside a call on that context or outside any call (calls
-// synchronise before they return, also when they fail); one released inside a call on
-// another context is freed with cudaFree, which waits.
-// Bounds: everything kept in the process is at most 16 GiB or a sixteenth of the
-// device's memory, whichever is less, oldest first out; an allocation that fails
-// gives it back to the device and tries again, and so does closing the last context.
-// Thread-safe.
-class MemPool {
- public:
-  MemPool(int device, cudaStream_t stream, size_t device_bytes);
-  ~MemPool();
-  void enter();  // a call on the context begins / ends (calls nest)
-  void leave();
-  void* take(size_t bytes, size_t* got);  // null: nothing fits
-  bool give(void* p, size_t bytes);       // false: not kept, the caller frees it
-  void close();                           // the context goes: keeps nothing more
-  static size_t kept();                   // bytes kept in the process
-  static void flush();                    // gives them back
- private:
-  int device_, depth_ = 0;
-  cudaStream_t stream_;
-  size_t cap_;
-  bool closed_ = false;
-};
-
 // The size an allocation is rounded up to, so that jobs of nearly equal sizes find
 // each other's blocks: whole driver pages from 1 MB on, steps of a sixteenth above
 // 32 MB and of 64 MB from 1 GB on.
@@ -96,9 +65,7 @@ inline size_t pool_size(size_t bytes) {
 // The pool of the context whose call runs on this thread (guard() sets it).
 inline thread_local const std::shared_ptr<MemPool>* g_pool = nullptr;
 
-// cudaMalloc, after giving back what the pools keep if it does not fit at first.
-cudaError_t device_malloc(void** p, size_t bytes);
-// Free device memory, counting what the pools keep.
+// Free and total memory of the current device, counting what its pools keep as free.
 void device_mem_info(size_t* free_bytes, size_t* total_bytes);
 
 // Owning device allocation (move-only).

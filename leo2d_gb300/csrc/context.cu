@@ -8,139 +8,11 @@ using namespace leo2d;
 
 namespace leo2d {
 
-// ---------------------------------------------------------------- device memory
-
-namespace {
-
-struct KeptBlock {
-  void* p;
-  size_t bytes;
-  int device;
-  const MemPool* owner;  // the context whose stream may still use it; null: anyone's
-};
-
-// Everything the process keeps, oldest first, under one lock.
-struct Kept {
-  std::mutex mu;
-  std::vector<KeptBlock> blocks;
-  size_t bytes = 0;
-  int contexts = 0;
-};
-Kept& kept_state() {
-  static Kept* k = new Kept();  // outlives every pool
-  return *k;
-}
-constexpr size_t kMaxBlocks = 1024;
-
-void drop_block(Kept& k, size_t i) {
-  cudaFree(k.blocks[i].p);  // waits for work that still uses it
-  k.bytes -= k.blocks[i].bytes;
-  k.blocks.erase(k.blocks.begin() + (std::ptrdiff_t)i);
-}
-
-}  // namespace
-
-MemPool::MemPool(int device, cudaStream_t stream, size_t device_bytes)
-    : device_(device), stream_(stream), cap_(std::min(device_bytes / 16, (size_t)16 << 30)) {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  ++k.contexts;
-}
-
-MemPool::~MemPool() { close(); }
-
-void MemPool::enter() {
-  std::lock_guard<std::mutex> lock(kept_state().mu);
-  ++depth_;
-}
-
-void MemPool::leave() {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (--depth_ != 0 || closed_) return;
-  bool mine = false;
-  for (const KeptBlock& b : k.blocks) mine |= b.owner == this;
-  if (!mine) return;
-  if (cudaStreamQuery(stream_) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  for (KeptBlock& b : k.blocks)
-    if (b.owner == this) b.owner = nullptr;
-}
-
-// The smallest block of at least `bytes` and at most a quarter (or 64 KB) more.
-void* MemPool::take(size_t bytes, size_t* got) {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  size_t best = k.blocks.size();
-  const size_t most = bytes + std::max(bytes / 4, (size_t)64 << 10);
-  for (size_t i = 0; i < k.blocks.size(); ++i) {
-    const KeptBlock& b = k.blocks[i];
-    if (b.device == device_ && (!b.owner || b.owner == this) && b.bytes >= bytes && b.bytes <= most &&
-        (best == k.blocks.size() || b.bytes < k.blocks[best].bytes))
-      best = i;
-  }
-  if (best == k.blocks.size()) return nullptr;
-  const KeptBlock b = k.blocks[best];
-  k.blocks.erase(k.blocks.begin() + (std::ptrdiff_t)best);
-  k.bytes -= b.bytes;
-  *got = b.bytes;
-  return b.p;
-}
-
-bool MemPool::give(void* p, size_t bytes) {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (closed_ || bytes > cap_) return false;
-  const MemPool* owner = this;
-  if (depth_ == 0) {  // outside any call: anyone's once the stream is idle
-    if (cudaStreamQuery(stream_) == cudaSuccess) owner = nullptr;
-    else cudaGetLastError();
-  }
-  while (!k.blocks.empty() && (k.bytes + bytes > cap_ || k.blocks.size() >= kMaxBlocks)) drop_block(k, 0);
-  try {
-    k.blocks.push_back(KeptBlock{p, bytes, device_, owner});
-  } catch (...) {
-    return false;
-  }
-  k.bytes += bytes;
-  return true;
-}
-
-void MemPool::close() {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (closed_) return;
-  closed_ = true;
-  --k.contexts;
-  for (size_t i = k.blocks.size(); i-- > 0;)
-    if (k.blocks[i].owner == this || k.contexts == 0) drop_block(k, i);
-}
-
-size_t MemPool::kept() {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  return k.bytes;
-}
-
-void MemPool::flush() {
-  Kept& k = kept_state();
-  std::lock_guard<std::mutex> lock(k.mu);
-  while (!k.blocks.empty()) drop_block(k, k.blocks.size() - 1);
-}
-
-cudaError_t device_malloc(void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaErrorMemoryAllocation || MemPool::kept() == 0) return e;
-  cudaGetLastError();
-  MemPool::flush();
-  return cudaMalloc(p, bytes);
-}
-
 void device_mem_info(size_t* free_bytes, size_t* total_bytes) {
+  int device = 0;
+  LEO_CUDA(cudaGetDevice(&device));
   LEO_CUDA(cudaMemGetInfo(free_bytes, total_bytes));
-  *free_bytes += MemPool::kept();
+  *free_bytes += MemPool::kept(device);
 }
 
 cudaEvent_t ctx_event(leo2d_ctx* ctx) {
