@@ -94,7 +94,7 @@ struct DevBuf {
                               " bytes exceeds the context's alloc_cap_mb");
     size_t got = pool_size(count * sizeof(T));
     void* q = g_pool ? (*g_pool)->take(got, &got) : nullptr;
-    if (!q) LEO_CUDA(device_malloc(&q, got));
+    if (!q) LEO_CUDA(device_malloc(&q, count * sizeof(T), &got));
     if (g_pool) home_ = *g_pool;
     p = static_cast<T*>(q);
     held_ = got;

@@ -41,8 +41,9 @@ class MemPool {
   bool closed_ = false;
 };
 
-// cudaMalloc on the current device, after giving back what is kept of it if it does
-// not fit at first.
-cudaError_t device_malloc(void** p, size_t bytes);
+// cudaMalloc of *got >= bytes (a rounded size) on the current device, after giving back
+// what is kept of it if that does not fit at first; of the bytes themselves (*got is set
+// to them) where the rounding is what does not fit.
+cudaError_t device_malloc(void** p, size_t bytes, size_t* got);
 
 }  // namespace leo2d

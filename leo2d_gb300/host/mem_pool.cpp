@@ -137,13 +137,20 @@ void MemPool::flush(int device) {
   while (!k.blocks.empty()) drop_block(k, k.blocks.size() - 1);
 }
 
-cudaError_t device_malloc(void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
+cudaError_t device_malloc(void** p, size_t bytes, size_t* got) {
+  cudaError_t e = cudaMalloc(p, *got);
   int device = 0;
-  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&device) != cudaSuccess || MemPool::kept(device) == 0) return e;
-  cudaGetLastError();
-  MemPool::flush(device);
-  return cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess && MemPool::kept(device) != 0) {
+    cudaGetLastError();
+    MemPool::flush(device);
+    e = cudaMalloc(p, *got);
+  }
+  if (e == cudaErrorMemoryAllocation && *got > bytes) {
+    cudaGetLastError();
+    *got = bytes;
+    e = cudaMalloc(p, *got);
+  }
+  return e;
 }
 
 }  // namespace leo2d

@@ -40,7 +40,8 @@ cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 static void* make(int device, size_t n) {
   g_current = device;
   void* p = nullptr;
-  return leo2d::device_malloc(&p, n) == cudaSuccess ? p : nullptr;
+  size_t got = n;
+  return leo2d::device_malloc(&p, n, &got) == cudaSuccess ? p : nullptr;
 }
 
 int main() {
@@ -79,6 +80,20 @@ int main() {
     CHECK(MemPool::kept(1) == 0 && MemPool::kept(0) == 200 * MB);
     MemPool::flush(0);
     CHECK(MemPool::kept(0) == 0);
+  }
+  {
+    // an allocation whose rounded size does not fit, but itself does
+    MemPool a(0, nullptr, 16 * 256 * MB);
+    void *p = make(0, 100 * MB), *q = nullptr;
+    CHECK(a.give(p, 100 * MB));
+    size_t got = 544 * MB;
+    CHECK(leo2d::device_malloc(&q, 510 * MB, &got) == cudaSuccess && got == 510 * MB && g_free[0] == 2 * MB);
+    cudaFree(q);
+    got = 512 * MB;
+    CHECK(leo2d::device_malloc(&q, 510 * MB, &got) == cudaSuccess && got == 512 * MB);
+    cudaFree(q);
+    got = 544 * MB;
+    CHECK(leo2d::device_malloc(&q, 513 * MB, &got) == cudaErrorMemoryAllocation);
   }
   CHECK(g_live.empty() && g_free[0] == 512 * MB && g_free[1] == 512 * MB);
   return 0;
