@@ -372,7 +372,6 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
     } catch (const Error& e) {
       // no room for the format beside the matrix: the tiled step needs none
       if (e.status != LEO2D_ERR_OOM) throw;
-      cudaGetLastError();
       row_release(mm, s.fp64);
       bar.release();
       x2.release();

@@ -150,6 +150,8 @@ cudaError_t device_malloc(void** p, size_t bytes, size_t* got) {
     *got = bytes;
     e = cudaMalloc(p, *got);
   }
+  // (the status says it; left behind, it would be taken for a failed launch of what runs next)
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
   return e;
 }
 

@@ -13,11 +13,12 @@ static int g_current = 0;
 static size_t g_free[2] = {512 * MB, 512 * MB};
 static std::map<void*, std::pair<int, size_t>> g_live;
 static int g_busy = 0;  // streams still run
+static cudaError_t g_last = cudaSuccess;
 
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = g_current; return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-  if (n > g_free[g_current]) return cudaErrorMemoryAllocation;
+  if (n > g_free[g_current]) return g_last = cudaErrorMemoryAllocation;
   *p = std::malloc(1);
   g_live[*p] = {g_current, n};
   g_free[g_current] -= n;
@@ -32,7 +33,11 @@ cudaError_t cudaFree(void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaStreamQuery(cudaStream_t) { return g_busy ? cudaErrorNotReady : cudaSuccess; }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void) {
+  const cudaError_t e = g_last;
+  g_last = cudaSuccess;
+  return e;
+}
 }
 
 #define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); return __LINE__; } } while (0)
@@ -94,6 +99,7 @@ int main() {
     cudaFree(q);
     got = 544 * MB;
     CHECK(leo2d::device_malloc(&q, 513 * MB, &got) == cudaErrorMemoryAllocation);
+    CHECK(cudaGetLastError() == cudaSuccess);  // nothing left for the next launch's check
   }
   CHECK(g_live.empty() && g_free[0] == 512 * MB && g_free[1] == 512 * MB);
   return 0;
