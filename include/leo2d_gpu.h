@@ -20,7 +20,9 @@
  *    returns (calls synchronise the context's stream before returning).
  *  - Device memory that a call or a handle releases is kept for later allocations
  *    of the process on that device (at most 16 GiB or a sixteenth of its memory), and
- *    given back when an allocation does not fit or the device's last context closes.
+ *    given back when an allocation does not fit, when the device's last context
+ *    closes, or when asked for (option "release_memory": another allocator of the
+ *    process, which cannot do it by itself, may want it).
  *  - One context = one CUDA device + one stream. A context may be used by one
  *    host thread at a time; use one context per thread.
  *  - Sizes and indices that can exceed 2^31 are 64-bit.
@@ -157,7 +159,8 @@ int64_t leo2d_ctx_launch_count(const leo2d_ctx* ctx);
  * block: 0 = autotuned, 8, or 16 with rt_stage 1, warps 12 or 16, depth 3),
  * "alloc_cap_mb" (the largest single device allocation a call on this context
  * may make, in MiB; a larger one fails with LEO2D_ERR_OOM and a message naming
- * its size; 0 = no limit, the default),
+ * its size; 0 = no limit, the default), "release_memory" (1 = give back now what the
+ * process keeps of the context's device, an action and not a setting),
  * "reorder_curve" (1 = inside each patch of the locality ordering, orbitals go
  * by sheet and along a Hilbert curve of 1/32-patch cells, the default; 0 = by
  * the reference index), "tile_warps" (8 or 24 warps per block of the tiled
