@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -305,6 +306,40 @@ T* ctx_scratch(leo2d_ctx* ctx, size_t count) {
   }
   return reinterpret_cast<T*>(ctx->scratch.p);
 }
+
+// Work space of one call in several parts: together in the context's scratch or, where
+// that would pass the context's limit on one allocation, an allocation each.
+class Scratch {
+ public:
+  Scratch(leo2d_ctx* ctx, std::initializer_list<size_t> bytes) {
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    size_t total = 0;
+    for (size_t b : bytes) total += up(b);
+    const bool apart = g_alloc_cap && total > g_alloc_cap;
+    char* p = apart ? nullptr : ctx_scratch<char>(ctx, total);
+    for (size_t b : bytes) {
+      if (n_ == kParts) fail(LEO2D_ERR_BAD_ARG, "too many parts of a work space");
+      if (apart) {
+        own_[n_].alloc(b);
+        part_[n_] = own_[n_].p;
+      } else {
+        part_[n_] = p;
+        p += up(b);
+      }
+      ++n_;
+    }
+  }
+  template <class T>
+  T* get(int i) const {
+    return reinterpret_cast<T*>(part_[i]);
+  }
+
+ private:
+  static constexpr int kParts = 5;
+  int n_ = 0;
+  DevBuf<char> own_[kParts];
+  char* part_[kParts] = {};
+};
 
 // tab[m] = cos(pi m / (2P)), 0 <= m < 4P (transform.cu).
 void cos_table(leo2d_ctx* ctx, int P, double* tab);

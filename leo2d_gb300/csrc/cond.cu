@@ -510,16 +510,19 @@ leo2d_status leo2d_cond_sigma(leo2d_ctx* ctx, const double* mu, int32_t M, const
     LEO_REQUIRE(M >= 2 && num_energies >= 0, "bad sizes");
     LEO_REQUIRE(rescale > 0 && std::isfinite(rescale) && std::isfinite(center), "bad rescale/center");
     LEO_CUDA(cudaSetDevice(ctx->device));
-    // energies in chunks whose t stays within 64 MB
-    const int64_t chunk = std::max<int64_t>(32, std::min<int64_t>(num_energies, (int64_t)(8 << 20) / M / 32 * 32));
+    // energies in chunks whose t stays within 64 MB (and within the limit on allocations)
+    const int64_t held = g_alloc_cap ? std::min<int64_t>((int64_t)8 << 20, (int64_t)(g_alloc_cap / sizeof(double))) : (int64_t)8 << 20;
+    const int64_t chunk = std::max<int64_t>(32, std::min<int64_t>(num_energies, held / M / 32 * 32));
     const int tiles = (int)((chunk + 31) / 32);
     // rows split over blocks so that every SM has work
     int splits = std::max(1, std::min(2 * ctx->sm_count / tiles, (M + kSigmaWarps * kSigmaRows - 1) / (kSigmaWarps * kSigmaRows)));
     const int rows_per = (M + splits - 1) / splits;
     splits = (M + rows_per - 1) / rows_per;
-    double* dmu = ctx_scratch<double>(ctx, (size_t)M * M + (size_t)chunk * (M + splits) + 2 * (size_t)num_energies);
-    double *dt = dmu + (size_t)M * M, *dpart = dt + (size_t)chunk * M, *dE = dpart + (size_t)chunk * splits;
-    double* dout = dE + num_energies;
+    const size_t points = (size_t)num_energies * sizeof(double);
+    const Scratch ws(ctx, {(size_t)M * M * sizeof(double), (size_t)chunk * M * sizeof(double),
+                           (size_t)chunk * splits * sizeof(double), points, points});
+    double *dmu = ws.get<double>(0), *dt = ws.get<double>(1), *dpart = ws.get<double>(2), *dE = ws.get<double>(3),
+           *dout = ws.get<double>(4);
     h2d(ctx, dmu, mu, (size_t)M * M);
     h2d(ctx, dE, energies, num_energies);
     for (int64_t e0 = 0; e0 < num_energies; e0 += chunk) {

@@ -882,12 +882,10 @@ leo2d_status leo2d_mlp_site_sum(leo2d_mlp* M, const leo2d_csr* csr, double twist
     // call in four allocations.
     const int64_t wave = (int64_t)ctx->sm_count * 2 * kGemmBM;
     const int64_t chunk = std::min<int64_t>(n, std::max<int64_t>(1, (2000000 / wave)) * wave);
-    const size_t part_n = std::max(mlp_fused_part(ctx), (size_t)tc_gemm_grid(ctx, (int)chunk, kOut) * kOut);
-    const size_t xw = ((size_t)chunk * kFeat * sizeof(__nv_bfloat16) + 255) / 256 * 256;
-    char* ws = ctx_scratch<char>(ctx, xw + (part_n + kOut) * sizeof(double));
-    __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(ws);
-    double* part = reinterpret_cast<double*>(ws + xw);
-    double* sums = part + part_n;
+    const size_t part_n = std::max(mlp_fused_part(ctx, chunk), (size_t)tc_gemm_grid(ctx, (int)chunk, kOut) * kOut);
+    const Scratch ws(ctx, {(size_t)chunk * kFeat * sizeof(__nv_bfloat16), part_n * sizeof(double), kOut * sizeof(double)});
+    __nv_bfloat16* X = ws.get<__nv_bfloat16>(0);
+    double *part = ws.get<double>(1), *sums = ws.get<double>(2);
     for (int64_t r0 = 0; r0 < n; r0 += chunk) {
       const int64_t rows = std::min(chunk, n - r0);
       launch(ctx, "mlp_features", [&] {

@@ -394,7 +394,12 @@ __global__ void __launch_bounds__(256) k_fused_site_sums(const double* __restric
 
 namespace leo2d {
 
-size_t mlp_fused_part(const leo2d_ctx* ctx) { return (size_t)ctx->sm_count * 4 * kWidth; }
+static int fused_grid(const leo2d_ctx* ctx, int64_t n) {
+  const int64_t tiles = (n + kRows - 1) / kRows;
+  return (int)std::min<int64_t>(ctx->sm_count, (tiles + 1) / 2);
+}
+
+size_t mlp_fused_part(const leo2d_ctx* ctx, int64_t n) { return (size_t)fused_grid(ctx, n) * 4 * kWidth; }
 
 void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap* tw, const float* const* bias,
                        int64_t n, float* Y, double* sums_dev, double* part, bool accumulate) {
@@ -412,7 +417,7 @@ void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap*
   a.tiles = (n + kRows - 1) / kRows;
   a.y = Y;
   a.status = ctx->status.p;
-  const int grid = (int)std::min<int64_t>(ctx->sm_count, (a.tiles + 1) / 2);
+  const int grid = fused_grid(ctx, n);
   a.part = part;
   launch(ctx, "mlp_fused", [&] { k_mlp_fused<<<grid, kThreads, kSmemBytes, ctx->stream>>>(a); });
   if (!Y)

@@ -574,7 +574,9 @@ void tc_gemm_f32x3_acc(leo2d_ctx* ctx, const float* A, const float* B, int M, in
   const int64_t tiles = (int64_t)g.m_tiles * g.n_tiles;
   const int64_t least = (nkb + kF3Chunk - 1) / kF3Chunk;
   const int64_t waves = (least * tiles + ctx->sm_count - 1) / ctx->sm_count;
-  const int64_t want = std::max(least, waves * ctx->sm_count / tiles);
+  int64_t want = std::max(least, waves * ctx->sm_count / tiles);
+  if (g_alloc_cap)  // (no more items' FP64 tiles than a limit on allocations leaves room for)
+    want = std::max(least, std::min<int64_t>(want, (int64_t)(g_alloc_cap / (F3_BM * F3_BN * sizeof(double))) / tiles));
   g.chunk_kb = std::min<int64_t>(kF3Chunk, ((nkb + want - 1) / want + kF3Flush - 1) / kF3Flush * kF3Flush);
   g.splits = (int)((nkb + g.chunk_kb - 1) / g.chunk_kb);
   const int64_t items = (int64_t)g.m_tiles * g.n_tiles * g.splits;

@@ -179,8 +179,8 @@ __device__ __forceinline__ void mlp_gelu2(float& a, float& b) {
 // the BF16 weights W_l [256][in_l] (boxes of 64 x 256); bias[l]: FP32 [256].
 // Writes Y (FP32 [n][256]) or, with Y null, sums_dev[256] (+)= the FP64 column
 // sums of the outputs over the n rows (added to with `accumulate`); `part` is then
-// work space of mlp_fused_part(ctx) doubles. n < 2^31. Only enqueues.
-size_t mlp_fused_part(const leo2d_ctx* ctx);
+// work space of mlp_fused_part(ctx, n) doubles. n < 2^31. Only enqueues.
+size_t mlp_fused_part(const leo2d_ctx* ctx, int64_t n);
 void mlp_forward_fused(leo2d_ctx* ctx, const CUtensorMap& tx, const CUtensorMap* tw, const float* const* bias,
                        int64_t n, float* Y, double* sums_dev, double* part, bool accumulate);
 

@@ -46,7 +46,9 @@ __global__ void k_cos_table(int P, double* __restrict__ tab) {
 constexpr int kDctWarps = 8;
 
 // A warp per pair of nodes k and P - 1 - k: the even and the odd terms, lanes over
-// j; then a thread per node of the block's pairs for the scale.
+// j; then a thread per node of the block's pairs for the scale. kTable false: each
+// cosine by itself (a limit on allocations that the table would pass).
+template <bool kTable>
 __global__ void __launch_bounds__(kDctWarps * 32) k_dct3_nodes(const double* __restrict__ in,
                                                                const double* __restrict__ tab, int P, double rescale,
                                                                double shift, double scale, double* __restrict__ dos,
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(kDctWarps * 32) k_dct3_nodes(const double* __r
       const int step = (int)((32 * q) % period);
       double s = 0.0;
       for (int j = 1 + lane; j < P; j += 32) {
-        s += in[j] * tab[m];
+        s += in[j] * (kTable ? tab[m] : cospi((double)m / (double)(2 * (int64_t)P)));
         m += step;
         if (m >= period) m -= period;
       }
@@ -132,16 +134,20 @@ leo2d_status leo2d_dos_transform(leo2d_ctx* ctx, const double* mu, int32_t poly_
     LEO_CUDA(cudaSetDevice(ctx->device));
     const int P = poly_order;
     LEO_REQUIRE(P < (1 << 29), "poly_order too large");
-    double* dmu = ctx_scratch<double>(ctx, (size_t)P * num_sets + 7 * (size_t)P);
-    double *din = dmu + (size_t)P * num_sets, *tab = din + P, *ddos = tab + 4 * (size_t)P, *dE = ddos + P;
+    const size_t row = (size_t)P * sizeof(double);
+    const bool table = !g_alloc_cap || 4 * row <= g_alloc_cap;
+    const Scratch ws(ctx, {row * num_sets, row, table ? 4 * row : 0, row, row});
+    double *dmu = ws.get<double>(0), *din = ws.get<double>(1), *tab = ws.get<double>(2), *ddos = ws.get<double>(3),
+           *dE = ws.get<double>(4);
     h2d(ctx, dmu, mu, (size_t)P * num_sets);
     // (a warp per block: FP64 functions of 1000 terms on one SM took 9 us)
     launch(ctx, "mean_jackson", [&] {
       k_mean_jackson<<<grid_for(P, 32), 32, 0, ctx->stream>>>(dmu, P, num_sets, std::tan(3.141592653589793 / P), din);
     });
-    cos_table(ctx, P, tab);
+    if (table) cos_table(ctx, P, tab);
+    auto nodes = table ? k_dct3_nodes<true> : k_dct3_nodes<false>;
     launch(ctx, "dct3_nodes", [&] {
-      k_dct3_nodes<<<grid_for((P + 1) / 2, kDctWarps, (int64_t)ctx->sm_count * 8), kDctWarps * 32, 0, ctx->stream>>>(
+      nodes<<<grid_for((P + 1) / 2, kDctWarps, (int64_t)ctx->sm_count * 8), kDctWarps * 32, 0, ctx->stream>>>(
           din, tab, P, rescale, shift, scale, ddos, dE);
     });
     d2h(ctx, dos_out, ddos, P);
@@ -159,8 +165,9 @@ leo2d_status leo2d_dos_reconstruct(leo2d_ctx* ctx, const double* mu, int32_t pol
     LEO_REQUIRE(rescale > 0 && std::isfinite(rescale) && std::isfinite(center), "bad rescale/center");
     LEO_CUDA(cudaSetDevice(ctx->device));
     const int P = poly_order;
-    double* dmu = ctx_scratch<double>(ctx, 2 * (size_t)P + 2 * (size_t)num_energies);
-    double *dg = dmu + P, *dE = dg + P, *dout = dE + num_energies;
+    const size_t terms = (size_t)P * sizeof(double), points = (size_t)num_energies * sizeof(double);
+    const Scratch ws(ctx, {terms, terms, points, points});
+    double *dmu = ws.get<double>(0), *dg = ws.get<double>(1), *dE = ws.get<double>(2), *dout = ws.get<double>(3);
     h2d(ctx, dmu, mu, P);
     h2d(ctx, dE, energies, num_energies);
     launch(ctx, "mean_jackson", [&] {
