@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "csr.cuh"
+#include "pair.cuh"
 #include "tc_gemm.cuh"
 
 using namespace leo2d;
@@ -43,36 +44,12 @@ __device__ __forceinline__ uint32_t mix32(uint64_t a, uint64_t b) {
   return (uint32_t)((z ^ (z >> 31)) >> 32);
 }
 
-// A value as an unevaluated sum of two FP32 numbers (about 2^-45 relative).
-struct Pair {
-  float h, l;
-};
-__device__ __forceinline__ Pair pair_fast_sum(float a, float b) {  // |a| >= |b|
-  const float s = __fadd_rn(a, b);
-  return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
-  const float p = __fmul_rn(a.h, b.h);
-  float e = __fmaf_rn(a.h, b.h, -p);
-  e = __fmaf_rn(a.h, b.l, e);
-  e = __fmaf_rn(a.l, b.h, e);
-  return {p, e};
-}
-// a + b rounded to FP32
-__device__ __forceinline__ float pair_sum(Pair a, Pair b) {
-  const float s = __fadd_rn(a.h, b.h);
-  const float t = __fsub_rn(s, a.h);
-  const float e = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, t)), __fsub_rn(b.h, t));
-  return __fadd_rn(s, __fadd_rn(e, __fadd_rn(a.l, b.l)));
-}
-__device__ __forceinline__ Pair pair_neg(Pair a) { return {-a.h, -a.l}; }
-
 // cos and sin of p 2^-64 turns. The quarter turn comes off exactly in integers;
 // the rest (at most 1/8 turn) goes through the Taylor series of sin and cos, their
 // first terms in pairs and the tail (below 1/60) in FP32: errors up to 5e-9, so
 // the rounded FP32 value is that of the FP64 function but for 3 in 1000 near ties
 // (then its neighbour).
-__device__ __forceinline__ void phase_cos_sin(uint64_t p, Pair& c, Pair& s) {
+__device__ __forceinline__ void phase_cos_sin(uint64_t p, FPair& c, FPair& s) {
   const uint32_t q = (uint32_t)((p + (1ull << 61)) >> 62);
   const int64_t r = (int64_t)(p - ((uint64_t)q << 62));
   const int32_t a = (int32_t)(r >> 32);
@@ -81,28 +58,28 @@ __device__ __forceinline__ void phase_cos_sin(uint64_t p, Pair& c, Pair& s) {
   // x = 2 pi (h + l) 2^-32
   constexpr double kTurn = 6.283185307179586476925 / 4294967296.0;
   constexpr float kTurnH = (float)kTurn, kTurnL = (float)(kTurn - (double)kTurnH);
-  const Pair u = pair_mul({h, l}, {kTurnH, kTurnL});
-  const Pair x = pair_fast_sum(u.h, u.l);
-  const Pair z = pair_mul(x, x);
+  const FPair u = fpair_mul({h, l}, {kTurnH, kTurnL});
+  const FPair x = fpair_fast_sum(u.h, u.l);
+  const FPair z = fpair_mul(x, x);
   constexpr double kSixth = -1.0 / 6.0;
   constexpr float kSixthH = (float)kSixth, kSixthL = (float)(kSixth - (double)kSixthH);
-  const Pair t = pair_mul(pair_mul(x, z), {kSixthH, kSixthL});
+  const FPair t = fpair_mul(fpair_mul(x, z), {kSixthH, kSixthL});
   float ts = __fmaf_rn(z.h, -1.0f / 39916800.0f, 1.0f / 362880.0f);
   ts = __fmaf_rn(z.h, ts, -1.0f / 5040.0f);
   ts = __fmaf_rn(z.h, ts, 1.0f / 120.0f);
   ts = __fmul_rn(ts, __fmul_rn(x.h, __fmul_rn(z.h, z.h)));
-  const Pair s0 = pair_fast_sum(x.h, t.h);
-  const Pair sn = pair_fast_sum(s0.h, __fadd_rn(s0.l, __fadd_rn(__fadd_rn(x.l, t.l), ts)));
+  const FPair s0 = fpair_fast_sum(x.h, t.h);
+  const FPair sn = fpair_fast_sum(s0.h, __fadd_rn(s0.l, __fadd_rn(__fadd_rn(x.l, t.l), ts)));
   float tc = __fmaf_rn(z.h, -1.0f / 3628800.0f, 1.0f / 40320.0f);
   tc = __fmaf_rn(z.h, tc, -1.0f / 720.0f);
   tc = __fmaf_rn(z.h, tc, 1.0f / 24.0f);
   tc = __fmul_rn(tc, __fmul_rn(z.h, z.h));
-  const Pair c0 = pair_fast_sum(1.0f, -0.5f * z.h);
-  const Pair cs = pair_fast_sum(c0.h, __fadd_rn(c0.l, __fmaf_rn(-0.5f, z.l, tc)));
+  const FPair c0 = fpair_fast_sum(1.0f, -0.5f * z.h);
+  const FPair cs = fpair_fast_sum(c0.h, __fadd_rn(c0.l, __fmaf_rn(-0.5f, z.l, tc)));
   c = (q & 1) ? sn : cs;
   s = (q & 1) ? cs : sn;
-  if (q == 1 || q == 2) c = pair_neg(c);
-  if (q >= 2) s = pair_neg(s);
+  if (q == 1 || q == 2) c = fpair_neg(c);
+  if (q >= 2) s = fpair_neg(s);
 }
 
 // BF16 features [n][16] of the sites first .. first + n - 1: site_features() with
@@ -117,26 +94,26 @@ __global__ void __launch_bounds__(256) k_site_rows(int64_t n, int64_t first, con
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
     const int4 g = __ldg(reinterpret_cast<const int4*>(grid4) + first + r);  // i, j, orbital, sheet
     const SitePhase& ph = g.w == 0 ? ph0 : ph1;
-    Pair c[2], s[2];
+    FPair c[2], s[2];
 #pragma unroll
     for (int d = 0; d < 2; ++d)
       phase_cos_sin(ph.c[d] + ph.mi[d] * (uint64_t)(int64_t)g.x + ph.mj[d] * (uint64_t)(int64_t)g.y, c[d], s[d]);
-    const Pair cc = pair_mul(c[0], c[1]), ss = pair_mul(s[0], s[1]);
-    const Pair sc = pair_mul(s[0], c[1]), cs = pair_mul(c[0], s[1]);
+    const FPair cc = fpair_mul(c[0], c[1]), ss = fpair_mul(s[0], s[1]);
+    const FPair sc = fpair_mul(s[0], c[1]), cs = fpair_mul(c[0], s[1]);
     float f[kFeat];
     f[0] = c[0].h;
     f[1] = s[0].h;
     f[2] = c[1].h;
     f[3] = s[1].h;
-    f[4] = pair_sum(cc, pair_neg(ss));
-    f[5] = pair_sum(sc, cs);
-    f[6] = pair_sum(cc, ss);
-    f[7] = pair_sum(sc, pair_neg(cs));
+    f[4] = fpair_sum(cc, fpair_neg(ss));
+    f[5] = fpair_sum(sc, cs);
+    f[6] = fpair_sum(cc, ss);
+    f[7] = fpair_sum(sc, fpair_neg(cs));
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
-      const Pair p = pair_mul(c[d], s[d]);
-      f[8 + 2 * d] = pair_sum(pair_mul(c[d], c[d]), pair_neg(pair_mul(s[d], s[d])));
-      f[9 + 2 * d] = pair_sum(p, p);
+      const FPair p = fpair_mul(c[d], s[d]);
+      f[8 + 2 * d] = fpair_sum(fpair_mul(c[d], c[d]), fpair_neg(fpair_mul(s[d], s[d])));
+      f[9 + 2 * d] = fpair_sum(p, p);
     }
     f[12] = twist_deg / 3.0f;
     f[13] = (float)g.w;
@@ -247,7 +224,7 @@ __global__ void __launch_bounds__(512) k_loss(int n, const float* __restrict__ Y
   const float scale = 2.0f / (float)n;
   const float4 w4 = *reinterpret_cast<const float4*>(w + j);
   const float wj[4] = {w4.x, w4.y, w4.z, w4.w};
-  float sh = 0.f, sl = 0.f;
+  PairSum sum;
 #pragma unroll
   for (int i = 0; i < kLossRows / 8; ++i) {
     const int rr = g8 + 8 * i;
@@ -262,15 +239,12 @@ __global__ void __launch_bounds__(512) k_loss(int n, const float* __restrict__ Y
       gr[k] = scale * wj[k] * d[k];
       b[k] = __float2bfloat16_rn(gr[k]);
       tile[j + k][rr] = b[k];
-      const Pair q = pair_mul({wj[k], 0.f}, pair_mul({d[k], 0.f}, {d[k], 0.f}));
-      const float s = __fadd_rn(sh, q.h), v = __fsub_rn(s, sh);  // two-sum
-      sl = __fadd_rn(sl, __fadd_rn(q.l, __fadd_rn(__fsub_rn(sh, __fsub_rn(s, v)), __fsub_rn(q.h, v))));
-      sh = s;
+      sum.add(fpair_mul({wj[k], 0.f}, fpair_mul({d[k], 0.f}, {d[k], 0.f})));
     }
     *reinterpret_cast<float4*>(dZ32 + e) = make_float4(gr[0], gr[1], gr[2], gr[3]);
     *reinterpret_cast<uint2*>(dZ + e) = *reinterpret_cast<const uint2*>(b);
   }
-  double acc = (double)sh + (double)sl;
+  double acc = sum.value();
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();

@@ -48,6 +48,7 @@
 
 #include <algorithm>
 
+#include "pair.cuh"
 #include "tc_gemm.cuh"
 
 using namespace leo2d;
@@ -250,7 +251,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
     // over the eight lanes of a column by halving exchanges, which leaves lane t the
     // columns 8 (t / 4) + 2 (t % 4) + c, in FP32 pairs (the FP64 pipe is narrow)
     constexpr int kAcc = kEpiCols / 4;
-    float acc[kAcc], sum_h[2] = {0.f, 0.f}, sum_l[2] = {0.f, 0.f};
+    float acc[kAcc];
+    PairSum sum[2];
 #pragma unroll
     for (int k = 0; k < kAcc; ++k) acc[k] = 0.f;
     auto flush = [&]() {
@@ -264,11 +266,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
         }
       }
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const float t = __fadd_rn(sum_h[k], acc[k]), d = __fsub_rn(t, sum_h[k]);
-        sum_l[k] += __fadd_rn(__fsub_rn(sum_h[k], __fsub_rn(t, d)), __fsub_rn(acc[k], d));
-        sum_h[k] = t;
-      }
+      for (int k = 0; k < 2; ++k) sum[k].add(acc[k]);
 #pragma unroll
       for (int k = 0; k < kAcc; ++k) acc[k] = 0.f;
     };
@@ -357,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fused(const __grid_constant
 #pragma unroll
       for (int k = 0; k < 2; ++k)
         a.part[((size_t)bid * 4 + q) * kWidth + h * kEpiCols + 8 * (lane >> 2) + 2 * (lane & 3) + k] =
-            (double)sum_h[k] + (double)sum_l[k];
+            sum[k].value();
     }
   }
   umma::fence_before_sync();

@@ -8,8 +8,14 @@
 #include <type_traits>
 
 #include "kpm.cuh"
+#include "pair.cuh"
 
 namespace {
+
+using leo2d::FPair;
+using leo2d::fpair_mul;
+using leo2d::fpair_two_sum;
+using leo2d::PairSum;
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
@@ -78,31 +84,6 @@ struct StepArgs {
   double* __restrict__ partials;             // this step: [grid][C][2]
   const double* __restrict__ prev_partials;  // previous step's partials, or null
   double* __restrict__ prev_dots;            // where the previous step's dots go
-};
-
-// A running sum of FP32 terms as an unevaluated pair hi + lo: Knuth's exact
-// addition (hi + x = s + e without rounding), e goes into lo. It keeps some 48 bits
-// where FP64 keeps 53, at FP32 cost: GB300's FP64 unit takes a warp's addition
-// every 16 cycles of an SM and answers late, so FP64 sums at the end of a step
-// (a chain over the warps) were microseconds of each step. Sums over CTAs are FP64.
-struct PairSum {
-  float h = 0.f, l = 0.f;
-  __device__ __forceinline__ void add(float x) {
-    const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
-    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b)));
-    h = s;
-  }
-  __device__ __forceinline__ void add(const PairSum& o) {
-    add(o.h);
-    l = __fadd_rn(l, o.l);
-  }
-  __device__ __forceinline__ PairSum shfl_xor(int o) const {
-    PairSum r;
-    r.h = __shfl_xor_sync(0xffffffffu, h, o);
-    r.l = __shfl_xor_sync(0xffffffffu, l, o);
-    return r;
-  }
-  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
 
 // Fixed-order reduction of partials[b][t] over b < nb into out[t], for the values
@@ -664,19 +645,6 @@ struct PhaseTable {
   }
 };
 
-struct FPair {
-  float h, l;
-};
-__device__ __forceinline__ FPair fpair_mul(FPair a, FPair b) {
-  const float p = __fmul_rn(a.h, b.h);
-  float e = __fmaf_rn(a.h, b.h, -p);
-  e = __fmaf_rn(a.h, b.l, e);
-  return {p, __fmaf_rn(a.l, b.h, e)};
-}
-__device__ __forceinline__ FPair fpair_two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
-}
 // a + a q + v, rounded to FP32
 __device__ __forceinline__ float fpair_turn(FPair a, FPair q, FPair v) {
   const FPair u = fpair_mul(a, q);
