@@ -210,8 +210,10 @@ __global__ void k_gather(int64_t n_train, int B, const __nv_bfloat16* __restrict
 // dY = (2/n) w (Y - T) -> BF16 [n][256], its transpose, FP32; per-block loss sums.
 // A block takes 32 rows; a thread 4 columns of 8 rows. The transpose goes through
 // shared memory: 2-byte stores a row length apart and six FP64 instructions an
-// element for the loss took 28 us at 8192 rows (10 now). w d^2 is summed as an
-// exact product in FP32 pairs (2^-45 relative), a thread's 32 terms, then in FP64.
+// element for the loss took 28 us at 8192 rows (10 now). w d^2 is a product in FP32
+// pairs (2^-45 relative), a thread's 16 terms are summed in pairs, then FP64. A thread
+// whose sum left the range where pairs hold that (an overflow, or low parts below
+// FP32's smallest) takes its terms again in FP64.
 constexpr int kLossRows = 32;
 __global__ void __launch_bounds__(512) k_loss(int n, const float* __restrict__ Y, const float* __restrict__ T,
                                               const float* __restrict__ w, __nv_bfloat16* __restrict__ dZ,
@@ -245,6 +247,16 @@ __global__ void __launch_bounds__(512) k_loss(int n, const float* __restrict__ Y
     *reinterpret_cast<uint2*>(dZ + e) = *reinterpret_cast<const uint2*>(b);
   }
   double acc = sum.value();
+  const float wmax = fmaxf(fmaxf(fabsf(wj[0]), fabsf(wj[1])), fmaxf(fabsf(wj[2]), fabsf(wj[3])));
+  if (!(isfinite(sum.h) && fabsf(sum.h) >= 1e-30f * fmaxf(1.0f, wmax))) {
+    acc = 0.0;
+    for (int i = 0; i < kLossRows / 8 && r0 + g8 + 8 * i < n; ++i)
+      for (int k = 0; k < 4; ++k) {
+        const size_t e = (size_t)(r0 + g8 + 8 * i) * kOut + j + k;
+        const float d = Y[e] - T[e];
+        acc += (double)w[j + k] * (double)d * (double)d;
+      }
+  }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();

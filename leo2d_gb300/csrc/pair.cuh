@@ -58,7 +58,8 @@ struct PairSum {
     r.l = __shfl_xor_sync(0xffffffffu, l, o);
     return r;
   }
-  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+  // (an infinite term leaves h infinite and l undefined: the sum is infinite, as in FP64)
+  __device__ __forceinline__ double value() const { return isfinite(h) ? (double)h + (double)l : (double)h; }
 };
 
 }  // namespace leo2d
