@@ -238,10 +238,14 @@ __device__ __forceinline__ bool row_step_end(const RowArgs<T>& a, const RowSum<T
     for (int t0 = 0; t0 < 2 * CS; t0 += 32) {
       const int t = t0 + lane;
       if (t < 2 * CS) {
-        RowSum<T> s;
-#pragma unroll 8
-        for (int w = 0; w < W; ++w) s.add(wsum[w][t]);
-        row_partials_of<T, CS>(a, k, slice, bid)[t] = s.value();
+        // four chains over the warps: a single one is most of an FP64 sum's rounding
+        RowSum<T> s[4];
+#pragma unroll
+        for (int w = 0; w < W; ++w) s[w & 3].add(wsum[w][t]);
+        s[0].add(s[1]);
+        s[2].add(s[3]);
+        s[0].add(s[2]);
+        row_partials_of<T, CS>(a, k, slice, bid)[t] = s[0].value();
       }
     }
     if (meet && lane == 0) *go = row_await(a, k, slice);
@@ -971,14 +975,25 @@ __global__ void __launch_bounds__(kPanWarps * 32 + 32, 1) k_cheb_pan(const __gri
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// dots[step][slice columns][2] = the CTAs' partials added in CTA order.
-__global__ void k_row_dots(const double* __restrict__ partials, int slices, int group, int w, int C2,
-                           double* __restrict__ dots) {
-  const int step = blockIdx.x, slice = blockIdx.y;
+// dots[step][slice columns][2] = the CTAs' partials added in a fixed order: 1024 / w
+// chains over the CTAs (w = 16, 32 or 64 values), then a tree. (One chain over 152 CTAs
+// made the moments of an FP64 run four times as inexact as the tiled step's, rms 3.3e-16
+// of the largest against 8e-17.)
+constexpr int kDotThreads = 1024;
+__global__ void __launch_bounds__(kDotThreads) k_row_dots(const double* __restrict__ partials, int slices, int group,
+                                                             int w, int C2, double* __restrict__ dots) {
+  __shared__ double red[kDotThreads];
+  const int step = blockIdx.x, slice = blockIdx.y, t = threadIdx.x % w, g = threadIdx.x / w, chains = kDotThreads / w;
   const double* p = partials + ((size_t)step * slices + slice) * group * w;
   double s = 0.0;
-  for (int b = 0; b < group; ++b) s += p[(size_t)b * w + threadIdx.x];
-  dots[(size_t)step * C2 + slice * w + threadIdx.x] = s;
+  for (int b = g; b < group; b += chains) s += p[(size_t)b * w + t];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = chains / 2; o > 0; o >>= 1) {
+    if (g < o) red[threadIdx.x] += red[threadIdx.x + o * w];
+    __syncthreads();
+  }
+  if (g == 0) dots[(size_t)step * C2 + slice * w + t] = red[t];
 }
 
 // ---------------------------------------------------------------- the formats
@@ -1661,7 +1676,7 @@ void row_run(leo2d_ctx* ctx, const leo2d_csr* csr, const RowShape& s, bool perm,
       LEO_CUDA(cudaMemsetAsync(bar, 0, sizeof(unsigned) * kRowBarWords, ctx->stream));
       row_coop_launch(ctx, kern, (unsigned)(s.slices * s.group), 32 * (1 + s.warps), s.smem, &a);
       launch(ctx, "row_dots", [&] {
-        k_row_dots<<<dim3((unsigned)(a.k1 - a.k0), (unsigned)s.slices), 2 * s.cs, 0, ctx->stream>>>(
+        k_row_dots<<<dim3((unsigned)(a.k1 - a.k0), (unsigned)s.slices), kDotThreads, 0, ctx->stream>>>(
             partials, s.slices, s.group, 2 * s.cs, 2 * cols, dots + (size_t)k0 * 2 * cols);
       });
     }
