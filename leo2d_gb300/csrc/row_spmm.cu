@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(kPanWarps * 32 + 32, 1) k_cheb_pan(const __gri
   using T = float;
   constexpr int W = kPanWarps;
   constexpr int VL = 4, LPE = CS / VL, RW = pan_blocks(CS), PC = pan_chunk(CS), RB = kPanRows;
-  constexpr int kSliceRows = RW * RB, kFlush = 4;  // items (16 rows a lane) of an FP32 sum
+  constexpr int kSliceRows = RW * RB;
   constexpr int kVal = PC * RW * 16, kIdx = PC * RW * 2, kSlot = kVal + kIdx;
   extern __shared__ __align__(128) unsigned char row_smem[];
   __shared__ RowSum<T> wsum[2][W][2 * CS];
@@ -865,11 +865,7 @@ __global__ void __launch_bounds__(kPanWarps * 32 + 32, 1) k_cheb_pan(const __gri
     const T* tn = (k & 1) ? a.x1 : a.x0;
     T* tp = (k & 1) ? a.x0 : a.x1;
     const T alpha = k == 0 ? T(1) : T(2);
-    T f[2 * VL];  // FP32 over kFlush items; [2 v + d]: column VL sub + v, dot d
-    RowSum<T> s[2 * VL];
-#pragma unroll
-    for (int v = 0; v < 2 * VL; ++v) f[v] = T(0);
-    int since = 0;
+    RowSum<T> s[2 * VL];  // [2 v + d]: column VL sub + v, dot d
     for (int t = 0; t < ntile; ++t) {
       // the tile's window
       const int64_t l0 = (t_first + t) * a.win_stride;
@@ -931,6 +927,10 @@ __global__ void __launch_bounds__(kPanWarps * 32 + 32, 1) k_cheb_pan(const __gri
               if (j + 4 * h < len) four(h);
           }
           const int64_t at = row0 * C + slice * CS + VL * sub;
+          // dots: FP32 over the item's 4 rows (as the tiled step; over 16 they lose two bits), then pairs
+          T f[2 * VL];
+#pragma unroll
+          for (int v = 0; v < 2 * VL; ++v) f[v] = T(0);
           float4 xn[RB], xp[RB];
 #pragma unroll
           for (int r = 0; r < RB; ++r) {
@@ -952,22 +952,14 @@ __global__ void __launch_bounds__(kPanWarps * 32 + 32, 1) k_cheb_pan(const __gri
             }
             if (row0 + r < a.n) y.store(tp + at + (int64_t)r * C);
           }
-          if (++since == kFlush) {
-            since = 0;
 #pragma unroll
-            for (int v = 0; v < 2 * VL; ++v) {
-              s[v].add(f[v]);
-              f[v] = T(0);
-            }
-          }
+          for (int v = 0; v < 2 * VL; ++v) s[v].add(f[v]);
         }
       }
       if (t + 1 < ntile) __syncthreads();  // the window is read
     }
     if (warp < W) {
       if (k + 1 < a.k1) restart();
-#pragma unroll
-      for (int v = 0; v < 2 * VL; ++v) s[v].add(f[v]);
       row_warp_sums<T, CS>(s, ws[warp], rl, sub);
     }
     if (!row_step_end<T, CS, W>(a, ws, k, slice, bid, &go)) break;

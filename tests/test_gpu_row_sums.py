@@ -34,3 +34,19 @@ def test_fp64_sums_are_a_tree(n, block):
         assert csr.step_kernel(cfg)[0] == 6
         mu = csr.kpm_dos(cfg, x)
     assert np.sqrt(np.mean(((mu[:, 0] - exact) / exact) ** 2)) <= 1.5e-16
+
+
+# (400,000 rows of 8 columns, 60,000 of 128: a lane of the panels takes several blocks a step)
+@pytest.mark.parametrize("n,R,block", [(3000, 8, 8), (3000, 32, 32), (9001, 16, 16), (12000, 64, 64), (400000, 8, 8),
+                                       (60000, 128, 128)])
+def test_fp32_sums_of_four_rows(n, R, block):
+    """Entries k / 2048 with 1024 <= k < 2048: the sum of four squares is a whole number of
+    2^-22 below 2^24 of them, exact in FP32 (of sixteen it is not), and so are the pairs
+    and the FP64 sums beyond. So T_0's norms are exact."""
+    k = np.random.default_rng(n + block).integers(1024, 2048, (R, n))
+    with L.Context(0) as ctx:
+        csr = ctx.upload_csr(*_ring(n))
+        cfg = L.kpm_cfg(64, R=R, kind=L.VEC_HOST, block=block)
+        assert csr.step_kernel(cfg)[0] == 6
+        mu = csr.kpm_dos(cfg, k / 2048.0)
+    np.testing.assert_array_equal(mu[:, 0], (k * k).sum(1) / 2.0**22)
