@@ -48,12 +48,6 @@ struct BatchParams {
 // kernel parameters may take up to 32764 bytes (CUDA 12.1+, sm_70+)
 static_assert(sizeof(BatchParams<float>) <= 32764, "batched step parameters exceed the parameter space");
 
-// Row slots of a block of the FP32 tiled step (as the single-matrix kernel).
-int batch_slots(int cols, int warps) {
-  const int v = cols == 8 ? 2 : 4;
-  return warps * (32 / (cols / v));
-}
-
 template <typename T, int V, int LPR, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 1)
     k_cheb_batch(const __grid_constant__ BatchParams<T> p) {
@@ -208,8 +202,8 @@ bool layout(leo2d_batch* b, const BatchShape& s) {
     G = ctx->sm_count;  // one CTA of 24 warps per SM
     for (int f = 0; f < F; ++f) tiles_of[f] = rb_tiles(b->fl[f].csr, s.warps);
   } else {
-    const int ns = batch_slots(s.cols, s.warps);
-    const int ri = s.rows_per_item > 0 ? s.rows_per_item : std::max(1, 32 / ns);
+    const int ns = tile_slots(s.cols, false, s.warps);
+    const int ri = s.rows_per_item > 0 ? s.rows_per_item : tile_default_rows(ns);
     b->tile_rows = ns * ri;
     int64_t mx = 0;
     for (auto& f : b->fl) mx = std::max(mx, tile_max_nnz(ctx, f.rowptr, f.n, b->tile_rows));

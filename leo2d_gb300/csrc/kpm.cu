@@ -103,13 +103,6 @@ void tile_dispatch<double>(leo2d_ctx* ctx, int cols, unsigned grid, size_t smem,
   fail(LEO2D_ERR_BAD_ARG, "FP64 block width must be 8, 16, 32 or 64 columns");
 }
 
-// Row slots of a block (warps x slots per warp) in the tiled kernel.
-int tile_slots(int cols, bool fp64, int warps) {
-  const int v = fp64 ? 2 : (cols == 8 ? 2 : 4);
-  const int lpr = cols / v;
-  return warps * (32 / lpr);
-}
-
 template <typename T>
 void launch_step(leo2d_ctx* ctx, int cols, unsigned grid, const StepArgs<T>& a);
 
@@ -433,7 +426,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
   }
   if (shape.tiled && !shape.tc && !shape.rb && !shape.rt) {
     const int ns = tile_slots(s.cols, s.fp64, s.warps);
-    const int ri = s.rows_per_item > 0 ? s.rows_per_item : std::max(1, 32 / ns);
+    const int ri = s.rows_per_item > 0 ? s.rows_per_item : tile_default_rows(ns);
     tile_rows = ns * ri;
     int& cached_rows = use_perm ? mm->perm_tile_rows : mm->tile_rows_cached;
     int64_t& cached_max = use_perm ? mm->perm_tile_max_nnz : mm->tile_max_nnz;
@@ -583,7 +576,7 @@ StepShape choose_shape(leo2d_ctx* ctx, const leo2d_csr* csr, bool fp64, int cols
   s.rows_per_item = requested_rows > 0 ? requested_rows : (it != g_shape_cache.end() ? it->second.rows : 0);
   if (ctx->tile_warps > 0) s.warps = ctx->tile_warps;
   else if (it != g_shape_cache.end() && it->second.warps > 0) s.warps = it->second.warps;
-  else s.warps = (!fp64 && (s.cols == 32 || s.cols == 64)) ? 24 : 8;
+  else s.warps = tile_default_warps(s.cols, fp64);
   s.tiled = ctx->kernel_variant != 1;
   const bool tc_ok = !fp64 && (s.cols == 32 || s.cols == 64);
   s.tc = tc_ok && (ctx->kernel_variant == 2 ||

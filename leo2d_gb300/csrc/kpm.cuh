@@ -31,6 +31,16 @@ struct StepShape {
   int cols_used = 0;       // columns that hold vectors (0: all); the row step leaves the other slices out
 };
 
+// The tiled step's shape: warps of a block by default, row slots of a block (warps x
+// slots per warp) and rows per slot by default. The row kernel's exact form groups its
+// dots as the default shape does.
+inline int tile_default_warps(int cols, bool fp64) { return !fp64 && (cols == 32 || cols == 64) ? 24 : 8; }
+inline int tile_slots(int cols, bool fp64, int warps) {
+  const int v = fp64 || cols == 8 ? 2 : 4;
+  return warps * (32 / (cols / v));
+}
+inline int tile_default_rows(int slots) { return slots >= 32 ? 1 : 32 / slots; }
+
 // Launch of the multi-step row kernel (row_spmm.cu): the columns in `slices` of
 // cs, `group` CTAs each, `chunk` steps per launch.
 constexpr int kRowSmall = 0, kRowSell = 1, kRowWin = 2;

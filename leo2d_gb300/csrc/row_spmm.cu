@@ -1566,10 +1566,8 @@ static RowShape row_shape(const leo2d_ctx* ctx, const leo2d_csr* csr, bool perm,
     // a slice (16 rows; panels: 64 of 8 columns, 16 of 32) per CTA and up: the rows'
     // latency and the shared-memory bandwidth are spread over every SM
     s.group = (int)std::min<int64_t>(most, (n + win_slice_rows(s) - 1) / win_slice_rows(s));
-    // the tiled step's row slots per tile and rows per slot (kpm.cu)
-    const int lpr = cols / (cols == 8 ? 2 : 4);
-    s.dot_slots = (cols == 32 || cols == 64 ? 24 : 8) * (32 / lpr);
-    s.dot_rows = std::max(1, 32 / s.dot_slots);
+    s.dot_slots = tile_slots(cols, false, tile_default_warps(cols, false));
+    s.dot_rows = tile_default_rows(s.dot_slots);
   } else {
     // The small form: one CTA up to 4 rows a warp (a barrier costs more than
     // three more rows), else about two thirds of a row per warp, so that no warp
