@@ -155,6 +155,7 @@ struct BatchShape {
 
 struct leo2d_batch {
   leo2d_ctx* ctx = nullptr;
+  int device = 0;  // (the batch may be destroyed after its context)
   std::vector<FlakeView> fl;
   int P = 0, steps = 0, R = 0, passes = 0;
   BatchShape shape;
@@ -506,6 +507,7 @@ leo2d_status leo2d_batch_create(leo2d_ctx* ctx, const leo2d_csr* const* csrs, in
     LEO_CUDA(cudaSetDevice(ctx->device));
     auto b = std::make_unique<leo2d_batch>();
     b->ctx = ctx;
+    b->device = ctx->device;
     b->stages = ctx->tile_stages;
     b->chunk = ctx->tile_chunk;
     b->P = cfg->poly_order;
@@ -636,7 +638,7 @@ leo2d_status leo2d_batch_info(const leo2d_batch* b, int32_t* block_cols, int32_t
 
 leo2d_status leo2d_batch_destroy(leo2d_batch* b) {
   if (!b) return LEO2D_OK;
-  cudaSetDevice(b->ctx->device);
+  cudaSetDevice(b->device);
   delete b;
   return LEO2D_OK;
 }

@@ -377,6 +377,7 @@ uint64_t splitmix(uint64_t& x) {
 
 struct leo2d_mlp {
   leo2d_ctx* ctx = nullptr;
+  int device = 0;  // (the network may be destroyed after its context)
   int64_t np = 0;
   int64_t w_off[kLayers], b_off[kLayers];
   DevBuf<float> p, g, m, v, lw;
@@ -651,6 +652,7 @@ leo2d_status leo2d_mlp_create(leo2d_ctx* ctx, uint64_t seed, leo2d_mlp** out) {
     LEO_CUDA(cudaSetDevice(ctx->device));
     auto M = std::make_unique<leo2d_mlp>();
     M->ctx = ctx;
+    M->device = ctx->device;
     int64_t off = 0;
     for (int l = 0; l < kLayers; ++l) {
       M->w_off[l] = off;
@@ -703,7 +705,7 @@ leo2d_status leo2d_mlp_create(leo2d_ctx* ctx, uint64_t seed, leo2d_mlp** out) {
 
 leo2d_status leo2d_mlp_destroy(leo2d_mlp* M) {
   if (!M) return LEO2D_OK;
-  cudaSetDevice(M->ctx->device);
+  cudaSetDevice(M->device);
   delete M;
   return LEO2D_OK;
 }
