@@ -494,8 +494,10 @@ leo2d_status leo2d_parse_input(const char* in_path, leo2d_geom* geom_out, int32_
  * about 5e5 orbitals. Larger problems return LEO2D_ERR_BAD_ARG.
  * The first call on a device looks up the array's device address with that
  * device current (set-up, once per device); make that first call before any
- * stream capture. All calls share the array: calls that overlap on the GPU
- * (other streams, other host threads) race and corrupt each other's results.
+ * stream capture. All calls share the array, so the work of calls on several
+ * streams or threads of a device runs one call after another. A call captured
+ * into a graph is not ordered against others: replays and calls that overlap on
+ * the GPU corrupt each other's results.
  * Status codes: LEO2D_ERR_BAD_ARG (null pointer, size, poly_order % 4 != 0,
  * problem too large), LEO2D_ERR_CUDA (no device, failed launch). */
 leo2d_status leo2d_kpm_dos_noalloc(const int64_t* rowptr, const int32_t* col, const float* val,

@@ -1102,6 +1102,9 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 // itself would name host memory, not the device array).
 std::mutex g_noalloc_mu;
 void* g_noalloc_ptr[64] = {nullptr};
+// The end of the last call's work on each device: the next call's stream waits for it,
+// since all calls share the array.
+cudaEvent_t g_noalloc_done[64] = {nullptr};
 
 __global__ void k_dots_to_moments(const double* __restrict__ dots, int cols, int steps, int n_vec,
                                   double* __restrict__ mu_out, int P) {
@@ -1140,19 +1143,19 @@ extern "C" leo2d_status leo2d_kpm_dos_noalloc(const int64_t* rowptr, const int32
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
     return bad(LEO2D_ERR_CUDA, "no current CUDA device");
-  void* base = nullptr;
-  {
+  // (held to the end: a call enqueues all of its work, from the wait for the last call's
+  // to the event of its own, before another one starts)
+  std::lock_guard<std::mutex> lk(g_noalloc_mu);
+  if (!g_noalloc_ptr[dev]) {
     // once per device, with that device current
-    std::lock_guard<std::mutex> lk(g_noalloc_mu);
-    if (!g_noalloc_ptr[dev]) {
-      cudaError_t e = cudaGetSymbolAddress(&g_noalloc_ptr[dev], g_noalloc_scratch);
-      if (e != cudaSuccess || !g_noalloc_ptr[dev]) {
-        g_noalloc_ptr[dev] = nullptr;
-        return bad(LEO2D_ERR_CUDA, "cudaGetSymbolAddress of the scratch array failed");
-      }
+    cudaError_t e = cudaEventCreateWithFlags(&g_noalloc_done[dev], cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&g_noalloc_ptr[dev], g_noalloc_scratch);
+    if (e != cudaSuccess || !g_noalloc_ptr[dev]) {
+      g_noalloc_ptr[dev] = nullptr;
+      return bad(LEO2D_ERR_CUDA, "set-up of the scratch array failed");
     }
-    base = g_noalloc_ptr[dev];
   }
+  void* base = g_noalloc_ptr[dev];
   cudaStream_t st = (cudaStream_t)stream;
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -1186,6 +1189,22 @@ extern "C" leo2d_status leo2d_kpm_dos_noalloc(const int64_t* rowptr, const int32
   if (cols == 0)
     return bad(LEO2D_ERR_BAD_ARG,
                "problem too large for the 32 MiB scratch array: n * 64 bytes plus moments must fit");
+  // a stream that is being captured cannot wait for work outside its graph
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    cap = cudaStreamCaptureStatusActive;
+  }
+  const bool ordered = cap == cudaStreamCaptureStatusNone;
+  if (ordered && cudaStreamWaitEvent(st, g_noalloc_done[dev], 0) != cudaSuccess)
+    return bad(LEO2D_ERR_CUDA, "cannot wait for the last call's work");
+  struct Done {  // also of a call that fails half-way
+    cudaEvent_t ev;
+    cudaStream_t st;
+    ~Done() {
+      if (ev) cudaEventRecord(ev, st);
+    }
+  } done{ordered ? g_noalloc_done[dev] : nullptr, st};
   unsigned char* sc = static_cast<unsigned char*>(base);
   float* x0 = reinterpret_cast<float*>(sc);
   float* x1 = reinterpret_cast<float*>(sc + off_x1);
