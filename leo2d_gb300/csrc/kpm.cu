@@ -345,10 +345,11 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
                      m->reorder_curve_req != ctx->reorder_curve))
       csr_build_reordered(ctx, mm, patch, s.fp64 || m->reorder_fp64, ctx->reorder_curve != 0);
   };
-  auto vectors = [&]() {
+  auto vectors = [&](size_t sums) {
     const size_t esz = s.fp64 ? sizeof(double) : sizeof(float);
     x0.alloc((size_t)n * s.cols * esz);
     x1.alloc((size_t)n * s.cols * esz);
+    partials.alloc(sums);
     dots.alloc((size_t)steps * 2 * s.cols);
   };
   if (shape.row) {
@@ -358,8 +359,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
       if (shape.row) {
         bar.alloc(kRowBarWords);
         if (rows.exact) x2.alloc((size_t)n * s.cols * sizeof(float));
-        partials.alloc(row_partials(rows, steps));
-        vectors();
+        vectors(row_partials(rows, steps));
         shape.tiled = false;
       }
     } catch (const Error& e) {
@@ -483,10 +483,7 @@ void Recursion::setup(leo2d_ctx* c, const leo2d_csr* m, StepShape s, int steps_)
     if (g > need) g = std::max<int64_t>(need, 1);
     grid = (unsigned)g;
   }
-  if (!shape.row) {
-    vectors();
-    partials.alloc((size_t)2 * grid * 2 * s.cols);
-  }
+  if (!shape.row) vectors((size_t)2 * grid * 2 * s.cols);
 }
 
 template <typename T>
