@@ -1014,7 +1014,8 @@ def main():
                    2: "k_cheb_tc (tensor cores)", 3: "k_cheb_rb (row blocks)",
                    4: "k_cheb_rbw (row blocks, shared-memory windows)",
                    5: "k_cheb_rt (8-row blocks, tensor cores)",
-                   6: "k_cheb_win (rows over shared-memory windows, every step in one launch)"}[kernel_id]
+                   6: ("k_cheb_win (rows" if csr.n <= 8000 else "k_cheb_pan (panels of 4 rows") +
+                      " over shared-memory windows, every step in one launch)"}[kernel_id]
 
     import torch
     torch.cuda.set_device(local)

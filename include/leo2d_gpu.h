@@ -286,7 +286,10 @@ leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2
 /* The step kernel a leo2d_kpm_dos call with this cfg would run on this matrix:
  * *kernel = 0 tiled CSR gathers, 1 register-streaming gathers, 2 tensor cores,
  * 3 row blocks, 4 row blocks over shared-memory windows, 5 row blocks of 8 rows
- * on the tensor cores, 6 every step in one launch over the CSR rows; *block = the
+ * on the tensor cores, 6 every step in one launch over the CSR rows (0 after a run
+ * found no format for this shape: windows that do not fit, a column stored twice,
+ * FP64 rows of very uneven length; before a first run that is not known, and a run
+ * without memory for the format takes 0 too); *block = the
  * vector-block width in columns. Builds nothing and
  * launches nothing. No counterpart in the reference. */
 leo2d_status leo2d_kpm_step_kernel(leo2d_ctx* ctx, const leo2d_csr* csr, const leo2d_kpm_cfg* cfg,

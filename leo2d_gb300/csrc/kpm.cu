@@ -612,10 +612,10 @@ StepShape choose_shape(leo2d_ctx* ctx, const leo2d_csr* csr, bool fp64, int cols
   s.rt_depth = ctx->rt_depth > 0 ? ctx->rt_depth : (cached && it->second.rt_depth > 0 ? it->second.rt_depth : 3);
   s.rt_rows = ctx->rt_rows > 0 ? ctx->rt_rows : (cached && it->second.rt ? it->second.rt_rows : 8);
   // 20 warps hide more of the epilogue where every warp has many blocks (10M
-  // orbitals: 2.26 ms against 2.34 with 16; 2.4M: 0.559 against 0.573), and cost
-  // more at the start and end of a short step (400k: 0.117 against 0.114; 150k:
-  // 0.060 against 0.055); the line between 400k and 2.4M was not searched for. Only
-  // the 8-row cp.async form of depth 3 is built for 20.
+  // orbitals: 2.26 ms against 2.34 with 16; 2.4M: 0.555 against 0.571), and cost
+  // more at the start and end of a short step (150k: 0.0486 against 0.0477; 400k: as
+  // fast); the line between 400k and 2.4M was not searched for. Only the 8-row
+  // cp.async form of depth 3 is built for 20.
   const bool form20 = s.rt_stage == 1 && s.rt_rows == 8 && s.rt_depth == 3;
   s.rt_warps = ctx->rt_warps > 0 ? ctx->rt_warps
                                  : (cached && it->second.rt_warps > 0 ? it->second.rt_warps
@@ -1004,9 +1004,9 @@ extern "C" leo2d_status leo2d_kpm_autotune(leo2d_ctx* ctx, const leo2d_csr* csr,
           (ctx->kernel_variant == -1 || ctx->kernel_variant == 5)) {
         struct RtTry { int warps, depth, stage, rows; };
         // (the TMA form, stage 2, is timed only when asked for: 1.8x slower)
-        // (16-row blocks: a third fewer k-steps on the 0.5 deg flakes but 1.7x the
-        // cost per k-step, 0.69 against 0.60 ms at 2.4M orbitals; kept as a
-        // candidate for denser matrices)
+        // (16-row blocks: a third fewer k-steps on the 0.5 deg flakes at half as much
+        // again for one, 0.547 against 0.555 ms at 2.4M orbitals with 16 warps, 0.591
+        // with 12, 0.110 against 0.107 at 400k; kept as a candidate for denser matrices)
         for (const RtTry t : {RtTry{16, 3, 1, 8}, RtTry{20, 3, 1, 8}, RtTry{12, 3, 1, 16}, RtTry{16, 2, 0, 8},
                               RtTry{16, 3, 2, 8}, RtTry{12, 7, 2, 8}}) {
           if (t.stage == 2 && ctx->rt_stage != 2) continue;

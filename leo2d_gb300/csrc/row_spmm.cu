@@ -32,7 +32,7 @@
 //   each other, LPE lanes own a row. Bound by the FP64 pipe (89 % active).
 // Measured per step, tiled step before -> now: the 11,908-orbital cell with 128
 //   columns 99 -> 16 us, a 2188-orbital cell with 12 targets 49 -> 8.2 us, 8 columns of
-//   a 200k-orbital flake 62 -> 22 us, FP64 with 32 columns of 52k orbitals 251 -> 223
+//   a 200k-orbital flake 62 -> 23 us, FP64 with 32 columns of 52k orbitals 251 -> 223
 //   us. The first and third, LPE lanes a row: 26 and 27 us over the window, 34 and 42
 //   with gathers through L1 (some misses in every group, about 1000 cycles each).
 //
@@ -757,7 +757,8 @@ __global__ void __launch_bounds__(kWinWarps * 32 + 32, 1) k_cheb_win(const __gri
 // Per step, the 11,908-orbital cell with 128 columns / 8 columns of a 200k flake:
 // 26 / 27 us row by row; panels in row order 23 / 35 (slices padded to their longest
 // block); blocks by size within a tile 19 / 24; chunks of 8 to 16 positions and warps
-// in fours 17.5 / 23; packed FMAs (half the issue slots of the products) 16 / 22.
+// in fours 17.5 / 23; packed FMAs (half the issue slots of the products) 16 / 22; the
+// dots of a block's 4 rows summed in pairs, not of 16 in FP32, 16 / 22.5.
 // The window and the entry ring are those of k_cheb_win.
 constexpr int kPanRows = 4;
 constexpr int kPanWarps = 15;  // + the service warp: 16 warps of 128 registers

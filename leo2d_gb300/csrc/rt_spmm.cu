@@ -45,7 +45,8 @@
 //   ((g & 1) << 2), of slots t and t + 4 with no bank conflicts (memory column
 //   4 cg + i is logical column g + 8 i of the MMA). At a block's last k-step
 //   the lane owns rows 2t and 2t + 1 of the block, columns 4 cg .. 4 cg + 3: it
-//   writes T_{n+1} and adds its moment dots (FP32 over 16 blocks, then FP64).
+//   writes T_{n+1} and adds its moment dots (FP32 over 16 blocks, then pairs of FP32
+//   over the CTA, FP64 over the CTAs).
 //   The T_n and T_{n-1} rows of that epilogue are copied into shared memory at
 //   the block's start (each lane its own 16-byte chunks, so its own wait orders
 //   them): held in registers through the block they cost 16 registers, and the
@@ -295,7 +296,7 @@ __device__ __forceinline__ void rt_body(const RtArgs& a, const int bid, const in
   constexpr int MS = 2 * XS;     // shared ring of matrix k-steps
   constexpr int DM = MS - 1 - D; // matrix lookahead beyond the rows'
   constexpr int kPf = STAGE == kRtCpAsync ? 8 : REGS ? 48 : 32;  // matrix k-steps prefetched into L2 ahead
-  constexpr int kDotFlush = 16;        // blocks summed in FP32 between FP64 flushes
+  constexpr int kDotFlush = 16;        // blocks summed in FP32 between flushes into pairs
   static_assert(REGS || ((XS & (XS - 1)) == 0 && DM >= D + 1), "power-of-two rings, matrix ahead of the rows");
   extern __shared__ __align__(1024) unsigned char rt_smem_raw[];
   // the 128-byte swizzle of TMA copies is a function of the address: ring
