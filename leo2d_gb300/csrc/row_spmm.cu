@@ -32,7 +32,7 @@
 //   each other, LPE lanes own a row. Bound by the FP64 pipe (89 % active).
 // Measured per step, tiled step before -> now: the 11,908-orbital cell with 128
 //   columns 99 -> 16 us, a 2188-orbital cell with 12 targets 49 -> 8.2 us, 8 columns of
-//   a 200k-orbital flake 62 -> 23 us, FP64 with 32 columns of 52k orbitals 251 -> 223
+//   a 200k-orbital flake 62 -> 23 us, FP64 with 32 columns of 52k orbitals 251 -> 220
 //   us. The first and third, LPE lanes a row: 26 and 27 us over the window, 34 and 42
 //   with gathers through L1 (some misses in every group, about 1000 cycles each).
 //
@@ -436,9 +436,9 @@ __global__ void __launch_bounds__(kSellWarps * 32 + 32, 1) k_cheb_sell(const __g
           xn.load(tn + at);
           if (k != 0) xp.load(tp + at);
         }
-        T acc[VL];
+        T part[2][VL];  // two sums of a row's entries: half the rounding of one chain
 #pragma unroll
-        for (int v = 0; v < VL; ++v) acc[v] = T(0);
+        for (int v = 0; v < VL; ++v) part[0][v] = part[1][v] = T(0);
         // the longest of this warp's rows (multiply-adds on the slice's padding
         // would cost as much as on entries)
         const int len = (int)__reduce_max_sync(
@@ -466,8 +466,11 @@ __global__ void __launch_bounds__(kSellWarps * 32 + 32, 1) k_cheb_sell(const __g
             if (j + U + u < len) load(u, j + U + u);
 #pragma unroll
           for (int u = 0; u < U; ++u)
-            if (j + u < len) row_fma<T>(acc, x[u], w2[u]);
+            if (j + u < len) row_fma<T>(part[u & 1], x[u], w2[u]);
         }
+        T acc[VL];
+#pragma unroll
+        for (int v = 0; v < VL; ++v) acc[v] = part[0][v] + part[1][v];
         if (in) {
           RowVec<T> y;
 #pragma unroll

@@ -7,6 +7,7 @@ before its last levels; one chain over 152 blocks to 4.4e-17 sqrt(152 / 3) = 3.1
 bound lies between: 1.5e-16 rms.
 """
 import math
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -34,6 +35,30 @@ def test_fp64_sums_are_a_tree(n, block):
         assert csr.step_kernel(cfg)[0] == 6
         mu = csr.kpm_dos(cfg, x)
     assert np.sqrt(np.mean(((mu[:, 0] - exact) / exact) ** 2)) <= 1.5e-16
+
+
+@pytest.mark.parametrize("n,block", [(3000, 8), (9001, 8), (9001, 16), (12000, 32)])
+def test_fp64_rows_are_not_one_chain(n, block):
+    """A row of 64 positive products, alone in the first moment: T_0 is 1 in its row and every
+    other row's values are zero. One chain of 64 additions errs by 4.4e-17 sqrt(64 / 3) =
+    2.0e-16 of the sum (rms), two of 32 and their sum by 4.4e-17 sqrt(32 / 3 / 2 + 1) =
+    1.1e-16. The bound lies between."""
+    rng = np.random.default_rng(n + block)
+    col = (np.arange(n)[:, None] + np.arange(1, 65)) % n
+    val = np.zeros((n, 64))
+    val[0] = rng.uniform(0.005, 0.015, 64)
+    x = rng.uniform(0.5, 1.5, (128, n))
+    x[:, 0] = 1.0
+    order = np.argsort(col, axis=1)
+    col, val = np.take_along_axis(col, order, 1), np.take_along_axis(val, order, 1)
+    with L.Context(0) as ctx:
+        csr = ctx.upload_csr(np.arange(n + 1) * 64, col.ravel(), val.ravel())
+        cfg = L.kpm_cfg(8, R=128, kind=L.VEC_HOST, precision=L.FP64, block=block)
+        assert csr.step_kernel(cfg)[0] == 6
+        mu = csr.kpm_dos(cfg, x)
+    exact = [sum((Fraction(w) * Fraction(v) for w, v in zip(val[0], r[col[0]])), Fraction(0)) for r in x]
+    err = [float((Fraction(m) - e) / e) for m, e in zip(mu[:, 1], exact)]
+    assert np.sqrt(np.mean(np.square(err))) <= 1.5e-16
 
 
 # (400,000 rows of 8 columns, 60,000 of 128: a lane of the panels takes several blocks a step)
